@@ -473,9 +473,11 @@ int link_plan_build(LinkPlan &plan, const uint32_t *src, const uint32_t *tgt, ui
   // level(e) = 1 + the largest level of an earlier link sharing a node, so
   // every link sees exactly the velocities its predecessors wrote.
   uint32_t nmax = 0;
+  bool self = false;
   for (uint32_t e = 0; e < m; ++e) {
     if (src[e] + 1 > nmax) nmax = src[e] + 1;
     if (tgt[e] + 1 > nmax) nmax = tgt[e] + 1;
+    self = self || src[e] == tgt[e];
   }
   std::vector<uint32_t> node_level(nmax, 0), level(m);
   uint32_t levels = 0;
@@ -486,52 +488,83 @@ int link_plan_build(LinkPlan &plan, const uint32_t *src, const uint32_t *tgt, ui
     node_level[tgt[e]] = l;
     if (l > levels) levels = l;
   }
-  std::vector<uint32_t> start(levels + 2, 0), order(m > 0 ? m : 1);
+  std::vector<uint32_t> start(levels + 2, 0), order(m > 0 ? m : 1), place(m > 0 ? m : 1);
   for (uint32_t e = 0; e < m; ++e) start[level[e]]++;
-  uint32_t run = 0;
+  uint32_t run = 0, width = 0;
   for (uint32_t l = 0; l <= levels + 1; ++l) {
     uint32_t c = start[l];
     start[l] = run;
     run += c;
+    width = c > width ? c : width;
   }
   std::vector<uint32_t> fill(start.begin(), start.end());
-  for (uint32_t e = 0; e < m; ++e) order[fill[level[e]]++] = e;
-  // per link, how many earlier links touch its source and its target: it may
-  // run once that many links on each have finished
-  std::vector<uint32_t> seen(nmax, 0), need_e(2 * (size_t)m), need(2 * (size_t)(m > 0 ? m : 1));
   for (uint32_t e = 0; e < m; ++e) {
-    need_e[2 * e] = seen[src[e]];
-    need_e[2 * e + 1] = seen[tgt[e]];
-    ++seen[src[e]];
-    ++seen[tgt[e]];
+    place[e] = fill[level[e]]++;
+    order[place[e]] = e;
   }
-  for (uint32_t p = 0; p < m; ++p) {
-    need[2 * p] = need_e[2 * order[p]];
-    need[2 * p + 1] = need_e[2 * order[p] + 1];
+  // per link in level order: its ends, each marked if no earlier link touches
+  // it, and where each end's velocity goes on to: the next link's input
+  // (2 x its place, + 1 for its target side) or nowhere (NONE: the last one)
+  std::vector<LinkEnds> ends(m > 0 ? m : 1);
+  std::vector<uint32_t> later(nmax, NONE);
+  for (uint32_t e = m; e-- > 0;) {
+    LinkEnds &r = ends[place[e]];
+    r.next_src = later[src[e]];
+    r.next_tgt = later[tgt[e]];
+    r.src = src[e];
+    r.tgt = tgt[e];
+    later[src[e]] = 2 * place[e];
+    later[tgt[e]] = 2 * place[e] + 1;
   }
+  for (uint32_t i = 0; i < nmax; ++i)
+    if (later[i] != NONE) {
+      LinkEnds &r = ends[later[i] >> 1];
+      if (later[i] & 1) r.tgt |= LINK_FIRST;
+      else r.src |= LINK_FIRST;
+    }
   link_plan_free(plan);
   D3_CUDA_OK(cudaMalloc(&plan.order, order.size() * 4));
   D3_CUDA_OK(cudaMalloc(&plan.level_start, start.size() * 4));
-  D3_CUDA_OK(cudaMalloc(&plan.need, need.size() * 4));
-  D3_CUDA_OK(cudaMalloc(&plan.done, (nmax > 0 ? nmax : 1) * 4ull));
+  D3_CUDA_OK(cudaMalloc(&plan.ends, ends.size() * sizeof(LinkEnds)));
+  D3_CUDA_OK(cudaMalloc(&plan.par, ends.size() * 3 * sizeof(double)));
+  D3_CUDA_OK(cudaMalloc(&plan.msg, ends.size() * 2 * sizeof(double2)));
+  D3_CUDA_OK(cudaMalloc(&plan.tally, 2 * sizeof(uint32_t)));
   D3_CUDA_OK(cudaMemcpy(plan.order, order.data(), order.size() * 4, cudaMemcpyHostToDevice));
   D3_CUDA_OK(cudaMemcpy(plan.level_start, start.data(), start.size() * 4, cudaMemcpyHostToDevice));
-  D3_CUDA_OK(cudaMemcpy(plan.need, need.data(), need.size() * 4, cudaMemcpyHostToDevice));
+  D3_CUDA_OK(cudaMemcpy(plan.ends, ends.data(), ends.size() * sizeof(LinkEnds), cudaMemcpyHostToDevice));
+  D3_CUDA_OK(cudaMemset(plan.msg, 0xff, ends.size() * 2 * sizeof(double2)));  // no message yet
+  D3_CUDA_OK(cudaMemset(plan.tally, 0, 2 * sizeof(uint32_t)));
   plan.h_level_start = new uint32_t[start.size()];
   for (size_t k = 0; k < start.size(); ++k) plan.h_level_start[k] = start[k];
   plan.m = m;
   plan.levels = levels;
   plan.nodes = nmax;
+  plan.width = width;
+  plan.self = self;
+  plan.gathered = false;
   return 0;
 }
 
 void link_plan_free(LinkPlan &plan) {
   cudaFree(plan.order);
   cudaFree(plan.level_start);
-  cudaFree(plan.need);
-  cudaFree(plan.done);
+  cudaFree(plan.ends);
+  cudaFree(plan.par);
+  cudaFree(plan.msg);
+  cudaFree(plan.tally);
   delete[] plan.h_level_start;
   plan = LinkPlan();
+}
+
+// The links' distance, strength and bias in plan order (three planes), once
+// per plan (an upload of the link force makes a new plan).
+__global__ void k_link_params(LinkArrays l, const uint32_t *order, double *par) {
+  const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= l.m) return;
+  const uint32_t e = order[p];
+  par[p] = l.distance[e];
+  par[(size_t)l.m + p] = l.strength[e];
+  par[2 * (size_t)l.m + p] = l.bias[e];
 }
 
 // One link, d3's statement order. Returns false (writing nothing) where d3
@@ -652,38 +685,22 @@ __global__ void k_link_serial_host(double *xs, double *ys, double *vxs, double *
   rng->pos += used;
 }
 
-// A link with everything about it that does not change during the pass
-// (e = NONE: no link).
-struct LinkPre {
-  uint32_t e, src, tgt;
-  double dist, str, bias, xt, yt, xsrc, ysrc;
-};
-
-__device__ inline void link_params(const LinkArrays &l, uint32_t e, LinkPre &p) {
-  p.e = e;
-  if (e == NONE) return;
-  p.src = l.source[e];
-  p.tgt = l.target[e];
-  p.dist = l.distance[e];
-  p.str = l.strength[e];
-  p.bias = l.bias[e];
-}
-
-__device__ inline void link_positions(const double *xs, const double *ys, LinkPre &p) {
-  if (p.e == NONE) return;
-  p.xt = xs[p.tgt];
-  p.yt = ys[p.tgt];
-  p.xsrc = xs[p.src];
-  p.ysrc = ys[p.src];
+__device__ inline unsigned long long globaltimer_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
 }
 
 struct LinkFlowArgs {
   const double *xs, *ys;
   double *vxs, *vys, *svx, *svy;
   LinkArrays l;
-  const uint32_t *order, *need;
-  uint32_t *done;
-  uint32_t n, nodes;
+  const LinkEnds *ends;
+  const double *par;           // distance, strength, bias planes
+  const uint32_t *level_start; // k_link_block
+  ulonglong2 *msg;             // k_link_flow: two inputs per link, all ones = nothing yet
+  uint32_t *tally;             // k_link_flow: blocks done, failure bits
+  uint32_t levels, nodes;
   double alpha, iterations;
   uint32_t *flag;
   Rng *rng;           // with serial_lcg: the serial pass's draws
@@ -692,110 +709,288 @@ struct LinkFlowArgs {
   unsigned sleep_ns;  // pause between polls of a wait (after the first eight)
 };
 
-__device__ inline unsigned long long globaltimer_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
+struct LinkPar {
+  double dist, str, bias;
+};
+
+// One link on the velocities of its ends, d3's statement order. False
+// (nothing changed) where d3 would draw from `random`.
+__device__ __forceinline__ bool link_apply(const LinkPar &c, double xt, double yt, double xs,
+                                           double ys, double alpha, double2 &vt, double2 &vs) {
+  double x = xt + vt.x - xs - vs.x;
+  double y = yt + vt.y - ys - vs.y;
+  if (x == 0 || x != x || y == 0 || y != y) return false;
+  double len = sqrt(x * x + y * y);
+  len = (len - c.dist) / len * alpha * c.str;
+  x *= len;
+  y *= len;
+  double b = c.bias;
+  vt.x -= x * b;
+  vt.y -= y * b;
+  b = 1 - b;
+  vs.x += x * b;
+  vs.y += y * b;
+  return true;
 }
 
-// A link's wait, bounded: until `ns` links on src and `nt` on tgt have
-// finished. False if it gave up (20 ms): the pass is then restored and run
-// serially.
-__device__ inline uint32_t ld_acquire_u32(const uint32_t *p) {
-  uint32_t v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+__device__ __forceinline__ LinkPar link_par(const LinkFlowArgs &a, uint32_t p) {
+  return {a.par[p], a.par[(size_t)a.l.m + p], a.par[2 * (size_t)a.l.m + p]};
+}
+
+// The pass of a graph whose nodes fit one SM: a block keeps every node's
+// velocity and position in shared memory and takes the links level by level,
+// a barrier between levels. A level costs the chain of one link (about 0.3 us:
+// shared loads, sqrt, division) and the barrier; its links' constants are
+// loaded during the level before. The node arrays are written only if no link
+// met a jiggle; if one did, they are still the pass's start for the serial
+// pass. A level's links share no node: at most half the nodes, so the block is
+// as wide as the widest level.
+constexpr uint32_t LINK_BLOCK_NODES = 7000;  // 32 bytes each in 227 KB
+
+__global__ void __launch_bounds__(1024) k_link_block(LinkFlowArgs a) {
+  extern __shared__ double2 link_smem[];
+  double2 *const V = link_smem, *const P = link_smem + a.nodes;
+  const uint32_t t = threadIdx.x, nt = blockDim.x, m = a.l.m;
+  for (uint32_t i = t; i < a.nodes; i += nt) {
+    V[i] = make_double2(a.vxs[i], a.vys[i]);
+    P[i] = make_double2(a.xs[i], a.ys[i]);
+  }
+  bool bad = false;
+  auto run = [&](const LinkEnds &r, const LinkPar &c) {
+    const uint32_t s = r.src & ~LINK_FIRST, d = r.tgt & ~LINK_FIRST;
+    const double2 pt = P[d], ps = P[s];
+    double2 vt = V[d], vs = V[s];
+    if (!link_apply(c, pt.x, pt.y, ps.x, ps.y, a.alpha, vt, vs)) {
+      bad = true;
+      return;
+    }
+    V[d] = vt;
+    V[s] = vs;
+  };
+  for (double k = 0; k < a.iterations; k += 1) {
+    uint32_t lo = 0, hi = a.level_start[2];  // level 1 starts at place 0
+    LinkEnds r;
+    LinkPar c;
+    if (t < hi) {
+      r = a.ends[t];
+      c = link_par(a, t);
+    }
+    __syncthreads();
+    for (uint32_t lv = 1; lv <= a.levels; ++lv) {
+      const uint32_t nhi = lv < a.levels ? a.level_start[lv + 2] : m;
+      LinkEnds rn;
+      LinkPar cn;
+      if (lv < a.levels && hi + t < nhi) {
+        rn = a.ends[hi + t];
+        cn = link_par(a, hi + t);
+      }
+      if (lo + t < hi) run(r, c);
+      for (uint32_t p = lo + nt + t; p < hi; p += nt) run(a.ends[p], link_par(a, p));
+      __syncthreads();
+      r = rn;
+      c = cn;
+      lo = hi;
+      hi = nhi;
+    }
+  }
+  bad = __syncthreads_or(bad);
+  if (t == 0) *a.flag = bad;
+  if (bad) {
+    if (a.serial_lcg && t == 0)
+      link_serial_lcg(a.xs, a.ys, a.vxs, a.vys, a.l, a.alpha, a.iterations, a.rng, a.status);
+    return;
+  }
+  for (uint32_t i = t; i < a.nodes; i += nt) {
+    a.vxs[i] = V[i].x;
+    a.vys[i] = V[i].y;
+  }
+}
+
+// A link's input from the link before it on one of its nodes, or all ones in
+// either half while that has not come. Each half is a 64-bit access and is
+// looked at by itself, so the halves need not arrive together; the value is
+// the message, so nothing else is ordered by it. (A velocity whose bits are
+// all ones, a NaN no arithmetic gives, runs the wait out: the serial pass.)
+__device__ __forceinline__ ulonglong2 msg_read(const ulonglong2 *p) {
+  ulonglong2 v;
+  asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p) : "memory");
   return v;
 }
-
-// A finished link's count on a node, ordered after its velocity writes.
-__device__ inline void red_release_add(uint32_t *p, uint32_t v) {
-  asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+__device__ __forceinline__ void msg_write(ulonglong2 *p, unsigned long long x, unsigned long long y) {
+  asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(x), "l"(y) : "memory");
 }
 
-__device__ inline bool link_wait(const uint32_t *done, uint32_t src, uint32_t ns, uint32_t tgt,
-                                 uint32_t nt, unsigned sleep_ns) {
-  // acquire loads: a count seen orders the counted links' writes before the
-  // velocities this link reads
-  if (ld_acquire_u32(&done[src]) >= ns && ld_acquire_u32(&done[tgt]) >= nt) return true;
-  const unsigned long long t0 = globaltimer_ns();
-  for (uint32_t it = 0;; ++it) {
-    if (ld_acquire_u32(&done[src]) >= ns && ld_acquire_u32(&done[tgt]) >= nt) return true;
-    if (it >= 8 && sleep_ns) __nanosleep(sleep_ns);
-    if ((it & 15) == 15 && globaltimer_ns() - t0 > 20000000ull) return false;
-  }
-}
+constexpr uint32_t LINK_MET_JIGGLE = 1, LINK_GAVE_UP = 2;
 
-// The pass as dataflow, in one cooperative launch: the pass-start snapshot,
-// then every link (threads take them in level order) once the links before
-// it on its two nodes have finished (per-node finished counts against the
-// plan's per-link counts; a link's parameters and endpoint positions are
-// loaded before its wait), then the snapshot back if a link met a zero or
-// NaN delta or a wait gave up (the serial kernel then runs the pass).
+// The pass as messages, in one cooperative launch, for any size: threads take
+// the links in level order; a link waits (bounded) for the velocities of its
+// two nodes from the links before it there, each a 16-byte message in a place
+// of its own, and hands them on to the links after it. A level costs one
+// message through L2 and one link's arithmetic (1.1 us; 5 us with finished
+// counts and the velocities read after an acquire). The first link on a node
+// reads its velocity and saves it, the last one writes it. A read message is
+// cleared for the next pass. If a link met a zero or NaN delta or gave up, the
+// last block puts the saved velocities back and runs the serial pass.
+// The work of a ready link is inside the polling loop: a lane never waits at
+// a convergence point for a lane that waits for its message.
 __global__ void __launch_bounds__(256) k_link_flow(LinkFlowArgs a) {
-  cg::grid_group g = cg::this_grid();
   const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
-  if (tid == 0) *a.flag = 0;
-  for (uint32_t i = tid; i < a.n; i += nth) {
-    a.svx[i] = a.vxs[i];
-    a.svy[i] = a.vys[i];
-  }
   const uint32_t m = a.l.m;
-  bool bad = false;
+  const unsigned long long none = ~0ull;
+  uint32_t bad = 0;
   for (double k = 0; k < a.iterations; k += 1) {
-    for (uint32_t i = tid; i < a.nodes; i += nth) a.done[i] = 0;
-    g.sync();  // the snapshot and the counts before any link runs
-    for (uint32_t p = tid; p < m; p += nth) {
-      LinkPre c;
-      link_params(a.l, a.order[p], c);
-      link_positions(a.xs, a.ys, c);
-      const uint32_t ns = a.need[2 * p], nt = a.need[2 * p + 1];
-      if (!link_wait(a.done, c.src, ns, c.tgt, nt, a.sleep_ns)) bad = true;
-      const double vxt = __ldcg(&a.vxs[c.tgt]), vyt = __ldcg(&a.vys[c.tgt]);
-      const double vxsrc = __ldcg(&a.vxs[c.src]), vysrc = __ldcg(&a.vys[c.src]);
-      double x = c.xt + vxt - c.xsrc - vxsrc;
-      double y = c.yt + vyt - c.ysrc - vysrc;
-      if (x == 0 || x != x || y == 0 || y != y) {
-        bad = true;
-      } else {
-        double len = sqrt(x * x + y * y);
-        len = (len - c.dist) / len * a.alpha * c.str;
-        x *= len;
-        y *= len;
-        double b = c.bias;
-        a.vxs[c.tgt] = vxt - x * b;
-        a.vys[c.tgt] = vyt - y * b;
-        b = 1 - b;
-        a.vxs[c.src] = vxsrc + x * b;
-        a.vys[c.src] = vysrc + y * b;
+    if (k > 0) cg::this_grid().sync();  // the last iteration's velocities and cleared messages
+    uint32_t p = tid;
+    LinkEnds r;
+    LinkPar c;
+    double2 pt, ps;
+    ulonglong2 in_s, in_t;
+    bool fresh = true;
+    unsigned long long t0 = 0;
+    uint32_t polls = 0;
+    while (p < m) {
+      if (fresh) {
+        fresh = false;
+        polls = 0;
+        r = a.ends[p];
+        c = link_par(a, p);
+        const uint32_t s = r.src & ~LINK_FIRST, d = r.tgt & ~LINK_FIRST;
+        pt = make_double2(a.xs[d], a.ys[d]);
+        ps = make_double2(a.xs[s], a.ys[s]);
+        in_s = in_t = make_ulonglong2(none, none);
+        if (r.src & LINK_FIRST) {
+          const double x = __ldcg(&a.vxs[s]), y = __ldcg(&a.vys[s]);
+          if (k == 0) {
+            a.svx[s] = x;
+            a.svy[s] = y;
+          }
+          in_s = make_ulonglong2(__double_as_longlong(x), __double_as_longlong(y));
+        }
+        if (r.tgt & LINK_FIRST) {
+          const double x = __ldcg(&a.vxs[d]), y = __ldcg(&a.vys[d]);
+          if (k == 0) {
+            a.svx[d] = x;
+            a.svy[d] = y;
+          }
+          in_t = make_ulonglong2(__double_as_longlong(x), __double_as_longlong(y));
+        }
       }
-      red_release_add(&a.done[c.src], 1u);
-      red_release_add(&a.done[c.tgt], 1u);
+      bool gave_up = false;
+      if (!(r.src & LINK_FIRST) && (in_s.x == none || in_s.y == none)) in_s = msg_read(&a.msg[2 * (size_t)p]);
+      if (!(r.tgt & LINK_FIRST) && (in_t.x == none || in_t.y == none)) in_t = msg_read(&a.msg[2 * (size_t)p + 1]);
+      const bool have_s = (r.src & LINK_FIRST) || (in_s.x != none && in_s.y != none);
+      const bool have_t = (r.tgt & LINK_FIRST) || (in_t.x != none && in_t.y != none);
+      if (!(have_s && have_t)) {
+        if (polls == 0) t0 = globaltimer_ns();
+        ++polls;
+        if (polls > 8 && a.sleep_ns) __nanosleep(a.sleep_ns);
+        gave_up = (polls & 15) == 0 && globaltimer_ns() - t0 > 20000000ull;
+      }
+      if ((have_s && have_t) || gave_up) {
+        const uint32_t s = r.src & ~LINK_FIRST, d = r.tgt & ~LINK_FIRST;
+        if (gave_up) bad |= LINK_GAVE_UP;
+        double2 vs = make_double2(__longlong_as_double(in_s.x), __longlong_as_double(in_s.y));
+        double2 vt = make_double2(__longlong_as_double(in_t.x), __longlong_as_double(in_t.y));
+        if (gave_up) vs = vt = make_double2(0, 0);  // the pass is put back: only keep the others going
+        else if (!link_apply(c, pt.x, pt.y, ps.x, ps.y, a.alpha, vt, vs)) bad |= LINK_MET_JIGGLE;
+        if (r.next_src != NONE) {
+          msg_write(&a.msg[r.next_src], __double_as_longlong(vs.x), __double_as_longlong(vs.y));
+        } else {
+          a.vxs[s] = vs.x;
+          a.vys[s] = vs.y;
+        }
+        if (r.next_tgt != NONE) {
+          msg_write(&a.msg[r.next_tgt], __double_as_longlong(vt.x), __double_as_longlong(vt.y));
+        } else {
+          a.vxs[d] = vt.x;
+          a.vys[d] = vt.y;
+        }
+        if (!(r.src & LINK_FIRST)) msg_write(&a.msg[2 * (size_t)p], none, none);
+        if (!(r.tgt & LINK_FIRST)) msg_write(&a.msg[2 * (size_t)p + 1], none, none);
+        p += nth;
+        fresh = true;
+      }
     }
-    g.sync();
   }
-  if (bad) atomicOr(a.flag, 1u);
-  g.sync();
-  if (__ldcg(a.flag)) {
-    for (uint32_t i = tid; i < a.n; i += nth) {
-      a.vxs[i] = __ldcg(&a.svx[i]);
-      a.vys[i] = __ldcg(&a.svy[i]);
-    }
-    if (a.serial_lcg) {
-      g.sync();
-      if (tid == 0) link_serial_lcg(a.xs, a.ys, a.vxs, a.vys, a.l, a.alpha, a.iterations, a.rng, a.status);
+  // the block that ends last sees every block's writes
+  __shared__ uint32_t bits;
+  const bool any_jiggle = __syncthreads_or(bad & LINK_MET_JIGGLE);
+  const bool any_gave_up = __syncthreads_or(bad & LINK_GAVE_UP);
+  if (threadIdx.x == 0) {
+    if (any_jiggle || any_gave_up)
+      atomicOr(&a.tally[1], (any_jiggle ? LINK_MET_JIGGLE : 0u) | (any_gave_up ? LINK_GAVE_UP : 0u));
+    __threadfence();
+    bits = NONE;
+    if (atomicAdd(&a.tally[0], 1u) == gridDim.x - 1) {
+      __threadfence();
+      bits = atomicExch(&a.tally[1], 0u);
+      a.tally[0] = 0;
+      *a.flag = bits != 0;
     }
   }
+  __syncthreads();
+  if (bits == NONE || bits == 0) return;
+  for (uint32_t p = threadIdx.x; p < m; p += blockDim.x) {
+    const LinkEnds r = a.ends[p];
+    const uint32_t s = r.src & ~LINK_FIRST, d = r.tgt & ~LINK_FIRST;
+    if (r.src & LINK_FIRST) {
+      a.vxs[s] = __ldcg(&a.svx[s]);
+      a.vys[s] = __ldcg(&a.svy[s]);
+    }
+    if (r.tgt & LINK_FIRST) {
+      a.vxs[d] = __ldcg(&a.svx[d]);
+      a.vys[d] = __ldcg(&a.svy[d]);
+    }
+    if (bits & LINK_GAVE_UP) {  // messages nobody took
+      msg_write(&a.msg[2 * (size_t)p], none, none);
+      msg_write(&a.msg[2 * (size_t)p + 1], none, none);
+    }
+  }
+  __syncthreads();
+  if (a.serial_lcg && threadIdx.x == 0)
+    link_serial_lcg(a.xs, a.ys, a.vxs, a.vys, a.l, a.alpha, a.iterations, a.rng, a.status);
 }
 
-static int g_link_blocks = 0;
+__global__ void k_link_flag(uint32_t *flag) { *flag = 1; }
 
-void link_exact(const NodeArrays &a, const LinkArrays &l, const LinkPlan &plan, double alpha,
+void link_exact(const NodeArrays &a, const LinkArrays &l, LinkPlan &plan, double alpha,
                 double iterations, Rng *rng, uint32_t *flag, uint32_t *status, bool serial_lcg,
                 cudaStream_t st) {
   if (l.m == 0) return;
   const uint32_t n = a.n;
-  if (!g_link_blocks) {
-    int dev = 0, sms = 0, per = 0;
+  if (plan.self) {
+    // a link from a node to itself always draws: the pass is serial
+    D3_LAUNCH(k_link_flag, 1, 1, 0, st)(flag);
+    if (serial_lcg) link_fallback_lcg(a, l, alpha, iterations, rng, flag, status, st);
+    return;
+  }
+  if (!plan.gathered) {
+    D3_LAUNCH(k_link_params, blocks_for(l.m, 256), 256, 0, st)(l, plan.order, plan.par);
+    plan.gathered = true;
+  }
+  LinkFlowArgs c;
+  c.xs = a.x; c.ys = a.y; c.vxs = a.vx; c.vys = a.vy; c.svx = a.snap_vx; c.svy = a.snap_vy;
+  c.l = l; c.ends = plan.ends; c.par = plan.par; c.level_start = plan.level_start;
+  c.msg = reinterpret_cast<ulonglong2 *>(plan.msg); c.tally = plan.tally;
+  c.levels = plan.levels; c.nodes = plan.nodes; c.alpha = alpha; c.iterations = iterations;
+  c.flag = flag; c.rng = rng; c.status = status; c.serial_lcg = serial_lcg;
+  c.sleep_ns = wait_sleep_ns();
+  // One SM when its shared memory holds the nodes: a level there takes a third
+  // of a message's time (1,000 nodes, 2,000 links: 12 us for 30; 5,003 nodes,
+  // 10,006 links: 22 us for 38).
+  if (plan.nodes <= LINK_BLOCK_NODES) {
+    static const bool attr =
+        cudaFuncSetAttribute(k_link_block, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)(LINK_BLOCK_NODES * 2 * sizeof(double2))) == cudaSuccess;
+    if (attr) {
+      const uint32_t w = plan.width > 1024 ? 1024 : (plan.width + 31) / 32 * 32;
+      D3_LAUNCH(k_link_block, 1, w, plan.nodes * 2 * sizeof(double2), st)(c);
+      return;
+    }
+  }
+  static int sms = 0, per_sm = 0;
+  if (!per_sm) {
+    int dev = 0, per = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_link_flow, 256, 0);
@@ -805,19 +1000,14 @@ void link_exact(const NodeArrays &a, const LinkArrays &l, const LinkPlan &plan, 
       const int v = atoi(e);
       if (v >= 1 && v <= per) want = v;
     }
-    g_link_blocks = sms * want;
+    per_sm = want;
   }
   {
-    LinkFlowArgs c;
-    c.xs = a.x; c.ys = a.y; c.vxs = a.vx; c.vys = a.vy; c.svx = a.snap_vx; c.svy = a.snap_vy;
-    c.l = l; c.order = plan.order; c.need = plan.need; c.done = plan.done;
-    c.n = n; c.nodes = plan.nodes; c.alpha = alpha; c.iterations = iterations; c.flag = flag;
-    c.sleep_ns = wait_sleep_ns();
-    c.rng = rng; c.status = status; c.serial_lcg = serial_lcg;
     void *params[] = {&c};
+    const unsigned most = (unsigned)(sms * per_sm), blocks = blocks_for(l.m, 256);
     ++g_launches;
-    if (cudaLaunchCooperativeKernel((const void *)k_link_flow, g_link_blocks, 256, params, 0, st) ==
-        cudaSuccess)
+    if (cudaLaunchCooperativeKernel((const void *)k_link_flow, blocks < most ? blocks : most, 256,
+                                    params, 0, st) == cudaSuccess)
       return;
     cudaGetLastError();
   }

@@ -56,14 +56,26 @@ void many_body_rerun(TreeDev &t, const NodeArrays &a, const double *strengths,
 
 // Link levels (computed on the host from source/target): links grouped by
 // level so that links sharing a node keep their order (link.zig:8-40).
+// A link in the plan's order (by level): its nodes (LINK_FIRST: no earlier
+// link touches that node) and the inputs that its nodes' velocities go on to
+// (2 x place + side of the next link on the node; NONE: it is the last one).
+constexpr uint32_t LINK_FIRST = 0x80000000u;
+struct alignas(16) LinkEnds {
+  uint32_t src, tgt, next_src, next_tgt;
+};
+
 struct LinkPlan {
   uint32_t m = 0, levels = 0, nodes = 0;
+  uint32_t width = 0;               // links of the widest level
+  bool self = false;                // some link joins a node with itself
+  bool gathered = false;            // par holds the current link arrays
   uint32_t *order = nullptr;        // device: link ids grouped by level
-  uint32_t *level_start = nullptr;  // device: levels + 1 offsets
+  uint32_t *level_start = nullptr;  // device: levels + 1 offsets (level 1 first at [1])
   uint32_t *h_level_start = nullptr;
-  uint32_t *need = nullptr;         // device: per position in order, the earlier links on
-                                    // its source, then on its target (2 per link)
-  uint32_t *done = nullptr;         // device: per node, links on it finished (this pass)
+  LinkEnds *ends = nullptr;         // device, in plan order
+  double *par = nullptr;            // device: distance, strength, bias planes in plan order
+  double2 *msg = nullptr;           // device: per link its two input messages
+  uint32_t *tally = nullptr;        // device: blocks done, failure bits of the running pass
 };
 int link_plan_build(LinkPlan &plan, const uint32_t *src, const uint32_t *tgt, uint32_t m);
 void link_plan_free(LinkPlan &plan);
@@ -75,10 +87,10 @@ struct LinkArrays {
 };
 
 // Exact link: Gauss-Seidel in dependency order. A link that meets a zero /
-// NaN delta (where d3 draws from `random`) sets *flag and the pass is undone
-// (velocities restored from the snapshot); with serial_lcg the serial pass on
-// the device LCG then runs in the same launch, otherwise the caller runs it.
-void link_exact(const NodeArrays &a, const LinkArrays &l, const LinkPlan &plan, double alpha,
+// NaN delta (where d3 draws from `random`) sets *flag and the velocities are
+// again those of the pass's start; with serial_lcg the serial pass on the
+// device LCG then runs in the same launch, otherwise the caller runs it.
+void link_exact(const NodeArrays &a, const LinkArrays &l, LinkPlan &plan, double alpha,
                 double iterations, Rng *rng, uint32_t *flag, uint32_t *status, bool serial_lcg,
                 cudaStream_t st);
 // The serial pass on the device LCG, only when *flag is set.
