@@ -98,11 +98,13 @@ __device__ inline uint32_t arrive_acq_rel(uint32_t *p) {
 // with a truthy |value|. Every cell's traversal record: the thread visiting
 // an internal cell writes its fixed part (width test, skip link); the climb
 // writes its centroid and charge.
-__global__ void k_mb_accumulate(Cell *cells, const uint32_t *parent, const uint8_t *pnch,
-                                uint32_t *counter, const uint32_t *perm, const uint32_t *skip,
-                                const double *xs, const double *ys, const double *strengths,
-                                double theta2, MRec *rec, const uint32_t *info) {
-  const uint32_t len = info[1];
+// BLOCK: all by one block, `counter` in its shared memory.
+template <bool BLOCK>
+__device__ __forceinline__ void accumulate(Cell *cells, const uint32_t *parent, const uint8_t *pnch,
+                                           uint32_t *counter, const uint32_t *perm,
+                                           const uint32_t *skip, const double *xs, const double *ys,
+                                           const double *strengths, double theta2, MRec *rec,
+                                           uint32_t len) {
   for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < len; c += gridDim.x * blockDim.x) {
     Cell *q = &cells[c];
     if (!is_leaf(*q)) {
@@ -185,13 +187,21 @@ __global__ void k_mb_accumulate(Cell *cells, const uint32_t *parent, const uint8
       uint32_t ch[4];
 #pragma unroll
       for (int k = 0; k < 4; ++k) ch[k] = cells[p].child[k];
-      if (arrive_acq_rel(&counter[p]) != up.nch - 1) break;
+      if (BLOCK) {
+        __threadfence_block();
+        const uint32_t old = atomicAdd(&counter[p], 1u);
+        __threadfence_block();
+        if (old != up.nch - 1) break;
+      } else if (arrive_acq_rel(&counter[p]) != up.nch - 1) {
+        break;
+      }
       double2 cxy[4], cvw[4];
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         if (ch[k] == NONE) continue;
-        cxy[k] = __ldcg((const double2 *)&rec[ch[k]].x);
-        cvw[k] = __ldcg((const double2 *)&rec[ch[k]].value);
+        const double2 *q0 = (const double2 *)&rec[ch[k]].x, *q1 = (const double2 *)&rec[ch[k]].value;
+        cxy[k] = BLOCK ? *q0 : __ldcg(q0);
+        cvw[k] = BLOCK ? *q1 : __ldcg(q1);
       }
       double st = 0, weight = 0, x = 0, y = 0;
 #pragma unroll
@@ -213,6 +223,34 @@ __global__ void k_mb_accumulate(Cell *cells, const uint32_t *parent, const uint8
       up = next;
     }
   }
+}
+
+__global__ void k_mb_accumulate(Cell *cells, const uint32_t *parent, const uint8_t *pnch,
+                                uint32_t *counter, const uint32_t *perm, const uint32_t *skip,
+                                const double *xs, const double *ys, const double *strengths,
+                                double theta2, MRec *rec, const uint32_t *info) {
+  accumulate<false>(cells, parent, pnch, counter, perm, skip, xs, ys, strengths, theta2, rec, info[1]);
+}
+
+// Small trees by one block: an arrival is a shared-memory atomic and the
+// children's values come from this SM's L1, where the grid's arrivals go
+// through L2 (1 us a level): 77 nodes 17 -> 12 us (event time). At 1,000
+// nodes the one SM is busy longer than the grid's chain takes (27 / 22 us).
+constexpr uint32_t ACC_BLOCK_NODES = 384, ACC_BLOCK_CELLS = 5120;  // (buffers of up to 1,024 nodes)
+
+__global__ void __launch_bounds__(512) k_mb_accumulate_block(
+    Cell *cells, const uint32_t *parent, const uint8_t *pnch, uint32_t *counter, const uint32_t *perm,
+    const uint32_t *skip, const double *xs, const double *ys, const double *strengths, double theta2,
+    MRec *rec, const uint32_t *info) {
+  __shared__ uint32_t count[ACC_BLOCK_CELLS];
+  const uint32_t len = info[1];
+  if (len > ACC_BLOCK_CELLS) {  // (cell buffers of a simulation that was larger before)
+    accumulate<false>(cells, parent, pnch, counter, perm, skip, xs, ys, strengths, theta2, rec, len);
+    return;
+  }
+  for (uint32_t c = threadIdx.x; c < len; c += blockDim.x) count[c] = 0;
+  __syncthreads();
+  accumulate<true>(cells, parent, pnch, count, perm, skip, xs, ys, strengths, theta2, rec, len);
 }
 
 // collide.zig:117-129 (prepare): leaf radius of its head, internal the largest
@@ -254,7 +292,7 @@ __global__ void k_collide_prep(Cell *cells, const uint32_t *parent, const uint32
 // jiggle, count the draws it would make, and do not write. Otherwise draws
 // come from the stream at `draw0`.
 template <bool RECORD>
-__device__ inline uint32_t mb_node(const MRec *rec, const uint32_t *perm,
+__device__ __forceinline__ uint32_t mb_node(const MRec *rec, const uint32_t *perm,
                                    uint32_t len, const double *xs, const double *ys,
                                    double *vxs, double *vys, const double *strengths,
                                    const ManyBodyParams p, uint32_t i, const Rng *rng,
@@ -332,6 +370,175 @@ __device__ inline uint32_t mb_node(const MRec *rec, const uint32_t *perm,
   return flagged ? draws : 0;
 }
 
+template <bool RECORD>
+__device__ __noinline__ uint32_t mb_node_call(const MRec *rec, const uint32_t *perm, uint32_t len,
+                                              const double *xs, const double *ys, double *vxs,
+                                              double *vys, const double *strengths,
+                                              const ManyBodyParams &p, uint32_t i, const Rng *rng,
+                                              uint64_t draw0) {
+  return mb_node<RECORD>(rec, perm, len, xs, ys, vxs, vys, strengths, p, i, rng, draw0);
+}
+
+// A warp's shared memory for one target (mb_warp): a bit per record, a stack
+// of cells to visit (later the accepted records in order), a window's terms.
+constexpr uint32_t MB_STACK = 1024;
+__host__ __device__ inline uint32_t mb_warp_words(uint32_t records) {
+  return MB_STACK + (records + 127) / 128 * 4;  // whole 16-byte units
+}
+
+// One target by a warp (all lanes with the same arguments). A thread per
+// target is a chain of dependent steps, one per visited record (500 cycles
+// each), and a small graph has no other targets to hide it; here the visit is
+// spread over the lanes and only the sum is a chain. The visit itself needs no
+// order: cells are popped 32 at a time from a stack, tested, and opened ones
+// push their children; a record that adds a term sets its bit. Records are in
+// preorder, so the set bits from the lowest up are the terms in visit order:
+// they are formed 32 at a time and added one after the other, which gives
+// mb_node's sums. (A stack that would overflow, at opening angles far below
+// d3's, leaves the target to mb_node on one lane.) Returns as mb_node does.
+template <bool RECORD>
+__device__ uint32_t mb_warp(const MRec *rec, const Cell *cells, const uint32_t *perm, uint32_t len,
+                            const double *xs, const double *ys, double *vxs, double *vys,
+                            const double *strengths, const ManyBodyParams &p, uint32_t i,
+                            const Rng *rng, uint64_t draw0, uint32_t *work, double2 *terms) {
+  const unsigned lane = threadIdx.x & 31, full = 0xffffffffu, before = (1u << lane) - 1u;
+  uint32_t *const stack = work, *const bits = work + MB_STACK;
+  const uint32_t words = (len + 31) / 32;
+  const double nx = xs[i], ny = ys[i];
+  for (uint32_t w = lane; w < words; w += 32) bits[w] = 0;
+  if (lane == 0) stack[0] = 0;
+  __syncwarp();
+  for (uint32_t sp = 1; sp;) {
+    const uint32_t take = sp < 32 ? sp : 32;
+    sp -= take;
+    const bool in = lane < take;
+    const uint32_t c = in ? stack[sp + lane] : 0;
+    __syncwarp();
+    uint2 ch[2] = {{NONE, NONE}, {NONE, NONE}};
+    if (in) {
+      const double x = rec[c].x - nx, y = rec[c].y - ny, value = rec[c].value, wt = rec[c].wt;
+      const uint32_t head = rec[c].head;
+      const double l = x * x + y * y;
+      if (value != 0 && value == value) {
+        if (wt < l) {
+          if (l < p.dmax2) atomicOr(&bits[c >> 5], 1u << (c & 31));
+        } else if (head != NONE) {
+          if (!(l >= p.dmax2) && (head != i || rec[c].count > 1)) atomicOr(&bits[c >> 5], 1u << (c & 31));
+        } else {
+          const uint2 *child = reinterpret_cast<const uint2 *>(cells[c].child);
+          ch[0] = child[0];
+          ch[1] = child[1];
+        }
+      }
+    }
+    const uint32_t nch = (ch[0].x != NONE) + (ch[0].y != NONE) + (ch[1].x != NONE) + (ch[1].y != NONE);
+    const unsigned b0 = __ballot_sync(full, nch & 1), b1 = __ballot_sync(full, nch & 2),
+                   b2 = __ballot_sync(full, nch & 4);
+    const uint32_t total = __popc(b0) + 2 * __popc(b1) + 4 * __popc(b2);
+    if (sp + total > MB_STACK) {
+      uint32_t d = 0;
+      if (lane == 0)
+        d = mb_node_call<RECORD>(rec, perm, len, xs, ys, vxs, vys, strengths, p, i, rng, draw0);
+      return __shfl_sync(full, d, 0);
+    }
+    uint32_t at = sp + __popc(b0 & before) + 2 * __popc(b1 & before) + 4 * __popc(b2 & before);
+    if (ch[0].x != NONE) stack[at++] = ch[0].x;
+    if (ch[0].y != NONE) stack[at++] = ch[0].y;
+    if (ch[1].x != NONE) stack[at++] = ch[1].x;
+    if (ch[1].y != NONE) stack[at++] = ch[1].y;
+    sp += total;
+    __syncwarp();
+  }
+  double vx = vxs[i], vy = vys[i];
+  uint32_t draws = 0;
+  for (uint32_t w0 = 0; w0 < words; w0 += 32) {
+    // the accepted records of 32 words, in order, into the stack's place
+    unsigned set = w0 + lane < words ? bits[w0 + lane] : 0;
+    if (!__any_sync(full, set)) continue;
+    uint32_t incl = __popc(set);
+    const uint32_t own = incl;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(full, incl, o);
+      if (lane >= (unsigned)o) incl += v;
+    }
+    const uint32_t count = __shfl_sync(full, incl, 31);
+    for (uint32_t at = incl - own; set; set &= set - 1) stack[at++] = (w0 + lane) * 32 + __ffs(set) - 1;
+    __syncwarp();
+    for (uint32_t k0 = 0; k0 < count; k0 += 32) {
+      const uint32_t nt = count - k0 < 32 ? count - k0 : 32;
+      const bool in = lane < nt;
+      double x = 0, y = 0, l = 1;
+      MRec q;
+      q.head = q.first = 0;
+      q.count = 1;
+      if (in) {
+        q = rec[stack[k0 + lane]];
+        x = q.x - nx;
+        y = q.y - ny;
+        l = x * x + y * y;
+      }
+      const bool far = in && q.wt < l, zx = in && x == 0, zy = in && y == 0;
+      if (__any_sync(full, zx || zy)) {
+        const unsigned bx = __ballot_sync(full, zx), by = __ballot_sync(full, zy);
+        if (!RECORD) {
+          uint64_t d = draw0 + draws + __popc(bx & before) + __popc(by & before);
+          if (zx) { x = (rng_draw_at(*rng, d++) - 0.5) * 1e-6; l += x * x; }
+          if (zy) { y = (rng_draw_at(*rng, d) - 0.5) * 1e-6; l += y * y; }
+        }
+        draws += __popc(bx) + __popc(by);
+      }
+      if (RECORD && draws) continue;  // flagged: only the draws still count
+      if (in && l < p.dmin2) l = sqrt(p.dmin2 * l);
+      if (in) {
+        // far: x value alpha / l, y value alpha / l; a leaf's point: x and y
+        // times strength alpha / l (the same two divisions for both kinds)
+        const double sv = far ? q.value : strengths[q.head];
+        const double a = far ? x * sv * p.alpha : sv * p.alpha, b = far ? y * sv * p.alpha : a;
+        const double qa = a / l, qb = b / l;
+        terms[lane] = make_double2(far ? qa : x * qa, far ? qb : y * qa);
+      }
+      const unsigned many = __ballot_sync(full, in && !far && q.count > 1);
+      __syncwarp();
+      if (!many && nt == 32) {
+#pragma unroll 8
+        for (uint32_t k = 0; k < 32; ++k) {
+          const double2 t = terms[k];
+          vx += t.x;
+          vy += t.y;
+        }
+      } else {
+        for (uint32_t k = 0; k < nt; ++k) {
+          if (!((many >> k) & 1u)) {
+            vx += terms[k].x;
+            vy += terms[k].y;
+            continue;
+          }
+          // a leaf of coincident points: its points one by one
+          const uint32_t first = __shfl_sync(full, q.first, k), points = __shfl_sync(full, q.count, k);
+          const double lx = __shfl_sync(full, x, k), ly = __shfl_sync(full, y, k);
+          const double ll = __shfl_sync(full, l, k);
+          for (uint32_t k2 = first + points; k2 > first;) {
+            --k2;
+            const uint32_t j = perm[k2];
+            if (j != i) {
+              const double wj = strengths[j] * p.alpha / ll;
+              vx += lx * wj;
+              vy += ly * wj;
+            }
+          }
+        }
+      }
+      __syncwarp();
+    }
+  }
+  if (RECORD && draws) return draws;  // flagged: nothing written
+  if (lane == 0) {
+    vxs[i] = vx;
+    vys[i] = vy;
+  }
+  return draws;
+}
+
 // Record pass over all nodes in Morton order (perm, then the NaN nodes).
 __global__ void __launch_bounds__(128) k_mb_traverse(const MRec *rec,
                                                      const uint32_t *perm, const uint32_t *info,
@@ -353,19 +560,69 @@ __global__ void __launch_bounds__(128) k_mb_traverse(const MRec *rec,
   if (d) atomicAdd(&counters[1], 1u);
 }
 
+// The same by a warp a target (mb_warp); `words` of shared memory a warp.
+__global__ void __launch_bounds__(128) k_mb_traverse_warp(
+    const MRec *rec, const Cell *cells, const uint32_t *perm, const uint32_t *info, const double *xs,
+    const double *ys, double *vxs, double *vys, const double *strengths, ManyBodyParams p, uint32_t n,
+    uint32_t *draws, uint32_t *counters, uint32_t words) {
+  extern __shared__ uint4 mb_smem[];
+  __shared__ double2 terms[4][32];
+  const uint32_t pos = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, warp = threadIdx.x >> 5;
+  if (pos >= n || info[5]) return;
+  const uint32_t len = info[1];
+  const uint32_t i = perm[pos];
+  uint32_t *work = reinterpret_cast<uint32_t *>(mb_smem) + (size_t)warp * words;
+  const uint32_t d = len ? mb_warp<true>(rec, cells, perm, len, xs, ys, vxs, vys, strengths, p, i,
+                                         nullptr, 0, work, terms[warp])
+                         : 0;
+  if ((threadIdx.x & 31) != 0) return;
+  draws[i] = d;
+  if (d) atomicAdd(&counters[1], 1u);
+}
+
+// The flagged ones of nodes i0 .. i0 + 31: one after the other by the whole
+// warp when a bit per record fits its `words` of shared memory (a flagged
+// node, 4 % of them where coincident ones are in play, is a chain that takes
+// one thread as long as the whole record pass), else a lane each.
+__device__ void mb_rerun_warp(const MRec *rec, const Cell *cells, const uint32_t *perm, uint32_t len,
+                              const double *xs, const double *ys, double *vxs, double *vys,
+                              const double *strengths, const ManyBodyParams &p, uint32_t n,
+                              uint32_t i0, const uint32_t *draws, const uint32_t *offsets,
+                              const Rng *rng, uint32_t *work, uint32_t words, double2 *terms) {
+  const uint32_t i = i0 + (threadIdx.x & 31);
+  const bool mine = i < n && __ldcg(&draws[i]) != 0;
+  const uint32_t off = mine ? __ldcg(&offsets[i]) : 0;
+  if (mb_warp_words(len) > words) {
+    if (mine) mb_node_call<false>(rec, perm, len, xs, ys, vxs, vys, strengths, p, i, rng, off);
+    return;
+  }
+  unsigned flagged = __ballot_sync(0xffffffffu, mine);
+  while (flagged) {
+    const unsigned b = __ffs(flagged) - 1;
+    flagged &= flagged - 1;
+    mb_warp<false>(rec, cells, perm, len, xs, ys, vxs, vys, strengths, p, i0 + b, rng,
+                   __shfl_sync(0xffffffffu, off, b), work, terms);
+    __syncwarp();
+  }
+}
+
 // Flagged nodes again, each from its own offset in the draw stream (the
 // exclusive scan of draws over node index = d3's draw order).
-__global__ void __launch_bounds__(128) k_mb_rerun(const MRec *rec,
+__global__ void __launch_bounds__(128) k_mb_rerun(const MRec *rec, const Cell *cells,
                                                   const uint32_t *perm, const uint32_t *info,
                                                   const double *xs, const double *ys, double *vxs,
                                                   double *vys, const double *strengths,
                                                   ManyBodyParams p, uint32_t n,
                                                   const uint32_t *draws, const uint32_t *offsets,
-                                                  const uint32_t *counters, const Rng *rng) {
+                                                  const uint32_t *counters, const Rng *rng,
+                                                  uint32_t words) {
+  extern __shared__ uint4 mb_smem[];
   if (counters[1] == 0 || info[5]) return;
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n || draws[i] == 0) return;
-  mb_node<false>(rec, perm, info[1], xs, ys, vxs, vys, strengths, p, i, rng, offsets[i]);
+  __shared__ double2 terms[4][32];
+  const uint32_t i0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u;
+  mb_rerun_warp(rec, cells, perm, info[1], xs, ys, vxs, vys, strengths, p, n, i0, draws, offsets, rng,
+                reinterpret_cast<uint32_t *>(mb_smem) + (size_t)(threadIdx.x >> 5) * words, words,
+                terms[threadIdx.x >> 5]);
 }
 
 // The jiggle draws of the flagged targets, after the record pass, in one
@@ -373,22 +630,25 @@ __global__ void __launch_bounds__(128) k_mb_rerun(const MRec *rec,
 // node index (d3's draw order), the flagged targets again from their stream
 // positions, then the LCG advanced past all the draws. Nothing to do (the
 // usual case) is decided by every block alike from the flagged count.
-__global__ void __launch_bounds__(256) k_mb_draws(const MRec *rec, const uint32_t *perm,
+__global__ void __launch_bounds__(256) k_mb_draws(const MRec *rec, const Cell *cells, const uint32_t *perm,
                                                   const uint32_t *info, const double *xs,
                                                   const double *ys, double *vxs, double *vys,
                                                   const double *strengths, ManyBodyParams p,
                                                   uint32_t n, const uint32_t *draws,
                                                   uint32_t *offsets, uint32_t *counters,
-                                                  uint32_t *bsum, Rng *rng) {
+                                                  uint32_t *bsum, Rng *rng, uint32_t words) {
+  extern __shared__ uint4 mb_smem[];
+  __shared__ double2 terms[8][32];
   if (__ldcg(&counters[1]) == 0 || __ldcg(&info[5])) return;
   cg::grid_group g = cg::this_grid();
   const uint32_t total = grid_excl_scan(g, draws, offsets, n, bsum);
   g.sync();
   const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
   const uint32_t len = info[1];
-  for (uint32_t i = tid; i < n; i += nth)
-    if (__ldcg(&draws[i]))
-      mb_node<false>(rec, perm, len, xs, ys, vxs, vys, strengths, p, i, rng, __ldcg(&offsets[i]));
+  for (uint32_t i0 = tid & ~31u; i0 < n; i0 += nth)
+    mb_rerun_warp(rec, cells, perm, len, xs, ys, vxs, vys, strengths, p, n, i0, draws, offsets, rng,
+                  reinterpret_cast<uint32_t *>(mb_smem) + (size_t)(threadIdx.x >> 5) * words, words,
+                  terms[threadIdx.x >> 5]);
   g.sync();
   if (tid == 0) {
     counters[0] = total;
@@ -410,6 +670,33 @@ static void climb_grid(unsigned &blocks, unsigned &threads, uint32_t cap) {
   if (blocks > 148 * 16) blocks = 148 * 16;
 }
 
+// Shared memory of k_mb_draws, two blocks of 8 warps an SM: a bit per record
+// up to 32,000 records (the trees of about 19,000 nodes). No more: the center
+// sum on the side stream holds 64 KB of one SM, and a cooperative launch waits
+// until all its blocks have room.
+constexpr size_t MB_DRAWS_SMEM = 64 * 1024;
+
+// The record pass: a warp per target up to MB_WARP_NODES nodes, a thread per
+// target above (event time, warp / thread: 77 nodes 22 / 41 us, 1,000 27 / 62,
+// 3,000 35 / 70, 5,003 56 / 72, 7,000 67 / 75, 10,000 113 / 80: a target takes
+// about 3,300 warp instructions, which 148 SMs issue in the time of the
+// longest serial visit at 8,000 targets).
+constexpr uint32_t MB_WARP_NODES = 7000;
+
+static void launch_traverse(TreeDev &t, const NodeArrays &a, const double *strengths,
+                            const ManyBodyParams &p, ForceScratch &s, cudaStream_t st) {
+  const uint32_t n = a.n;
+  const MRec *rec = (const MRec *)t.rec;
+  // four warps a block: at most 42 KB (the cell buffers may be larger than n asks for)
+  const uint32_t words = mb_warp_words(t.cells_cap);
+  if (n <= MB_WARP_NODES && 16 * words <= 42 * 1024)
+    D3_LAUNCH(k_mb_traverse_warp, blocks_for(n * 32ull, 128), 128, 16 * words, st)(
+        rec, t.cells, t.perm, t.info, a.x, a.y, a.vx, a.vy, strengths, p, n, s.draws, s.counters, words);
+  else
+    D3_LAUNCH(k_mb_traverse, blocks_for(n, 128), 128, 0, st)(rec, t.perm, t.info, a.x, a.y, a.vx, a.vy,
+                                                          strengths, p, n, s.draws, s.counters);
+}
+
 void many_body_exact(TreeDev &t, const NodeArrays &a, const double *strengths,
                      const ManyBodyParams &p, Rng *rng, ForceScratch &s, uint32_t *status,
                      bool host_draws, cudaStream_t st, const std::function<void(int)> &mark) {
@@ -419,13 +706,16 @@ void many_body_exact(TreeDev &t, const NodeArrays &a, const double *strengths,
   if (n == 0) return;
   unsigned cb, ct;
   climb_grid(cb, ct, t.cells_cap);
-  D3_LAUNCH(k_mb_accumulate, cb, ct, 0, st)(t.cells, t.parent, t.pnch, t.counter, t.perm, t.skip, a.x,
-                                     a.y, strengths, p.theta2, (MRec *)t.rec, t.info);
+  if (n <= ACC_BLOCK_NODES)
+    D3_LAUNCH(k_mb_accumulate_block, 1, 512, 0, st)(
+        t.cells, t.parent, t.pnch, t.counter, t.perm, t.skip, a.x, a.y, strengths, p.theta2,
+        (MRec *)t.rec, t.info);
+  else
+    D3_LAUNCH(k_mb_accumulate, cb, ct, 0, st)(t.cells, t.parent, t.pnch, t.counter, t.perm, t.skip, a.x,
+                                       a.y, strengths, p.theta2, (MRec *)t.rec, t.info);
   if (mark) mark(1);
   cudaMemsetAsync(s.counters, 0, 2 * sizeof(uint32_t), st);
-  D3_LAUNCH(k_mb_traverse, blocks_for(n, 128), 128, 0, st)((const MRec *)t.rec, t.perm, t.info, a.x, a.y,
-                                                    a.vx, a.vy, strengths, p, n, s.draws,
-                                                    s.counters);
+  launch_traverse(t, a, strengths, p, s, st);
   if (host_draws) {
     scan_u32(s.draws, s.offsets, n, s.scan_part, s.counters, st);
     return;
@@ -435,21 +725,24 @@ void many_body_exact(TreeDev &t, const NodeArrays &a, const double *strengths,
     int dev = 0, sms = 0, per = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_mb_draws, 256, 0);
+    cudaFuncSetAttribute(k_mb_draws, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MB_DRAWS_SMEM);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_mb_draws, 256, MB_DRAWS_SMEM);
     blocks = sms * (per >= 2 ? 2 : (per > 0 ? per : 1));
   }
   const MRec *rec = (const MRec *)t.rec;
+  const Cell *cells = t.cells;
   const uint32_t *perm = t.perm, *info = t.info;
   const double *x = a.x, *y = a.y;
   double *vx = a.vx, *vy = a.vy;
   ManyBodyParams pp = p;
-  uint32_t nn = n;
+  uint32_t nn = n, words = (uint32_t)(MB_DRAWS_SMEM / 32);  // of 8 warps
   const uint32_t *draws = s.draws;
   uint32_t *offsets = s.offsets, *counters = s.counters, *bsum = s.scan_part;
-  void *params[] = {&rec, &perm, &info, &x, &y, &vx, &vy, &strengths, &pp, &nn, &draws, &offsets,
-                    &counters, &bsum, &rng};
+  void *params[] = {&rec, &cells, &perm, &info, &x, &y, &vx, &vy, &strengths, &pp, &nn, &draws,
+                    &offsets, &counters, &bsum, &rng, &words};
   ++g_launches;
-  if (cudaLaunchCooperativeKernel((const void *)k_mb_draws, blocks, 256, params, 0, st) != cudaSuccess) {
+  if (cudaLaunchCooperativeKernel((const void *)k_mb_draws, blocks, 256, params, MB_DRAWS_SMEM, st) !=
+      cudaSuccess) {
     cudaGetLastError();
     scan_u32(s.draws, s.offsets, n, s.scan_part, s.counters, st);
     many_body_rerun(t, a, strengths, p, rng, s, st);
@@ -459,9 +752,10 @@ void many_body_exact(TreeDev &t, const NodeArrays &a, const double *strengths,
 void many_body_rerun(TreeDev &t, const NodeArrays &a, const double *strengths,
                      const ManyBodyParams &p, Rng *rng, ForceScratch &s, cudaStream_t st) {
   const uint32_t n = a.n;
-  D3_LAUNCH(k_mb_rerun, blocks_for(n, 128), 128, 0, st)((const MRec *)t.rec, t.perm, t.info, a.x, a.y, a.vx,
-                                                 a.vy, strengths, p, n, s.draws, s.offsets,
-                                                 s.counters, rng);
+  constexpr uint32_t words = 48 * 1024 / 16;  // of 4 warps, 47 KB in all
+  D3_LAUNCH(k_mb_rerun, blocks_for(n, 128), 128, (words - 256) * 16, st)(
+      (const MRec *)t.rec, t.cells, t.perm, t.info, a.x, a.y, a.vx, a.vy, strengths, p, n, s.draws,
+      s.offsets, s.counters, rng, words - 256);
   D3_LAUNCH(k_rng_advance, 1, 1, 0, st)(rng, s.counters);
 }
 

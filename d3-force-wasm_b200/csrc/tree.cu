@@ -31,6 +31,18 @@ __device__ inline uint32_t ldc(const uint32_t *p) { return __ldcg(p); }
 __device__ inline int8_t ldc(const int8_t *p) { return (int8_t)__ldcg((const signed char *)p); }
 __device__ inline uint8_t ldc(const uint8_t *p) { return (uint8_t)__ldcg((const unsigned char *)p); }
 
+// How a build step reads what other threads of its launch wrote: through L2
+// (the grid-wide build), or plainly (the one-block build, whose arrays are in
+// shared memory or this SM's L1).
+struct GridLoads {
+  template <typename T>
+  __device__ static T ld(const T *p) { return ldc(p); }
+};
+struct BlockLoads {
+  template <typename T>
+  __device__ static T ld(const T *p) { return *p; }
+};
+
 struct BoxPart {
   double v[4];   // min x, min y, max x, max y
   uint32_t i[4]; // index of the point that set each
@@ -64,9 +76,9 @@ __device__ inline void box_merge(double *v, uint32_t *ix, uint32_t &m, const dou
 // The block's merged box (every thread gets it): warp shuffles, then the
 // warps' results by warp 0 (the merge is commutative and associative).
 __device__ void block_box_reduce(double *v, uint32_t *ix, uint32_t &m) {
-  __shared__ double sv[BOX_THREADS / 32][4];
-  __shared__ uint32_t si[BOX_THREADS / 32][4];
-  __shared__ uint32_t sm[BOX_THREADS / 32];
+  __shared__ double sv[32][4];
+  __shared__ uint32_t si[32][4];
+  __shared__ uint32_t sm[32];
   const unsigned lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
   auto warp_reduce = [&]() {
     for (int o = 16; o > 0; o >>= 1) {
@@ -242,10 +254,11 @@ __device__ void keys_at(uint32_t i, const double *xs, const double *ys, const do
 // perm (sorted node indices, then the NaN nodes in index order), and per
 // sorted point the levels its key shares with the previous one: -1 for the
 // first, 64 for the same position (no boundary), else min(32, clz / 2).
+template <class M>
 __device__ void runs_at(uint32_t k, uint32_t m, const double *xs, const double *ys,
                         const uint64_t *keys, const uint32_t *sv, uint32_t *perm, int8_t *lcpx,
                         uint32_t *leaf_of) {
-  uint32_t p = ldc(&sv[k]) & 0x7fffffffu;
+  uint32_t p = M::ld(&sv[k]) & 0x7fffffffu;
   perm[k] = p;
   if (k >= m) {
     leaf_of[p] = NONE;
@@ -255,18 +268,19 @@ __device__ void runs_at(uint32_t k, uint32_t m, const double *xs, const double *
     lcpx[0] = -1;
     return;
   }
-  uint32_t q = ldc(&sv[k - 1]) & 0x7fffffffu;
+  uint32_t q = M::ld(&sv[k - 1]) & 0x7fffffffu;
   if (xs[p] == xs[q] && ys[p] == ys[q]) {
     lcpx[k] = 64;
     return;
   }
-  uint64_t d = ldc(&keys[k]) ^ ldc(&keys[k - 1]);
+  uint64_t d = M::ld(&keys[k]) ^ M::ld(&keys[k - 1]);
   int l = d ? (__clzll(d) >> 1) : 32;
   lcpx[k] = (int8_t)(l < 32 ? l : 32);
 }
 
+template <class M>
 __device__ inline bool is_start(const int8_t *lcpx, uint32_t k) {
-  int l = ldc(&lcpx[k]);
+  int l = M::ld(&lcpx[k]);
   return k == 0 || l < 32;  // -1 only at k = 0; 32 and 64 are not starts
 }
 
@@ -292,6 +306,7 @@ __device__ inline int quadrant(double x, double y, double xm, double ym) {
 // count mode (write = false) returns the number of cells below depth 32;
 // write mode emits them from c32 + 1 in preorder and sets their skip indices.
 // Frames live in frames[4 lo, 4 hi): at most one frame per point is pending.
+template <class M>
 __device__ uint32_t deep_group(bool write, uint32_t lo, uint32_t hi, uint32_t c32, uint64_t key,
                                const double *extent, const double *xs, const double *ys,
                                uint32_t *perm, uint32_t *perm_tmp, Frame *frames, Cell *cells,
@@ -327,14 +342,14 @@ __device__ uint32_t deep_group(bool write, uint32_t lo, uint32_t hi, uint32_t c3
       f.parent = me;
       // allSame by position (tree.zig:437-444); the depth guard of tree.zig:33
       bool same = true;
-      uint32_t p0 = ldc(&perm[f.lo]);
+      uint32_t p0 = M::ld(&perm[f.lo]);
       for (uint32_t k = f.lo + 1; k < f.hi; ++k) {
-        uint32_t p = ldc(&perm[k]);
+        uint32_t p = M::ld(&perm[k]);
         if (xs[p] != xs[p0] || ys[p] != ys[p0]) { same = false; break; }
       }
       if (f.depth >= MAX_DEPTH || same) {
         if (write)
-          for (uint32_t k = f.lo; k < f.hi; ++k) leaf_of[ldc(&perm[k])] = me;
+          for (uint32_t k = f.lo; k < f.hi; ++k) leaf_of[M::ld(&perm[k])] = me;
         continue;
       }
     }
@@ -343,17 +358,17 @@ __device__ uint32_t deep_group(bool write, uint32_t lo, uint32_t hi, uint32_t c3
     double xm = (f.x0 + f.x1) / 2, ym = (f.y0 + f.y1) / 2;
     uint32_t counts[4] = {0, 0, 0, 0}, off[4], b[5];
     for (uint32_t k = f.lo; k < f.hi; ++k) {
-      uint32_t p = ldc(&perm[k]);
+      uint32_t p = M::ld(&perm[k]);
       counts[quadrant(xs[p], ys[p], xm, ym)]++;
     }
     uint32_t sum = f.lo;
     for (int q = 0; q < 4; ++q) { off[q] = sum; b[q] = sum; sum += counts[q]; }
     b[4] = f.hi;
     for (uint32_t k = f.lo; k < f.hi; ++k) {
-      uint32_t p = ldc(&perm[k]);
+      uint32_t p = M::ld(&perm[k]);
       perm_tmp[off[quadrant(xs[p], ys[p], xm, ym)]++] = p;
     }
-    for (uint32_t k = f.lo; k < f.hi; ++k) perm[k] = ldc(&perm_tmp[k]);
+    for (uint32_t k = f.lo; k < f.hi; ++k) perm[k] = M::ld(&perm_tmp[k]);
     uint32_t nq = 0;
     for (int q = 0; q < 4; ++q) nq += b[q] != b[q + 1];
     for (int q = 3; q >= 0; --q) {
@@ -383,6 +398,7 @@ __device__ uint32_t deep_group(bool write, uint32_t lo, uint32_t hi, uint32_t c3
 
 // Cells starting at each sorted point: per start k, depths d0..leaf, plus the
 // cells below depth 32 of a deep group.
+template <class M>
 __device__ void count_at(uint32_t k, uint32_t m, const double *xs, const double *ys,
                          const uint64_t *keys, const int8_t *lcpx, const double *extent,
                          uint32_t *perm, uint32_t *perm_tmp, Frame *frames, uint32_t *cnt,
@@ -391,14 +407,14 @@ __device__ void count_at(uint32_t k, uint32_t m, const double *xs, const double 
     cnt[k] = 0;  // points with a NaN coordinate start no cell
     return;
   }
-  if (!is_start(lcpx, k)) {
+  if (!is_start<M>(lcpx, k)) {
     cnt[k] = 0;
     return;
   }
-  int d0 = k == 0 ? 0 : ldc(&lcpx[k]) + 1;
+  int d0 = k == 0 ? 0 : M::ld(&lcpx[k]) + 1;
   uint32_t j = k + 1;
-  while (j < m && ldc(&lcpx[j]) == 64) ++j;
-  int lr = j < m ? ldc(&lcpx[j]) : -1;
+  while (j < m && M::ld(&lcpx[j]) == 64) ++j;
+  int lr = j < m ? M::ld(&lcpx[j]) : -1;
   if (lr < 32) {
     int ld = lr + 1 > d0 ? lr + 1 : d0;
     leafd[k] = (uint8_t)ld;
@@ -407,10 +423,10 @@ __device__ void count_at(uint32_t k, uint32_t m, const double *xs, const double 
     return;
   }
   uint32_t g1 = j;
-  while (g1 < m && ldc(&lcpx[g1]) >= 32) ++g1;
+  while (g1 < m && M::ld(&lcpx[g1]) >= 32) ++g1;
   leafd[k] = 33;
   run_end[k] = g1;
-  uint32_t deep = deep_group(false, k, g1, 0, ldc(&keys[k]), extent, xs, ys, perm, perm_tmp, frames,
+  uint32_t deep = deep_group<M>(false, k, g1, 0, M::ld(&keys[k]), extent, xs, ys, perm, perm_tmp, frames,
                              nullptr, nullptr, nullptr, nullptr, 0, nullptr, nullptr);
   cnt[k] = (uint32_t)(32 - d0 + 1) + deep;
 }
@@ -478,40 +494,43 @@ constexpr int TB_TOP_D = 4;
 // depth-32 cell emits them after it).
 constexpr uint32_t OWN_TAG = 0x80000000u;
 
+template <class M>
 __device__ void own_at(uint32_t k, uint32_t m, const int8_t *lcpx, const uint32_t *base,
                        const uint32_t *cnt, const uint8_t *leafd, uint32_t *owner, uint32_t *info,
                        uint32_t *top) {
-  if (!is_start(lcpx, k)) return;
-  const int d0 = k == 0 ? 0 : ldc(&lcpx[k]) + 1;
-  const int ld = ldc(&leafd[k]);
+  if (!is_start<M>(lcpx, k)) return;
+  const int d0 = k == 0 ? 0 : M::ld(&lcpx[k]) + 1;
+  const int ld = M::ld(&leafd[k]);
   const int dlast = ld == 33 ? 32 : ld;
-  const uint32_t c0 = ldc(&base[k]);
+  const uint32_t c0 = M::ld(&base[k]);
   for (int d = d0; d <= dlast; ++d) owner[c0 + (d - d0)] = k | OWN_TAG;
-  for (int d = d0; d <= dlast && d < TB_TOP_D; ++d) top[atomicAdd(&info[8], 1u)] = c0 + (d - d0);
-  const uint32_t chain = (uint32_t)(dlast - d0 + 1), all = ldc(&cnt[k]);
+  if (top)
+    for (int d = d0; d <= dlast && d < TB_TOP_D; ++d) top[atomicAdd(&info[8], 1u)] = c0 + (d - d0);
+  const uint32_t chain = (uint32_t)(dlast - d0 + 1), all = M::ld(&cnt[k]);
   for (uint32_t c = c0 + chain; c < c0 + all; ++c) owner[c] = NONE;
   atomicMax(&info[2], (uint32_t)dlast);
 }
 
-template <bool WARP>
+// TOPS: the top cells are left to whole warps (WARP).
+template <class M, bool WARP, bool TOPS>
 __device__ void emit_cell(uint32_t c, uint32_t m, uint32_t total, const double *xs, const double *ys,
                           const uint64_t *keys, const int8_t *lcpx, const double *extent,
                           uint32_t *perm, uint32_t *perm_tmp, Frame *frames, const uint32_t *base,
                           const uint32_t *run_end, const uint8_t *leafd, Cell *cells, uint32_t *skip,
                           uint32_t *parent, uint8_t *pnch, uint32_t *counter, uint32_t *info,
                           uint32_t *leaf_of) {
-  const uint32_t own = ldc(&counter[c]);
+  const uint32_t own = M::ld(&counter[c]);
   if (own == NONE || !(own & OWN_TAG)) return;
   const uint32_t k = own & ~OWN_TAG;
-  const uint64_t key = ldc(&keys[k]);
-  const int d0 = k == 0 ? 0 : ldc(&lcpx[k]) + 1;
-  const int ld = ldc(&leafd[k]);
+  const uint64_t key = M::ld(&keys[k]);
+  const int d0 = k == 0 ? 0 : M::ld(&lcpx[k]) + 1;
+  const int ld = M::ld(&leafd[k]);
   const bool deep = ld == 33;
-  const uint32_t c0 = ldc(&base[k]);
+  const uint32_t c0 = M::ld(&base[k]);
   const int d = d0 + (int)(c - c0);
-  if (!WARP && d < TB_TOP_D) return;  // a top cell: emitted by a warp
+  if (!WARP && TOPS && d < TB_TOP_D) return;  // a top cell: emitted by a warp
   const bool writer = !WARP || (threadIdx.x & 31) == 0;
-  const uint32_t rend = ldc(&run_end[k]);
+  const uint32_t rend = M::ld(&run_end[k]);
   double x0, y0, x1, y1;
   path_bounds(extent, key, d, x0, y0, x1, y1);
   if (c == 0 && writer) {
@@ -536,7 +555,7 @@ __device__ void emit_cell(uint32_t c, uint32_t m, uint32_t total, const double *
   cell.count = end - k;
   cell.x0 = x0; cell.y0 = y0; cell.x1 = x1; cell.y1 = y1;
   cell.x = cell.y = cell.value = cell.r = 0;
-  const uint32_t sk = end < m ? ldc(&base[end]) : total;
+  const uint32_t sk = end < m ? M::ld(&base[end]) : total;
   if (writer) skip[c] = sk;
   if (!leaf && d < 32) {
     const uint64_t top = d == 0 ? 0 : (key >> (64 - 2 * d)) << (64 - 2 * d);
@@ -553,8 +572,8 @@ __device__ void emit_cell(uint32_t c, uint32_t m, uint32_t total, const double *
     for (int q = 0; q < 4; ++q) {
       if (b[q] == b[q + 1]) continue;
       uint32_t a = b[q];
-      int cd0 = a == k ? d0 : ldc(&lcpx[a]) + 1;
-      uint32_t ch = ldc(&base[a]) + (uint32_t)(d + 1 - cd0);
+      int cd0 = a == k ? d0 : M::ld(&lcpx[a]) + 1;
+      uint32_t ch = M::ld(&base[a]) + (uint32_t)(d + 1 - cd0);
       cell.child[q] = ch;
       parent[ch] = c;
       pnch[ch] = nch;
@@ -564,10 +583,10 @@ __device__ void emit_cell(uint32_t c, uint32_t m, uint32_t total, const double *
   cells[c] = cell;
   counter[c] = 0;
   if (leaf)
-    for (uint32_t p = k; p < rend; ++p) leaf_of[ldc(&perm[p])] = c;
+    for (uint32_t p = k; p < rend; ++p) leaf_of[M::ld(&perm[p])] = c;
   if (deep && d == 32) {
-    const uint32_t after = rend < m ? ldc(&base[rend]) : total;
-    const uint32_t emitted = deep_group(true, k, rend, c, key, extent, xs, ys, perm, perm_tmp,
+    const uint32_t after = rend < m ? M::ld(&base[rend]) : total;
+    const uint32_t emitted = deep_group<M>(true, k, rend, c, key, extent, xs, ys, perm, perm_tmp,
                                         frames, cells, parent, pnch, skip, after, &info[2], leaf_of);
     for (uint32_t q = c + 1; q <= c + emitted; ++q) counter[q] = 0;
   }
@@ -852,11 +871,11 @@ __global__ void __launch_bounds__(TB_THREADS) k_tree_build(TreeBuildArgs a) {
   tb_stamp(a, 3);
   // 4. perm and the shared levels; 5. cells per start
   for (uint32_t k = tid; k < n; k += nth)
-    runs_at(k, m, X, Y, fk, fv, a.perm, a.lcpx, a.leaf_of);
+    runs_at<GridLoads>(k, m, X, Y, fk, fv, a.perm, a.lcpx, a.leaf_of);
   g.sync();
   tb_stamp(a, 4);
   for (uint32_t k = tid; k < n; k += nth)
-    count_at(k, m, X, Y, fk, a.lcpx, se, a.perm, a.perm_tmp, a.frames, a.cnt, a.run_end,
+    count_at<GridLoads>(k, m, X, Y, fk, a.lcpx, se, a.perm, a.perm_tmp, a.frames, a.cnt, a.run_end,
              a.leafd);
   g.sync();
   tb_stamp(a, 5);
@@ -881,22 +900,187 @@ __global__ void __launch_bounds__(TB_THREADS) k_tree_build(TreeBuildArgs a) {
   }
   uint32_t *top = reinterpret_cast<uint32_t *>(a.parts);  // the box partials are done with
   for (uint32_t k = tid; k < m; k += nth)
-    own_at(k, m, a.lcpx, a.base, a.cnt, a.leafd, a.counter, a.info, top);
+    own_at<GridLoads>(k, m, a.lcpx, a.base, a.cnt, a.leafd, a.counter, a.info, top);
   g.sync();
   tb_stamp(a, 7);
   for (uint32_t c = tid; c < total; c += nth)
-    emit_cell<false>(c, m, total, X, Y, fk, a.lcpx, se, a.perm, a.perm_tmp, a.frames, a.base,
+    emit_cell<GridLoads, false, true>(c, m, total, X, Y, fk, a.lcpx, se, a.perm, a.perm_tmp, a.frames, a.base,
                      a.run_end, a.leafd, a.cells, a.skip, a.parent, a.pnch, a.counter, a.info,
                      a.leaf_of);
   {
     const uint32_t ntop = ldc(&a.info[8]), gw = tid >> 5, nw = nth >> 5;
     for (uint32_t k = gw; k < ntop; k += nw)
-      emit_cell<true>(ldc(&top[k]), m, total, X, Y, fk, a.lcpx, se, a.perm, a.perm_tmp,
+      emit_cell<GridLoads, true, true>(ldc(&top[k]), m, total, X, Y, fk, a.lcpx, se, a.perm, a.perm_tmp,
                       a.frames, a.base, a.run_end, a.leafd, a.cells, a.skip, a.parent, a.pnch,
                       a.counter, a.info, a.leaf_of);
   }
   __syncthreads();
   tb_stamp(a, 8);  // block 0's cells only
+}
+
+// ---- the build in one block --------------------------------------------------
+
+// Small trees: the same steps by one block, whose barriers cost 0.03 us where
+// the grid's cost 2 us each (some 16 of them: the grid build takes 60 us at any
+// size up to 5,000 points). Keys, values and the per-start arrays stay in
+// shared memory. The sort is a bitonic network over one 64-bit word a thread:
+// the key's top 53 bits and the index; the rare runs equal in those bits are
+// then ranked by the whole key and the index, which is the stable sort's order
+// (points with a NaN coordinate get the largest key and bit 31 in their value:
+// last, in index order). Event time, this / grid: 77 points 16 / 61 us, 384
+// 24 / 64 us, 1,000 37 / 67 us; the coordinates' 32 levels (4.6 us) and the
+// cells (14 us) are then bound by the one SM, which at 2,000 points takes as
+// long as the grid.
+constexpr uint32_t TREE_SMALL_MAX = 1024;
+constexpr uint32_t TREE_SMALL_CELLS = 4 * TREE_SMALL_MAX + 1024;
+constexpr unsigned TREE_SMALL_THREADS = 1024;
+
+struct TreeSmallShared {
+  uint64_t keys[TREE_SMALL_MAX], raw[TREE_SMALL_MAX], word[TREE_SMALL_MAX];
+  uint32_t sv[TREE_SMALL_MAX], rawv[TREE_SMALL_MAX];
+  uint32_t cnt[TREE_SMALL_MAX], base[TREE_SMALL_MAX], run_end[TREE_SMALL_MAX];
+  uint8_t leafd[TREE_SMALL_MAX];
+  int8_t lcpx[TREE_SMALL_MAX];
+  uint32_t owner[TREE_SMALL_CELLS];
+  uint32_t info[16];
+  double extent[4];
+};
+
+__global__ void __launch_bounds__(TREE_SMALL_THREADS) k_tree_small(TreeBuildArgs a) {
+  extern __shared__ __align__(16) unsigned char tree_smem[];
+  TreeSmallShared &S = *reinterpret_cast<TreeSmallShared *>(tree_smem);
+  __shared__ uint32_t sw[32];
+  const uint32_t t = threadIdx.x, nt = blockDim.x, n = a.n;
+  tb_stamp(a, 0);
+  // 1. the box
+  double v[4] = {INFINITY, INFINITY, -INFINITY, -INFINITY};
+  uint32_t ix[4] = {NONE, NONE, NONE, NONE};
+  uint32_t m = 0;
+  for (uint32_t i = t; i < n; i += nt) {
+    double x = a.xs[i], y = a.ys[i];
+    if (a.vxs) {
+      x += a.vxs[i];
+      y += a.vys[i];
+      a.pxs[i] = x;
+      a.pys[i] = y;
+    }
+    if (x != x || y != y) continue;
+    double pv[4] = {x, y, x, y};
+    uint32_t pi[4] = {i, i, i, i};
+    box_merge(v, ix, m, pv, pi, 1);
+  }
+  block_box_reduce(v, ix, m);
+  if (t < 16) S.info[t] = 0;
+  if (t == 0) {
+    double e[4] = {NAN, NAN, NAN, NAN};
+    if (!(v[0] > v[2] || v[1] > v[3])) {
+      cover(e, v[0], v[1]);
+      cover(e, v[2], v[3]);
+    }
+    for (int q = 0; q < 4; ++q) a.extent[q] = S.extent[q] = e[q];
+  }
+  __syncthreads();
+  tb_stamp(a, 1);
+  const double *X = a.vxs ? a.pxs : a.xs, *Y = a.vxs ? a.pys : a.ys;
+  // 2. keys (a thread per point from here on: n <= blockDim)
+  uint64_t w = ~0ull;
+  if (t < n) {
+    keys_at(t, X, Y, S.extent, S.raw, S.rawv);
+    if (S.rawv[t] >> 31) S.raw[t] = ~0ull;
+    w = (S.raw[t] & ~2047ull) | t;
+  }
+  tb_stamp(a, 2);
+  // 3. the sort; words at most 16 threads apart by shuffles
+  static_assert(TREE_SMALL_MAX <= 2048, "the index takes 11 bits of the word");
+  for (uint32_t k = 2; k / 2 < n; k <<= 1) {
+    for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+      uint64_t o;
+      if (j >= 32) {
+        __syncthreads();
+        S.word[t] = w;
+        __syncthreads();
+        o = S.word[t ^ j];
+      } else {
+        o = __shfl_xor_sync(0xffffffffu, w, j);
+      }
+      const bool lower = (t & j) == 0, up = (t & k) == 0;
+      if ((o < w) == (lower == up)) w = o;
+    }
+  }
+  __syncthreads();
+  S.word[t] = w;
+  __syncthreads();
+  if (t < n) {
+    // its run: the words with the same top bits (a word alone: itself)
+    const uint64_t top = w >> 11;
+    uint32_t lo = t, hi = t + 1;
+    while (lo > 0 && (S.word[lo - 1] >> 11) == top) --lo;
+    while (hi < n && (S.word[hi] >> 11) == top) ++hi;
+    const uint32_t i = (uint32_t)w & 2047u, v = S.rawv[i];
+    const uint64_t key = S.raw[i];
+    uint32_t at = lo;
+    if (hi - lo > 1)
+      for (uint32_t q = lo; q < hi; ++q) {
+        const uint32_t iq = (uint32_t)S.word[q] & 2047u;
+        const uint64_t kq = S.raw[iq];
+        at += kq < key || (kq == key && S.rawv[iq] < v);
+      }
+    S.keys[at] = key;
+    S.sv[at] = v;
+  }
+  __syncthreads();
+  tb_stamp(a, 3);
+  // 4. perm and the shared levels; 5. cells per start
+  for (uint32_t k = t; k < n; k += nt)
+    runs_at<BlockLoads>(k, m, X, Y, S.keys, S.sv, a.perm, S.lcpx, a.leaf_of);
+  __syncthreads();
+  tb_stamp(a, 4);
+  for (uint32_t k = t; k < n; k += nt)
+    count_at<BlockLoads>(k, m, X, Y, S.keys, S.lcpx, S.extent, a.perm, a.perm_tmp, a.frames, S.cnt,
+                         S.run_end, S.leafd);
+  __syncthreads();
+  tb_stamp(a, 5);
+  // 6. cell indices
+  uint32_t total = 0;
+  for (uint32_t b = 0; b < n; b += nt) {
+    uint32_t tot;
+    const uint32_t ex = block_excl(b + t < n ? S.cnt[b + t] : 0, sw, tot);
+    if (b + t < n) S.base[b + t] = total + ex;
+    total += tot;
+  }
+  __syncthreads();
+  tb_stamp(a, 6);
+  const bool fits = total <= a.cells_cap;
+  // (a simulation that was larger before has room for more cells than fit here)
+  uint32_t *const owner = total <= TREE_SMALL_CELLS ? S.owner : a.counter;
+  // 7. the cells
+  if (fits)
+    for (uint32_t k = t; k < m; k += nt)
+      own_at<BlockLoads>(k, m, S.lcpx, S.base, S.cnt, S.leafd, owner, S.info, nullptr);
+  __syncthreads();
+  tb_stamp(a, 7);
+  if (fits)
+    for (uint32_t c = t; c < total; c += nt)
+      emit_cell<BlockLoads, false, false>(c, m, total, X, Y, S.keys, S.lcpx, S.extent, a.perm, a.perm_tmp,
+                                          a.frames, S.base, S.run_end, S.leafd, a.cells, a.skip,
+                                          a.parent, a.pnch, owner, S.info, a.leaf_of);
+  if (fits && owner != a.counter)
+    for (uint32_t c = t; c < total; c += nt) a.counter[c] = 0;  // as after a grid build
+  __syncthreads();
+  if (t == 0) {
+    // as the grid build leaves them (info[6]: the count the tree needed)
+    a.info[0] = m;
+    a.info[1] = fits ? total : 0;
+    a.info[2] = S.info[2];
+    a.info[3] = m ? 0 : NONE;
+    a.info[4] = 0;
+    a.info[5] = fits ? 0 : 1;
+    a.info[6] = total;
+    a.info[7] = 0;
+    a.info[8] = 0;
+    if (!fits) atomicOr(a.status, ST_DEEP_STACK);
+  }
+  tb_stamp(a, 8);
 }
 
 int tree_reserve(TreeDev &t, uint32_t n) {
@@ -1002,6 +1186,17 @@ void tree_build_shifted(TreeDev &t, const double *xs, const double *ys, const do
   a.bsum = a.dtot + 256;
   a.extent = t.extent; a.info = t.info; a.status = status;
   a.stamps = t.stamps;
+  if (n > 0 && n <= TREE_SMALL_MAX) {
+    static const bool attr =
+        cudaFuncSetAttribute(k_tree_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sizeof(TreeSmallShared)) == cudaSuccess;
+    if (attr) {
+      unsigned threads = 64;
+      while (threads < n) threads <<= 1;
+      D3_LAUNCH(k_tree_small, 1, threads, sizeof(TreeSmallShared), st)(a);
+      return;
+    }
+  }
   void *params[] = {&a};
   ++g_launches;
   if (cudaLaunchCooperativeKernel((const void *)k_tree_build, g_tree_blocks, TB_THREADS, params, 0,
