@@ -6,19 +6,20 @@
 // weights to bf16, biases stay FP32), weights stored [out][in]:
 //   W1 [64][12] | b1 [64] | W2 [64][64] | b2 [64] | W3 [2][64] | b3 [2]
 //
-// Training kernel (CUDA cores): a CTA of 128 threads takes tiles of 128
-// samples, a thread per sample for the forward pass and the input gradients
-// (activations in shared memory, unit-major with a padded stride so the
-// threads' reads fall in distinct banks), then the weight gradients as
-// sums over the tile's samples, a thread per weight row; a CTA keeps its
-// gradient sums in shared memory over all its tiles and adds them to the
-// global sums once. Loss: mean over samples of sum_o (y_o - t_o)^2.
+// Training (CUDA cores, FP32): a CTA of 256 threads takes tiles of 64 samples;
+// the three 64 x 64 x 64 products of a tile (layer 2 forward, its input
+// gradient, its weight gradient) and layer 1 are register tiles of 4 x 4 over
+// operands in shared memory, both k-major; gelu' and the gradient sums stay
+// in registers over all of a CTA's tiles. The CTAs' sums are added in CTA
+// order by the kernel that applies them (the result does not depend on
+// timing). Loss: mean over samples of sum_o (y_o - t_o)^2.
 // Inference (tcgen05, mlp_infer_tc): a CTA per 128 samples, the three layers
 // as MMAs of M = 128 with the activations staged as bf16 in shared memory,
 // GELU and the biases applied between them from the TMEM accumulators.
 #include <cuda_bf16.h>
 
 #include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <vector>
@@ -30,8 +31,7 @@
 namespace d3 {
 namespace {
 
-constexpr int TT = 128;       // samples per tile
-constexpr int SP = TT + 1;    // padded stride of unit-major activation rows
+constexpr int TT = 128;       // samples per inference tile
 
 __device__ __forceinline__ float bf(float w) { return __bfloat162float(__float2bfloat16(w)); }
 __device__ __forceinline__ float gelu(float z) { return 0.5f * z * (1.f + erff(z * 0.70710678f)); }
@@ -39,140 +39,256 @@ __device__ __forceinline__ float gelu_d(float z) {
   return 0.5f * (1.f + erff(z * 0.70710678f)) + z * 0.39894228f * expf(-0.5f * z * z);
 }
 
-struct TrainSmem {
-  float w1[MLP_H][MLP_IN], w2[MLP_H][MLP_H], w3[MLP_OUT][MLP_H];  // bf16-rounded
-  float b1[MLP_H], b2[MLP_H], b3[MLP_OUT];
-  float x[MLP_IN][SP];
-  float a1[MLP_H][SP], g1[MLP_H][SP];  // activation, gelu'(z); g reused for dz
-  float a2[MLP_H][SP], g2[MLP_H][SP];
-  float dy[MLP_OUT][SP];
-  float gsum[MLP_PARAMS];  // this CTA's gradient sums
-  float loss;
-};
+constexpr int GT = 64;            // samples per training tile
+constexpr int GTHREADS = 256;     // 16 x 16 threads, 4 samples x 4 units each
+constexpr int PART = (MLP_PARAMS + 1 + 31) / 32 * 32;  // a CTA's sums: the gradient, then the loss
+static_assert(MLP_H == GT, "the tiles are square");
 
-// Gradient of the loss over samples [0, n) (sum over samples of the per-
-// sample loss, divided by `norm`), added into grad (zeroed by the caller);
-// loss_sum gets the summed loss.
-__global__ void __launch_bounds__(TT) k_mlp_grad(const float *x, const float *y, uint32_t n,
-                                                 const float *params, float norm, float *grad,
-                                                 float *loss_sum) {
-  extern __shared__ float mlp_smem[];
+// Rows are read 16 bytes at a time; GS floats a row (17 x 16 bytes), so the
+// rows that a warp's lanes read or write side by side start in other banks.
+constexpr int GS = 68;
+struct TrainSmem {
+  float w1t[MLP_IN][GS];              // bf16-rounded, [in][out]
+  float w2[MLP_H][GS], w2t[MLP_H][GS];  // [out][in] and [in][out]
+  float w3[MLP_OUT][GS];
+  float a1[GT][GS], a2[GT][GS];       // a row per sample
+  float d1[GT][GS], d2[GT][GS];       // dz1, dz2
+  float x[GT][MLP_IN];
+  float b1[MLP_H], b2[MLP_H];
+  float dy[MLP_OUT][GT];
+  float b3[MLP_OUT], loss[GTHREADS / 32];
+};
+static_assert(offsetof(TrainSmem, w2) % 16 == 0 && offsetof(TrainSmem, w2t) % 16 == 0 &&
+                  offsetof(TrainSmem, w3) % 16 == 0 && offsetof(TrainSmem, a1) % 16 == 0 &&
+                  offsetof(TrainSmem, a2) % 16 == 0 && offsetof(TrainSmem, d1) % 16 == 0 &&
+                  offsetof(TrainSmem, d2) % 16 == 0 && offsetof(TrainSmem, x) % 16 == 0 &&
+                  MLP_IN % 4 == 0 && GS % 4 == 0,
+              "16-byte rows");
+
+// c[i][j] += sum_k A[i0 + i][k] B[k][j0 + j]; A's rows `stride` floats apart.
+template <int K>
+__device__ __forceinline__ void tile_product(const float *A, int stride, const float (*B)[GS], int i0,
+                                             int j0, float c[4][4]) {
+#pragma unroll 4
+  for (int k = 0; k < K; k += 4) {
+    float a[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float4 v = *reinterpret_cast<const float4 *>(A + (i0 + i) * stride + k);
+      a[i][0] = v.x; a[i][1] = v.y; a[i][2] = v.z; a[i][3] = v.w;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float4 b = *reinterpret_cast<const float4 *>(&B[k + q][j0]);
+      const float bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) c[i][j] += a[i][q] * bv[j];
+    }
+  }
+}
+
+// c[i][j] += sum_s A[s][i0 + i] B[s][j0 + j]
+__device__ __forceinline__ void tile_outer(const float (*A)[GS], const float (*B)[GS], int i0, int j0,
+                                           float c[4][4]) {
+#pragma unroll 8
+  for (int s = 0; s < GT; ++s) {
+    const float4 a = *reinterpret_cast<const float4 *>(&A[s][i0]);
+    const float4 b = *reinterpret_cast<const float4 *>(&B[s][j0]);
+    const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) c[i][j] += av[i] * bv[j];
+  }
+}
+
+__device__ __forceinline__ void put_tile(const float v[4][4], int i0, int j0, float (*R)[GS]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    *reinterpret_cast<float4 *>(&R[i0 + i][j0]) = make_float4(v[i][0], v[i][1], v[i][2], v[i][3]);
+}
+
+// Sums over samples [0, n) of the per-sample loss and its gradient divided by
+// `norm`: each CTA's own into part[blockIdx][PART].
+//
+// A step of 8,192 samples (128 tiles, an SM each) takes 26 us with its Adam
+// kernel (127 us before: 64 CTAs of a thread per sample, atomic gradient
+// sums, a host synchronisation per step); it is bound by the tile's chain of
+// products (3 x 1,024 FMA a thread) and the 32 erf and exp a thread takes.
+__global__ void __launch_bounds__(GTHREADS) k_mlp_grad(const float *x, const float *y, uint32_t n,
+                                                       const float *params, float norm, float *part) {
+  extern __shared__ __align__(16) float mlp_smem[];
   TrainSmem &S = *reinterpret_cast<TrainSmem *>(mlp_smem);
-  const int t = threadIdx.x;
-  for (int k = t; k < MLP_H * MLP_IN; k += TT) (&S.w1[0][0])[k] = bf(params[P_W1 + k]);
-  for (int k = t; k < MLP_H * MLP_H; k += TT) (&S.w2[0][0])[k] = bf(params[P_W2 + k]);
-  for (int k = t; k < MLP_OUT * MLP_H; k += TT) (&S.w3[0][0])[k] = bf(params[P_W3 + k]);
-  for (int k = t; k < MLP_H; k += TT) {
-    S.b1[k] = params[P_B1 + k];
-    S.b2[k] = params[P_B2 + k];
+  const int t = threadIdx.x, i0 = (t >> 4) * 4, j0 = (t & 15) * 4;
+  for (int e = t; e < MLP_H * MLP_IN; e += GTHREADS) S.w1t[e % MLP_IN][e / MLP_IN] = bf(params[P_W1 + e]);
+  for (int e = t; e < MLP_H * MLP_H; e += GTHREADS) {
+    const float w = bf(params[P_W2 + e]);
+    S.w2[e / MLP_H][e % MLP_H] = w;
+    S.w2t[e % MLP_H][e / MLP_H] = w;
+  }
+  for (int e = t; e < MLP_OUT * MLP_H; e += GTHREADS) S.w3[e / MLP_H][e % MLP_H] = bf(params[P_W3 + e]);
+  if (t < MLP_H) {
+    S.b1[t] = params[P_B1 + t];
+    S.b2[t] = params[P_B2 + t];
   }
   if (t < MLP_OUT) S.b3[t] = params[P_B3 + t];
-  for (int k = t; k < MLP_PARAMS; k += TT) S.gsum[k] = 0;
-  if (t == 0) S.loss = 0;
-  __syncthreads();
   const float inv = 1.f / norm;
-  float my_loss = 0;
-  for (uint32_t base = blockIdx.x * TT; base < n; base += gridDim.x * TT) {
-    const uint32_t i = base + t;
-    const bool act = i < n;
-    // forward, a thread per sample
-    float xi[MLP_IN];
-#pragma unroll
-    for (int k = 0; k < MLP_IN; ++k) {
-      xi[k] = act ? x[(size_t)i * MLP_IN + k] : 0.f;
-      S.x[k][t] = __bfloat162float(__float2bfloat16(xi[k]));
-    }
-    for (int j = 0; j < MLP_H; ++j) {
-      float z = S.b1[j];
-#pragma unroll
-      for (int k = 0; k < MLP_IN; ++k) z += S.w1[j][k] * S.x[k][t];
-      S.a1[j][t] = bf(gelu(z));
-      S.g1[j][t] = gelu_d(z);
-    }
-    for (int j = 0; j < MLP_H; ++j) {
-      float z = S.b2[j];
-      for (int k = 0; k < MLP_H; ++k) z += S.w2[j][k] * S.a1[k][t];
-      S.a2[j][t] = bf(gelu(z));
-      S.g2[j][t] = gelu_d(z);
-    }
-    for (int o = 0; o < MLP_OUT; ++o) {
-      float z = S.b3[o];
-      for (int k = 0; k < MLP_H; ++k) z += S.w3[o][k] * S.a2[k][t];
-      const float d = act ? z - y[(size_t)i * MLP_OUT + o] : 0.f;
-      my_loss += d * d;
-      S.dy[o][t] = 2.f * d * inv;
-    }
-    // input gradients: dz2 = (W3^T dy) gelu'(z2), dz1 = (W2^T dz2) gelu'(z1)
-    for (int k = 0; k < MLP_H; ++k) {
-      float s = 0;
-      for (int o = 0; o < MLP_OUT; ++o) s += S.w3[o][k] * S.dy[o][t];
-      S.g2[k][t] *= s;  // g2 now holds dz2
-    }
-    for (int k = 0; k < MLP_H; ++k) {
-      float s = 0;
-      for (int j = 0; j < MLP_H; ++j) s += S.w2[j][k] * S.g2[j][t];
-      S.g1[k][t] *= s;  // g1 now holds dz1
+  // gradient sums: W2 tile (rows i0.., columns j0..), W1 (row gj, columns gk ..
+  // gk + 2), W3 and the biases by the threads that take their columns
+  const int gj = t & 63, gk = (t >> 6) * 3;
+  float gw2[4][4] = {}, gw1[3] = {}, gw3 = 0, gb1 = 0, gb2 = 0, gb3 = 0, my_loss = 0;
+  for (uint32_t base = blockIdx.x * GT; base < n; base += gridDim.x * GT) {
+    __syncthreads();  // the weights; the last tile's reads
+    for (int e = t; e < GT * MLP_IN; e += GTHREADS) {
+      const uint32_t i = base + e / MLP_IN;
+      S.x[e / MLP_IN][e % MLP_IN] = i < n ? bf(x[(size_t)base * MLP_IN + e]) : 0.f;
     }
     __syncthreads();
-    // weight gradients: sums over the tile's samples, a thread per row
-    if (t < MLP_H) {
-      const int j = t;
-      float gb1 = 0, gw1[MLP_IN] = {};
-      for (int s = 0; s < TT; ++s) {
-        const float d = S.g1[j][s];
-        gb1 += d;
+    // layer 1
+    float g1[4][4], g2[4][4], v[4][4];
 #pragma unroll
-        for (int k = 0; k < MLP_IN; ++k) gw1[k] += d * S.x[k][s];
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) v[i][j] = S.b1[j0 + j];
+    tile_product<MLP_IN>(&S.x[0][0], MLP_IN, S.w1t, i0, j0, v);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        g1[i][j] = gelu_d(v[i][j]);
+        v[i][j] = bf(gelu(v[i][j]));
       }
-      S.gsum[P_B1 + j] += gb1;
+    put_tile(v, i0, j0, S.a1);
+    __syncthreads();
+    // layer 2
 #pragma unroll
-      for (int k = 0; k < MLP_IN; ++k) S.gsum[P_W1 + j * MLP_IN + k] += gw1[k];
-    } else {
-      const int j = t - MLP_H;
-      float gb2 = 0;
-      for (int s = 0; s < TT; ++s) gb2 += S.g2[j][s];
-      S.gsum[P_B2 + j] += gb2;
-      for (int k0 = 0; k0 < MLP_H; k0 += 16) {
-        float acc[16] = {};
-        for (int s = 0; s < TT; ++s) {
-          const float d = S.g2[j][s];
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
-          for (int k = 0; k < 16; ++k) acc[k] += d * S.a1[k0 + k][s];
-        }
+      for (int j = 0; j < 4; ++j) v[i][j] = S.b2[j0 + j];
+    tile_product<MLP_H>(&S.a1[0][0], GS, S.w2t, i0, j0, v);
 #pragma unroll
-        for (int k = 0; k < 16; ++k) S.gsum[P_W2 + j * MLP_H + k0 + k] += acc[k];
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        g2[i][j] = gelu_d(v[i][j]);
+        v[i][j] = bf(gelu(v[i][j]));
       }
+    put_tile(v, i0, j0, S.a2);
+    __syncthreads();
+    // the output layer, a thread per sample and output
+    if (t < MLP_OUT * GT) {
+      const int smp = t & 63, o = t >> 6;
+      const uint32_t i = base + smp;
+      float z = S.b3[o];
+#pragma unroll 4
+      for (int k = 0; k < MLP_H; k += 4) {
+        const float4 a = *reinterpret_cast<const float4 *>(&S.a2[smp][k]);
+        const float4 w = *reinterpret_cast<const float4 *>(&S.w3[o][k]);
+        z += w.x * a.x;
+        z += w.y * a.y;
+        z += w.z * a.z;
+        z += w.w * a.w;
+      }
+      const float d = i < n ? z - y[(size_t)i * MLP_OUT + o] : 0.f;
+      my_loss += d * d;
+      S.dy[o][smp] = 2.f * d * inv;
+    }
+    __syncthreads();
+    // dz2 = (W3^T dy) gelu'(z2)
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        v[i][j] = g2[i][j] * fmaf(S.w3[1][j0 + j], S.dy[1][i0 + i], S.w3[0][j0 + j] * S.dy[0][i0 + i]);
+    put_tile(v, i0, j0, S.d2);
+    __syncthreads();
+    // dz1 = (W2^T dz2) gelu'(z1); W2's gradient over the tile's samples
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) v[i][j] = 0;
+    tile_product<MLP_H>(&S.d2[0][0], GS, S.w2, i0, j0, v);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) v[i][j] *= g1[i][j];
+    put_tile(v, i0, j0, S.d1);
+    tile_outer(S.d2, S.a1, i0, j0, gw2);
+    __syncthreads();
+    // the other gradients, a column of samples each
+    for (int s = 0; s < GT; ++s) {
+      const float d = S.d1[s][gj];
+      if (gk == 0) gb1 += d;
+#pragma unroll
+      for (int q = 0; q < 3; ++q) gw1[q] += d * S.x[s][gk + q];
     }
     if (t < MLP_OUT * MLP_H) {
       const int o = t / MLP_H, k = t % MLP_H;
-      float g = 0;
-      for (int s = 0; s < TT; ++s) g += S.dy[o][s] * S.a2[k][s];
-      S.gsum[P_W3 + o * MLP_H + k] += g;
+      for (int s = 0; s < GT; ++s) gw3 += S.dy[o][s] * S.a2[s][k];
+    } else if (t < MLP_OUT * MLP_H + MLP_H) {
+      for (int s = 0; s < GT; ++s) gb2 += S.d2[s][t - MLP_OUT * MLP_H];
+    } else if (t < MLP_OUT * MLP_H + MLP_H + MLP_OUT) {
+      for (int s = 0; s < GT; ++s) gb3 += S.dy[t - MLP_OUT * MLP_H - MLP_H][s];
     }
-    if (t < MLP_OUT) {
-      float g = 0;
-      for (int s = 0; s < TT; ++s) g += S.dy[t][s];
-      S.gsum[P_B3 + t] += g;
-    }
-    __syncthreads();
   }
-  atomicAdd(&S.loss, my_loss);
+  float *g = part + (size_t)blockIdx.x * PART;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) g[P_W2 + (i0 + i) * MLP_H + j0 + j] = gw2[i][j];
+#pragma unroll
+  for (int q = 0; q < 3; ++q) g[P_W1 + gj * MLP_IN + gk + q] = gw1[q];
+  if (gk == 0) g[P_B1 + gj] = gb1;
+  if (t < MLP_OUT * MLP_H) g[P_W3 + t] = gw3;
+  else if (t < MLP_OUT * MLP_H + MLP_H) g[P_B2 + t - MLP_OUT * MLP_H] = gb2;
+  else if (t < MLP_OUT * MLP_H + MLP_H + MLP_OUT) g[P_B3 + t - MLP_OUT * MLP_H - MLP_H] = gb3;
+  for (int o = 16; o > 0; o >>= 1) my_loss += __shfl_xor_sync(0xffffffffu, my_loss, o);
+  if ((t & 31) == 0) S.loss[t >> 5] = my_loss;
   __syncthreads();
-  for (int k = t; k < MLP_PARAMS; k += TT) atomicAdd(&grad[k], S.gsum[k]);
-  if (t == 0) atomicAdd(loss_sum, S.loss);
+  if (t == 0) {
+    float l = 0;
+    for (int w = 0; w < GTHREADS / 32; ++w) l += S.loss[w];
+    g[MLP_PARAMS] = l;
+  }
 }
 
-// Adam (Kingma & Ba 2015) on the FP32 master parameters.
-__global__ void k_mlp_adam(float *params, float *m, float *v, const float *grad, float lr,
-                           float b1, float b2, float eps, float c1, float c2) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= MLP_PARAMS) return;
-  const float g = grad[k];
-  const float mk = b1 * m[k] + (1 - b1) * g;
-  const float vk = b2 * v[k] + (1 - b2) * g * g;
-  m[k] = mk;
-  v[k] = vk;
-  params[k] -= lr * (mk / c1) / (sqrtf(vk / c2) + eps);
+struct AdamArgs {
+  float *params, *m, *v;
+  float lr, b1, b2, eps, c1, c2;
+};
+
+// The sum over the CTAs' parts, in CTA order within each of the block's 8
+// warps (a warp every eighth part, a lane per parameter): into grad and *loss,
+// or (ADAM) straight into an Adam step (Kingma & Ba 2015) on the FP32 master
+// parameters, *loss then the mean over nb samples.
+template <bool ADAM>
+__global__ void __launch_bounds__(256) k_mlp_apply(const float *part, int parts, float *grad, float *loss,
+                                                   AdamArgs a, float nb) {
+  __shared__ float sum[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, k = blockIdx.x * 32 + lane;
+  float g = 0;
+#pragma unroll 4
+  for (int c = warp; c < parts; c += 8) g += part[(size_t)c * PART + k];
+  sum[warp][lane] = g;
+  __syncthreads();
+  if (warp != 0 || k > MLP_PARAMS) return;
+  g = 0;
+  for (int w = 0; w < 8; ++w) g += sum[w][lane];
+  if (k == MLP_PARAMS) {
+    if (loss) *loss = ADAM ? __fdiv_rn(g, nb) : g;
+    return;
+  }
+  if (!ADAM) {
+    grad[k] = g;
+    return;
+  }
+  const float mk = a.b1 * a.m[k] + (1 - a.b1) * g;
+  const float vk = a.b2 * a.v[k] + (1 - a.b2) * g * g;
+  a.m[k] = mk;
+  a.v[k] = vk;
+  a.params[k] -= a.lr * (mk / a.c1) / (sqrtf(vk / a.c2) + a.eps);
 }
 
 // The forward pass on CUDA cores (a thread per sample): the check of the
@@ -344,40 +460,48 @@ using namespace d3;
 
 namespace {
 
-int grad_launch(const float *x, const float *y, uint32_t n, const float *params, float *grad,
-                float *loss, cudaStream_t st) {
-  static int blocks = 0;
-  if (!blocks) {
+// CTAs of a gradient launch over n samples: a tile each, at most one an SM.
+int grad_ctas(uint32_t n) {
+  static int sms = 0;
+  if (!sms) {
+    int dev = 0, count = 0;
     cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)sizeof(TrainSmem));
-    int dev = 0, sms = 0;
     cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    blocks = sms;
+    cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev);
+    sms = count;
   }
-  unsigned b = blocks_for(n, TT);
-  if (b > (unsigned)blocks) b = blocks;
-  if (cudaMemsetAsync(grad, 0, MLP_PARAMS * 4, st) != cudaSuccess ||
-      cudaMemsetAsync(loss, 0, 4, st) != cudaSuccess)
-    return -1;
-  D3_LAUNCH(k_mlp_grad, b, TT, sizeof(TrainSmem), st)(x, y, n, params, (float)n, grad, loss);
+  const unsigned b = blocks_for(n, GT);
+  return b < (unsigned)sms ? (int)b : sms;
+}
+
+int grad_launch(const float *x, const float *y, uint32_t n, const float *params, float *part, int ctas,
+                cudaStream_t st) {
+  D3_LAUNCH(k_mlp_grad, ctas, GTHREADS, sizeof(TrainSmem), st)(x, y, n, params, (float)n, part);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
+
+constexpr unsigned APPLY_BLOCKS = PART / 32;
 
 }  // namespace
 
 extern "C" int32_t d3_mlp_grad(const float *x, const float *y, uint32_t n, const float *params,
                                float *grad, float *loss) {
   if (!x || !y || !params || !grad || !loss || n == 0) return D3_BAD_ARGUMENT;
+  const int ctas = grad_ctas(n);
   float *d = nullptr;
-  if (cudaMalloc(&d, (2 * MLP_PARAMS + 1) * 4) != cudaSuccess) return D3_OUT_OF_MEMORY;
-  float *dp = d, *dg = d + MLP_PARAMS, *dl = d + 2 * MLP_PARAMS;
+  if (cudaMalloc(&d, (2 * MLP_PARAMS + 1 + (size_t)ctas * PART) * 4) != cudaSuccess) return D3_OUT_OF_MEMORY;
+  float *dp = d, *dg = d + MLP_PARAMS, *dl = d + 2 * MLP_PARAMS, *part = dl + 1;
   int32_t rc = D3_OK;
   if (cudaMemcpy(dp, params, MLP_PARAMS * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
-      grad_launch(x, y, n, dp, dg, dl, 0) ||
-      cudaMemcpy(grad, dg, MLP_PARAMS * 4, cudaMemcpyDeviceToHost) != cudaSuccess ||
-      cudaMemcpy(loss, dl, 4, cudaMemcpyDeviceToHost) != cudaSuccess)
+      grad_launch(x, y, n, dp, part, ctas, 0))
     rc = D3_WORKER_FAILED;
+  if (rc == D3_OK) {
+    D3_LAUNCH(k_mlp_apply<false>, APPLY_BLOCKS, 256, 0, 0)(part, ctas, dg, dl, AdamArgs{}, 1.f);
+    if (cudaMemcpy(grad, dg, MLP_PARAMS * 4, cudaMemcpyDeviceToHost) != cudaSuccess ||
+        cudaMemcpy(loss, dl, 4, cudaMemcpyDeviceToHost) != cudaSuccess)
+      rc = D3_WORKER_FAILED;
+  }
   *loss /= (float)n;
   cudaFree(d);
   return rc;
@@ -386,39 +510,38 @@ extern "C" int32_t d3_mlp_grad(const float *x, const float *y, uint32_t n, const
 extern "C" int32_t d3_mlp_train(const float *x, const float *y, uint32_t n, uint32_t batch,
                                 uint32_t steps, float lr, float *params, float *losses) {
   if (!x || !y || !params || n == 0 || batch == 0) return D3_BAD_ARGUMENT;
+  const uint32_t nb = batch < n ? batch : n;
+  const int ctas = grad_ctas(nb);
   float *d = nullptr;
-  if (cudaMalloc(&d, (4 * MLP_PARAMS + 1) * 4) != cudaSuccess) return D3_OUT_OF_MEMORY;
-  float *dp = d, *dm = d + MLP_PARAMS, *dv = d + 2 * MLP_PARAMS, *dg = d + 3 * MLP_PARAMS,
-        *dl = d + 4 * MLP_PARAMS;
+  if (cudaMalloc(&d, (3 * MLP_PARAMS + (size_t)ctas * PART + steps) * 4) != cudaSuccess)
+    return D3_OUT_OF_MEMORY;
+  float *dp = d, *dm = d + MLP_PARAMS, *dv = d + 2 * MLP_PARAMS, *part = d + 3 * MLP_PARAMS,
+        *dl = part + (size_t)ctas * PART;
   int32_t rc = D3_OK;
   cudaStream_t st = 0;
   if (cudaMemcpy(dp, params, MLP_PARAMS * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaMemset(dm, 0, 2 * MLP_PARAMS * 4) != cudaSuccess)
     rc = D3_WORKER_FAILED;
-  const float b1 = 0.9f, b2 = 0.999f;
+  AdamArgs a{dp, dm, dv, lr, 0.9f, 0.999f, 1e-8f, 0, 0};
   float c1 = 1, c2 = 1;
   uint32_t off = 0;
   for (uint32_t s = 0; s < steps && rc == D3_OK; ++s) {
-    const uint32_t nb = batch < n ? batch : n;
     if (off + nb > n) off = 0;  // batches walk the (pre-shuffled) samples in order
-    if (grad_launch(x + (size_t)off * MLP_IN, y + (size_t)off * MLP_OUT, nb, dp, dg, dl, st)) {
+    if (grad_launch(x + (size_t)off * MLP_IN, y + (size_t)off * MLP_OUT, nb, dp, part, ctas, st)) {
       rc = D3_WORKER_FAILED;
       break;
     }
     off += nb;
-    c1 *= b1;
-    c2 *= b2;
-    D3_LAUNCH(k_mlp_adam, blocks_for(MLP_PARAMS, 256), 256, 0, st)(dp, dm, dv, dg, lr, b1, b2,
-                                                                    1e-8f, 1 - c1, 1 - c2);
-    if (losses) {
-      float l = 0;
-      if (cudaMemcpyAsync(&l, dl, 4, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-          cudaStreamSynchronize(st) != cudaSuccess)
-        rc = D3_WORKER_FAILED;
-      losses[s] = l / (float)nb;
-    }
+    c1 *= a.b1;
+    c2 *= a.b2;
+    a.c1 = 1 - c1;
+    a.c2 = 1 - c2;
+    D3_LAUNCH(k_mlp_apply<true>, APPLY_BLOCKS, 256, 0, st)(part, ctas, nullptr, dl + s, a, (float)nb);
   }
-  if (rc == D3_OK && (cudaMemcpy(params, dp, MLP_PARAMS * 4, cudaMemcpyDeviceToHost) != cudaSuccess))
+  // the step losses come back once, with the parameters
+  if (rc == D3_OK && (cudaMemcpy(params, dp, MLP_PARAMS * 4, cudaMemcpyDeviceToHost) != cudaSuccess ||
+                      (losses && steps &&
+                       cudaMemcpy(losses, dl, steps * 4ull, cudaMemcpyDeviceToHost) != cudaSuccess)))
     rc = D3_WORKER_FAILED;
   cudaFree(d);
   return rc;
