@@ -70,12 +70,22 @@ constexpr uint32_t TC_CLASS_MAX = 192;
 constexpr uint32_t TC_THREADS = 256;
 constexpr uint32_t TC_WARPS = TC_THREADS / 32;
 constexpr uint32_t TC_TILE = 128;     // target cells per M2L tile (the MMA's M)
-constexpr uint32_t TC_STACK = 64;
 constexpr uint32_t TC_NONE = 0xFFFFFFFFu;
 constexpr uint32_t TC_NEAR_FLAG = 0x8000u;
 // info words
-enum : uint32_t { TI_POOL_P2P = 0, TI_POOL_W, TI_POOL_X, TI_POOL_C, TI_OVF, TI_GROUP = 8,
+enum : uint32_t { TI_POOL_P2P = 0, TI_POOL_W, TI_POOL_X, TI_POOL_C, TI_OVF, TI_SEG_P2P, TI_SEG_W,
+                  TI_GROUP = 8,
                   TI_LEAVES = 12, TI_ERR = 16, TI_WORDS = 32 };
+// A leaf's P2P and W lists are taken in segments: the leaf's own
+// warp (near field) or threads (far field) take the first, further warps the
+// others, each into a partial sum of its own, added in segment order. Beside a
+// dense cluster a list has thousands of entries where most have 13, and one
+// warp's list was the pass's time. Leaves of more than SEG_POINTS points (the
+// deepest level's clumps) are not split.
+constexpr uint32_t SEG_P2P = 32, SEG_W = 8, SEG_POINTS = 64;
+__host__ __device__ inline uint32_t more_segments(uint32_t entries, uint32_t points, uint32_t seg) {
+  return entries > seg && points <= SEG_POINTS ? (entries - 1) / seg : 0;
+}
 // The learned correction's output unit: the network predicts
 // (L'_0 at order 12 - L'_0 at order 4) / sc * LEARN_TARGET_SCALE.
 constexpr float LEARN_TARGET_SCALE = 1000.f;
@@ -141,6 +151,13 @@ struct TcDev {
   double2 *chk_part = nullptr;               // the check's partial direct sums
   uint32_t chk_cap = 0;                      // entries chk_part holds
   float2 *nearbuf = nullptr;                 // per sorted point: the learned pass's near field
+  // segments past the first: per cell where its P2P and W segments are, the
+  // segments (cell, number), and their points' sums
+  uint32_t *seg_at = nullptr;                // 2 per cell
+  uint2 *seg_p2p = nullptr, *seg_w = nullptr;  // pool_cap / SEG_P2P and / SEG_W
+  float2 *part_p2p = nullptr;                // SEG_POINTS per segment
+  double2 *part_w = nullptr;
+  size_t part_p2p_cap = 0, part_w_cap = 0;   // segments
   uint32_t *leafidx = nullptr;               // per sorted point: its leaf's index in the leaf list
   float *mlp = nullptr;              // installed network parameters (device)
   uint32_t ncells_last = 0;
@@ -177,6 +194,10 @@ struct TcArgs {
   size_t pool_cap;
   float *feat, *mlp_x, *mlp_y;
   uint32_t *leaves;
+  uint32_t *seg_at;
+  uint2 *seg_p2p, *seg_w;
+  float2 *part_p2p;
+  double2 *part_w;
   uint32_t *leafidx;  // per sorted point: its leaf's index in the leaf list (near pass)
   double2 *kick;  // non-null: the many-body kick goes here instead of into vx, vy
   double *vx, *vy;
@@ -422,76 +443,98 @@ __device__ __forceinline__ bool separated(const TcArgs &a, const TcCell &A, cons
   return dx * dx + dy * dy >= thr * thr;
 }
 
-// Per-lane list events. WRITE false: counts; true: writes from the offsets.
+// Per-lane list events.
 struct Ev {
   uint32_t np, nw, nx, nc;
 };
 
-// Leaf A against the subtree of B (not a leaf, near A): M2P for the cells
-// separated from A, P2P for the leaves that are not.
+// The walks of leaf A through the subtrees of the lanes' cells b (not leaves,
+// near A; NONE: none), by the whole warp: M2P for the cells separated from A,
+// P2P for the leaves that are not, counted into np and nw (the same on every
+// lane) and, WRITE, written from op + np and ow + nw on. Beside a dense
+// cluster a sparse leaf's walk passes thousands of cells: a lane alone took up
+// to half a millisecond for it (0.4 us a cell), the warp tests 32 at a time.
+// The cells to visit are on a stack in shared memory; near its limit they are
+// taken one at a time, which adds at most 3 a level, so it cannot overflow.
+constexpr uint32_t WALK_STACK = 512, WALK_SOFT = 352;
+static_assert(WALK_SOFT - 32 + 4 * 32 + 3 * 17 <= WALK_STACK, "levels 0 .. 16");
+
 template <bool WRITE>
-__device__ bool tc_walk(const TcArgs &a, const TcCell &A, uint32_t b, Ev &e, uint32_t op,
-                        uint32_t ow) {
-  uint32_t stack[TC_STACK];
+__device__ void tc_walk(const TcArgs &a, const TcCell &A, uint32_t b, uint32_t *stack, uint32_t &np,
+                        uint32_t &nw, uint32_t op, uint32_t ow) {
+  const unsigned lane = threadIdx.x & 31, full = 0xffffffffu, lt = (1u << lane) - 1;
   uint32_t sp = 0;
-  const TcCell B = a.cells[b];
-  for (uint32_t j = 0; j < 4; ++j) {
-    const uint32_t ch = child_at(B, 3 - j);
-    if (ch != TC_NONE) stack[sp++] = ch;
-  }
+  // the children of the lanes' opened cells onto the stack
+  auto push = [&](const TcCell &C, bool open) {
+    const uint32_t n = open ? C.nchild : 0;
+    const unsigned b0 = __ballot_sync(full, n & 1), b1 = __ballot_sync(full, n & 2),
+                   b2 = __ballot_sync(full, n & 4);
+    uint32_t at = sp + __popc(b0 & lt) + 2 * __popc(b1 & lt) + 4 * __popc(b2 & lt);
+    for (uint32_t j = 0; j < n; ++j) stack[at + j] = C.child0 + j;
+    sp += __popc(b0) + 2 * __popc(b1) + 4 * __popc(b2);
+    __syncwarp();
+  };
+  TcCell C;
+  C.nchild = 0;
+  if (b != TC_NONE) C = a.cells[b];
+  push(C, b != TC_NONE);
   while (sp) {
-    const uint32_t c = stack[--sp];
-    const TcCell C = a.cells[c];
-    if (separated(a, A, C)) {
-      if (WRITE) a.pool[ow + e.nw] = c;
-      ++e.nw;
-    } else if (C.nchild == 0) {
-      if (WRITE) a.pool[op + e.np] = c;
-      ++e.np;
-    } else {
-      if (sp + 4 > TC_STACK) return false;
-      for (uint32_t j = 0; j < 4; ++j) {
-        const uint32_t ch = child_at(C, 3 - j);
-        if (ch != TC_NONE) stack[sp++] = ch;
-      }
+    const uint32_t take = sp > WALK_SOFT ? 1 : min(sp, 32u);
+    sp -= take;
+    const bool in = lane < take;
+    const uint32_t c = in ? stack[sp + lane] : 0;
+    __syncwarp();
+    bool far = false, near = false;
+    if (in) {
+      C = a.cells[c];
+      far = separated(a, A, C);
+      near = !far && C.nchild == 0;
     }
+    const unsigned mw = __ballot_sync(full, far), mp = __ballot_sync(full, near);
+    if (WRITE) {
+      if (far) a.pool[ow + nw + __popc(mw & lt)] = c;
+      if (near) a.pool[op + np + __popc(mp & lt)] = c;
+    }
+    nw += __popc(mw);
+    np += __popc(mp);
+    push(C, in && !far && !near);
   }
-  return true;
 }
 
 // The events of candidate u of cell c (u < 4 nnear: a child of a parent's
-// near cell; beyond: the parent's coarse leaf u - 4 nnear).
+// near cell; beyond: the parent's coarse leaf u - 4 nnear). Returns the cell
+// whose subtree a walk has to look through, or NONE.
 template <bool WRITE>
-__device__ bool tc_candidate(const TcArgs &a, uint32_t c, const TcCell &A, uint32_t u, Ev &e,
-                             const uint32_t *o4) {
+__device__ uint32_t tc_candidate(const TcArgs &a, uint32_t c, const TcCell &A, uint32_t u, Ev &e,
+                                 const uint32_t *o4) {
   const uint32_t nn = a.tab->nnear;
   const bool leaf = A.nchild == 0;
   uint32_t coarse = TC_NONE;
   if (u < 4 * nn) {
     const uint32_t o = u >> 2, b = u & 3;
     const uint32_t pb = __ldcg(&a.near[(size_t)A.parent * nn + o]);
-    if (pb == TC_NONE) return true;
+    if (pb == TC_NONE) return TC_NONE;
     const TcCell PB = a.cells[pb];
     if (PB.nchild == 0) {
-      if (b != 0) return true;
+      if (b != 0) return TC_NONE;
       coarse = pb;  // a near leaf of the parent: seen from A as a coarse leaf
     } else {
       const uint32_t B = child_at(PB, b);
-      if (B == TC_NONE) return true;
+      if (B == TC_NONE) return TC_NONE;
       const uint32_t e16 = a.tab->map[A.quad][o][b];
       if (!(e16 & TC_NEAR_FLAG)) {
         if (WRITE) a.m2l[(size_t)c * a.tab->sstride + e16] = B;
-        return true;
+        return TC_NONE;
       }
       if (WRITE) a.near[(size_t)c * nn + (e16 & 0xFF)] = B;
-      if (!leaf) return true;
+      if (!leaf) return TC_NONE;
       const TcCell Bc = a.cells[B];
       if (Bc.nchild == 0) {
         if (WRITE) a.pool[o4[0] + e.np] = B;
         ++e.np;
-        return true;
+        return TC_NONE;
       }
-      return tc_walk<WRITE>(a, A, B, e, o4[0], o4[1]);
+      return B;
     }
   } else {
     const uint32_t k = u - 4 * nn;
@@ -508,7 +551,7 @@ __device__ bool tc_candidate(const TcArgs &a, uint32_t c, const TcCell &A, uint3
     if (WRITE) a.pool[o4[3] + e.nc] = coarse;
     ++e.nc;
   }
-  return true;
+  return TC_NONE;
 }
 
 
@@ -523,38 +566,25 @@ __device__ __forceinline__ uint32_t warp_excl_sum(uint32_t v, uint32_t &total) {
   return incl - v;
 }
 
-// One candidate's pool event: its kind (0 none, 1 P2P leaf, 2 W cell, 3 X
-// leaf, 4 coarse leaf passed down, 5 a walk of the subtree of `id`) and cell.
+// One candidate's pool event: its kind (0 none, 1 P2P leaf, 3 X leaf, 4 coarse
+// leaf passed down, 5 a walk of the subtree of `id`) and cell.
 struct Cand {
   uint32_t kind, id;
 };
 
-// The events of an evaluated candidate: counted into e, or (WRITE) written
-// from the offsets o4 (p2p, w, x, coarse) plus e's counts so far.
+// The event of an evaluated candidate (not a walk): counted into e, or
+// (WRITE) written from the offsets o4 (p2p, w, x, coarse).
 template <bool WRITE>
-__device__ __forceinline__ bool cand_events(const TcArgs &a, const TcCell &A, Cand cd, Ev &e,
-                                            const uint32_t *o4) {
-  switch (cd.kind) {
-    case 1:
-      if (WRITE) a.pool[o4[0] + e.np] = cd.id;
-      ++e.np;
-      return true;
-    case 2:
-      if (WRITE) a.pool[o4[1] + e.nw] = cd.id;
-      ++e.nw;
-      return true;
-    case 3:
-      if (WRITE) a.pool[o4[2] + e.nx] = cd.id;
-      ++e.nx;
-      return true;
-    case 4:
-      if (WRITE) a.pool[o4[3] + e.nc] = cd.id;
-      ++e.nc;
-      return true;
-    case 5:
-      return tc_walk<WRITE>(a, A, cd.id, e, o4[0], o4[1]);
-    default:
-      return true;
+__device__ __forceinline__ void cand_event(const TcArgs &a, Cand cd, Ev &e, const uint32_t *o4) {
+  if (cd.kind == 1) {
+    if (WRITE) a.pool[o4[0]] = cd.id;
+    ++e.np;
+  } else if (cd.kind == 3) {
+    if (WRITE) a.pool[o4[2]] = cd.id;
+    ++e.nx;
+  } else if (cd.kind == 4) {
+    if (WRITE) a.pool[o4[3]] = cd.id;
+    ++e.nc;
   }
 }
 
@@ -565,10 +595,10 @@ constexpr uint32_t LIST_KEEP = 4;
 
 struct ListState {
   Ev tot;
-  bool ok;
   uint32_t mode, ncand;
   Cand kept[LIST_KEEP];
   uint32_t off[LIST_KEEP][4];
+  uint32_t walk[LIST_KEEP][2];  // where a round's walk starts in the P2P and W lists
 };
 
 // The per-kind totals of one round of events: tot += the warp's sums, off[k]
@@ -596,7 +626,8 @@ __device__ __forceinline__ void round_offsets(const Ev &e, Ev &tot, uint32_t *of
 // candidates' loads by dependency level for all rounds at once (the parent's
 // near cell or coarse leaf, its cell, then for a leaf the near cell's child);
 // the M2L table and near list entries are written here.
-__device__ void tc_list_count_kept(const TcArgs &a, uint32_t c, const TcCell &A, ListState &S) {
+__device__ void tc_list_count_kept(const TcArgs &a, uint32_t c, const TcCell &A, ListState &S,
+                                   uint32_t *stack) {
   const unsigned lane = threadIdx.x & 31;
   const uint32_t nn = a.tab->nnear, ncand = S.ncand;
   const bool leaf = A.nchild == 0;
@@ -651,35 +682,42 @@ __device__ void tc_list_count_kept(const TcArgs &a, uint32_t c, const TcCell &A,
     if (r >= rounds) break;
     Ev e{0, 0, 0, 0};
     const uint32_t z4[4] = {0, 0, 0, 0};
-    if (!cand_events<false>(a, A, S.kept[r], e, z4)) S.ok = false;
+    cand_event<false>(a, S.kept[r], e, z4);
     round_offsets(e, S.tot, S.off[r]);
+    S.walk[r][0] = S.tot.np;
+    S.walk[r][1] = S.tot.nw;
+    if (__any_sync(0xffffffffu, S.kept[r].kind == 5))
+      tc_walk<false>(a, A, S.kept[r].kind == 5 ? S.kept[r].id : TC_NONE, stack, S.tot.np, S.tot.nw, 0, 0);
   }
 }
 
 // Count phase of a cell with more candidates than the lanes keep.
-__device__ void tc_list_count_general(const TcArgs &a, uint32_t c, const TcCell &A, ListState &S) {
+__device__ void tc_list_count_general(const TcArgs &a, uint32_t c, const TcCell &A, ListState &S,
+                                      uint32_t *stack) {
   const unsigned lane = threadIdx.x & 31;
   const uint32_t zero4[4] = {0, 0, 0, 0};
   for (uint32_t u0 = 0; u0 < S.ncand; u0 += 32) {
     const uint32_t u = u0 + lane;
     Ev e{0, 0, 0, 0};
-    if (u < S.ncand && !tc_candidate<false>(a, c, A, u, e, zero4)) S.ok = false;
+    const uint32_t b = u < S.ncand ? tc_candidate<false>(a, c, A, u, e, zero4) : TC_NONE;
     uint32_t off[4];
     round_offsets(e, S.tot, off);
+    if (__any_sync(0xffffffffu, b != TC_NONE))
+      tc_walk<false>(a, A, b, stack, S.tot.np, S.tot.nw, 0, 0);
   }
 }
 
 // Write phase of the general case: evaluate again, each lane's events after
 // those of the candidates before it.
 __device__ void tc_list_write_general(const TcArgs &a, uint32_t c, const TcCell &A,
-                                      const ListState &S, uint32_t *o4) {
+                                      const ListState &S, const uint32_t *o4, uint32_t *stack) {
   const unsigned lane = threadIdx.x & 31;
   const uint32_t zero4[4] = {0, 0, 0, 0};
   Ev run{0, 0, 0, 0};
   for (uint32_t u0 = 0; u0 < S.ncand; u0 += 32) {
     const uint32_t u = u0 + lane;
     Ev e{0, 0, 0, 0};
-    if (u < S.ncand) tc_candidate<false>(a, c, A, u, e, zero4);
+    const uint32_t b = u < S.ncand ? tc_candidate<false>(a, c, A, u, e, zero4) : TC_NONE;
     uint32_t off[4];
     round_offsets(e, run, off);
     if (u < S.ncand) {
@@ -687,6 +725,8 @@ __device__ void tc_list_write_general(const TcArgs &a, uint32_t c, const TcCell 
       const uint32_t w4[4] = {o4[0] + off[0], o4[1] + off[1], o4[2] + off[2], o4[3] + off[3]};
       tc_candidate<true>(a, c, A, u, w, w4);
     }
+    if (__any_sync(0xffffffffu, b != TC_NONE))
+      tc_walk<true>(a, A, b, stack, run.np, run.nw, o4[0], o4[1]);
   }
 }
 
@@ -701,13 +741,13 @@ __device__ void tc_list_write_general(const TcArgs &a, uint32_t c, const TcCell 
 constexpr uint32_t LIST_THREADS = 128, LIST_WARPS = LIST_THREADS / 32;
 __global__ void __launch_bounds__(LIST_THREADS, 8) k_tc_lists(TcArgs a, uint32_t c0, uint32_t c1) {
   __shared__ uint32_t wsum[LIST_WARPS + 1];
+  __shared__ uint32_t stacks[LIST_WARPS][WALK_STACK];
   const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t c = c0 + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   const bool active = c < c1;  // warp-uniform
   const uint32_t nn = a.tab->nnear;
   ListState S;
   S.tot = {0, 0, 0, 0};
-  S.ok = true;
   S.mode = 0;
   S.ncand = 0;
   TcCell A;
@@ -723,12 +763,11 @@ __global__ void __launch_bounds__(LIST_THREADS, 8) k_tc_lists(TcArgs a, uint32_t
       S.ncand = 4 * nn + __ldcg(&a.loff[(size_t)A.parent * 8 + 7]);
       if (S.ncand <= 32 * LIST_KEEP) {
         S.mode = 1;
-        tc_list_count_kept(a, c, A, S);
+        tc_list_count_kept(a, c, A, S, stacks[warp]);
       } else {
         S.mode = 2;
-        tc_list_count_general(a, c, A, S);
+        tc_list_count_general(a, c, A, S, stacks[warp]);
       }
-      S.ok = __all_sync(0xffffffffu, S.ok);
     }
     all = S.tot.np + S.tot.nw + S.tot.nx + S.tot.nc;
   }
@@ -749,9 +788,9 @@ __global__ void __launch_bounds__(LIST_THREADS, 8) k_tc_lists(TcArgs a, uint32_t
   const uint32_t o4[4] = {base, base + S.tot.np, base + S.tot.np + S.tot.nw,
                           base + S.tot.np + S.tot.nw + S.tot.nx};
   uint32_t *lo = a.loff + (size_t)c * 8;
-  if (!S.ok || (size_t)base + all > a.pool_cap) {
+  if ((size_t)base + all > a.pool_cap) {
     if (lane == 0) {
-      atomicOr(&a.info[TI_OVF], S.ok ? 1u : 2u);
+      atomicOr(&a.info[TI_OVF], 1u);
       lo[0] = lo[2] = lo[4] = lo[6] = 0;
       lo[1] = lo[3] = lo[5] = lo[7] = 0;
     }
@@ -762,6 +801,23 @@ __global__ void __launch_bounds__(LIST_THREADS, 8) k_tc_lists(TcArgs a, uint32_t
     lo[2] = o4[1]; lo[3] = S.tot.nw;
     lo[4] = o4[2]; lo[5] = S.tot.nx;
     lo[6] = o4[3]; lo[7] = S.tot.nc;
+  }
+  if (A.nchild == 0) {
+    // the further segments of its lists (the pool holds their entries, so
+    // there are at most pool_cap / SEG_P2P and pool_cap / SEG_W of them)
+    const uint32_t mp = more_segments(S.tot.np, A.count, SEG_P2P),
+                   mw = more_segments(S.tot.nw, A.count, SEG_W);
+    if (mp | mw) {
+      uint32_t ap = 0, aw = 0;
+      if (lane == 0) {
+        if (mp) ap = a.seg_at[2 * (size_t)c] = atomicAdd(&a.info[TI_SEG_P2P], mp);
+        if (mw) aw = a.seg_at[2 * (size_t)c + 1] = atomicAdd(&a.info[TI_SEG_W], mw);
+      }
+      ap = __shfl_sync(0xffffffffu, ap, 0);
+      aw = __shfl_sync(0xffffffffu, aw, 0);
+      for (uint32_t j = lane; j < mp; j += 32) a.seg_p2p[ap + j] = make_uint2(c, j + 1);
+      for (uint32_t j = lane; j < mw; j += 32) a.seg_w[aw + j] = make_uint2(c, j + 1);
+    }
   }
   if (S.mode == 0) {
     if (lane == 0) {
@@ -778,12 +834,14 @@ __global__ void __launch_bounds__(LIST_THREADS, 8) k_tc_lists(TcArgs a, uint32_t
         const uint32_t w4[4] = {o4[0] + S.off[r][0], o4[1] + S.off[r][1], o4[2] + S.off[r][2],
                                 o4[3] + S.off[r][3]};
         Ev w{0, 0, 0, 0};
-        cand_events<true>(a, A, S.kept[r], w, w4);
+        cand_event<true>(a, S.kept[r], w, w4);
       }
+      if (__any_sync(0xffffffffu, S.kept[r].kind == 5))
+        tc_walk<true>(a, A, S.kept[r].kind == 5 ? S.kept[r].id : TC_NONE, stacks[warp], S.walk[r][0],
+                      S.walk[r][1], o4[0], o4[1]);
     }
   } else {
-    uint32_t o[4] = {o4[0], o4[1], o4[2], o4[3]};
-    tc_list_write_general(a, c, A, S, o);
+    tc_list_write_general(a, c, A, S, o4, stacks[warp]);
   }
 }
 
@@ -791,16 +849,21 @@ __global__ void __launch_bounds__(LIST_THREADS, 8) k_tc_lists(TcArgs a, uint32_t
 
 // M2L CTA: 256 gathering threads (two per target row: the bf16 hi and the lo
 // half of the row) and one warp whose first lane only issues the MMAs.
-constexpr uint32_t M2L_STAGES = 3;
-constexpr uint32_t M2L_AHEAD = 2;  // slots of copies in flight per gathering thread
-static_assert(M2L_AHEAD <= M2L_STAGES, "a stage is landed before it is reused");
+// Stages of the ring and slots of copies in flight per gathering thread: 3 and
+// 2 let three CTAs share an SM, which hides the gathers' latency when there
+// are tiles enough; with at most one tile an SM a CTA takes the SM's memory for
+// itself and keeps 6 slots in flight (32 tiles, 39 slots: 84 -> 48 us).
+constexpr uint32_t M2L_STAGES = 3, M2L_AHEAD = 2, M2L_FEW_STAGES = 8, M2L_FEW_AHEAD = 6;
+static_assert(M2L_AHEAD <= M2L_STAGES && M2L_FEW_AHEAD <= M2L_FEW_STAGES,
+              "a stage is landed before it is reused");
 constexpr uint32_t M2L_PRODUCERS = 2 * TC_TILE;
 constexpr uint32_t M2L_THREADS = M2L_PRODUCERS + 32;
 
+template <uint32_t STAGES>
 struct M2lSmem {
-  unsigned char a[M2L_STAGES][2][TC_TILE * TC_KN * 2];  // [stage][hi, lo] 128 x 32 bf16
-  unsigned char b[M2L_STAGES][2][TC_KN * TC_KN * 2];    // [stage][hi, lo] 32 x 32 bf16
-  uint64_t full[M2L_STAGES], empty[M2L_STAGES], done;
+  unsigned char a[STAGES][2][TC_TILE * TC_KN * 2];  // [stage][hi, lo] 128 x 32 bf16
+  unsigned char b[STAGES][2][TC_KN * TC_KN * 2];    // [stage][hi, lo] 32 x 32 bf16
+  uint64_t full[STAGES], empty[STAGES], done;
   uint32_t tmem;
   uint32_t tgt[TC_TILE];
   uint32_t err;
@@ -809,9 +872,10 @@ struct M2lSmem {
 // Budget of a wait on a barrier the tile's own threads complete.
 constexpr uint64_t TC_WAIT_NS = 50ull * 1000 * 1000;
 
+template <uint32_t STAGES, uint32_t AHEAD>
 __global__ void __launch_bounds__(M2L_THREADS) k_tc_m2l(TcArgs a) {
   extern __shared__ __align__(1024) unsigned char tc_m2l_smem[];
-  M2lSmem &S = *reinterpret_cast<M2lSmem *>(tc_m2l_smem);
+  M2lSmem<STAGES> &S = *reinterpret_cast<M2lSmem<STAGES> *>(tc_m2l_smem);
   volatile uint32_t *abort = &S.err;
   const uint32_t t = threadIdx.x, warp = t >> 5;
   // this CTA's tile: group g, rows base .. base + 127
@@ -827,7 +891,7 @@ __global__ void __launch_bounds__(M2L_THREADS) k_tc_m2l(TcArgs a) {
   const uint32_t nslot = a.tab->nslot[g], sstride = a.tab->sstride;
   if (t < TC_TILE) S.tgt[t] = base + t < cnt ? a.groups[(size_t)g * a.ccap + base + t] : TC_NONE;
   if (t == 0) {
-    for (uint32_t s = 0; s < M2L_STAGES; ++s) {
+    for (uint32_t s = 0; s < STAGES; ++s) {
       tc::mbar_init(&S.full[s], M2L_PRODUCERS);
       tc::mbar_init(&S.empty[s], 1);
     }
@@ -872,18 +936,18 @@ __global__ void __launch_bounds__(M2L_THREADS) k_tc_m2l(TcArgs a) {
     // wait for them, make them visible to the tensor core, arrive
     auto land = [&](uint32_t j, bool all) {
       if (all) tc::cp_async_wait<0>();
-      else tc::cp_async_wait<M2L_AHEAD - 1>();
+      else tc::cp_async_wait<AHEAD - 1>();
       tc::fence_proxy_async();
-      tc::mbar_arrive(&S.full[j % M2L_STAGES]);
+      tc::mbar_arrive(&S.full[j % STAGES]);
     };
     uint32_t src = source(0), landed = 0;
     for (uint32_t j = 0; j < nslot; ++j) {
-      const uint32_t s = j % M2L_STAGES, use = j / M2L_STAGES;
+      const uint32_t s = j % STAGES, use = j / STAGES;
       const uint32_t next = source(j + 1);
       // the stage is free once the MMAs that read it (slot j - STAGES) are done
       if (use > 0 && !tc::mbar_wait(&S.empty[s], (use - 1) & 1, abort, TC_WAIT_NS)) break;
       copy(j, s, src);
-      if (j + 1 >= M2L_AHEAD) land(landed++, false);
+      if (j + 1 >= AHEAD) land(landed++, false);
       src = next;
     }
     // the slots still in flight (also after a wait that gave up: every copy
@@ -895,7 +959,7 @@ __global__ void __launch_bounds__(M2L_THREADS) k_tc_m2l(TcArgs a) {
     const uint32_t idesc = tc::idesc_bf16_f32(TC_TILE, TC_KN);
     const uint32_t alb = (TC_TILE / 8) * 128, blb = (TC_KN / 8) * 128;
     for (uint32_t j = 0; j < nslot; ++j) {
-      const uint32_t s = j % M2L_STAGES, use = j / M2L_STAGES;
+      const uint32_t s = j % STAGES, use = j / STAGES;
       if (!tc::mbar_wait(&S.full[s], use & 1, abort, TC_WAIT_NS)) break;
       tc::fence_after_sync();
       const uint32_t a_hi = tc::smem_addr(S.a[s][0]), a_lo = tc::smem_addr(S.a[s][1]);
@@ -1288,36 +1352,18 @@ __device__ __forceinline__ float4 staged_point(const float4 *sg, uint32_t k) {
   return make_float4(p[h], p[2 + h], p[4 + h], p[6 + h]);
 }
 
-// The far field at target point k of leaf C: L2P of the leaf's final local
-// expansion (Lsh: 2q floats, L'_0 possibly corrected) by Horner in FP32 (the
-// L2P of downwardCell, fmm.zig:851-886),
-//     phi = (1/s) sum_l L'_l w^l,   w = (u - c) / s,
-// and M2P from each cell of the leaf's W list (z from an FP64 shift, the
-// series in FP32; the adaptive list has no reference counterpart),
-//     phi += (1/s_W) sum_k M'_k / z^(k+1),   z = (u - c_W) / s_W.
-// Returns the kick's far part in world units; (wr, wi) = w for the feature row.
-__device__ __forceinline__ float2 tc_far(const TcArgs &a, uint32_t k, double cx, double cy,
-                                         double inv_s, const float *Lsh, float c0r, float c0i,
-                                         uint32_t nw, uint32_t ow, float &wr, float &wi) {
+// M2P at (ux, uy) from the W-list cells pool[ow ..  ow + nw): z from an FP64
+// shift, the series in FP32 (|1/z| < 1 for a separated cell),
+//     g += (1/s_W) sum_k M'_k / z^(k+1),   z = (u - c_W) / s_W.
+__device__ __forceinline__ void tc_m2p(const TcArgs &a, double ux, double uy, uint32_t nw, uint32_t ow,
+                                       double &gr, double &gi) {
   const uint32_t q = a.q;
-  const double ux = a.ux[k], uy = a.uy[k];
-  wr = (float)((ux - cx) * inv_s);
-  wi = (float)((uy - cy) * inv_s);
-  // L'_0 + (c0r, c0i): the learned form's correction (zero otherwise)
-  float ar = Lsh[q - 1] + (q == 1 ? c0r : 0.f), ai = Lsh[2 * q - 1] + (q == 1 ? c0i : 0.f);
-  for (int l = (int)q - 2; l >= 0; --l) {
-    const float nr = ar * wr - ai * wi + Lsh[l] + (l == 0 ? c0r : 0.f);
-    ai = ar * wi + ai * wr + Lsh[q + l] + (l == 0 ? c0i : 0.f);
-    ar = nr;
-  }
-  double gr = (double)ar * inv_s, gi = (double)ai * inv_s;
   for (uint32_t e = 0; e < nw; ++e) {
     const uint32_t cc = a.pool[ow + e];
     const TcCell W = a.cells[cc];
     double wx, wy;
     cell_centre(W, wx, wy);
     const double winv = pow2((int)W.level);
-    // z in FP64 (the shift), the series in FP32: |1/z| < 1 for a separated cell
     const float zr = (float)((ux - wx) * winv), zi = (float)((uy - wy) * winv);
     const float d2 = zr * zr + zi * zi;
     const float ir = __fdividef(zr, d2), ii = -__fdividef(zi, d2);
@@ -1333,6 +1379,54 @@ __device__ __forceinline__ float2 tc_far(const TcArgs &a, uint32_t k, double cx,
     }
     gr += (double)sr * winv;
     gi += (double)si * winv;
+  }
+}
+
+// The further segments of the W lists, a warp each, a lane per point of the
+// leaf (and 32 on): their M2P sums into part_w, for tc_far.
+__global__ void __launch_bounds__(128) k_tc_m2p_segments(TcArgs a, uint32_t segments) {
+  const uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (k >= segments) return;
+  const uint2 it = a.seg_w[k];
+  const TcCell C = a.cells[it.x];
+  const uint32_t nw = a.loff[(size_t)it.x * 8 + 3], ow = a.loff[(size_t)it.x * 8 + 2];
+  const uint32_t e0 = it.y * SEG_W, n = min(SEG_W, nw - e0);
+  for (uint32_t j = threadIdx.x & 31; j < C.count; j += 32) {
+    double gr = 0, gi = 0;
+    tc_m2p(a, a.ux[C.first + j], a.uy[C.first + j], n, ow + e0, gr, gi);
+    a.part_w[(size_t)k * SEG_POINTS + j] = make_double2(gr, gi);
+  }
+}
+
+// The far field at target point k of leaf C: L2P of the leaf's final local
+// expansion (Lsh: 2q floats, L'_0 possibly corrected) by Horner in FP32 (the
+// L2P of downwardCell, fmm.zig:851-886),
+//     phi = (1/s) sum_l L'_l w^l,   w = (u - c) / s,
+// and M2P from each cell of the leaf's W list (the adaptive list has no
+// reference counterpart): the first `nw` cells here, the further segments'
+// sums from `part`.
+// Returns the kick's far part in world units; (wr, wi) = w for the feature row.
+__device__ __forceinline__ float2 tc_far(const TcArgs &a, uint32_t k, double cx, double cy,
+                                         double inv_s, const float *Lsh, float c0r, float c0i,
+                                         uint32_t nw, uint32_t ow, const double2 *part, uint32_t parts,
+                                         float &wr, float &wi) {
+  const uint32_t q = a.q;
+  const double ux = a.ux[k], uy = a.uy[k];
+  wr = (float)((ux - cx) * inv_s);
+  wi = (float)((uy - cy) * inv_s);
+  // L'_0 + (c0r, c0i): the learned form's correction (zero otherwise)
+  float ar = Lsh[q - 1] + (q == 1 ? c0r : 0.f), ai = Lsh[2 * q - 1] + (q == 1 ? c0i : 0.f);
+  for (int l = (int)q - 2; l >= 0; --l) {
+    const float nr = ar * wr - ai * wi + Lsh[l] + (l == 0 ? c0r : 0.f);
+    ai = ar * wi + ai * wr + Lsh[q + l] + (l == 0 ? c0i : 0.f);
+    ar = nr;
+  }
+  double gr = (double)ar * inv_s, gi = (double)ai * inv_s;
+  tc_m2p(a, ux, uy, nw, ow, gr, gi);
+  for (uint32_t j = 0; j < parts; ++j) {
+    const double2 v = part[(size_t)j * SEG_POINTS];
+    gr += v.x;
+    gi += v.y;
   }
   return make_float2((float)(-gr * a.inv_w), (float)(gi * a.inv_w));
 }
@@ -1351,7 +1445,9 @@ __device__ __forceinline__ float2 tc_far(const TcArgs &a, uint32_t k, double cx,
 // pair loop takes two sources per step in packed FP32 (tc_pair2), each half
 // of a target's sums adding every other source; there the lane groups take
 // alternate source pairs.
-__global__ void __launch_bounds__(NEAR_THREADS, 8) k_tc_near(TcArgs a, float2 *nearbuf) {
+// Warps past the leaf list take the further segments of long P2P lists
+// (`segments` of them) into part_p2p, which k_tc_far adds.
+__global__ void __launch_bounds__(NEAR_THREADS, 8) k_tc_near(TcArgs a, float2 *nearbuf, uint32_t segments) {
   __shared__ float4 stage[NEAR_WARPS][P2P_STAGE];
   __shared__ float4 red[NEAR_WARPS][32];
   const unsigned lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
@@ -1361,10 +1457,14 @@ __global__ void __launch_bounds__(NEAR_THREADS, 8) k_tc_near(TcArgs a, float2 *n
   const float fl = 1e-18f * fmaxf(1e-18f, a.dmin2f);
   const uint32_t nleaf = __ldcg(&a.info[TI_LEAVES]);
   float4 *sg = stage[wl];
-  for (uint32_t e0 = gw; e0 < nleaf; e0 += nwarps) {
-    const uint32_t c = a.leaves[e0];
+  for (uint32_t e0 = gw; e0 < nleaf + segments; e0 += nwarps) {
+    const uint2 it = e0 < nleaf ? make_uint2(a.leaves[e0], 0) : a.seg_p2p[e0 - nleaf];
+    const uint32_t c = it.x;
     const TcCell A = a.cells[c];
-    const uint32_t np = a.loff[(size_t)c * 8 + 1], op = a.loff[(size_t)c * 8];
+    const uint32_t all = a.loff[(size_t)c * 8 + 1], op = a.loff[(size_t)c * 8];
+    // this item's entries of the list
+    const uint32_t np0 = it.y * SEG_P2P;
+    const uint32_t np = more_segments(all, A.count, SEG_P2P) ? min(all, np0 + SEG_P2P) : all;
     // lane groups: a lane holds two targets (slots gl and W + gl of the
     // round), W = ceil(count / 2) lanes a group, G = 32 / W groups (lanes
     // past G W idle); a leaf of more than 64 points takes several rounds
@@ -1393,7 +1493,7 @@ __global__ void __launch_bounds__(NEAR_THREADS, 8) k_tc_near(TcArgs a, float2 *n
       const float2 nx1 = make_float2(-x1, -x1), ny1 = make_float2(-y1, -y1);
       // targets 0 and 1; the halves sum the even and the odd sources
       float2 ax0 = make_float2(0.f, 0.f), ay0 = ax0, ax1 = ax0, ay1 = ax0;
-      for (uint32_t eb = 0; eb < np; eb += 32) {
+      for (uint32_t eb = np0; eb < np; eb += 32) {
         // this batch's source leaves: lane j holds leaf j's first point and
         // the running count before it
         const uint32_t ne = min(32u, np - eb);
@@ -1463,6 +1563,12 @@ __global__ void __launch_bounds__(NEAR_THREADS, 8) k_tc_near(TcArgs a, float2 *n
           v1x += v.z;
           v1y += v.w;
         }
+        if (it.y) {
+          float2 *part = a.part_p2p + (size_t)(e0 - nleaf) * SEG_POINTS;
+          if (act0) part[t0 - A.first] = make_float2(v0x, v0y);
+          if (act1) part[t1 - A.first] = make_float2(v1x, v1y);
+          continue;
+        }
         if (act0) {
           nearbuf[t0] = make_float2(v0x, v0y);
           a.leafidx[t0] = e0;
@@ -1500,9 +1606,20 @@ __global__ void __launch_bounds__(TC_THREADS) k_tc_far(TcArgs a, const float2 *n
     c0i = sc * a.mlp_y[(size_t)e * 2 + 1];
   }
   float wr, wi;
-  const float2 f =
-      tc_far(a, k, cx, cy, inv_s, a.lco + (size_t)c * TC_KN, c0r, c0i, nw, ow, wr, wi);
-  const float2 nv = nearbuf[k];
+  const uint32_t mw = more_segments(nw, C.count, SEG_W);
+  const float2 f = tc_far(a, k, cx, cy, inv_s, a.lco + (size_t)c * TC_KN, c0r, c0i, mw ? SEG_W : nw, ow,
+                          mw ? a.part_w + (size_t)a.seg_at[2 * (size_t)c + 1] * SEG_POINTS + (k - C.first)
+                             : nullptr,
+                          mw, wr, wi);
+  float2 nv = nearbuf[k];
+  const uint32_t mp = more_segments(a.loff[(size_t)c * 8 + 1], C.count, SEG_P2P);
+  if (mp) {
+    const float2 *part = a.part_p2p + (size_t)a.seg_at[2 * (size_t)c] * SEG_POINTS + (k - C.first);
+    for (uint32_t j = 0; j < mp; ++j) {
+      nv.x += part[(size_t)j * SEG_POINTS].x;
+      nv.y += part[(size_t)j * SEG_POINTS].y;
+    }
+  }
   const double kx = (double)nv.x + (double)f.x, ky = (double)nv.y + (double)f.y;
   if (a.kick) {
     a.kick[k] = make_double2(kx, ky);
@@ -1803,6 +1920,8 @@ int reserve(TcDev &d, uint32_t ncells, uint32_t m) {
     D3_CUDA_OK(cudaMalloc(&d.loff, (size_t)cap * 8 * 4));
     cudaFree(d.arrive);
     D3_CUDA_OK(cudaMalloc(&d.arrive, (size_t)cap * 4));
+    cudaFree(d.seg_at);
+    D3_CUDA_OK(cudaMalloc(&d.seg_at, (size_t)cap * 2 * 4));
     d.ccap = cap;
   }
   if (m > d.pcap) {
@@ -1823,6 +1942,19 @@ int reserve(TcDev &d, uint32_t ncells, uint32_t m) {
     D3_CUDA_OK(cudaMalloc(&d.mlp_y, (size_t)d.ccap * 2 * 4));
     d.lcap = d.ccap;
   }
+  return 0;
+}
+
+// Room for `segments` segments' partial sums, with headroom.
+template <typename T>
+int grow_parts(T *&p, size_t &cap, size_t segments) {
+  if (segments <= cap) return 0;
+  cudaFree(p);
+  p = nullptr;
+  cap = 0;
+  const size_t want = segments + segments / 4 + 64;
+  D3_CUDA_OK(cudaMalloc(&p, want * SEG_POINTS * sizeof(T)));
+  cap = want;
   return 0;
 }
 
@@ -1857,8 +1989,11 @@ TcDev *tc_dev(FastScratch &s) {
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaFuncSetAttribute(k_tc_m2l, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)sizeof(M2lSmem));
+  cudaFuncSetAttribute(k_tc_m2l<M2L_STAGES, M2L_AHEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)sizeof(M2lSmem<M2L_STAGES>));
+  cudaFuncSetAttribute(k_tc_m2l<M2L_FEW_STAGES, M2L_FEW_AHEAD>,
+                       cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)sizeof(M2lSmem<M2L_FEW_STAGES>));
   d->sms = sms;
   bool ok = cudaStreamCreateWithFlags(&d->side, cudaStreamNonBlocking) == cudaSuccess;
   for (cudaEvent_t *e : {&d->ev_geom, &d->ev_up, &d->ev_lists, &d->ev_near, &d->ev_down,
@@ -1916,15 +2051,21 @@ int tc_order_pass(TcDev &d, TcArgs &g, const TcTabSet &ts, uint32_t tiles, bool 
     cudaEventRecord(d.ev_lists, st);
     cudaStreamWaitEvent(d.side, d.ev_lists, 0);
     cudaEventRecord(d.ev[7], d.side);
-    D3_LAUNCH(k_tc_near, blocks_for((size_t)nleaf * 32, NEAR_THREADS), NEAR_THREADS, 0, d.side)(
-        g, d.nearbuf);
+    const uint32_t segments = d.h_info[TI_SEG_P2P];
+    D3_LAUNCH(k_tc_near, blocks_for(((size_t)nleaf + segments) * 32, NEAR_THREADS), NEAR_THREADS, 0,
+              d.side)(g, d.nearbuf, segments);
     cudaEventRecord(d.ev[8], d.side);
     cudaEventRecord(d.ev_near, d.side);
   }
   if (upward_done) cudaStreamWaitEvent(st, d.ev_up, 0);
   else tc_upward(d, g, ts, false, st);
   cudaEventRecord(d.ev[3], st);
-  if (tiles) D3_LAUNCH(k_tc_m2l, tiles, M2L_THREADS, sizeof(M2lSmem), st)(g);
+  if (tiles > (uint32_t)d.sms)
+    D3_LAUNCH((k_tc_m2l<M2L_STAGES, M2L_AHEAD>), tiles, M2L_THREADS, sizeof(M2lSmem<M2L_STAGES>),
+              st)(g);
+  else if (tiles)
+    D3_LAUNCH((k_tc_m2l<M2L_FEW_STAGES, M2L_FEW_AHEAD>), tiles, M2L_THREADS,
+              sizeof(M2lSmem<M2L_FEW_STAGES>), st)(g);
   cudaEventRecord(d.ev[4], st);
   d.last_tiles = tiles;
   if (!d.last_args) d.last_args = new TcArgs;
@@ -1945,6 +2086,8 @@ int tc_order_pass(TcDev &d, TcArgs &g, const TcTabSet &ts, uint32_t tiles, bool 
     D3_LAUNCH(k_tc_features, lw, TC_THREADS, 0, d.side)(g);
     cudaEventRecord(d.ev_feat, d.side);
   }
+  if (const uint32_t segments = d.h_info[TI_SEG_W])
+    D3_LAUNCH(k_tc_m2p_segments, blocks_for(segments * 32ull, 128), 128, 0, st)(g, segments);
   cudaEventRecord(d.ev[11], st);
   if (!far_only) cudaStreamWaitEvent(st, d.ev_near, 0);
   D3_LAUNCH(k_tc_far, blocks_for(g.m, TC_THREADS), TC_THREADS, 0, st)(g, d.nearbuf, learned ? 1 : 0);
@@ -1969,6 +2112,8 @@ void fmm_tc_free(FastScratch &s) {
   cudaFree(d->feat); cudaFree(d->leaves); cudaFree(d->mlp_x); cudaFree(d->mlp_y);
   cudaFree(d->kick); cudaFree(d->chk); cudaFreeHost(d->h_chk); cudaFree(d->mlp);
   cudaFree(d->chk_part); cudaFree(d->nearbuf); cudaFree(d->leafidx);
+  cudaFree(d->seg_at); cudaFree(d->seg_p2p); cudaFree(d->seg_w); cudaFree(d->part_p2p);
+  cudaFree(d->part_w);
   for (cudaEvent_t e : d->ev)
     if (e) cudaEventDestroy(e);
   if (d->side) {
@@ -2103,6 +2248,7 @@ int tc_run(FastScratch &s, TreeDev &t, const NodeArrays &a, const double *streng
   g.near = d.near; g.m2l = d.m2l; g.groups = d.groups; g.loff = d.loff;
   g.feat = d.feat; g.leaves = d.leaves; g.mlp_x = d.mlp_x; g.mlp_y = d.mlp_y;
   g.leafidx = d.leafidx;
+  g.seg_at = d.seg_at;
   g.kick = learned ? d.kick : nullptr;
   g.vx = a.vx; g.vy = a.vy;
   g.info = d.info;
@@ -2125,10 +2271,17 @@ int tc_run(FastScratch &s, TreeDev &t, const NodeArrays &a, const double *streng
       cudaFree(d.pool);
       d.pool = nullptr;
       d.pool_cap = need;
+      cudaFree(d.seg_p2p);
+      cudaFree(d.seg_w);
+      d.seg_p2p = d.seg_w = nullptr;
       D3_CUDA_OK(cudaMalloc(&d.pool, d.pool_cap * 4));
+      D3_CUDA_OK(cudaMalloc(&d.seg_p2p, (d.pool_cap / SEG_P2P + 1) * sizeof(uint2)));
+      D3_CUDA_OK(cudaMalloc(&d.seg_w, (d.pool_cap / SEG_W + 1) * sizeof(uint2)));
     }
     g.pool = d.pool;
     g.pool_cap = d.pool_cap;
+    g.seg_p2p = d.seg_p2p;
+    g.seg_w = d.seg_w;
     if (cudaMemsetAsync(d.info, 0, 8 * 4, st) != cudaSuccess) return -1;
     for (uint32_t lev = 0; lev < pr.nlev; ++lev) {
       const uint32_t c0 = pr.lvl[lev], c1 = pr.lvl[lev + 1];
@@ -2144,9 +2297,14 @@ int tc_run(FastScratch &s, TreeDev &t, const NodeArrays &a, const double *streng
       d.last_pool = used;
       break;
     }
-    if ((d.h_info[TI_OVF] & 2) || attempt > 6) return -1;  // a walk's stack overflowed
+    if (attempt > 6) return -1;
     need = 2 * (size_t)(used > need ? used : need);
   }
+  if (grow_parts(d.part_p2p, d.part_p2p_cap, d.h_info[TI_SEG_P2P]) ||
+      grow_parts(d.part_w, d.part_w_cap, d.h_info[TI_SEG_W]))
+    return -1;
+  g.part_p2p = d.part_p2p;
+  g.part_w = d.part_w;
   cudaEventRecord(d.ev[2], st);
   uint32_t tiles = 0;
   for (uint32_t q4 = 0; q4 < 4; ++q4) tiles += (d.h_info[TI_GROUP + q4] + TC_TILE - 1) / TC_TILE;
