@@ -27,7 +27,7 @@ int fast_reserve(FastScratch &s, uint32_t n) {
   if (n <= s.cap && s.cap) return 0;
   uint32_t cap = n < 1024 ? 1024 : n;
   cudaFree(s.g_keys); cudaFree(s.g_keys_tmp); cudaFree(s.g_items); cudaFree(s.g_items_tmp);
-  cudaFree(s.g_cell_of); cudaFree(s.g_start); cudaFree(s.g_hist); cudaFree(s.g_part);
+  cudaFree(s.g_cell_of); cudaFree(s.g_start); cudaFree(s.g_hist);
   D3_CUDA_OK(cudaMalloc(&s.g_keys, cap * 8ull));
   D3_CUDA_OK(cudaMalloc(&s.g_keys_tmp, cap * 8ull));
   D3_CUDA_OK(cudaMalloc(&s.g_items, cap * 4ull));
@@ -35,7 +35,6 @@ int fast_reserve(FastScratch &s, uint32_t n) {
   D3_CUDA_OK(cudaMalloc(&s.g_cell_of, cap * 4ull));
   D3_CUDA_OK(cudaMalloc(&s.g_start, (4ull * cap + 24) * 4));
   D3_CUDA_OK(cudaMalloc(&s.g_hist, sort_hist_words(cap) * 4));
-  D3_CUDA_OK(cudaMalloc(&s.g_part, scan_partial_words(sort_hist_words(cap)) * 4));
   s.cap = cap;
   return 0;
 }
@@ -45,7 +44,7 @@ void fmm_free(FastScratch &s);
 void fast_free(FastScratch &s) {
   cudaFree(s.seed); cudaFree(s.g_keys); cudaFree(s.g_keys_tmp); cudaFree(s.g_items);
   cudaFree(s.g_items_tmp); cudaFree(s.g_cell_of); cudaFree(s.g_start); cudaFree(s.g_hist);
-  cudaFree(s.g_part); cudaFree(s.g_box); cudaFree(s.g_info); cudaFree(s.g_geom);
+  cudaFree(s.g_box); cudaFree(s.g_info); cudaFree(s.g_geom);
   fmm_free(s);
   fmm_tc_free(s);
   s = FastScratch();
@@ -380,7 +379,7 @@ void fast_collide(FastScratch &s, const NodeArrays &a, const double *radii, doub
   if (n == 0) return;
   unsigned gb = blocks_for(n, GRID_THREADS * 4);
   if (gb > GRID_BLOCKS_MAX) gb = GRID_BLOCKS_MAX;
-  SortScratch ss{s.g_keys_tmp, s.g_items_tmp, s.g_hist, s.g_part};
+  SortScratch ss{s.g_keys_tmp, s.g_items_tmp, s.g_hist};
   for (double k = 0; k < iterations; k += 1) {
     D3_LAUNCH(k_grid_bounds, gb, GRID_THREADS, 0, st)(a.x, a.y, a.vx, a.vy, a.px, a.py, radii, n, s.g_box,
                                                 s.g_info, s.g_geom);

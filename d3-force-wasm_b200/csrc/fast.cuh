@@ -16,7 +16,7 @@ struct FastScratch {
   // grid collide
   uint64_t *g_keys = nullptr, *g_keys_tmp = nullptr;
   uint32_t *g_items = nullptr, *g_items_tmp = nullptr, *g_cell_of = nullptr, *g_start = nullptr;
-  uint32_t *g_hist = nullptr, *g_part = nullptr;
+  uint32_t *g_hist = nullptr;
   double *g_box = nullptr;      // per-block partial bounds
   uint32_t *g_info = nullptr;   // grid geometry: gx, gy, cells, m, active, ticket
   double *g_geom = nullptr;     // x0, y0, inv_h

@@ -1123,7 +1123,7 @@ int fmm_prepare(FastScratch &s, TreeDev &t, const NodeArrays &a, const double *s
   // keys: square extent, quantised Morton keys, stable sort (NaN nodes last)
   fast_box(t, a.x, a.y, n, f.square, st);
   D3_LAUNCH(k_fmm_keys, blocks_for(n, 256), 256, 0, st)(a.x, a.y, n, f.square, t.keys, t.sv);
-  SortScratch ss{t.keys_tmp, t.sv_tmp, t.hist, t.scan_part};
+  SortScratch ss{t.keys_tmp, t.sv_tmp, t.hist};
   radix_sort_u64(t.keys, t.sv, n, 0, 4, true, ss, st);
   // the geometry, the point count and the gather stay on the device: the
   // host reads them with the cell counts, in one synchronisation

@@ -44,7 +44,6 @@ constexpr size_t NA_SIZES[] = {
     (size_t)NA_CELLS, 64ull * NA_CELLS,           // pnch, rec
     4ull * NA_CAP,                                // leaf_of
     NA_BOX_BYTES,                                 // box partials
-    4 * na_scan_words(na_hist_words > NA_CAP + 1 ? na_hist_words : NA_CAP + 1),  // tree scan
     4 * na_hist_words,                            // hist
     4 * sizeof(double), 16 * sizeof(uint32_t),    // extent, info
     4ull * (NA_CAP + 1), 4ull * (NA_CAP + 1),     // draws, offsets
@@ -153,7 +152,6 @@ extern "C" int32_t d3_many_body_exact_noalloc(const double *x, const double *y, 
   t.rec = c.take<unsigned char>();
   t.leaf_of = c.take<uint32_t>();
   t.box_part = c.take<uint32_t>();
-  t.scan_part = c.take<uint32_t>();
   t.hist = c.take<uint32_t>();
   t.extent = c.take<double>();
   t.info = c.take<uint32_t>();

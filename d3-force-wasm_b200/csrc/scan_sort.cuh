@@ -2,9 +2,10 @@
 //
 // The sort is the reference's algorithm (sort.zig:55-91: stable LSD radix,
 // 8-bit digits, per-chunk histograms turned into offsets that keep equal
-// digits in input order) laid out for the GPU: one tile of TILE keys per CTA,
-// a digit-major histogram (digit * tiles + tile) so one exclusive scan yields
-// every tile's base per digit, and a stable in-tile ranking with warp match.
+// digits in input order) laid out for the GPU: the counts of all passes first,
+// then one launch a pass, a tile of SORT_TILE keys per CTA with a stable in-tile
+// ranking by warp match; a tile gets its place in each digit's run from the
+// counts the tiles before it publish.
 #pragma once
 
 #include <cooperative_groups.h>
@@ -93,16 +94,17 @@ void scan_u32(const uint32_t *in, uint32_t *out, uint32_t n, uint32_t *partials,
 constexpr unsigned SORT_TILE = 2048;
 constexpr unsigned SORT_THREADS = 256;
 
-// Stable sort of (keys, vals)[0..n) by key bytes [byte_lo, byte_hi), then (if
-// `partition_hi_bit`) a stable partition on bit 31 of the value, zeros first
-// (folded into the last byte pass as a 9-bit digit). Results end in
-// keys/vals. Scratch: keys_tmp, vals_tmp (n each) and hist of at least
-// 512 * tiles + 1 words plus scan partials.
+constexpr int SORT_PASSES = 4;  // key bytes a sort may take
+
+// Stable sort of (keys, vals)[0..n), n < 2^30, by at most SORT_PASSES key
+// bytes [byte_lo, byte_hi), then (if `partition_hi_bit`) a stable partition on
+// bit 31 of the value, zeros first (folded into the last byte pass as a 9-bit
+// digit). Results end in keys/vals. Scratch: keys_tmp, vals_tmp (n each) and
+// hist of sort_hist_words(n).
 struct SortScratch {
   uint64_t *keys_tmp;
   uint32_t *vals_tmp;
-  uint32_t *hist;      // 512 * tiles
-  uint32_t *partials;  // scan partials
+  uint32_t *hist;
 };
 void radix_sort_u64(uint64_t *keys, uint32_t *vals, uint32_t n, int byte_lo, int byte_hi,
                     bool partition_hi_bit, const SortScratch &s, cudaStream_t st);
@@ -110,7 +112,7 @@ void radix_sort_u64(uint64_t *keys, uint32_t *vals, uint32_t n, int byte_lo, int
 inline size_t sort_hist_words(uint32_t n) {
   size_t tiles = (n + SORT_TILE - 1) / SORT_TILE;
   if (!tiles) tiles = 1;
-  return 512 * tiles + 1;
+  return SORT_PASSES * (513 + 512 * tiles) + 1;
 }
 inline size_t scan_partial_words(size_t n) { return blocks_for(n, SCAN_BLOCK * 4) + 2; }
 

@@ -1097,7 +1097,7 @@ int tree_reserve(TreeDev &t, uint32_t n) {
   cudaFree(t.keys); cudaFree(t.keys_tmp); cudaFree(t.sv); cudaFree(t.sv_tmp); cudaFree(t.perm);
   cudaFree(t.perm_tmp); cudaFree(t.lcpx); cudaFree(t.cnt); cudaFree(t.base); cudaFree(t.run_end);
   cudaFree(t.leafd); cudaFree(t.frames); cudaFree(t.cells); cudaFree(t.skip); cudaFree(t.parent);
-  cudaFree(t.counter); cudaFree(t.scan_part); cudaFree(t.hist); cudaFree(t.leaf_of);
+  cudaFree(t.counter); cudaFree(t.hist); cudaFree(t.leaf_of);
   cudaFree(t.pnch); cudaFree(t.rec);
   size_t cells = 4 * (size_t)cap + 1024;
   D3_CUDA_OK(cudaMalloc(&t.keys, cap * 8ull));
@@ -1119,8 +1119,6 @@ int tree_reserve(TreeDev &t, uint32_t n) {
   D3_CUDA_OK(cudaMalloc(&t.pnch, cells));
   D3_CUDA_OK(cudaMalloc(&t.rec, cells * 64));
   D3_CUDA_OK(cudaMalloc(&t.leaf_of, cap * 4ull));
-  size_t sp = scan_partial_words(sort_hist_words(cap) > cap + 1 ? sort_hist_words(cap) : cap + 1);
-  D3_CUDA_OK(cudaMalloc(&t.scan_part, sp * 4));
   D3_CUDA_OK(cudaMalloc(&t.hist, tree_hist_words(cap) * 4));
   t.cap = cap;
   t.cells_cap = (uint32_t)cells;
@@ -1131,7 +1129,7 @@ void tree_free(TreeDev &t) {
   cudaFree(t.keys); cudaFree(t.keys_tmp); cudaFree(t.sv); cudaFree(t.sv_tmp); cudaFree(t.perm);
   cudaFree(t.perm_tmp); cudaFree(t.lcpx); cudaFree(t.cnt); cudaFree(t.base); cudaFree(t.run_end);
   cudaFree(t.leafd); cudaFree(t.frames); cudaFree(t.cells); cudaFree(t.skip); cudaFree(t.parent);
-  cudaFree(t.counter); cudaFree(t.scan_part); cudaFree(t.hist); cudaFree(t.info);
+  cudaFree(t.counter); cudaFree(t.hist); cudaFree(t.info);
   cudaFree(t.leaf_of); cudaFree(t.pnch); cudaFree(t.rec);
   cudaFree(t.extent); cudaFree(t.box_part); cudaFree(t.stamps);
   t = TreeDev();

@@ -33,7 +33,6 @@ struct TreeDev {
   void *rec = nullptr;           // per cell: the current traversal's 64-byte record
   uint32_t *leaf_of = nullptr;   // per node: the leaf cell holding it (NONE: NaN coordinate)
   uint32_t *box_part = nullptr;  // per-block bbox partials
-  uint32_t *scan_part = nullptr;
   uint32_t *hist = nullptr;
   double *extent = nullptr;      // 4
   uint32_t *info = nullptr;      // 0 m, 1 cells, 2 depth, 3 root, 4 ticket, 5 overflow
