@@ -66,7 +66,7 @@ struct FmmParams {
 
 // fmm.zig:68-78 (a cell of the fast tree, level order, children contiguous),
 // with the parent index in the spare word.
-struct FCell {
+struct alignas(16) FCell {
   double cx, cy, r;
   uint32_t first, count, child0, nchild, depth, parent;
 };
@@ -83,7 +83,6 @@ struct FmmPrep {
   const double *px = nullptr, *py = nullptr, *ps = nullptr, *ux = nullptr, *uy = nullptr;
   FCell *cells = nullptr;
   uint32_t *info = nullptr;  // device: FI_LVL + d = first cell of level d
-  int coop_blocks = 0;
 };
 
 // The fast tree of fmm.zig:247-330 up to the cells: square extent, 16-bit

@@ -11,30 +11,26 @@
 //           depth 16, children contiguous (fmm.zig:685-717); all levels at
 //           once from each point's shared digits (four launches, no level
 //           barriers).
-//  upward   per level from the deepest: bounding box, centre and radius
-//           (fmm.zig:721-754), P2M at leaves and M2M from the children
-//           (fmm.zig:757-806), then M_k /= k! (fmm.zig:629-642).
-//  lists    the recursion's calls, expanded level by level. A call (A, B)
+//  upward   from the leaves: bounding box, centre and radius (fmm.zig:721-754),
+//           P2M at leaves and M2M from the children (fmm.zig:757-806), then
+//           M_k /= k! (fmm.zig:629-642).
+//  lists    the recursion's calls, each cell's after its parent's. A call (A, B)
 //           either ends (M2L of B into A, P2P of B into A's points, or nothing
 //           past distanceMax), or splits B (the calls (A, B_j) follow at once,
 //           in order), or splits A (the call goes to every child of A). So
 //           every child of A receives the same ordered list of B's — the
 //           "forward" list of A — and each cell's M2L and P2P lists come out
 //           in the order the serial recursion meets them.
-//  m2l      per cell, its M2L sources in list order: one lane per (source,
-//           l) computes the two-lane correlation of fmm.zig:561-610, then one
+//  m2l      per cell, its M2L sources in list order: a lane per (source, three
+//           l) computes the two-lane correlation of fmm.zig:561-610, then a
 //           lane per coefficient adds the sources in order; L_l is unscaled by
 //           (-1)^l / l! (fmm.zig:645-657).
-//  p2p      per leaf, one lane per target point runs fmm.zig:477-553 against
-//           each source leaf of its list in order.
-//  downward per level from the root: L2L into the children
-//           (fmm.zig:823-849), L2P at leaves (fmm.zig:853-886).
-#include <cooperative_groups.h>
-
+//  p2p      per leaf, one to four lanes per target point run fmm.zig:477-553
+//           against each source leaf of its list in order.
+//  downward per cell with leaf children: L2L along its path from the root and
+//           into the children (fmm.zig:823-849), L2P there (fmm.zig:853-886).
 #include "fast.cuh"
 #include "scan_sort.cuh"
-
-namespace cg = cooperative_groups;
 
 namespace d3 {
 
@@ -45,21 +41,23 @@ constexpr uint32_t FMM_LEAF = 32;
 constexpr uint32_t FMM_LEVELS = 16;
 constexpr double FMM_MIN_SEP2 = 1e-28;
 constexpr uint32_t FMM_TAB = 2 * FMM_MAX_ORDER + 2;  // rows of the binomial table
-constexpr unsigned FMM_THREADS = 256;
-constexpr unsigned FMM_WARPS = FMM_THREADS / 32;
+constexpr unsigned LISTS_THREADS = 128;
+constexpr unsigned UP_THREADS = 64, M2L_THREADS = 32, P2P_THREADS = 32, DOWN_THREADS = 64;
+constexpr uint32_t P2P_FEW_CELLS = 4096;  // some 30,000 nodes; measured at k_fmm_p2p
 constexpr uint32_t FMM_STACK = 64;
 
 
 struct FmmTables {
   double fact[FMM_TAB];
+  double ifact[FMM_TAB];            // 1 / fact
   double binom[FMM_TAB * FMM_TAB];  // binom[n * FMM_TAB + k]
 };
 
 // info words (device, mirrored to the host after the cell build)
-// (FI_LIST_OVERFLOW + level parity: a level's overflow is read at the start of
-// the next level, while that level writes the other word.)
 enum : uint32_t { FI_CELLS = 0, FI_OVERFLOW, FI_LEVELS, FI_POOL_M2L, FI_POOL_P2P, FI_POOL_FWD,
-                  FI_LIST_OVERFLOW, FI_LVL = 8,  // FI_LVL + d: first cell of level d
+                  FI_LIST_OVERFLOW,              // 1: a pool, 2: a call stack or a wait
+                  FI_TICKET,                     // k_fmm_lists' blocks so far
+                  FI_LVL = 8,  // FI_LVL + d: first cell of level d
                   FI_M = 40,                     // points to act on (0 when the extent is bad)
                   FI_BAD = 41 };                 // 1: the extent is not finite and positive
 
@@ -75,12 +73,12 @@ struct FmmDev {
   double *mco = nullptr, *lco = nullptr;
   FmmTables *tab = nullptr;
   uint32_t tab_p = 0;
-  uint32_t *info = nullptr, *bsum = nullptr;
+  uint32_t *info = nullptr, *arrive = nullptr;
+  cudaEvent_t lists_read = nullptr;  // the lists' words are in h_info
   double *square = nullptr;      // box x0, y0, side
   uint32_t *h_info = nullptr;    // pinned mirror of info
   double *h_geom = nullptr;      // pinned: the geometry read back (w, 1 / w, ox, oy)
   double *geom = nullptr;        // device: w, 1 / w, ox, oy (k_fmm_geom)
-  int coop_blocks = 0;
   size_t last_m2l = 0, last_p2p = 0, last_fwd = 0;  // list sizes of the previous run
   // the cell build: per-block counts per level, each cell's start and level
   uint32_t *cb_count = nullptr, *start_of = nullptr;
@@ -100,9 +98,9 @@ struct FmmArgs {
   double *vx, *vy;
   uint32_t *m2l, *p2p, *fwd;
   uint32_t *m2l_off, *m2l_cnt, *p2p_off, *p2p_cnt, *fwd_off, *fwd_cnt;
-  uint32_t *info;
+  uint32_t *info, *arrive;
   size_t cap_m2l, cap_p2p, cap_fwd;
-  uint32_t ncells, nlev, p, q, stride;
+  uint32_t ncells, p;
   double mac_far, dmax_scaled, dmin_scaled, dmin2, dmax2, inv_w;
   int ring, has_dmax;
   const double *seed;
@@ -412,7 +410,8 @@ __global__ void __launch_bounds__(CB_THREADS) k_cells_place(const uint16_t *leve
 __global__ void __launch_bounds__(CB_THREADS) k_cells_fill(const uint64_t *keys,
                                                            const uint32_t *start_of,
                                                            const uint8_t *level_of,
-                                                           const uint32_t *info, FCell *cells) {
+                                                           const uint32_t *info, FCell *cells,
+                                                           uint32_t *arrive, uint32_t *fwd_cnt) {
   const uint32_t m = info[FI_M];
   const uint32_t total = __ldcg(&info[FI_CELLS]);
   if (__ldcg(&info[FI_OVERFLOW])) return;
@@ -460,6 +459,8 @@ __global__ void __launch_bounds__(CB_THREADS) k_cells_fill(const uint64_t *keys,
     f.parent = a - 1;
   }
   cells[c] = f;
+  arrive[c] = 0;       // children k_fmm_upward has finished
+  fwd_cnt[c] = NONE;   // k_fmm_lists' forward list is not there yet
 }
 
 // ---- upward: geometry, P2M, M2M, scale ------------------------------------------
@@ -488,14 +489,46 @@ __device__ inline void minmax_merge(double &mn, uint32_t &imn, double &mx, uint3
   if (omx > mx || (omx == mx && oimx < imx)) { mx = omx; imx = oimx; }
 }
 
-// One cell, by one warp. ws: this warp's shared scratch (32 * stride doubles).
-__device__ void upward_cell(const FmmArgs &a, uint32_t c, double *ws) {
-  const unsigned lane = threadIdx.x & 31;
-  const uint32_t p = a.p, q = a.q, stride = a.stride;
-  const uint32_t first = a.cells[c].first, count = a.cells[c].count;
-  const uint32_t nchild = ldg_cg(&a.cells[c].nchild), child0 = ldg_cg(&a.cells[c].child0);
-  double x0, y0, x1, y1;
-  if (nchild == 0) {
+__device__ inline void write_box(const FmmArgs &a, uint32_t c, double x0, double y0, double x1,
+                                 double y1, double cx, double cy) {
+  a.bx0[c] = x0; a.by0[c] = y0; a.bx1[c] = x1; a.by1[c] = y1;
+  const double dx = x1 - x0, dy = y1 - y0;
+  a.cells[c].cx = cx;
+  a.cells[c].cy = cy;
+  a.cells[c].r = 0.5 * sqrt(dx * dx + dy * dy);
+}
+
+// Real r of cell c's multipole; the root's, which no parent reads, scaled.
+__device__ inline void store_sums(const FmmArgs &a, uint32_t c, uint32_t q, uint32_t r, double v) {
+  if (r >= 2 * q) return;
+  const uint32_t o = r % q;
+  a.mco[(size_t)c * 2 * q + r] = c == 0 && o >= 2 ? v * a.tab->ifact[o] : v;
+}
+
+// Shared doubles a warp of k_fmm_upward needs: 32 rows of a point's terms (odd
+// rows: no bank conflicts), more than four children's coefficients, powers and
+// sums take.
+__host__ __device__ constexpr uint32_t up_row(uint32_t stride) { return stride | 1; }
+
+// A warp per leaf: box, centre and P2M. The warp that finishes a cell's last
+// child (`arrive` counts them) goes on with the cell: box from the children's,
+// M2M with a lane per (child, coefficient), up to the root. A plain launch, and
+// a chain of one or two microseconds a level: with a grid barrier a level, the
+// children one after another and the coefficients read from L2 inside the sums
+// it was a chain of 16 us a level (6,000 nodes: 98 -> 31 us; 1 M: 358 ->
+// 193 us). A parent is the last reader of its children's sums, so it also
+// scales them (fmm.zig:629-642: M_k /= k!); no pass of its own. P fixes the
+// order at compile time (0: the order of the arguments) so that the sums unroll.
+template <uint32_t P>
+__global__ void __launch_bounds__(UP_THREADS) k_fmm_upward(FmmArgs a) {
+  extern __shared__ double fmm_smem[];
+  const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t p = P ? P : a.p, q = p + 1, stride = 2 * q, row = up_row(stride);
+  double *ws = fmm_smem + warp * 32 * row;
+  uint32_t c = blockIdx.x * (UP_THREADS / 32) + warp;
+  if (c >= a.ncells || a.cells[c].nchild) return;
+  {
+    const uint32_t first = a.cells[c].first, count = a.cells[c].count;
     double mnx = INFINITY, mxx = -INFINITY, mny = INFINITY, mxy = -INFINITY;
     uint32_t imnx = NONE, imxx = NONE, imny = NONE, imxy = NONE;
     for (uint32_t k = first + lane; k < first + count; k += 32) {
@@ -513,26 +546,8 @@ __device__ void upward_cell(const FmmArgs &a, uint32_t c, double *ws) {
       minmax_merge(mnx, imnx, mxx, imxx, a0, i0, a1, i1);
       minmax_merge(mny, imny, mxy, imxy, b0, j0, b1, j1);
     }
-    x0 = mnx; x1 = mxx; y0 = mny; y1 = mxy;
-  } else {
-    x0 = INFINITY; y0 = INFINITY; x1 = -INFINITY; y1 = -INFINITY;
-    for (uint32_t ch = child0; ch < child0 + nchild; ++ch) {
-      x0 = zmin(x0, ldg_cg(&a.bx0[ch]));
-      x1 = zmax(x1, ldg_cg(&a.bx1[ch]));
-      y0 = zmin(y0, ldg_cg(&a.by0[ch]));
-      y1 = zmax(y1, ldg_cg(&a.by1[ch]));
-    }
-  }
-  const double cx = (x0 + x1) / 2, cy = (y0 + y1) / 2;
-  if (lane == 0) {
-    a.bx0[c] = x0; a.by0[c] = y0; a.bx1[c] = x1; a.by1[c] = y1;
-    const double dx = x1 - x0, dy = y1 - y0;
-    a.cells[c].cx = cx;
-    a.cells[c].cy = cy;
-    a.cells[c].r = 0.5 * sqrt(dx * dx + dy * dy);
-  }
-  double *mco = a.mco + (size_t)c * stride;
-  if (nchild == 0) {
+    const double cx = (mnx + mxx) / 2, cy = (mny + mxy) / 2;
+    if (lane == 0) write_box(a, c, mnx, mny, mxx, mxy, cx, cy);
     // P2M (fmm.zig:757-780): lane t holds point t's terms; then lane r adds
     // real r (re 0..q-1, im q..2q-1) over the points in order.
     double acc0 = 0, acc1 = 0;
@@ -540,87 +555,107 @@ __device__ void upward_cell(const FmmArgs &a, uint32_t c, double *ws) {
     for (uint32_t base = first; base < first + count; base += 32) {
       const uint32_t k = base + lane;
       const uint32_t np = min(32u, first + count - base);
-      double *row = ws + lane * stride;
+      double *rt = ws + lane * row;
       if (k < first + count) {
         const double sv = a.ps[k];
         if (sv != sv) {
-          row[0] = NAN;  // skipped point
+          rt[0] = NAN;  // skipped point
         } else {
           const double zre = a.ux[k] - cx, zim = a.uy[k] - cy;
           double pre = 1, pim = 0;
-          row[0] = sv;
-          row[q] = 0;
+          rt[0] = sv;
+          rt[q] = 0;
+#pragma unroll 8
           for (uint32_t o = 1; o < q; ++o) {
             const double nre = pre * zre - pim * zim;
             const double nim = pre * zim + pim * zre;
             pre = nre;
             pim = nim;
-            row[o] = sv * pre;
-            row[q + o] = sv * pim;
+            rt[o] = sv * pre;
+            rt[q + o] = sv * pim;
           }
         }
       }
       __syncwarp();
+#pragma unroll 4
       for (uint32_t t = 0; t < np; ++t) {
-        const double *rt = ws + t * stride;
-        const double sv = rt[0];
+        const double *ot = ws + t * row;
+        const double sv = ot[0];
         if (sv != sv) continue;
-        if (r0 < stride && r0 != q) acc0 += rt[r0];
-        if (r1 < stride && r1 != q) acc1 += rt[r1];
+        if (r0 < stride && r0 != q) acc0 += ot[r0];
+        if (r1 < stride && r1 != q) acc1 += ot[r1];
       }
       __syncwarp();
     }
-    if (r0 < stride) mco[r0] = acc0;
-    if (r1 < stride) mco[r1] = acc1;
-  } else {
-    // M2M (fmm.zig:782-806): lane nn sums the children in order.
-    double sre_acc = 0, sim_acc = 0;
-    const uint32_t nn = lane;
-    for (uint32_t ch = child0; ch < child0 + nchild; ++ch) {
-      if (lane == 0) shift_powers(ldg_cg(&a.cells[ch].cx) - cx, ldg_cg(&a.cells[ch].cy) - cy, p, ws);
-      __syncwarp();
-      if (nn < q) {
-        const double *cre = a.mco + (size_t)ch * stride, *cim = cre + q;
-        double sre = 0, sim = 0;
-        for (uint32_t k = 0; k <= nn; ++k) {
-          const double b = a.tab->binom[nn * FMM_TAB + k];
-          const double xre = ldg_cg(&cre[k]) * b, xim = ldg_cg(&cim[k]) * b;
-          sre += xre * ws[nn - k] - xim * ws[q + nn - k];
-          sim += xre * ws[q + nn - k] + xim * ws[nn - k];
-        }
-        sre_acc += sre;
-        sim_acc += sim;
+    store_sums(a, c, q, r0, acc0);
+    store_sums(a, c, q, r1, acc1);
+  }
+  const uint32_t S = 32 / q, nn = lane % q;
+  double bn[P + 1];  // the lane's row of the binomials, on its way during the first wait
+  if (P) {
+#pragma unroll
+    for (uint32_t k = 0; k <= P; ++k) bn[k] = a.tab->binom[nn * FMM_TAB + k];
+  }
+  while (c != 0) {
+    const uint32_t parent = a.cells[c].parent;
+    const uint32_t nchild = a.cells[parent].nchild, child0 = a.cells[parent].child0;
+    __threadfence();
+    __syncwarp();
+    uint32_t before = 0;
+    if (lane == 0) before = atomicAdd(&a.arrive[parent], 1u);
+    if (__shfl_sync(0xffffffffu, before, 0) + 1 != nchild) return;
+    __threadfence();
+    c = parent;
+    // the box: lane j holds child j's
+    double b0 = 0, b1 = 0, b2 = 0, b3 = 0, ccx = 0, ccy = 0;
+    if (lane < nchild) {
+      const uint32_t ch = child0 + lane;
+      b0 = ldg_cg(&a.bx0[ch]); b1 = ldg_cg(&a.by0[ch]);
+      b2 = ldg_cg(&a.bx1[ch]); b3 = ldg_cg(&a.by1[ch]);
+      ccx = ldg_cg(&a.cells[ch].cx); ccy = ldg_cg(&a.cells[ch].cy);
+    }
+    double *Ms = ws, *pw = ws + 4 * stride, *Cs = ws + 8 * stride;
+    for (uint32_t idx = lane; idx < nchild * stride; idx += 32) {
+      double *m = a.mco + (size_t)child0 * stride + idx;
+      const uint32_t o = idx % q;  // stride is 2 q
+      const double v = ldg_cg(m);
+      Ms[idx] = v;
+      if (o >= 2) *m = v * a.tab->ifact[o];
+    }
+    double x0 = INFINITY, y0 = INFINITY, x1 = -INFINITY, y1 = -INFINITY;
+    for (uint32_t j = 0; j < nchild; ++j) {
+      x0 = zmin(x0, __shfl_sync(0xffffffffu, b0, j));
+      y0 = zmin(y0, __shfl_sync(0xffffffffu, b1, j));
+      x1 = zmax(x1, __shfl_sync(0xffffffffu, b2, j));
+      y1 = zmax(y1, __shfl_sync(0xffffffffu, b3, j));
+    }
+    const double cx = (x0 + x1) / 2, cy = (y0 + y1) / 2;
+    if (lane == 0) write_box(a, c, x0, y0, x1, y1, cx, cy);
+    if (lane < nchild) shift_powers(ccx - cx, ccy - cy, p, pw + lane * stride);
+    __syncwarp();
+    // M2M (fmm.zig:782-806): lane (child, nn) its sum over k, then lane r the
+    // children in order
+    for (uint32_t j = lane / q; j < nchild && lane < S * q; j += S) {
+      const double *cre = Ms + j * stride, *cim = cre + q, *w = pw + j * stride;
+      double sre = 0, sim = 0;
+#pragma unroll
+      for (uint32_t k = 0; k < (P ? P + 1 : nn + 1); ++k) {
+        if (k > nn) continue;
+        const double b = P ? bn[P ? k : 0] : a.tab->binom[nn * FMM_TAB + k];
+        const double xre = cre[k] * b, xim = cim[k] * b;
+        sre += xre * w[nn - k] - xim * w[q + nn - k];
+        sim += xre * w[q + nn - k] + xim * w[nn - k];
       }
-      __syncwarp();
+      Cs[j * stride + nn] = sre;
+      Cs[j * stride + q + nn] = sim;
     }
-    if (nn < q) {
-      mco[nn] = sre_acc;
-      mco[q + nn] = sim_acc;
+    __syncwarp();
+    for (uint32_t r = lane; r < stride; r += 32) {
+      double acc = 0;
+      for (uint32_t j = 0; j < nchild; ++j) acc += Cs[j * stride + r];
+      store_sums(a, c, q, r, acc);
     }
-  }
-}
-
-__global__ void __launch_bounds__(FMM_THREADS) k_fmm_upward(FmmArgs a) {
-  extern __shared__ double fmm_smem[];
-  cg::grid_group g = cg::this_grid();
-  const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-  double *ws = fmm_smem + (threadIdx.x >> 5) * 32 * a.stride;
-  const uint32_t *lvl = a.info + FI_LVL;
-  for (int lev = (int)a.nlev - 1; lev >= 0; --lev) {
-    for (uint32_t c = lvl[lev] + gw; c < lvl[lev + 1]; c += nwarps) upward_cell(a, c, ws);
-    g.sync();
-  }
-  // fmm.zig:629-642: M_k /= k! for k >= 2
-  const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
-  const size_t total = (size_t)a.ncells * a.q;
-  for (size_t idx = tid; idx < total; idx += nth) {
-    const uint32_t c = (uint32_t)(idx / a.q), o = (uint32_t)(idx % a.q);
-    if (o < 2) continue;
-    double *m = a.mco + (size_t)c * a.stride;
-    const double inv = 1 / a.tab->fact[o];
-    m[o] = ldg_cg(&m[o]) * inv;
-    m[a.q + o] = ldg_cg(&m[a.q + o]) * inv;
+    __syncwarp();
   }
 }
 
@@ -685,6 +720,20 @@ __device__ bool expand_call(const FmmArgs &a, uint32_t c, const FCell &A, uint32
   return true;
 }
 
+__device__ inline unsigned long long fmm_timer_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+__device__ inline uint32_t ld_acquire(const uint32_t *p) {
+  uint32_t v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ inline void st_release(uint32_t *p, uint32_t v) {
+  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
 __device__ inline uint32_t warp_excl(uint32_t v, uint32_t &total) {
   const unsigned lane = threadIdx.x & 31;
   uint32_t incl = v;
@@ -696,26 +745,95 @@ __device__ inline uint32_t warp_excl(uint32_t v, uint32_t &total) {
   return incl - v;
 }
 
-// The calls of cell c (its parent's forward list in order, or (root, root)),
-// by one warp: lane k expands calls k, k + 32, ...; each call's events are
-// placed after those of the calls before it (a warp scan of the counts).
-// Counts, then a reservation in the pools, then counts again and the writes.
-__device__ void warp_expand_cell(const FmmArgs &a, uint32_t c, uint32_t *ovf) {
-  const unsigned lane = threadIdx.x & 31;
-  const FCell A = a.cells[c];
-  const uint32_t *in = nullptr;
-  uint32_t nin = 1;
-  if (c != 0) {
-    in = a.fwd + ldg_cg(&a.fwd_off[A.parent]);
-    nin = ldg_cg(&a.fwd_cnt[A.parent]);
+// A cell in three 16-byte loads.
+__device__ inline FCell load_cell(const FCell *p) {
+  union {
+    uint4 w[3];
+    FCell c;
+  } u;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) u.w[i] = reinterpret_cast<const uint4 *>(p)[i];
+  return u.c;
+}
+
+// What cell c's call with B comes to: an event, B's children in its place
+// (n of them from v), or nothing. The decision of expand_call above.
+constexpr uint32_t EV_CALL = 0, EV_M2L = 1u << 30, EV_P2P = 2u << 30, EV_FWD = 3u << 30;
+constexpr uint32_t EV_CELL = EV_M2L - 1;
+
+__device__ inline uint32_t decide_call(const FmmArgs &a, uint32_t c, const FCell &A, uint32_t B,
+                                       uint32_t &v) {
+  const bool la = A.nchild == 0;
+  if (B == c) {
+    v = la ? c | EV_P2P : A.child0 | EV_FWD;
+    return la ? 1 : A.nchild;
   }
+  const FCell Bc = load_cell(a.cells + B);
+  const double ra = A.r, rb = Bc.r;
+  const double dx = A.cx - Bc.cx, dy = A.cy - Bc.cy;
+  const double d2 = dx * dx + dy * dy;
+  const double rmax = zmax(ra, rb), rmin = zmin(ra, rb);
+  const double thr = a.mac_far * rmax + rmin;
+  if (d2 > FMM_MIN_SEP2 && d2 >= thr * thr) {
+    bool separated = true;
+    if (a.ring) {
+      const double gap = sqrt(d2) - ra - rb;
+      if (gap >= a.dmax_scaled) return 0;
+      if (gap + 2 * (ra + rb) > a.dmax_scaled || gap < a.dmin_scaled) separated = false;
+    }
+    if (separated) {
+      v = B | EV_M2L;
+      return 1;
+    }
+  }
+  const bool lb = Bc.nchild == 0;
+  if (la && lb) {
+    v = B | EV_P2P;
+    return 1;
+  }
+  if (la || (!lb && rb > ra)) {
+    v = Bc.child0;
+    return Bc.nchild;
+  }
+  v = B | EV_FWD;
+  return 1;
+}
+
+// Reserves cell c's places in the pools; false if they do not fit.
+__device__ bool reserve_lists(const FmmArgs &a, uint32_t c, uint32_t tm, uint32_t tp, uint32_t tf,
+                              uint32_t &om, uint32_t &op, uint32_t &of) {
+  const unsigned lane = threadIdx.x & 31;
+  uint32_t at = 0;
+  if (lane < 3) {
+    const uint32_t t = lane == 0 ? tm : lane == 1 ? tp : tf;
+    if (t) at = atomicAdd(&a.info[FI_POOL_M2L + lane], t);
+    (lane == 0 ? a.m2l_off : lane == 1 ? a.p2p_off : a.fwd_off)[c] = at;
+    if (lane < 2) (lane == 0 ? a.m2l_cnt : a.p2p_cnt)[c] = t;
+  }
+  om = __shfl_sync(0xffffffffu, at, 0);
+  op = __shfl_sync(0xffffffffu, at, 1);
+  of = __shfl_sync(0xffffffffu, at, 2);
+  if ((size_t)om + tm > a.cap_m2l || (size_t)op + tp > a.cap_p2p || (size_t)of + tf > a.cap_fwd) {
+    if (lane == 0) atomicOr(&a.info[FI_LIST_OVERFLOW], 1u);
+    return false;
+  }
+  return true;
+}
+
+// The calls of cell c (`in`, in order; null: (root, root)) by one warp, where
+// their expansion passes the shared lists: lane k expands calls k, k + 32, ...
+// depth first; each call's events are placed after those of the calls before
+// it (a warp scan of the counts). Counts, then a reservation in the pools, then
+// counts again and the writes. Returns the forward list's length.
+__device__ uint32_t expand_long(const FmmArgs &a, uint32_t c, const FCell &A, const uint32_t *in,
+                                uint32_t nin) {
+  const unsigned lane = threadIdx.x & 31;
   uint32_t tm = 0, tp = 0, tf = 0;
   bool ok = true;
   for (uint32_t u0 = 0; u0 < nin; u0 += 32) {
     const uint32_t u = u0 + lane;
     uint32_t nm = 0, np = 0, nf = 0;
-    if (u < nin && !expand_call<false>(a, c, A, c == 0 ? 0 : ldg_cg(&in[u]), nm, np, nf, 0, 0, 0))
-      ok = false;
+    if (u < nin && !expand_call<false>(a, c, A, in ? ldg_cg(&in[u]) : 0, nm, np, nf, 0, 0, 0)) ok = false;
     uint32_t t;
     warp_excl(nm, t); tm += t;
     warp_excl(np, t); tp += t;
@@ -724,28 +842,13 @@ __device__ void warp_expand_cell(const FmmArgs &a, uint32_t c, uint32_t *ovf) {
   ok = __all_sync(0xffffffffu, ok);
   if (!ok) {
     tm = tp = tf = 0;
-    if (lane == 0) atomicOr(ovf, 2u);
+    if (lane == 0) atomicOr(&a.info[FI_LIST_OVERFLOW], 2u);
   }
-  uint32_t om = 0, op = 0, of = 0;
-  if (lane == 0) {
-    om = atomicAdd(&a.info[FI_POOL_M2L], tm);
-    op = atomicAdd(&a.info[FI_POOL_P2P], tp);
-    of = atomicAdd(&a.info[FI_POOL_FWD], tf);
-    a.m2l_off[c] = om; a.m2l_cnt[c] = tm;
-    a.p2p_off[c] = op; a.p2p_cnt[c] = tp;
-    a.fwd_off[c] = of; a.fwd_cnt[c] = tf;
-  }
-  om = __shfl_sync(0xffffffffu, om, 0);
-  op = __shfl_sync(0xffffffffu, op, 0);
-  of = __shfl_sync(0xffffffffu, of, 0);
-  if (!ok) return;
-  if ((size_t)om + tm > a.cap_m2l || (size_t)op + tp > a.cap_p2p || (size_t)of + tf > a.cap_fwd) {
-    if (lane == 0) atomicOr(ovf, 1u);
-    return;
-  }
+  uint32_t om, op, of;
+  if (!reserve_lists(a, c, tm, tp, tf, om, op, of) || !ok) return 0;
   for (uint32_t u0 = 0; u0 < nin; u0 += 32) {
     const uint32_t u = u0 + lane;
-    const uint32_t b = u < nin ? (c == 0 ? 0 : ldg_cg(&in[u])) : 0;
+    const uint32_t b = u < nin && in ? ldg_cg(&in[u]) : 0;
     uint32_t nm = 0, np = 0, nf = 0;
     if (u < nin) expand_call<false>(a, c, A, b, nm, np, nf, 0, 0, 0);
     uint32_t t0, t1, t2;
@@ -758,114 +861,262 @@ __device__ void warp_expand_cell(const FmmArgs &a, uint32_t c, uint32_t *ovf) {
     op += t1;
     of += t2;
   }
+  return tf;
 }
 
-// Level by level from the root, a warp per cell; a grid barrier between
-// levels (a cell's calls are its parent's forward list).
-__global__ void __launch_bounds__(FMM_THREADS) k_fmm_lists(FmmArgs a) {
-  cg::grid_group g = cg::this_grid();
-  const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
-  const uint32_t gw = tid >> 5, nwarps = nth >> 5;
-  const uint32_t *lvl = a.info + FI_LVL;
-  for (uint32_t lev = 0; lev < a.nlev; ++lev) {
-    // the previous level's word: nobody writes it during this level, so every
-    // thread takes the same branch
-    if (lev && ldg_cg(&a.info[FI_LIST_OVERFLOW + ((lev - 1) & 1)])) break;
-    uint32_t *ovf = &a.info[FI_LIST_OVERFLOW + (lev & 1)];
-    for (uint32_t c = lvl[lev] + gw; c < lvl[lev + 1]; c += nwarps) warp_expand_cell(a, c, ovf);
-    g.sync();
+// The same in shared memory: the calls as one ordered list, and in each round
+// every call in it (a lane each) is replaced by what it comes to, until only
+// events are left. Each cell is read once, by as many lanes as there are calls;
+// the depth-first form reads it three times, in one lane's chain of dependent
+// loads a call. `buf` holds two lists of LIST_CAP words; a longer list (a leaf
+// beside a far denser region) takes the depth-first form.
+constexpr uint32_t LIST_CAP = 512;
+__device__ uint32_t expand_cell(const FmmArgs &a, uint32_t c, const FCell &A, const uint32_t *in,
+                                uint32_t nin, uint32_t *buf) {
+  const unsigned lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1;
+  if (nin > LIST_CAP) return expand_long(a, c, A, in, nin);
+  for (uint32_t u = lane; u < nin; u += 32) buf[u] = in ? ldg_cg(&in[u]) : 0;
+  __syncwarp();
+  uint32_t cnt = nin, tm = 0, tp = 0;
+  uint32_t *src = buf, *dst = buf + LIST_CAP;
+  for (bool more = true; more;) {
+    more = false;
+    tm = tp = 0;
+    uint32_t out = 0;
+    for (uint32_t w0 = 0; w0 < cnt; w0 += 32) {
+      uint32_t k = 0, v = 0;
+      if (w0 + lane < cnt) {
+        v = src[w0 + lane];
+        k = 1;
+        if (v < EV_M2L) k = decide_call(a, c, A, v, v);
+      }
+      const unsigned b0 = __ballot_sync(0xffffffffu, k & 1), b1 = __ballot_sync(0xffffffffu, k & 2),
+                     b2 = __ballot_sync(0xffffffffu, k & 4);
+      const uint32_t at = out + __popc(b0 & lt) + 2 * __popc(b1 & lt) + 4 * __popc(b2 & lt);
+      out += __popc(b0) + 2 * __popc(b1) + 4 * __popc(b2);
+      if (out > LIST_CAP) return expand_long(a, c, A, in, nin);
+      for (uint32_t j = 0; j < k; ++j) dst[at + j] = v + j;
+      const uint32_t type = v & ~EV_CELL;
+      tm += __popc(__ballot_sync(0xffffffffu, k && type == EV_M2L));
+      tp += __popc(__ballot_sync(0xffffffffu, k && type == EV_P2P));
+      if (__any_sync(0xffffffffu, k && type == EV_CALL)) more = true;
+    }
+    __syncwarp();
+    cnt = out;
+    uint32_t *t = src; src = dst; dst = t;
+  }
+  const uint32_t tf = cnt - tm - tp;
+  uint32_t om, op, of;
+  if (!reserve_lists(a, c, tm, tp, tf, om, op, of)) return 0;
+  for (uint32_t w0 = 0; w0 < cnt; w0 += 32) {
+    const uint32_t v = w0 + lane < cnt ? src[w0 + lane] : 0;
+    const uint32_t type = v & ~EV_CELL;
+    const unsigned bm = __ballot_sync(0xffffffffu, type == EV_M2L),
+                   bp = __ballot_sync(0xffffffffu, type == EV_P2P),
+                   bf = __ballot_sync(0xffffffffu, type == EV_FWD);
+    if (type == EV_M2L) a.m2l[om + __popc(bm & lt)] = v & EV_CELL;
+    if (type == EV_P2P) a.p2p[op + __popc(bp & lt)] = v & EV_CELL;
+    if (type == EV_FWD) a.fwd[of + __popc(bf & lt)] = v & EV_CELL;
+    om += __popc(bm);
+    op += __popc(bp);
+    of += __popc(bf);
+  }
+  return tf;
+}
+
+// A warp per cell, in level order (blocks numbered as they start, so a block's
+// cells wait only for cells of running blocks): a cell waits for its parent's
+// forward list (`fwd_cnt`, NONE until the list is there) and no level waits as
+// a whole. With a grid barrier a level and the depth-first form 6,000 nodes
+// took 174 us (now 37), 1 M 584 us (now 151). The wait is bounded
+// (20 ms, then the run fails).
+__global__ void __launch_bounds__(LISTS_THREADS) k_fmm_lists(FmmArgs a) {
+  __shared__ uint32_t buf[LISTS_THREADS / 32][2 * LIST_CAP];
+  __shared__ uint32_t ticket;
+  const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) ticket = atomicAdd(&a.info[FI_TICKET], 1u);
+  __syncthreads();
+  const uint32_t c = ticket * (LISTS_THREADS / 32) + warp;
+  if (c >= a.ncells) return;
+  const FCell A = load_cell(a.cells + c);
+  const uint32_t *in = nullptr;
+  uint32_t nin = 1;
+  if (c != 0) {
+    if (lane == 0) {
+      nin = ld_acquire(&a.fwd_cnt[A.parent]);
+      if (nin == NONE) {
+        const unsigned long long t0 = fmm_timer_ns();
+        while ((nin = ld_acquire(&a.fwd_cnt[A.parent])) == NONE) {
+          if (fmm_timer_ns() - t0 > 20000000ull) {
+            atomicOr(&a.info[FI_LIST_OVERFLOW], 2u);
+            nin = 0;
+            break;
+          }
+          __nanosleep(64);
+        }
+      }
+    }
+    nin = __shfl_sync(0xffffffffu, nin, 0);
+    in = a.fwd + (nin ? ldg_cg(&a.fwd_off[A.parent]) : 0);
+  }
+  const uint32_t tf = expand_cell(a, c, A, in, nin, buf[warp]);
+  if (A.nchild) {
+    __threadfence();
+    __syncwarp();
+    if (lane == 0) st_release(&a.fwd_cnt[c], tf);
   }
 }
 
 // ---- M2L (fmm.zig:561-610) and the unscale of L (fmm.zig:645-657) --------------------
 
-__global__ void __launch_bounds__(FMM_THREADS) k_fmm_m2l(FmmArgs a) {
-  extern __shared__ double fmm_smem[];
-  const unsigned lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
-  const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-  const uint32_t p = a.p, q = a.q, stride = a.stride, nt = 2 * p + 1;
-  const uint32_t S = 32 / q;  // sources per step
-  // per warp: T [S][2 nt], M [S][stride], C [S][stride]
-  double *ws = fmm_smem + wl * (size_t)S * (2 * nt + 2 * stride);
-  double *Ts = ws, *Ms = ws + S * 2 * nt, *Cs = Ms + S * stride;
-  const uint32_t s = lane / q, l = lane % q;
-  for (uint32_t c = gw; c < a.ncells; c += nwarps) {
-    const double acx = a.cells[c].cx, acy = a.cells[c].cy;
-    const uint32_t cnt = a.m2l_cnt[c], off = a.m2l_off[c];
-    double acc_re = 0, acc_im = 0;
-    for (uint32_t base = 0; base < cnt; base += S) {
-      const uint32_t ns = min(S, cnt - base);
-      if (lane < ns) {
-        const uint32_t B = a.m2l[off + base + lane];
-        const double dx = acx - a.cells[B].cx, dy = acy - a.cells[B].cy;
-        const double d2 = dx * dx + dy * dy;
-        const double ire = dx / d2, iim = -dy / d2;
-        double are = ire, aim = iim;
-        double *tr = Ts + lane * 2 * nt, *ti = tr + nt;
-        tr[0] = are;
-        ti[0] = aim;
-        for (uint32_t mm = 1; mm < nt; ++mm) {
-          const double nre = are * ire - aim * iim;
-          const double nim = are * iim + aim * ire;
-          are = nre;
-          aim = nim;
-          tr[mm] = are * a.tab->fact[mm];
-          ti[mm] = aim * a.tab->fact[mm];
-        }
+// A warp per cell. The powers T of 32 sources' offsets at a time, a lane per
+// source; then per source M2L_R of the q outputs a lane, so that a T and an M
+// read from shared memory (both as (re, im) pairs) feed M2L_R multiplications
+// and S = 32 / ceil(q / M2L_R) sources run side by side; then a lane per real
+// adds the sources in order. One output a lane and three sources at a time,
+// three lanes busy in the powers, were bound by shared-memory reads and by those
+// idle lanes: 1 M nodes 731 -> 256 us, 6,000 36 -> 10 us.
+constexpr uint32_t M2L_R = 3;
+__host__ __device__ constexpr uint32_t m2l_lanes(uint32_t q) { return (q + M2L_R - 1) / M2L_R; }
+__host__ __device__ constexpr uint32_t m2l_side(uint32_t q) { return 32 / m2l_lanes(q); }
+__host__ __device__ constexpr uint32_t m2l_chunk(uint32_t q) { return 32 / m2l_side(q) * m2l_side(q); }
+// doubles a warp: T (and a lane's reads past the last row), M, C
+__host__ __device__ constexpr uint32_t m2l_words(uint32_t q) {
+  return 2 * (m2l_chunk(q) * (2 * q - 1) + 2 * M2L_R) + 4 * m2l_side(q) * q;
+}
+
+template <uint32_t P>
+__global__ void __launch_bounds__(M2L_THREADS, 18) k_fmm_m2l(FmmArgs a) {
+  extern __shared__ __align__(16) double fmm_smem[];
+  if (a.info[FI_LIST_OVERFLOW]) return;
+  const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t p = P ? P : a.p, q = p + 1, stride = 2 * q, nt = 2 * p + 1;
+  const uint32_t G = m2l_lanes(q), S = m2l_side(q), CH = m2l_chunk(q);
+  double2 *T = reinterpret_cast<double2 *>(fmm_smem + (size_t)warp * m2l_words(q));
+  double2 *M = T + CH * nt + 2 * M2L_R;
+  double *C = reinterpret_cast<double *>(M + S * q);
+  const uint32_t s = lane / G, l0 = lane % G * M2L_R;
+  const uint32_t c = blockIdx.x * (M2L_THREADS / 32) + warp;
+  if (c >= a.ncells) return;
+  const double acx = a.cells[c].cx, acy = a.cells[c].cy;
+  const uint32_t cnt = a.m2l_cnt[c], off = a.m2l_off[c];
+  double acc0 = 0, acc1 = 0;
+  for (uint32_t base = 0; base < cnt; base += CH) {
+    const uint32_t nc = min(CH, cnt - base);
+    uint32_t B = 0;
+    if (lane < nc) {
+      B = a.m2l[off + base + lane];
+      const double dx = acx - a.cells[B].cx, dy = acy - a.cells[B].cy;
+      const double d2 = dx * dx + dy * dy;
+      const double ire = dx / d2, iim = -dy / d2;
+      double are = ire, aim = iim;
+      double2 *t = T + lane * nt;
+      t[0] = make_double2(are, aim);
+#pragma unroll
+      for (uint32_t mm = 1; mm < (P ? 2 * P + 1 : nt); ++mm) {
+        const double nre = are * ire - aim * iim;
+        const double nim = are * iim + aim * ire;
+        are = nre;
+        aim = nim;
+        const double f = a.tab->fact[mm];
+        t[mm] = make_double2(are * f, aim * f);
       }
-      for (uint32_t idx = lane; idx < ns * stride; idx += 32) {
-        const uint32_t ss = idx / stride, r = idx % stride;
-        const uint32_t B = a.m2l[off + base + ss];
-        Ms[ss * stride + r] = a.mco[(size_t)B * stride + r];
+    }
+    // a round's multipoles: real idx of S x stride a lane, the next round's
+    // (default order) loaded while this one's are multiplied
+    constexpr uint32_t LOADS = P ? (m2l_side(P + 1) * 2 * (P + 1) + 31) / 32 : 1;
+    double next[LOADS];
+    auto load = [&](uint32_t r0, uint32_t i) {
+      const uint32_t ss = (i * 32 + lane) / stride, r = (i * 32 + lane) % stride;
+      const uint32_t Bs = __shfl_sync(0xffffffffu, B, (r0 + ss) & 31);
+      return ss < S && r0 + ss < nc ? a.mco[(size_t)Bs * stride + r] : 0.0;
+    };
+    auto put = [&](uint32_t i, double v) {
+      const uint32_t ss = (i * 32 + lane) / stride, r = (i * 32 + lane) % stride;
+      if (ss < S) reinterpret_cast<double *>(M + ss * q + r % q)[r / q] = v;
+    };
+    if (P) {
+#pragma unroll
+      for (uint32_t i = 0; i < LOADS; ++i) next[i] = load(0, i);
+    }
+    for (uint32_t r0 = 0; r0 < nc; r0 += S) {
+      const uint32_t ns = min(S, nc - r0);
+      if (P) {
+#pragma unroll
+        for (uint32_t i = 0; i < LOADS; ++i) {
+          put(i, next[i]);
+          next[i] = load(r0 + S, i);
+        }
+      } else {
+        for (uint32_t i = 0; i * 32 < ns * stride; ++i) put(i, load(r0, i));
       }
       __syncwarp();
       if (s < ns) {
-        const double *tr = Ts + s * 2 * nt, *ti = tr + nt;
-        const double *mre = Ms + s * stride, *mim = mre + q;
-        double v0re = 0, v1re = 0, v0im = 0, v1im = 0;
+        const double2 *t = T + (r0 + s) * nt + l0, *m = M + s * q;
+        double vre[2][M2L_R], vim[2][M2L_R];
+        double2 w[M2L_R];
+#pragma unroll
+        for (uint32_t j = 0; j < M2L_R; ++j) {
+          vre[0][j] = vre[1][j] = vim[0][j] = vim[1][j] = 0;
+          w[j] = t[j];
+        }
         uint32_t k = 0;
-        for (; k + 2 <= q; k += 2) {
-          v0re += mre[k] * tr[l + k] - mim[k] * ti[l + k];
-          v1re += mre[k + 1] * tr[l + k + 1] - mim[k + 1] * ti[l + k + 1];
-          v0im += mre[k] * ti[l + k] + mim[k] * tr[l + k];
-          v1im += mre[k + 1] * ti[l + k + 1] + mim[k + 1] * tr[l + k + 1];
+#pragma unroll
+        for (; k + 2 <= (P ? P + 1 : q); k += 2) {
+#pragma unroll
+          for (uint32_t h = 0; h < 2; ++h) {
+            const double2 mk = m[k + h];
+#pragma unroll
+            for (uint32_t j = 0; j < M2L_R; ++j) {
+              vre[h][j] += mk.x * w[j].x - mk.y * w[j].y;
+              vim[h][j] += mk.x * w[j].y + mk.y * w[j].x;
+            }
+#pragma unroll
+            for (uint32_t j = 0; j + 1 < M2L_R; ++j) w[j] = w[j + 1];
+            w[M2L_R - 1] = t[k + h + M2L_R];
+          }
         }
-        double sre = v0re + v1re, sim = v0im + v1im;
-        if (k < q) {
-          sre += mre[k] * tr[l + k] - mim[k] * ti[l + k];
-          sim += mre[k] * ti[l + k] + mim[k] * tr[l + k];
+#pragma unroll
+        for (uint32_t j = 0; j < M2L_R; ++j) {
+          double sre = vre[0][j] + vre[1][j], sim = vim[0][j] + vim[1][j];
+          if (k < q) {
+            const double2 mk = m[k];
+            sre += mk.x * w[j].x - mk.y * w[j].y;
+            sim += mk.x * w[j].y + mk.y * w[j].x;
+          }
+          if (l0 + j < q) {
+            C[s * stride + l0 + j] = sre;
+            C[s * stride + q + l0 + j] = sim;
+          }
         }
-        Cs[s * stride + l] = sre;
-        Cs[s * stride + q + l] = sim;
       }
       __syncwarp();
-      if (lane < q) {
-        for (uint32_t t = 0; t < ns; ++t) {
-          acc_re += Cs[t * stride + lane];
-          acc_im += Cs[t * stride + q + lane];
-        }
+#pragma unroll 4
+      for (uint32_t t = 0; t < ns; ++t) {
+        if (lane < stride) acc0 += C[t * stride + lane];
+        if (lane + 32 < stride) acc1 += C[t * stride + lane + 32];
       }
       __syncwarp();
     }
-    if (lane < q) {
-      const double inv = ((lane & 1) ? -1.0 : 1.0) / a.tab->fact[lane];
-      double *L = a.lco + (size_t)c * stride;
-      L[lane] = acc_re * inv;
-      L[q + lane] = acc_im * inv;
-    }
+  }
+  double *L = a.lco + (size_t)c * stride;
+  for (uint32_t r = lane; r < stride; r += 32) {
+    const uint32_t l = r % q;
+    const double inv = ((l & 1) ? -1.0 : 1.0) / a.tab->fact[l];
+    L[r] = (r < 32 ? acc0 : acc1) * inv;
   }
 }
 
 // ---- P2P (fmm.zig:477-553) ------------------------------------------------------------
 
-__device__ inline void fmm_pair(const FmmArgs &a, uint64_t seed, uint32_t ti, uint32_t tj, double xi,
-                                double yi, double &vx, double &vy) {
-  if (tj == ti) return;
-  const double sj = a.ps[tj];
-  double x = a.px[tj] - xi, y = a.py[tj] - yi;
+// One pair's term, or false where it has none.
+__device__ inline bool pair_term(const FmmArgs &a, uint64_t seed, uint32_t ti, uint32_t tj, double sj,
+                                 double xj, double yj, double xi, double yi, double &tx, double &ty) {
+  if (tj == ti) return false;
+  double x = xj - xi, y = yj - yi;
   double l = x * x + y * y;
-  if (l >= a.dmax2) return;
+  if (l >= a.dmax2) return false;
   if (x == 0 || y == 0) {
     const uint32_t i = a.perm[ti], j = a.perm[tj];
     if (x == 0) { x = hash_jiggle(seed, i, j, 0); l += x * x; }
@@ -873,36 +1124,48 @@ __device__ inline void fmm_pair(const FmmArgs &a, uint64_t seed, uint32_t ti, ui
   }
   if (l < a.dmin2) l = sqrt(a.dmin2 * l);
   const double wj = sj / l;
-  vx += x * wj;
-  vy += y * wj;
+  tx = x * wj;
+  ty = y * wj;
+  return true;
 }
 
-// One target against sources [b0, b1), four pairs per division on two lanes
-// (lane 0: k, k + 2; lane 1: k + 1, k + 3).
-__device__ void fmm_target(const FmmArgs &a, uint64_t seed, uint32_t ti, uint32_t b0, uint32_t b1,
-                           double xi, double yi, double &vxr, double &vyr) {
-  double vx = vxr, vy = vyr;
-  double ax0 = 0, ax1 = 0, ay0 = 0, ay1 = 0;
-  uint32_t k = b0;
-  for (; k + 4 <= b1; k += 4) {
-    const double sa0 = a.ps[k], sa1 = a.ps[k + 1], sb0 = a.ps[k + 2], sb1 = a.ps[k + 3];
-    const double xa0 = a.px[k] - xi, xa1 = a.px[k + 1] - xi;
-    const double ya0 = a.py[k] - yi, ya1 = a.py[k + 1] - yi;
-    const double xb0 = a.px[k + 2] - xi, xb1 = a.px[k + 3] - xi;
-    const double yb0 = a.py[k + 2] - yi, yb1 = a.py[k + 3] - yi;
+// The points of a source leaf, up to 32 at a time, in a warp's shared memory.
+struct Sources {
+  double x[32], y[32], s[32];
+};
+
+// A target's sums within one source leaf: four pairs per division on two lanes
+// (sum 0: k, k + 2; sum 1: k + 1, k + 3), pairs that cannot go that way added to
+// the velocity one by one.
+// One thread has both sums; `b0` is the chunk's first point.
+__device__ inline void leaf_one(const FmmArgs &a, uint64_t seed, uint32_t ti, uint32_t b0, uint32_t cn,
+                                const Sources &src, double xi, double yi, double &vx, double &vy,
+                                double &ax0, double &ay0, double &ax1, double &ay1) {
+  uint32_t k = 0;
+  for (; k + 4 <= cn; k += 4) {
+    const double xa0 = src.x[k] - xi, xa1 = src.x[k + 1] - xi;
+    const double ya0 = src.y[k] - yi, ya1 = src.y[k + 1] - yi;
+    const double xb0 = src.x[k + 2] - xi, xb1 = src.x[k + 3] - xi;
+    const double yb0 = src.y[k + 2] - yi, yb1 = src.y[k + 3] - yi;
     const double la0 = xa0 * xa0 + ya0 * ya0, la1 = xa1 * xa1 + ya1 * ya1;
     const double lb0 = xb0 * xb0 + yb0 * yb0, lb1 = xb1 * xb1 + yb1 * yb1;
     const double z0 = xa0 * ya0 * xb0 * yb0, z1 = xa1 * ya1 * xb1 * yb1;
     const double mn = zmin(zmin(la0, lb0), zmin(la1, lb1));
-    if (z0 == 0 || z1 == 0 || !(mn >= a.dmin2) || (ti >= k && ti < k + 4)) {
-      for (uint32_t u = 0; u < 4; ++u) fmm_pair(a, seed, ti, k + u, xi, yi, vx, vy);
+    if (z0 == 0 || z1 == 0 || !(mn >= a.dmin2) || ti - (b0 + k) < 4) {
+#pragma unroll 1
+      for (uint32_t u = 0; u < 4; ++u) {
+        double tx, ty;
+        if (pair_term(a, seed, ti, b0 + k + u, src.s[k + u], src.x[k + u], src.y[k + u], xi, yi, tx, ty)) {
+          vx += tx;
+          vy += ty;
+        }
+      }
       continue;
     }
-    const double pa0 = la0 * la1, pa1 = la1 * la0;
-    const double pb0 = lb0 * lb1, pb1 = lb1 * lb0;
-    const double inv0 = 1 / (pa0 * pb0), inv1 = 1 / (pa1 * pb1);
-    double wa0 = sa0 * la1 * pb0 * inv0, wa1 = sa1 * la0 * pb1 * inv1;
-    double wb0 = sb0 * lb1 * pa0 * inv0, wb1 = sb1 * lb0 * pa1 * inv1;
+    const double pa = la0 * la1, pb = lb0 * lb1;
+    const double inv = 1 / (pa * pb);
+    double wa0 = src.s[k] * la1 * pb * inv, wa1 = src.s[k + 1] * la0 * pb * inv;
+    double wb0 = src.s[k + 2] * lb1 * pa * inv, wb1 = src.s[k + 3] * lb0 * pa * inv;
     if (a.has_dmax) {
       if (!(la0 < a.dmax2)) wa0 = 0;
       if (!(la1 < a.dmax2)) wa1 = 0;
@@ -914,31 +1177,178 @@ __device__ void fmm_target(const FmmArgs &a, uint64_t seed, uint32_t ti, uint32_
     ay0 += ya0 * wa0 + yb0 * wb0;
     ay1 += ya1 * wa1 + yb1 * wb1;
   }
-  for (; k < b1; ++k) fmm_pair(a, seed, ti, k, xi, yi, vx, vy);
-  vxr = vx + (ax0 + ax1);
-  vyr = vy + (ay0 + ay1);
+#pragma unroll 1
+  for (; k < cn; ++k) {
+    double tx, ty;
+    if (pair_term(a, seed, ti, b0 + k, src.s[k], src.x[k], src.y[k], xi, yi, tx, ty)) {
+      vx += tx;
+      vy += ty;
+    }
+  }
 }
 
-__global__ void __launch_bounds__(FMM_THREADS, 4) k_fmm_p2p(FmmArgs a) {
-  const unsigned lane = threadIdx.x & 31;
-  const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-  const uint64_t seed = (uint64_t)__double_as_longlong(*a.seed);
-  for (uint32_t c = gw; c < a.ncells; c += nwarps) {
-    const uint32_t cnt = a.p2p_cnt[c];
-    if (!cnt) continue;
-    const uint32_t off = a.p2p_off[c], first = a.cells[c].first, count = a.cells[c].count;
-    for (uint32_t base = first; base < first + count; base += 32) {
-      const uint32_t ti = base + lane;
-      if (ti >= first + count) continue;
-      const uint32_t i = a.perm[ti];
-      const double xi = a.px[ti], yi = a.py[ti];
-      double vx = a.vx[i], vy = a.vy[i];
-      for (uint32_t e = 0; e < cnt; ++e) {
-        const uint32_t B = a.p2p[off + e];
-        const uint32_t b0 = a.cells[B].first, b1 = b0 + a.cells[B].count;
-        fmm_target(a, seed, ti, b0, b1, xi, yi, vx, vy);
+// Pairs [k, k + np), np <= 4, of a target that LANES neighbouring lanes hold
+// (all keep the whole velocity): each takes every LANES-th pair, the terms are
+// added in order. Every lane of the warp calls it; `mine` says whose terms count.
+template <uint32_t LANES>
+__device__ inline void pairs_many(const FmmArgs &a, uint64_t seed, uint32_t ti, uint32_t b0, uint32_t k,
+                                  uint32_t np, const Sources &src, double xi, double yi, bool mine,
+                                  double &vx, double &vy) {
+  constexpr uint32_t PER = 4 / LANES;
+  const uint32_t lane = threadIdx.x & 31, r = lane % LANES, l0 = lane - r;
+  double tx[PER], ty[PER];
+  uint32_t has = 0;
+#pragma unroll
+  for (uint32_t i = 0; i < PER; ++i) {
+    const uint32_t u = i * LANES + r, j = (k + u) & 31;
+    tx[i] = ty[i] = 0;
+    if (mine && u < np &&
+        pair_term(a, seed, ti, b0 + j, src.s[j], src.x[j], src.y[j], xi, yi, tx[i], ty[i]))
+      has |= 1u << u;
+  }
+#pragma unroll
+  for (uint32_t o = 1; o < LANES; o <<= 1) has |= __shfl_xor_sync(0xffffffffu, has, o);
+#pragma unroll
+  for (uint32_t u = 0; u < 4; ++u) {
+    const double x = __shfl_sync(0xffffffffu, tx[u / LANES], l0 + u % LANES),
+                 y = __shfl_sync(0xffffffffu, ty[u / LANES], l0 + u % LANES);
+    if (has >> u & 1u) {
+      vx += x;
+      vy += y;
+    }
+  }
+}
+
+// leaf_one for a target that LANES neighbouring lanes hold: LANES / 2 groups of
+// four pairs at a time, a lane per group and sum; both sums are kept by every
+// second lane, the groups' terms added in order. (The pairs that go to the
+// velocity one by one do not meet the sums before the leaf ends.)
+template <uint32_t LANES>
+__device__ inline void leaf_many(const FmmArgs &a, uint64_t seed, uint32_t ti, uint32_t b0, uint32_t cn,
+                                 const Sources &src, double xi, double yi, double &vx, double &vy,
+                                 double &ax, double &ay) {
+  constexpr uint32_t G = LANES / 2;
+  const uint32_t lane = threadIdx.x & 31, h = lane & 1, g = lane % LANES / 2, l0 = lane - lane % LANES;
+  for (uint32_t k = 0; k + 4 <= cn; k += 4 * G) {
+    const bool in = G == 1 || k + 4 * g + 4 <= cn;
+    const uint32_t ja = in ? k + 4 * g + h : h, jb = ja + 2;
+    const double xa = src.x[ja] - xi, ya = src.y[ja] - yi;
+    const double xb = src.x[jb] - xi, yb = src.y[jb] - yi;
+    const double la = xa * xa + ya * ya, lb = xb * xb + yb * yb;
+    const double oa = __shfl_xor_sync(0xffffffffu, la, 1), ob = __shfl_xor_sync(0xffffffffu, lb, 1);
+    const double z = xa * ya * xb * yb;
+    const double mn = zmin(zmin(la, lb), zmin(oa, ob));
+    int bad = z == 0 || !(mn >= a.dmin2) || ti - (b0 + k + 4 * g) < 4;
+    bad |= __shfl_xor_sync(0xffffffffu, bad, 1);
+    const double pa = la * oa, pb = lb * ob;
+    const double inv = 1 / (pa * pb);
+    double wa = src.s[ja] * oa * pb * inv, wb = src.s[jb] * ob * pa * inv;
+    if (a.has_dmax) {
+      if (!(la < a.dmax2)) wa = 0;
+      if (!(lb < a.dmax2)) wb = 0;
+    }
+    const double tx = xa * wa + xb * wb, ty = ya * wa + yb * wb;
+    if (G == 1) {
+      if (!bad) {
+        ax += tx;
+        ay += ty;
       }
+      if (__any_sync(0xffffffffu, bad))
+        pairs_many<LANES>(a, seed, ti, b0, k, 4, src, xi, yi, bad, vx, vy);
+    } else {
+      const int state = in ? 1 + bad : 0;
+#pragma unroll
+      for (uint32_t gg = 0; gg < G; ++gg) {
+        const uint32_t from = l0 + 2 * gg + h;
+        const double x = __shfl_sync(0xffffffffu, tx, from), y = __shfl_sync(0xffffffffu, ty, from);
+        const int st = __shfl_sync(0xffffffffu, state, from);
+        if (st == 1) {
+          ax += x;
+          ay += y;
+        }
+        if (__any_sync(0xffffffffu, st == 2))
+          pairs_many<LANES>(a, seed, ti, b0, k + 4 * gg, 4, src, xi, yi, st == 2, vx, vy);
+      }
+    }
+  }
+  if (cn & 3) pairs_many<LANES>(a, seed, ti, b0, cn & ~3u, cn & 3, src, xi, yi, true, vx, vy);
+}
+
+// A warp per leaf: the source leaves of its list one after another, the next
+// one's points on their way into registers while this one's, in shared memory,
+// are summed. A lane holds a target, or two lanes where the leaf has at most 16
+// (six in ten leaves of evenly spread nodes: half the lanes were idle). Sources
+// read from L2 as the sums went, a chain of three loads a source leaf, took 104
+// us at 6,000 nodes (now 52) and 759 us at 1 M (now 620). FEW: four warps
+// a leaf, eight targets each and four lanes a target, where the leaves do not
+// fill the chip: shorter chains for a sixth more work. Against a lane or two a
+// target, evenly spread / clustered: 6,000 nodes 25 / 64 us for 37 / 84; 20,000
+// 39 / 150 for 35 / 200; 80,000 104 / 360 for 68 / 478 (one leaf's long list).
+template <bool FEW>
+__global__ void __launch_bounds__(P2P_THREADS) k_fmm_p2p(FmmArgs a) {
+  __shared__ Sources sources[P2P_THREADS / 32];
+  if (a.info[FI_LIST_OVERFLOW]) return;
+  const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  Sources &src = sources[warp];
+  const uint64_t seed = (uint64_t)__double_as_longlong(*a.seed);
+  const uint32_t gw = blockIdx.x * (P2P_THREADS / 32) + warp;
+  const uint32_t c = FEW ? gw >> 2 : gw, skip = FEW ? (gw & 3) * 8 : 0;
+  if (c >= a.ncells) return;
+  const uint32_t cnt = a.p2p_cnt[c];
+  if (!cnt) return;
+  const uint32_t off = a.p2p_off[c], first = a.cells[c].first, count = a.cells[c].count;
+  const bool two = count <= 16;
+  for (uint32_t base = first + skip; base < first + count; base += 32) {
+    const uint32_t at = base + (FEW ? lane >> 2 : two ? lane >> 1 : lane);
+    const bool live = at < first + count;
+    const uint32_t ti = live ? at : first;
+    const uint32_t i = a.perm[ti];
+    const double xi = a.px[ti], yi = a.py[ti];
+    double vx = a.vx[i], vy = a.vy[i];
+    for (uint32_t e0 = 0; e0 < cnt; e0 += 32) {
+      const uint32_t ne = min(32u, cnt - e0);
+      uint32_t lb = 0, ln = 0;
+      if (lane < ne) {
+        const uint32_t B = a.p2p[off + e0 + lane];
+        lb = a.cells[B].first;
+        ln = a.cells[B].count;
+      }
+      uint32_t b0 = __shfl_sync(0xffffffffu, lb, 0), bn = __shfl_sync(0xffffffffu, ln, 0);
+      double rx = 0, ry = 0, rs = 0;
+      if (lane < bn) { rx = a.px[b0 + lane]; ry = a.py[b0 + lane]; rs = a.ps[b0 + lane]; }
+      double ax0 = 0, ax1 = 0, ay0 = 0, ay1 = 0;
+      for (uint32_t e = 0; e < ne;) {
+        const uint32_t cb = b0, cn = min(32u, bn);
+        __syncwarp();
+        src.x[lane] = rx;
+        src.y[lane] = ry;
+        src.s[lane] = rs;
+        __syncwarp();
+        const bool ends = bn <= 32;  // this source leaf ends with this chunk
+        if (ends) {
+          ++e;
+          b0 = __shfl_sync(0xffffffffu, lb, e & 31);
+          bn = __shfl_sync(0xffffffffu, ln, e & 31);
+        } else {
+          b0 += 32;
+          bn -= 32;
+        }
+        if (e < ne && lane < bn) { rx = a.px[b0 + lane]; ry = a.py[b0 + lane]; rs = a.ps[b0 + lane]; }
+        if (FEW) leaf_many<4>(a, seed, ti, cb, cn, src, xi, yi, vx, vy, ax0, ay0);
+        else if (two) leaf_many<2>(a, seed, ti, cb, cn, src, xi, yi, vx, vy, ax0, ay0);
+        else leaf_one(a, seed, ti, cb, cn, src, xi, yi, vx, vy, ax0, ay0, ax1, ay1);
+        if (ends) {
+          if (FEW || two) {
+            ax1 = __shfl_xor_sync(0xffffffffu, ax0, 1);
+            ay1 = __shfl_xor_sync(0xffffffffu, ay0, 1);
+          }
+          vx += ax0 + ax1;
+          vy += ay0 + ay1;
+          ax0 = ax1 = ay0 = ay1 = 0;
+        }
+      }
+    }
+    if (live && (FEW ? lane % 4 == 0 : !two || lane % 2 == 0)) {
       a.vx[i] = vx;
       a.vy[i] = vy;
     }
@@ -947,61 +1357,116 @@ __global__ void __launch_bounds__(FMM_THREADS, 4) k_fmm_p2p(FmmArgs a) {
 
 // ---- downward: L2L (fmm.zig:823-849), L2P (fmm.zig:853-886) ---------------------------
 
-__global__ void __launch_bounds__(FMM_THREADS) k_fmm_down(FmmArgs a) {
+// L2L's sum for one coefficient: local `L` (re 0..q-1, im q..) shifted by the
+// powers `pw`.
+template <uint32_t P>
+__device__ inline void l2l_sum(const FmmArgs &a, const double *L, const double *pw, uint32_t mm,
+                               uint32_t q, double &sre, double &sim) {
+  sre = sim = 0;
+#pragma unroll
+  for (uint32_t u = 0; u < (P ? P + 1 : q - mm); ++u) {
+    const uint32_t l = mm + u;
+    if (l >= q) continue;
+    const double b = a.tab->binom[l * FMM_TAB + mm];
+    const double xre = L[l] * b, xim = L[q + l] * b;
+    sre += xre * pw[u] - xim * pw[q + u];
+    sim += xre * pw[q + u] + xim * pw[u];
+  }
+}
+
+// Rows of a warp's shared memory: a local and the powers of the step to it for
+// each cell of the path from the root and for four children.
+constexpr uint32_t DOWN_ROWS = FMM_LEVELS + 1 + 4;
+
+// A warp per cell with leaf children: it takes the locals down the path from
+// the root itself, in shared memory, then to its children, and on to their
+// points. The path's upper cells are recomputed by every warp below them (the
+// same operations on the same values): eight short sums a warp at 1 M nodes,
+// where a grid barrier a level and a cell's children one after another made a
+// chain of 19 us a level (6,000 nodes: 116 -> 15 us; 1 M: 415 -> 106 us).
+template <uint32_t P>
+__global__ void __launch_bounds__(DOWN_THREADS) k_fmm_down(FmmArgs a) {
   extern __shared__ double fmm_smem[];
-  cg::grid_group g = cg::this_grid();
-  const unsigned lane = threadIdx.x & 31;
-  const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-  const uint32_t p = a.p, q = a.q, stride = a.stride;
-  double *ws = fmm_smem + (threadIdx.x >> 5) * 2 * (size_t)stride;  // L of the cell, then powers
-  double *Lw = ws, *pw = ws + stride;
-  const uint32_t *lvl = a.info + FI_LVL;
-  for (uint32_t lev = 0; lev < a.nlev; ++lev) {
-    for (uint32_t c = lvl[lev] + gw; c < lvl[lev + 1]; c += nwarps) {
-      const double cx = a.cells[c].cx, cy = a.cells[c].cy;
-      const uint32_t nchild = a.cells[c].nchild, child0 = a.cells[c].child0;
-      for (uint32_t r = lane; r < stride; r += 32) Lw[r] = ldg_cg(&a.lco[(size_t)c * stride + r]);
-      __syncwarp();
-      if (nchild == 0) {
-        const uint32_t first = a.cells[c].first, count = a.cells[c].count;
-        for (uint32_t k = first + lane; k < first + count; k += 32) {
-          const uint32_t j = a.perm[k];
-          const double wre = a.ux[k] - cx, wim = a.uy[k] - cy;
-          double are = Lw[p], aim = Lw[q + p];
-          for (uint32_t l = p; l > 0;) {
-            --l;
-            const double nre = are * wre - aim * wim + Lw[l];
-            const double nim = are * wim + aim * wre + Lw[q + l];
-            are = nre;
-            aim = nim;
-          }
-          a.vx[j] = a.vx[j] - are * a.inv_w;
-          a.vy[j] = a.vy[j] + aim * a.inv_w;
-        }
-      } else {
-        for (uint32_t ch = child0; ch < child0 + nchild; ++ch) {
-          if (lane == 0) shift_powers(a.cells[ch].cx - cx, a.cells[ch].cy - cy, p, pw);
-          __syncwarp();
-          const uint32_t mm = lane;
-          if (mm < q) {
-            double sre = 0, sim = 0;
-            for (uint32_t l = mm; l < q; ++l) {
-              const double b = a.tab->binom[l * FMM_TAB + mm];
-              const double xre = Lw[l] * b, xim = Lw[q + l] * b;
-              sre += xre * pw[l - mm] - xim * pw[q + l - mm];
-              sim += xre * pw[q + l - mm] + xim * pw[l - mm];
-            }
-            double *C = a.lco + (size_t)ch * stride;
-            C[mm] = C[mm] + sre;
-            C[q + mm] = C[q + mm] + sim;
-          }
-          __syncwarp();
-        }
-      }
-      __syncwarp();
+  if (a.info[FI_LIST_OVERFLOW]) return;
+  const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t p = P ? P : a.p, q = p + 1, stride = 2 * q, row = up_row(stride);
+  double *Ls = fmm_smem + (size_t)warp * 2 * DOWN_ROWS * row, *pw = Ls + DOWN_ROWS * row;
+  const uint32_t c = blockIdx.x * (DOWN_THREADS / 32) + warp;
+  if (c >= a.ncells) return;
+  const FCell A = load_cell(a.cells + c);
+  if (A.nchild == 0 && c != 0) return;
+  const uint32_t d = A.depth;  // path rows 0 .. d, children's rows d + 1 ..
+  // lane k: the path's cell at depth k, then the children
+  uint32_t id = c, at = c;
+  for (uint32_t k = d; k-- > 0;) {
+    at = a.cells[at].parent;
+    if (k == lane) id = at;
+  }
+  if (lane > d && lane <= d + A.nchild) id = A.child0 + lane - d - 1;
+  const uint32_t rows = d + 1 + A.nchild;
+  FCell mine = {};
+  if (lane < rows) mine = load_cell(a.cells + id);
+  const unsigned leaves = __ballot_sync(0xffffffffu, lane < rows && mine.nchild == 0);
+  if (!leaves) return;
+  for (uint32_t i0 = 0; i0 < rows * stride; i0 += 32) {
+    const uint32_t k = (i0 + lane) / stride, r = (i0 + lane) % stride;
+    const uint32_t from = __shfl_sync(0xffffffffu, id, k & 31);
+    if (k < rows) Ls[k * row + r] = a.lco[(size_t)from * stride + r];
+  }
+  {
+    // the step to row k: from the row before, or from c to a child
+    const uint32_t before = lane > d ? d : lane ? lane - 1 : 0;
+    const double bx = __shfl_sync(0xffffffffu, mine.cx, before),
+                 by = __shfl_sync(0xffffffffu, mine.cy, before);
+    if (lane > 0 && lane < rows) shift_powers(mine.cx - bx, mine.cy - by, p, pw + lane * row);
+  }
+  __syncwarp();
+  for (uint32_t k = 1; k <= d; ++k) {
+    if (lane < q) {
+      double sre, sim;
+      l2l_sum<P>(a, Ls + (k - 1) * row, pw + k * row, lane, q, sre, sim);
+      double *L = Ls + k * row;
+      L[lane] = L[lane] + sre;
+      L[q + lane] = L[q + lane] + sim;
     }
-    g.sync();
+    __syncwarp();
+  }
+  const uint32_t S = 32 / q;
+  for (uint32_t j = lane / q; j < A.nchild && lane < S * q; j += S) {
+    const uint32_t k = d + 1 + j, mm = lane % q;
+    double sre, sim;
+    l2l_sum<P>(a, Ls + d * row, pw + k * row, mm, q, sre, sim);
+    double *L = Ls + k * row;
+    L[mm] = L[mm] + sre;
+    L[q + mm] = L[q + mm] + sim;
+  }
+  __syncwarp();
+  // the leaves' points, one leaf after another over the lanes
+  const uint32_t held = leaves >> lane & 1u ? mine.count : 0;
+  for (uint32_t k0 = 0;; k0 += 32) {
+    uint32_t rk = 0, k = NONE, before = 0;
+    for (uint32_t j = d; j < rows; ++j) {
+      const uint32_t n = __shfl_sync(0xffffffffu, held, j), f = __shfl_sync(0xffffffffu, mine.first, j);
+      if (k0 + lane - before < n) { rk = j; k = f + k0 + lane - before; }
+      before += n;
+    }
+    if (k0 >= before) break;
+    const double cx = __shfl_sync(0xffffffffu, mine.cx, rk), cy = __shfl_sync(0xffffffffu, mine.cy, rk);
+    if (k == NONE) continue;
+    const double *L = Ls + rk * row;
+    const uint32_t j = a.perm[k];
+    const double wre = a.ux[k] - cx, wim = a.uy[k] - cy;
+    double are = L[p], aim = L[q + p];
+#pragma unroll 8
+    for (uint32_t l = p; l > 0;) {
+      --l;
+      const double nre = are * wre - aim * wim + L[l];
+      const double nim = are * wim + aim * wre + L[q + l];
+      are = nre;
+      aim = nim;
+    }
+    a.vx[j] = a.vx[j] - are * a.inv_w;
+    a.vy[j] = a.vy[j] + aim * a.inv_w;
   }
 }
 
@@ -1038,7 +1503,7 @@ int fmm_reserve_cells(FmmDev &f, uint32_t ccap) {
   if (ccap <= f.ccap && f.ccap) return 0;
   cudaFree(f.cells); cudaFree(f.bx0); cudaFree(f.by0); cudaFree(f.bx1); cudaFree(f.by1);
   cudaFree(f.m2l_off); cudaFree(f.m2l_cnt); cudaFree(f.p2p_off);
-  cudaFree(f.p2p_cnt); cudaFree(f.fwd_off); cudaFree(f.fwd_cnt);
+  cudaFree(f.p2p_cnt); cudaFree(f.fwd_off); cudaFree(f.fwd_cnt); cudaFree(f.arrive);
   D3_CUDA_OK(cudaMalloc(&f.cells, ccap * sizeof(FCell)));
   D3_CUDA_OK(cudaMalloc(&f.bx0, ccap * 8ull));
   D3_CUDA_OK(cudaMalloc(&f.by0, ccap * 8ull));
@@ -1050,6 +1515,7 @@ int fmm_reserve_cells(FmmDev &f, uint32_t ccap) {
   D3_CUDA_OK(cudaMalloc(&f.p2p_cnt, ccap * 4ull));
   D3_CUDA_OK(cudaMalloc(&f.fwd_off, ccap * 4ull));
   D3_CUDA_OK(cudaMalloc(&f.fwd_cnt, ccap * 4ull));
+  D3_CUDA_OK(cudaMalloc(&f.arrive, ccap * 4ull));
   f.ccap = ccap;
   return 0;
 }
@@ -1063,19 +1529,18 @@ void fmm_free(FastScratch &s) {
   cudaFree(f->m2l_off); cudaFree(f->m2l_cnt); cudaFree(f->p2p_off);
   cudaFree(f->p2p_cnt); cudaFree(f->fwd_off); cudaFree(f->fwd_cnt); cudaFree(f->m2l);
   cudaFree(f->p2p); cudaFree(f->fwd); cudaFree(f->mco); cudaFree(f->lco); cudaFree(f->tab);
-  cudaFree(f->info); cudaFree(f->bsum); cudaFree(f->square); cudaFree(f->geom);
+  cudaFree(f->info); cudaFree(f->arrive); cudaFree(f->square); cudaFree(f->geom);
   cudaFree(f->cb_count); cudaFree(f->start_of); cudaFree(f->level_of);
   cudaFreeHost(f->h_info); cudaFreeHost(f->h_geom);
+  if (f->lists_read) cudaEventDestroy(f->lists_read);
   delete f;
   s.fmm = nullptr;
 }
 
-static int coop_launch(const void *fn, int blocks, size_t smem, FmmArgs &args, cudaStream_t st) {
-  void *params[] = {&args};
-  ++g_launches;
-  return cudaLaunchCooperativeKernel(fn, blocks, FMM_THREADS, params, smem, st) == cudaSuccess ? 0
-                                                                                                  : -1;
-}
+// Dynamic shared memory of a block, at q coefficients.
+static int up_smem(uint32_t q) { return (int)(UP_THREADS / 32 * 32 * up_row(2 * q) * 8); }
+static int m2l_smem(uint32_t q) { return (int)(M2L_THREADS / 32 * m2l_words(q) * 8); }
+static int down_smem(uint32_t q) { return (int)(DOWN_THREADS / 32 * 2 * DOWN_ROWS * up_row(2 * q) * 8); }
 
 static int sync_read(FmmDev &f, cudaStream_t st) {
   if (cudaMemcpyAsync(f.h_info, f.info, 64 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st) !=
@@ -1098,25 +1563,17 @@ int fmm_prepare(FastScratch &s, TreeDev &t, const NodeArrays &a, const double *s
     D3_CUDA_OK(cudaMalloc(&f->geom, 4 * sizeof(double)));
     D3_CUDA_OK(cudaHostAlloc(&f->h_info, 64 * sizeof(uint32_t), cudaHostAllocDefault));
     D3_CUDA_OK(cudaHostAlloc(&f->h_geom, 8 * sizeof(double), cudaHostAllocDefault));
-    int dev = 0, sms = 0, per = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    // the largest dynamic shared memory any of the kernels asks for (order 24)
-    const size_t smax = FMM_WARPS * 32 * (size_t)(2 * (FMM_MAX_ORDER + 1)) * 8;
-    cudaFuncSetAttribute(k_fmm_upward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smax);
-    cudaFuncSetAttribute(k_fmm_m2l, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smax);
-    int per_up = 0, per_lists = 0, per_down = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_up, k_fmm_upward, FMM_THREADS, smax);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_lists, k_fmm_lists, FMM_THREADS, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_down, k_fmm_down, FMM_THREADS,
-                                                  FMM_WARPS * 2 * (size_t)(2 * (FMM_MAX_ORDER + 1)) * 8);
-    per = per_up;
-    if (per_lists < per) per = per_lists;
-    if (per_down < per) per = per_down;
-    if (per > 2) per = 2;
-    if (per < 1) per = 1;
-    f->coop_blocks = sms * per;
-    D3_CUDA_OK(cudaMalloc(&f->bsum, (size_t)f->coop_blocks * 4));
+    D3_CUDA_OK(cudaEventCreateWithFlags(&f->lists_read, cudaEventDisableTiming));
+    // shared memory past the default 48 KB (up to order 24)
+    int up = 0, m2l = 0, down = 0;
+    for (uint32_t q = 2; q <= FMM_MAX_ORDER + 1; ++q) {
+      if (up_smem(q) > up) up = up_smem(q);
+      if (m2l_smem(q) > m2l) m2l = m2l_smem(q);
+      if (down_smem(q) > down) down = down_smem(q);
+    }
+    cudaFuncSetAttribute(k_fmm_upward<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, up);
+    cudaFuncSetAttribute(k_fmm_m2l<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, m2l);
+    cudaFuncSetAttribute(k_fmm_down<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, down);
   }
   FmmDev &f = *static_cast<FmmDev *>(s.fmm);
   if (fmm_reserve_points(f, n)) return -1;
@@ -1145,7 +1602,7 @@ int fmm_prepare(FastScratch &s, TreeDev &t, const NodeArrays &a, const double *s
       D3_LAUNCH(k_cells_place, nb, CB_THREADS, 0, st)(f.pt_levels, f.cb_count, f.info, f.start_of,
                                                     f.level_of);
       D3_LAUNCH(k_cells_fill, blocks_for(f.ccap, CB_THREADS), CB_THREADS, 0, st)(
-          t.keys, f.start_of, f.level_of, f.info, f.cells);
+          t.keys, f.start_of, f.level_of, f.info, f.cells, f.arrive, f.fwd_cnt);
     }
     if (cudaMemcpyAsync(f.h_geom, f.geom, 4 * sizeof(double), cudaMemcpyDeviceToHost, st) !=
             cudaSuccess ||
@@ -1172,7 +1629,6 @@ int fmm_prepare(FastScratch &s, TreeDev &t, const NodeArrays &a, const double *s
   out.px = f.px; out.py = f.py; out.ps = f.ps; out.ux = f.ux; out.uy = f.uy;
   out.cells = f.cells;
   out.info = f.info;
-  out.coop_blocks = f.coop_blocks;
   return 1;
 }
 
@@ -1204,6 +1660,7 @@ int fmm_run(FastScratch &s, TreeDev &t, const NodeArrays &a, const double *stren
     }
     h.fact[0] = 1;
     for (size_t k = 1; k < nmax; ++k) h.fact[k] = h.fact[k - 1] * (double)k;
+    for (size_t k = 0; k < nmax; ++k) h.ifact[k] = 1 / h.fact[k];
     if (cudaMemcpyAsync(f.tab, &h, sizeof h, cudaMemcpyHostToDevice, st) != cudaSuccess ||
         cudaStreamSynchronize(st) != cudaSuccess)
       return -1;
@@ -1218,7 +1675,7 @@ int fmm_run(FastScratch &s, TreeDev &t, const NodeArrays &a, const double *stren
   args.tab = f.tab;
   args.vx = a.vx; args.vy = a.vy;
   args.info = f.info;
-  args.p = p; args.q = q; args.stride = stride;
+  args.p = p;
   args.inv_w = pr.inv_w;
   args.mac_far = 2 * kappa - 1;
   double dmax_scaled = INFINITY;
@@ -1231,11 +1688,10 @@ int fmm_run(FastScratch &s, TreeDev &t, const NodeArrays &a, const double *stren
   args.dmin2 = prm.dmin2;
   args.dmax2 = prm.dmax2;
   args.seed = seed;
-  const uint32_t ncells = pr.ncells, nlev = pr.nlev;
+  const uint32_t ncells = pr.ncells;
   args.cells = f.cells;
   args.bx0 = f.bx0; args.by0 = f.by0; args.bx1 = f.bx1; args.by1 = f.by1;
   args.ncells = ncells;
-  args.nlev = nlev;
   if ((size_t)ncells * stride > f.coef_cap || !f.mco) {
     cudaFree(f.mco);
     cudaFree(f.lco);
@@ -1246,11 +1702,15 @@ int fmm_run(FastScratch &s, TreeDev &t, const NodeArrays &a, const double *stren
   }
   args.mco = f.mco;
   args.lco = f.lco;
+  args.arrive = f.arrive;
   args.m2l_off = f.m2l_off; args.m2l_cnt = f.m2l_cnt;
   args.p2p_off = f.p2p_off; args.p2p_cnt = f.p2p_cnt;
   args.fwd_off = f.fwd_off; args.fwd_cnt = f.fwd_cnt;
-  const size_t smem_up = FMM_WARPS * 32 * (size_t)stride * 8;
-  if (coop_launch((const void *)k_fmm_upward, f.coop_blocks, smem_up, args, st)) return -1;
+  const bool dflt = p == FMM_DEFAULT_ORDER;  // its own kernels: the sums unroll
+  const unsigned ub = blocks_for(ncells, UP_THREADS / 32), mb = blocks_for(ncells, M2L_THREADS / 32),
+                 pb = blocks_for(ncells, P2P_THREADS / 32), db = blocks_for(ncells, DOWN_THREADS / 32);
+  if (dflt) D3_LAUNCH(k_fmm_upward<FMM_DEFAULT_ORDER>, ub, UP_THREADS, up_smem(q), st)(args);
+  else D3_LAUNCH(k_fmm_upward<0>, ub, UP_THREADS, up_smem(q), st)(args);
   // interaction lists; grow the pools and redo on overflow
   // first guesses from the cell count, then what the previous run needed
   size_t need_m2l = (size_t)ncells * 48 + 1024, need_p2p = (size_t)ncells * 16 + 1024,
@@ -1267,27 +1727,34 @@ int fmm_run(FastScratch &s, TreeDev &t, const NodeArrays &a, const double *stren
     args.m2l = f.m2l; args.p2p = f.p2p; args.fwd = f.fwd;
     args.cap_m2l = f.cap_m2l; args.cap_p2p = f.cap_p2p; args.cap_fwd = f.cap_fwd;
     if (cudaMemsetAsync(f.info + FI_POOL_M2L, 0, 5 * sizeof(uint32_t), st) != cudaSuccess) return -1;
-    if (coop_launch((const void *)k_fmm_lists, f.coop_blocks, 0, args, st)) return -1;
-    if (sync_read(f, st)) return -1;
-    const uint32_t ovf = f.h_info[FI_LIST_OVERFLOW] | f.h_info[FI_LIST_OVERFLOW + 1];
+    if (attempt && cudaMemsetAsync(f.fwd_cnt, 0xFF, (size_t)ncells * 4, st) != cudaSuccess) return -1;
+    D3_LAUNCH(k_fmm_lists, blocks_for(ncells, LISTS_THREADS / 32), LISTS_THREADS, 0, st)(args);
+    // the rest follows at once (it does nothing where a list overflowed), and
+    // the host reads the lists' words while it runs
+    if (cudaMemcpyAsync(f.h_info, f.info, 8 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st) !=
+            cudaSuccess ||
+        cudaEventRecord(f.lists_read, st) != cudaSuccess)
+      return -1;
+    if (dflt) D3_LAUNCH(k_fmm_m2l<FMM_DEFAULT_ORDER>, mb, M2L_THREADS, m2l_smem(q), st)(args);
+    else D3_LAUNCH(k_fmm_m2l<0>, mb, M2L_THREADS, m2l_smem(q), st)(args);
+    if (ncells <= P2P_FEW_CELLS)
+      D3_LAUNCH(k_fmm_p2p<true>, blocks_for(4 * ncells, P2P_THREADS / 32), P2P_THREADS, 0, st)(args);
+    else D3_LAUNCH(k_fmm_p2p<false>, pb, P2P_THREADS, 0, st)(args);
+    if (dflt) D3_LAUNCH(k_fmm_down<FMM_DEFAULT_ORDER>, db, DOWN_THREADS, down_smem(q), st)(args);
+    else D3_LAUNCH(k_fmm_down<0>, db, DOWN_THREADS, down_smem(q), st)(args);
+    if (cudaEventSynchronize(f.lists_read) != cudaSuccess) return -1;
+    const uint32_t ovf = f.h_info[FI_LIST_OVERFLOW];
     if (!ovf) {
       f.last_m2l = f.h_info[FI_POOL_M2L];
       f.last_p2p = f.h_info[FI_POOL_P2P];
       f.last_fwd = f.h_info[FI_POOL_FWD];
       break;
     }
-    if ((ovf & 2) || attempt > 8) return -1;  // a call stack overflowed
+    if ((ovf & 2) || attempt > 8) return -1;  // a call stack overflowed, or a wait ran out
     need_m2l = 2 * (size_t)(f.h_info[FI_POOL_M2L] > need_m2l ? f.h_info[FI_POOL_M2L] : need_m2l);
     need_p2p = 2 * (size_t)(f.h_info[FI_POOL_P2P] > need_p2p ? f.h_info[FI_POOL_P2P] : need_p2p);
     need_fwd = 2 * (size_t)(f.h_info[FI_POOL_FWD] > need_fwd ? f.h_info[FI_POOL_FWD] : need_fwd);
   }
-  const uint32_t S = 32 / q;
-  const size_t smem_m2l = FMM_WARPS * (size_t)S * (2 * (2 * p + 1) + 2 * stride) * 8;
-  const unsigned wblocks = blocks_for((size_t)ncells * 32, FMM_THREADS);
-  D3_LAUNCH(k_fmm_m2l, wblocks, FMM_THREADS, smem_m2l, st)(args);
-  D3_LAUNCH(k_fmm_p2p, wblocks, FMM_THREADS, 0, st)(args);
-  const size_t smem_down = FMM_WARPS * 2 * (size_t)stride * 8;
-  if (coop_launch((const void *)k_fmm_down, f.coop_blocks, smem_down, args, st)) return -1;
   return cudaGetLastError() == cudaSuccess ? 1 : -1;
 }
 
