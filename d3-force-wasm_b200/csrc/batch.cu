@@ -35,10 +35,13 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
+#include <thread>
 #include <vector>
 
 #include "common.cuh"
@@ -715,6 +718,139 @@ void build_btables(BTables &T) {
   }
 }
 
+// Reads of device arrays into the caller's (pageable, often untouched) memory.
+// One cudaMemcpy stages through one thread, which also takes every page fault:
+// 96 MB take 25 ms, 4 GB/s. Here up to READ_WORKERS threads take pieces of
+// READ_PIECE bytes in turn, each with two pinned slots (one being filled by the
+// copy engine while the other is copied out): 9 ms. The slots, 8 MB at most,
+// stay with the batch and go with it. Reads under READ_MIN take cudaMemcpy:
+// pinning the slots costs the first read 4 to 9 ms, which later reads of 32 MB
+// (4.3 ms as they are, 3.1 to 4.6 with the threads: the allocator hands out
+// memory of that size that is mapped already) do not win back.
+constexpr unsigned READ_WORKERS = 8, READ_SLOTS = 2;
+constexpr size_t READ_PIECE = 1u << 19, READ_MIN = 48u << 20;
+
+struct ReadSpan {
+  void *dst;
+  const void *src;
+  size_t bytes;
+};
+
+class Reader {
+ public:
+  // Copies the spans; false on a CUDA error. One call at a time (a second
+  // thread waits).
+  bool read(const ReadSpan *spans, unsigned count) {
+    size_t total = 0;
+    for (unsigned i = 0; i < count; ++i) total += spans[i].bytes;
+    std::lock_guard<std::mutex> hold(lock_);
+    if (total < READ_MIN || !reserve()) {
+      for (unsigned i = 0; i < count; ++i)
+        if (cudaMemcpy(spans[i].dst, spans[i].src, spans[i].bytes, cudaMemcpyDeviceToHost) !=
+            cudaSuccess)
+          return false;
+      return true;
+    }
+    int dev = 0;
+    cudaGetDevice(&dev);
+    spans_ = spans;
+    count_ = count;
+    next_ = 0;
+    failed_ = false;
+    std::thread threads[READ_WORKERS - 1];
+    unsigned started = 0;
+    try {
+      for (; started + 1 < workers_; ++started)
+        threads[started] = std::thread([this, dev, started] {
+          if (cudaSetDevice(dev) == cudaSuccess) work(started + 1);
+          else failed_ = true;
+        });
+    } catch (...) {  // no more threads: those that run take the pieces
+    }
+    work(0);
+    for (unsigned t = 0; t < started; ++t) threads[t].join();
+    return !failed_;
+  }
+
+  ~Reader() {
+    if (stream_) cudaStreamDestroy(stream_);
+    for (unsigned w = 0; w < READ_WORKERS; ++w)
+      for (unsigned q = 0; q < READ_SLOTS; ++q)
+        if (filled_[w][q]) cudaEventDestroy(filled_[w][q]);
+    if (slots_) cudaFreeHost(slots_);
+  }
+
+ private:
+  // The pinned slots, once. (A blocking stream: it waits for work on the
+  // default stream, as cudaMemcpy does.)
+  bool reserve() {
+    if (workers_) return true;
+    const unsigned cores = std::thread::hardware_concurrency();
+    const unsigned n = cores && cores < READ_WORKERS ? cores : READ_WORKERS;
+    bool ok = slots_ || cudaHostAlloc(reinterpret_cast<void **>(&slots_), n * READ_SLOTS * READ_PIECE,
+                                      cudaHostAllocDefault) == cudaSuccess;
+    ok = ok && (stream_ || cudaStreamCreate(&stream_) == cudaSuccess);
+    for (unsigned w = 0; ok && w < n; ++w)
+      for (unsigned q = 0; ok && q < READ_SLOTS; ++q)
+        ok = filled_[w][q] ||
+             cudaEventCreateWithFlags(&filled_[w][q], cudaEventDisableTiming) == cudaSuccess;
+    if (ok) workers_ = n;
+    else cudaGetLastError();
+    return ok;
+  }
+
+  // Piece `i` of the spans in order; false past the last.
+  bool piece(size_t i, ReadSpan &out) const {
+    for (unsigned k = 0; k < count_; ++k) {
+      const size_t pieces = (spans_[k].bytes + READ_PIECE - 1) / READ_PIECE;
+      if (i < pieces) {
+        const size_t at = i * READ_PIECE;
+        out = {static_cast<char *>(spans_[k].dst) + at, static_cast<const char *>(spans_[k].src) + at,
+               std::min(READ_PIECE, spans_[k].bytes - at)};
+        return true;
+      }
+      i -= pieces;
+    }
+    return false;
+  }
+
+  void work(unsigned w) {
+    ReadSpan held[READ_SLOTS];
+    bool full[READ_SLOTS] = {};
+    auto fill = [&](unsigned q) {
+      full[q] = !failed_ && piece(next_++, held[q]);
+      if (full[q] && (cudaMemcpyAsync(slot(w, q), held[q].src, held[q].bytes, cudaMemcpyDeviceToHost,
+                                      stream_) != cudaSuccess ||
+                      cudaEventRecord(filled_[w][q], stream_) != cudaSuccess)) {
+        failed_ = true;
+        full[q] = false;
+      }
+    };
+    for (unsigned q = 0; q < READ_SLOTS; ++q) fill(q);
+    for (unsigned q = 0; full[q]; q = (q + 1) % READ_SLOTS) {
+      if (cudaEventSynchronize(filled_[w][q]) != cudaSuccess) {
+        failed_ = true;
+        break;
+      }
+      std::memcpy(held[q].dst, slot(w, q), held[q].bytes);
+      fill(q);
+    }
+    if (failed_) cudaStreamSynchronize(stream_);  // no copy into a slot is left behind
+  }
+
+  char *slot(unsigned w, unsigned q) const { return slots_ + (w * READ_SLOTS + q) * READ_PIECE; }
+
+  std::mutex lock_;
+  unsigned workers_ = 0;
+  char *slots_ = nullptr;
+  cudaStream_t stream_ = nullptr;
+  cudaEvent_t filled_[READ_WORKERS][READ_SLOTS] = {};
+  const ReadSpan *spans_ = nullptr;
+  unsigned count_ = 0;
+  std::atomic<size_t> next_{0};
+  std::atomic<bool> failed_{false};
+};
+
 struct Batch {
   uint32_t graphs = 0, nodes = 0;
   std::vector<uint32_t> h_off, h_order;
@@ -737,6 +873,7 @@ struct Batch {
   cudaStream_t st = nullptr;
   cudaGraphExec_t graph = nullptr;
   uint32_t graph_ticks = 0;
+  Reader reader;
 };
 
 std::vector<Batch *> g_batches;
@@ -1030,23 +1167,22 @@ int32_t batch_kick(uint32_t h, float *out, double *alpha_used) {
   if (alpha_used) *alpha_used = (float)al;
   if (cudaMemsetAsync(b->queues, 0, 4, b->st) != cudaSuccess ||
       launch_tick(*b, (float)al, b->tick, b->queues, b->kick) ||
-      cudaMemcpyAsync(out, b->kick, b->nodes * sizeof(float2), cudaMemcpyDeviceToHost, b->st) !=
-          cudaSuccess ||
       cudaStreamSynchronize(b->st) != cudaSuccess)
     return D3_WORKER_FAILED;
-  return D3_OK;
+  const ReadSpan span{out, b->kick, b->nodes * sizeof(float2)};
+  return b->reader.read(&span, 1) ? D3_OK : D3_WORKER_FAILED;
 }
 
 int32_t batch_read(uint32_t h, float *x, float *y, float *vx, float *vy) {
   Batch *b = get_batch(h);
   if (!b) return D3_BAD_HANDLE;
   const size_t bytes = b->nodes * 4ull;
-  if ((x && cudaMemcpy(x, b->x, bytes, cudaMemcpyDeviceToHost) != cudaSuccess) ||
-      (y && cudaMemcpy(y, b->y, bytes, cudaMemcpyDeviceToHost) != cudaSuccess) ||
-      (vx && cudaMemcpy(vx, b->vx, bytes, cudaMemcpyDeviceToHost) != cudaSuccess) ||
-      (vy && cudaMemcpy(vy, b->vy, bytes, cudaMemcpyDeviceToHost) != cudaSuccess))
-    return D3_WORKER_FAILED;
-  return D3_OK;
+  const ReadSpan all[4] = {{x, b->x, bytes}, {y, b->y, bytes}, {vx, b->vx, bytes}, {vy, b->vy, bytes}};
+  ReadSpan spans[4];
+  unsigned count = 0;
+  for (const ReadSpan &sp : all)
+    if (sp.dst) spans[count++] = sp;
+  return b->reader.read(spans, count) ? D3_OK : D3_WORKER_FAILED;
 }
 
 // Autotuner: times `ticks` ticks (from a copy of the current state, which is
