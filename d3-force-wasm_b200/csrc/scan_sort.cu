@@ -113,6 +113,19 @@ __device__ inline uint32_t digit_of(uint64_t k, uint32_t v, int shift) {
   return MODE == PART_BYTE ? ((v >> 31) << 8) | b : b;
 }
 
+// The lanes whose digit of `bits` bits is this lane's, among the valid ones: a
+// ballot a bit (a warp match takes a turn per distinct digit, up to 32).
+__device__ inline unsigned same_digit(uint32_t d, bool valid, int bits) {
+  unsigned peers = __ballot_sync(0xffffffffu, valid);
+#pragma unroll
+  for (int b = 0; b < 9; ++b) {
+    if (b >= bits) break;
+    const unsigned on = __ballot_sync(0xffffffffu, d >> b & 1u);
+    peers &= d >> b & 1u ? on : ~on;
+  }
+  return peers;
+}
+
 // The whole array's digit counts of every pass (they do not depend on the
 // order), so that a pass is one launch: tot[pass * 512 + digit].
 __global__ void __launch_bounds__(SORT_THREADS) k_sort_totals(const uint64_t *keys, const uint32_t *vals,
@@ -192,7 +205,7 @@ __device__ bool look_back(const uint32_t *words, uint32_t tile, uint32_t d, uint
 // Stable scatter of one tile of SORT_TILE keys: warp w takes the tile's
 // w-th run of 32 x PER keys, in PER rounds of 32. In a round a key's rank
 // among equal digits is the warp's count of that digit so far plus the lanes
-// below it with the same digit (warp match). The warps' counts then give
+// below it with the same digit (same_digit). The warps' counts then give
 // each key its place in the tile sorted by digit (stable); the tile is
 // reordered in shared memory and written in that order, so consecutive
 // threads write consecutive places of one digit's run. Where the tile's run of
@@ -202,7 +215,7 @@ __device__ bool look_back(const uint32_t *words, uint32_t tile, uint32_t d, uint
 // pass and three scan launches came first. Tiles are numbered in the order
 // their blocks start (`ticket`), so a tile only waits for running blocks; where
 // a wait runs out all the same, the tile counts the keys before it itself. A pass over
-// 1 M keys 37 -> 31 us, over 41,000 24 -> 12 us, its share of k_sort_totals
+// 1 M keys 37 -> 27 us, over 41,000 24 -> 11 us, its share of k_sort_totals
 // in it.
 template <int MODE>
 __global__ void __launch_bounds__(SORT_THREADS) k_sort_scatter(const uint64_t *keys, const uint32_t *vals,
@@ -250,7 +263,7 @@ __global__ void __launch_bounds__(SORT_THREADS) k_sort_scatter(const uint64_t *k
   for (unsigned r = 0; r < PER; ++r) {
     const bool valid = wbase + r * 32 + lane < n;
     const uint32_t d = valid ? digit_of<MODE>(k[r], v[r], shift) : NB + lane;  // never matches
-    const unsigned peers = __match_any_sync(0xffffffffu, d);
+    const unsigned peers = same_digit(d, valid, MODE == PART_BYTE ? 9 : 8);
     const unsigned below = __popc(peers & lt);
     const uint32_t cnt = valid ? wh[warp][d] : 0;
     __syncwarp();
@@ -361,9 +374,127 @@ __global__ void __launch_bounds__(SORT_THREADS) k_sort_scatter(const uint64_t *k
   }
 }
 
+// Up to SORT_BLOCK_MAX keys: all passes in one block, keys (the sorted bytes,
+// at most 32 bits) and values in registers and shared memory. A pass is the
+// ranking above without the other tiles: no launch, no wait. Four passes: 3,000
+// keys 35 us, 8,192 41 us, for 39 us and the gaps of six launches; the one SM's
+// ranking rounds grow with the keys, the tiles' time does not, so the line is
+// what registers and shared memory hold.
+constexpr uint32_t SORT_BLOCK_MAX = 8192;
+constexpr unsigned SB_THREADS = 1024, SB_WARPS = SB_THREADS / 32,
+                   SB_PER = SORT_BLOCK_MAX / SB_THREADS;
+constexpr size_t SB_SMEM = SORT_BLOCK_MAX * 8 + SB_WARPS * 512 * 2;
+
+__global__ void __launch_bounds__(SB_THREADS) k_sort_block(uint64_t *keys, uint32_t *vals, uint32_t n,
+                                                           int byte_lo, int passes, int part) {
+  extern __shared__ uint32_t sb_smem[];
+  uint32_t *skey = sb_smem, *sval = skey + SORT_BLOCK_MAX;
+  uint16_t *wh = reinterpret_cast<uint16_t *>(sval + SORT_BLOCK_MAX);  // [warp][digit]
+  __shared__ uint32_t seg[SB_THREADS], lstart[512], wsum[16];
+  const unsigned tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const unsigned lt = (1u << lane) - 1;
+  const uint32_t base = warp * 32 * SB_PER + lane;
+  uint32_t k[SB_PER], v[SB_PER];
+  uint16_t rk[SB_PER];
+#pragma unroll
+  for (unsigned r = 0; r < SB_PER; ++r) {
+    const uint32_t i = base + r * 32;
+    k[r] = i < n ? (uint32_t)(keys[i] >> (8 * byte_lo)) : 0;
+    v[r] = i < n ? vals[i] : 0;
+  }
+  for (int p = 0; p < passes; ++p) {
+    const bool wide = part && p + 1 == passes;  // the partition's bit on top of the byte
+    const unsigned nb = wide ? 512 : 256;
+    uint16_t *mine = wh + warp * nb;
+    for (unsigned d = lane; d < nb; d += 32) mine[d] = 0;
+    __syncwarp();
+#pragma unroll
+    for (unsigned r = 0; r < SB_PER; ++r) {
+      const bool valid = base + r * 32 < n;
+      const uint32_t b = (k[r] >> (8 * p)) & 255u;
+      const uint32_t d = !valid ? nb + lane : wide ? (v[r] >> 31) << 8 | b : b;
+      const unsigned peers = same_digit(d, valid, wide ? 9 : 8);
+      const unsigned below = __popc(peers & lt);
+      const uint32_t cnt = valid ? mine[d] : 0;
+      __syncwarp();
+      if (valid && below == 0) mine[d] = (uint16_t)(cnt + __popc(peers));
+      __syncwarp();
+      rk[r] = (uint16_t)(cnt + below);
+    }
+    __syncthreads();
+    // per digit: the earlier warps' counts (in place) and the count of all,
+    // the warps in SB_THREADS / nb stretches
+    const unsigned d = tid & (nb - 1), part_of = tid / nb, stretch = SB_WARPS * nb / SB_THREADS;
+    uint32_t run = 0;
+#pragma unroll 4
+    for (unsigned w = part_of * stretch; w < (part_of + 1) * stretch; ++w) {
+      const uint32_t t = wh[w * nb + d];
+      wh[w * nb + d] = (uint16_t)run;
+      run += t;
+    }
+    seg[tid] = run;
+    __syncthreads();
+    uint32_t before = 0, total = 0;
+    for (unsigned q = 0; q < SB_THREADS / nb; ++q) {
+      if (q < part_of) before += seg[q * nb + d];
+      total += seg[q * nb + d];
+    }
+    // every key has the same digit: the order stands
+    if (__syncthreads_or(total == n)) continue;
+    uint32_t in = total;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, in, o);
+      if (lane >= (unsigned)o) in += y;
+    }
+    if (tid < nb && lane == 31) wsum[warp] = in;
+    seg[tid] = before;
+    __syncthreads();
+    if (tid < nb) {
+      uint32_t pre = 0;
+      for (unsigned w = 0; w < warp; ++w) pre += wsum[w];
+      lstart[tid] = pre + in - total;
+    }
+    __syncthreads();
+#pragma unroll
+    for (unsigned r = 0; r < SB_PER; ++r) {
+      if (base + r * 32 < n) {
+        const uint32_t b = (k[r] >> (8 * p)) & 255u;
+        const uint32_t dd = wide ? (v[r] >> 31) << 8 | b : b;
+        const uint32_t to = lstart[dd] + seg[warp / stretch * nb + dd] + mine[dd] + rk[r];
+        skey[to] = k[r];
+        sval[to] = v[r];
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (unsigned r = 0; r < SB_PER; ++r) {
+      const uint32_t i = base + r * 32;
+      if (i < n) {
+        k[r] = skey[i];
+        v[r] = sval[i];
+      }
+    }
+    // (the next pass writes skey only after its own barriers)
+  }
+#pragma unroll
+  for (unsigned r = 0; r < SB_PER; ++r) {
+    const uint32_t i = base + r * 32;
+    if (i < n) {
+      keys[i] = (uint64_t)k[r] << (8 * byte_lo);
+      vals[i] = v[r];
+    }
+  }
+}
+
 void radix_sort_u64(uint64_t *keys, uint32_t *vals, uint32_t n, int byte_lo, int byte_hi,
                     bool partition_hi_bit, const SortScratch &s, cudaStream_t st) {
   if (n == 0) return;
+  if (n <= SORT_BLOCK_MAX && cudaFuncSetAttribute(k_sort_block, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                  (int)SB_SMEM) == cudaSuccess) {
+    D3_LAUNCH(k_sort_block, 1, SB_THREADS, SB_SMEM, st)(keys, vals, n, byte_lo, byte_hi - byte_lo,
+                                                        partition_hi_bit);
+    return;
+  }
   uint64_t *ak = keys, *bk = s.keys_tmp;
   uint32_t *av = vals, *bv = s.vals_tmp;
   const uint32_t tiles = (n + SORT_TILE - 1) / SORT_TILE;

@@ -4,7 +4,7 @@
 // 8-bit digits, per-chunk histograms turned into offsets that keep equal
 // digits in input order) laid out for the GPU: the counts of all passes first,
 // then one launch a pass, a tile of SORT_TILE keys per CTA with a stable in-tile
-// ranking by warp match; a tile gets its place in each digit's run from the
+// ranking by warp ballots; a tile gets its place in each digit's run from the
 // counts the tiles before it publish.
 #pragma once
 
@@ -97,7 +97,7 @@ constexpr unsigned SORT_THREADS = 256;
 constexpr int SORT_PASSES = 4;  // key bytes a sort may take
 
 // Stable sort of (keys, vals)[0..n), n < 2^30, by at most SORT_PASSES key
-// bytes [byte_lo, byte_hi), then (if `partition_hi_bit`) a stable partition on
+// bytes [byte_lo, byte_hi) (the keys have no other bits), then (if `partition_hi_bit`) a stable partition on
 // bit 31 of the value, zeros first (folded into the last byte pass as a 9-bit
 // digit). Results end in keys/vals. Scratch: keys_tmp, vals_tmp (n each) and
 // hist of sort_hist_words(n).

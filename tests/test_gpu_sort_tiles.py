@@ -1,4 +1,5 @@
-"""The device sort at its tiles' edges (2,048 keys), with counts that come from
+"""The device sort at its tiles' edges (2,048 keys), at the most one block takes
+(8,192) and one more, with counts that come from
 many tiles before (more than one read of the look-back), all keys of a pass
 equal (the copy pass) and NaN nodes (the partition): fast many-body and fast
 collide order their sums by it, so positions equal the oracle's bit for bit."""
@@ -13,7 +14,9 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("n,spread", [(1, 9.0), (2, 9.0), (2047, 400.0), (2048, 1e-3), (2049, 400.0),
-                                      (40961, 3000.0), (300001, 8000.0)])
+                                      (8191, 900.0), (8192, 900.0), (8193, 900.0),
+                                      (10240, 900.0), (10241, 900.0), (40961, 3000.0),
+                                      (300001, 8000.0)])
 def test_gpu_sort_tiles(ocore, gcore, n, spread):
     def setup(core):
         rnd = sc.generator(n)
