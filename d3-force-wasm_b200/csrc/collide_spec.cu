@@ -63,6 +63,7 @@ enum : uint32_t {
   C_FAIL_READ, C_FAIL_WRITE, C_FAIL_MOVED, C_FAST_TURNS, C_SLOW_TURNS, C_TIMEOUT,
   C_ALLOC = 16, C_BIGFILL, C_BIGLINK, C_VWORK, C_DONE = 32, C_CLAIM = 64, C_COUNTERS = 128
 };
+constexpr uint32_t GUESS_WARP_NODES = 8192;  // measured at warp_guess
 constexpr uint32_t PR_SLOTS = SPEC_CAP + 1;  // a node's entries: its heads, then itself
 
 // A cell as the collide traversals read it, in one 64-byte load: its box and
@@ -182,9 +183,10 @@ __device__ uint32_t start_cell(const SpecArgs &a, uint32_t i, double xi, double 
   const double slack = (fabs(xi) + fabs(yi) + R) * 0x1p-40 + 1e-300;
   const double h = R + slack;
   while (c != 0 && c != NONE) {
+    const uint32_t up = a.parent[c];  // on its way with the record
     const CRec &q = a.rec[c];
     if (q.x0 < xi - h && q.x1 > xi + h && q.y0 < yi - h && q.y1 > yi + h) break;
-    c = a.parent[c];
+    c = up;
   }
   return c == NONE ? 0 : c;
 }
@@ -251,6 +253,149 @@ __device__ bool spec_guess(const SpecArgs &a, uint32_t i, double margin, bool al
   a.emask[i] = em;
   a.vcount[i] = nv <= VISIT_CAP ? (uint16_t)nv : VISIT_NONE;
   return true;
+}
+
+// The same by a warp: the walk as one list in preorder, every cell of it not
+// yet decided tested by a lane of its own and replaced by nothing (pruned), by
+// itself (a leaf) or by itself and its children, until all are decided: a load
+// latency a level of the tree instead of one a cell. `list` holds two lists of
+// GUESS_CAP entries; 1 done, 0 the guess overflows (as spec_guess), -1 the list
+// does (the caller takes spec_guess). For few nodes (GUESS_WARP_NODES), whose
+// walks in a thread each leave the chip idle: the phase takes 65 to 107 us with
+// a thread a node (chains of 60 to 150 loads, the same at 5,003 and at 50,000
+// nodes), with a warp 45 to 61 us at 5,003 nodes, 67 to 97 at 10,000, 84 to 115
+// at 16,000.
+constexpr uint32_t GUESS_CAP = 320;  // two lists of 8 bytes each: a warp's boxes' place
+constexpr uint32_t G_DECIDED = 1u << 31, G_EXACT = 1u << 30, G_WRITE = 1u << 29, G_HEAD = 1u << 28,
+                   G_CELL = G_HEAD - 1;
+
+__device__ int warp_guess(const SpecArgs &a, uint32_t i, double margin, uint2 *list) {
+  const unsigned lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1;
+  const uint32_t len = a.info[1];
+  const double xi = a.px[i], yi = a.py[i], ri = a.radii[i];
+  if (len > G_CELL) return -1;
+  if (lane == 0) {
+    a.rcount[i] = 0;
+    a.wmask[i] = 0;
+    a.emask[i] = 0;
+    a.vcount[i] = 0;
+    a.mdelta[i] = margin;
+  }
+  if (len == 0 || xi != xi || yi != yi) {
+    if (lane == 0) a.start[i] = 0;
+    return 1;
+  }
+  const double rmax = a.rec[0].r;
+  const uint32_t c0 = start_cell(a, i, xi, yi, ri + rmax + margin);
+  if (lane == 0) {
+    a.start[i] = c0;
+    list[0] = make_uint2(c0 | G_EXACT, 0);
+  }
+  __syncwarp();
+  uint2 *src = list, *dst = list + GUESS_CAP;
+  uint32_t cnt = 1;
+  for (bool more = true; more;) {
+    more = false;
+    uint32_t out = 0;
+    for (uint32_t w0 = 0; w0 < cnt; w0 += 32) {
+      uint2 e = make_uint2(0, 0);
+      uint32_t k = 0, ch[4], nch = 0, childs = 0;
+      if (w0 + lane < cnt) {
+        e = src[w0 + lane];
+        k = 1;
+        if (!(e.x & G_DECIDED)) {
+          const uint32_t c = e.x & G_CELL;
+          const CRec q = a.rec[c];
+          const uint32_t *cp = a.cells[c].child;
+#pragma unroll
+          for (int t = 0; t < 4; ++t) ch[t] = cp[t];
+          const double r = ri + q.r;
+          e.y = q.link;
+          if (rec_leaf(q)) {
+            e.x |= G_DECIDED;
+            const uint32_t j = q.link & ~LEAF_TAG;
+            if (j > i) {
+              e.x |= G_HEAD;
+              const double dx = xi - q.hx, dy = yi - q.hy;
+              const double rr = r + margin + (double)q.margin;
+              if (dx * dx + dy * dy < rr * rr) e.x |= G_WRITE;
+            }
+          } else if (pruned(q, xi, yi, r + margin)) {
+            k = 0;
+          } else {
+            childs = e.x & G_EXACT && !pruned(q, xi, yi, r) ? G_EXACT : 0;
+            e.x |= G_DECIDED;
+#pragma unroll
+            for (int t = 0; t < 4; ++t) nch += ch[t] != NONE;
+          }
+        }
+      }
+      const uint32_t put = k ? 1 + nch : 0;
+      const unsigned b0 = __ballot_sync(FULL, put & 1), b1 = __ballot_sync(FULL, put & 2),
+                     b2 = __ballot_sync(FULL, put & 4);
+      uint32_t at = out + __popc(b0 & lt) + 2 * __popc(b1 & lt) + 4 * __popc(b2 & lt);
+      out += __popc(b0) + 2 * __popc(b1) + 4 * __popc(b2);
+      if (out > GUESS_CAP) return -1;
+      if (k) dst[at++] = e;
+      if (nch) {
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+          if (ch[t] != NONE) dst[at++] = make_uint2(ch[t] | childs, 0);
+      }
+      if (__any_sync(FULL, nch != 0)) more = true;
+    }
+    __syncwarp();
+    cnt = out;
+    uint2 *t = src; src = dst; dst = t;
+  }
+  uint32_t *rl = a.rlist + (size_t)i * SPEC_CAP;
+  uint32_t *vl = a.vlist + (size_t)i * VISIT_CAP;
+  uint32_t *va = a.vaux + (size_t)i * VISIT_CAP;
+  uint32_t nr = 0;
+  uint64_t wm = 0, em = 0;
+  for (uint32_t w0 = 0; w0 < cnt; w0 += 32) {
+    const uint32_t t = w0 + lane;
+    const uint2 e = t < cnt ? src[t] : make_uint2(0, 0);
+    if (t < cnt && t < VISIT_CAP) {
+      vl[t] = e.x & G_CELL;
+      va[t] = e.y;
+    }
+    const unsigned hb = __ballot_sync(FULL, e.x & G_HEAD);
+    const uint32_t h = nr + __popc(hb & lt);
+    nr += __popc(hb);
+    if (nr > SPEC_CAP) return 0;
+    if (e.x & G_HEAD) {
+      rl[h] = e.y & ~LEAF_TAG;
+      if (e.x & G_WRITE) wm |= 1ull << h;
+      if (e.x & G_EXACT) em |= 1ull << h;
+    }
+  }
+  wm = (uint64_t)__reduce_or_sync(FULL, (uint32_t)(wm >> 32)) << 32 | __reduce_or_sync(FULL, (uint32_t)wm);
+  em = (uint64_t)__reduce_or_sync(FULL, (uint32_t)(em >> 32)) << 32 | __reduce_or_sync(FULL, (uint32_t)em);
+  if (lane == 0) {
+    a.rcount[i] = (uint8_t)nr;
+    a.wmask[i] = wm;
+    a.emask[i] = em;
+    a.vcount[i] = cnt <= VISIT_CAP ? (uint16_t)cnt : VISIT_NONE;
+  }
+  __syncwarp();
+  return 1;
+}
+
+// spec_guess_fit by a warp.
+__device__ bool warp_guess_fit(const SpecArgs &a, uint32_t i, double margin, uint2 *list) {
+  for (;;) {
+    int res = warp_guess(a, i, margin, list);
+    if (res < 0) {
+      __syncwarp();
+      if ((threadIdx.x & 31) == 0) res = spec_guess(a, i, margin, false);
+      res = __shfl_sync(FULL, res, 0);
+    }
+    if (res) return true;
+    if (!(margin > a.delta0)) return false;
+    margin = margin * 0.5 > a.delta0 ? margin * 0.5 : a.delta0;
+  }
 }
 
 // Which guessed heads node i examines from (xi, yi), once i has moved: a mask
@@ -321,8 +466,8 @@ __device__ bool warp_replay(const SpecArgs &a, uint32_t i, double xi, double yi,
     }
     ex = max(ex, upto[u]);
   }
-  for (int o = 16; o > 0; o >>= 1) m |= __shfl_xor_sync(0xffffffffu, m, o);
-  mask = m;
+  mask = (uint64_t)__reduce_or_sync(0xffffffffu, (uint32_t)(m >> 32)) << 32 |
+         __reduce_or_sync(0xffffffffu, (uint32_t)m);
   return true;
 }
 
@@ -773,21 +918,26 @@ __device__ void warp_link(const SpecArgs &a, uint32_t base) {
   }
 }
 
-__device__ inline uint8_t ld_acquire_u8(const uint8_t *p) {
-  uint16_t v;
-  asm volatile("ld.acquire.gpu.global.u8 %0, [%1];" : "=h"(v) : "l"(p) : "memory");
-  return (uint8_t)v;
+__device__ inline uint32_t ld_acquire(const uint32_t *p) {
+  uint32_t v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ inline void st_relaxed(uint32_t *p, uint32_t v) {
+  asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
 // A lane's wait on the turns of one wait range (see wait_range; `first`: the
-// first turn's node, already known): until none is pending any more. dmax gets their largest depth. Gives up (false) after
+// first turn's node, already known): until each has its depth (`lev`, zero
+// until the turn is done). dmax gets the largest. Gives up (false) after
 // SPEC_WAIT_NS in which no turn anywhere finished.
 __device__ bool wait_on(const SpecArgs &a, uint64_t r, uint32_t first, uint32_t &dmax,
                         unsigned long long &t0, uint32_t &seen) {
   const uint32_t c = (uint32_t)r & 0x7fffffffu;
   for (uint32_t t = 0; t < c; ++t) {
     const uint32_t x = t ? (uint32_t)(rd(&a.ents[(r >> 32) + t]) >> 32) : first;
-    for (uint32_t it = 0; ld_acquire_u8(&a.state[x]) == 1; ++it) {
+    uint32_t lv;
+    for (uint32_t it = 0; (lv = ld_acquire(&a.lev[x])) == 0; ++it) {
       if (it >= 4 && a.sleep_ns) __nanosleep(a.sleep_ns);
       if ((it & 15) == 15) {
         const uint32_t d = ld_relaxed(&a.counters[C_DONE]);
@@ -800,7 +950,7 @@ __device__ bool wait_on(const SpecArgs &a, uint64_t r, uint32_t first, uint32_t 
         }
       }
     }
-    dmax = max(dmax, ld_relaxed(&a.lev[x]));
+    dmax = max(dmax, lv);
   }
   return true;
 }
@@ -810,7 +960,13 @@ struct TurnTally {
   uint32_t fast = 0, slow = 0, depth = 0;
 };
 
-// Node i's turn, by one warp: everything about it that cannot change (its
+// Node i's turn, by one warp. Turns that wait on one another follow each other
+// by a message through L2 (write, fence, `lev`, read), and that chain bounds
+// the phase, so what is not needed for it stays out: the depth is the flag that
+// is waited on, all velocities are asked for before the first is used, and the
+// tallies of the check are added after the flag. A link of the chain took 3.3 to
+// 5.6 us, now 2.3 to 4.4 (5,003 nodes, depth 33: 120 -> 90 us; 50,000 nodes,
+// depth 86: 652 -> 515 us). Everything about the node that cannot change (its
 // guessed heads, lane k holding heads k and k + 32, with their positions and
 // radii; its record; its masks and pass-start velocity; the first turn each
 // of its accesses waits on) is loaded first; then the warp waits until every
@@ -880,18 +1036,11 @@ __device__ void warp_pull(const SpecArgs &a, uint32_t i, bool stamp, TurnTally &
   for (int k = 0; k < 3; ++k)
     if (waited) waited = wait_on(a, ww[k], first[k], dmax, t0, seen);
   if (!__all_sync(FULL, waited) && lane == 0) atomicAdd(&a.counters[C_TIMEOUT], 1u);
-  for (int o = 16; o > 0; o >>= 1) dmax = max(dmax, __shfl_xor_sync(FULL, dmax, o));
   // the velocities, each read by the lane whose acquiring waits cover it: the
   // node's own by lane 0 (it waited on the node's own accesses), its heads'
   // by their lanes (no other turn writes the heads of a running turn: the
   // values loaded here are what its pushes update)
-  double vi = 0, wi = 0;
-  if (lane == 0) {
-    vi = rd(&a.vxs[i]);
-    wi = rd(&a.vys[i]);
-  }
-  vi = __shfl_sync(FULL, vi, 0);
-  wi = __shfl_sync(FULL, wi, 0);
+  // (all loads are on their way before the first value is used)
   double hv[2], hw[2];
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
@@ -900,6 +1049,14 @@ __device__ void warp_pull(const SpecArgs &a, uint32_t i, bool stamp, TurnTally &
     hv[h] = rd(&a.vxs[jj[h]]);
     hw[h] = rd(&a.vys[jj[h]]);
   }
+  double vi = 0, wi = 0;
+  if (lane == 0) {
+    vi = rd(&a.vxs[i]);
+    wi = rd(&a.vys[i]);
+  }
+  dmax = __reduce_max_sync(FULL, dmax);
+  vi = __shfl_sync(FULL, vi, 0);
+  wi = __shfl_sync(FULL, wi, 0);
   const bool unmoved = same_bits(vi, svi) && same_bits(wi, swi);
   // per head: the offset (x, y) = (xi - xs[j] - vxs[j], ...) of the turn,
   // formed as the turn forms it
@@ -962,7 +1119,8 @@ __device__ void warp_pull(const SpecArgs &a, uint32_t i, bool stamp, TurnTally &
   }
   fail = __any_sync(FULL, fail);
   jig = __any_sync(FULL, jig);
-  for (int o = 16; o > 0; o >>= 1) over |= __shfl_xor_sync(FULL, over, o);
+  over = (uint64_t)__reduce_or_sync(FULL, (uint32_t)(over >> 32)) << 32 |
+         __reduce_or_sync(FULL, (uint32_t)over);
   __syncwarp();
   uint8_t result = 2;
   const bool holds = !(fail_read || fail || jig);
@@ -997,18 +1155,24 @@ __device__ void warp_pull(const SpecArgs &a, uint32_t i, bool stamp, TurnTally &
       const uint32_t j = jj[h];
       a.vxs[j] = hv[h] - pdx[h];
       a.vys[j] = hw[h] - pdy[h];
-      atomicAdd(&a.push[j], sqrt(pdx[h] * pdx[h] + pdy[h] * pdy[h]));
-      atomicMin(&a.min_pusher[j], i);
-      atomicMax(&a.max_pusher[j], i);
     }
   }
-  // done: after the writes (a turn that wrote nothing has finished its reads)
+  // done: after the writes (a turn that wrote nothing has finished its reads).
+  // What only the check reads comes after it, out of the chain of turns.
   if (holds && over) __threadfence();
   __syncwarp();
   const uint32_t lv = dmax + 1;
   tally.depth = max(tally.depth, lv);
+  if (lane == 0) st_relaxed(&a.lev[i], lv);
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    if (!holds || !pushed[h]) continue;
+    const uint32_t j = jj[h];
+    atomicAdd(&a.push[j], sqrt(pdx[h] * pdx[h] + pdy[h] * pdy[h]));
+    atomicMin(&a.min_pusher[j], i);
+    atomicMax(&a.max_pusher[j], i);
+  }
   if (lane == 0) {
-    a.lev[i] = lv;
     a.state[i] = result;
     atomicAdd(&a.counters[C_DONE], 1u);
     if (stamp) {
@@ -1061,6 +1225,16 @@ __device__ void spec_serial(const SpecArgs &a) {
   a.rng->lcg = s;
 }
 
+// The node's pass-start snapshot and tallies.
+__device__ inline void reset_node(const SpecArgs &a, uint32_t i) {
+  a.svx[i] = a.vxs[i];
+  a.svy[i] = a.vys[i];
+  a.push[i] = 0;
+  a.min_pusher[i] = NONE;
+  a.max_pusher[i] = 0;
+  a.aflag[i] = 0;
+}
+
 __global__ void __launch_bounds__(SPEC_THREADS, 2) k_collide_spec(SpecArgs a) {
   __shared__ double contrib[SPEC_WARPS][2][SPEC_CAP];
   extern __shared__ Box boxes_all[];  // SPEC_WARPS * VISIT_CAP (dynamic)
@@ -1105,28 +1279,42 @@ __global__ void __launch_bounds__(SPEC_THREADS, 2) k_collide_spec(SpecArgs a) {
   }
   g.sync();
   // G, plus per-node resets, the pass-start snapshot and the access counts.
-  for (uint32_t i = tid; i < n; i += nth) {
-    a.svx[i] = a.vxs[i];
-    a.svy[i] = a.vys[i];
-    a.push[i] = 0;
-    a.min_pusher[i] = NONE;
-    a.max_pusher[i] = 0;
-    a.aflag[i] = 0;
-    if (!spec_guess_fit(a, i, margin_of(a, i), false)) {
-      atomicAdd(&a.counters[C_OVERFLOW], 1u);
-      a.state[i] = 0;
-      continue;
+  if (n <= GUESS_WARP_NODES) {
+    for (uint32_t i = gw; i < n; i += nwarps) {
+      const bool fits = warp_guess_fit(a, i, margin_of(a, i),
+                                       reinterpret_cast<uint2 *>(boxes_all + (size_t)wl * VISIT_CAP));
+      __syncwarp();
+      const uint64_t wm = fits ? rd(&a.wmask[i]) : 0;
+      if (lane == 0) {
+        reset_node(a, i);
+        if (!fits) atomicAdd(&a.counters[C_OVERFLOW], 1u);
+        a.state[i] = wm ? 1 : 0;
+        if (wm) {
+          a.active[atomicAdd(&a.counters[C_ACTIVE], 1u)] = i;
+          a.aflag[i] = 1;
+        }
+      }
+      if (wm) warp_count(a, i);
     }
-    if (a.wmask[i]) {
-      a.state[i] = 1;
-      a.active[atomicAdd(&a.counters[C_ACTIVE], 1u)] = i;
-      a.aflag[i] = 1;
-      const uint32_t *rl = a.rlist + (size_t)i * SPEC_CAP;
-      const uint32_t nr = a.rcount[i];
-      for (uint32_t h = 0; h < nr; ++h) atomicAdd(&a.cnt[rl[h]], 1u);
-      atomicAdd(&a.cnt[i], 1u);
-    } else {
-      a.state[i] = 0;
+  } else {
+    for (uint32_t i = tid; i < n; i += nth) {
+      reset_node(a, i);
+      if (!spec_guess_fit(a, i, margin_of(a, i), false)) {
+        atomicAdd(&a.counters[C_OVERFLOW], 1u);
+        a.state[i] = 0;
+        continue;
+      }
+      if (a.wmask[i]) {
+        a.state[i] = 1;
+        a.active[atomicAdd(&a.counters[C_ACTIVE], 1u)] = i;
+        a.aflag[i] = 1;
+        const uint32_t *rl = a.rlist + (size_t)i * SPEC_CAP;
+        const uint32_t nr = a.rcount[i];
+        for (uint32_t h = 0; h < nr; ++h) atomicAdd(&a.cnt[rl[h]], 1u);
+        atomicAdd(&a.cnt[i], 1u);
+      } else {
+        a.state[i] = 0;
+      }
     }
   }
   g.sync();
@@ -1262,6 +1450,7 @@ __global__ void __launch_bounds__(SPEC_THREADS, 2) k_collide_spec(SpecArgs a) {
 static int g_spec_blocks = 0;
 // Dynamic shared memory of k_collide_spec: the staged boxes, per warp.
 constexpr size_t SPEC_DYN_SMEM = (size_t)SPEC_WARPS * VISIT_CAP * sizeof(Box);
+static_assert(2 * GUESS_CAP * sizeof(uint2) <= VISIT_CAP * sizeof(Box), "the guess's lists");
 
 // Every device array of the scratch, with its bytes per node of capacity.
 template <class F>
