@@ -203,8 +203,30 @@ void fast_link(const NodeArrays &a, const LinkArrays &l, FastLink &c, double alp
 
 // ---- grid.zig --------------------------------------------------------------
 
+// A block's minimum x, y, maximum x, y, largest radius (b) and count (m), left
+// in thread 0's place of sb and sm.
+__device__ inline void grid_reduce(const double (&b)[5], uint32_t m, double (*sb)[5], uint32_t *sm) {
+  const unsigned t = threadIdx.x;
+  for (int q = 0; q < 5; ++q) sb[t][q] = b[q];
+  sm[t] = m;
+  __syncthreads();
+  for (unsigned s = GRID_THREADS / 2; s > 0; s >>= 1) {
+    if (t < s) {
+      if (sb[t + s][0] < sb[t][0]) sb[t][0] = sb[t + s][0];
+      if (sb[t + s][1] < sb[t][1]) sb[t][1] = sb[t + s][1];
+      if (sb[t + s][2] > sb[t][2]) sb[t][2] = sb[t + s][2];
+      if (sb[t + s][3] > sb[t][3]) sb[t][3] = sb[t + s][3];
+      if (sb[t + s][4] > sb[t][4]) sb[t][4] = sb[t + s][4];
+      sm[t] += sm[t + s];
+    }
+    __syncthreads();
+  }
+}
+
 // Shifted positions, bounds, largest radius and point count; the last block
-// sizes the grid (grid.zig:66-91, 224-258).
+// merges the blocks' and sizes the grid (grid.zig:66-91, 224-258). (Merged by
+// one thread, a load latency a block, the merge was most of the kernel: 6,001
+// nodes 16 -> 13 us, 1 M 626 -> 20 us.)
 __global__ void __launch_bounds__(GRID_THREADS) k_grid_bounds(const double *x, const double *y,
                                                               const double *vx, const double *vy,
                                                               double *px, double *py,
@@ -229,20 +251,7 @@ __global__ void __launch_bounds__(GRID_THREADS) k_grid_bounds(const double *x, c
   __shared__ double sb[GRID_THREADS][5];
   __shared__ uint32_t sm[GRID_THREADS];
   const unsigned t = threadIdx.x;
-  for (int q = 0; q < 5; ++q) sb[t][q] = b[q];
-  sm[t] = m;
-  __syncthreads();
-  for (unsigned s = GRID_THREADS / 2; s > 0; s >>= 1) {
-    if (t < s) {
-      if (sb[t + s][0] < sb[t][0]) sb[t][0] = sb[t + s][0];
-      if (sb[t + s][1] < sb[t][1]) sb[t][1] = sb[t + s][1];
-      if (sb[t + s][2] > sb[t][2]) sb[t][2] = sb[t + s][2];
-      if (sb[t + s][3] > sb[t][3]) sb[t][3] = sb[t + s][3];
-      if (sb[t + s][4] > sb[t][4]) sb[t][4] = sb[t + s][4];
-      sm[t] += sm[t + s];
-    }
-    __syncthreads();
-  }
+  grid_reduce(b, m, sb, sm);
   __shared__ bool last;
   if (t == 0) {
     for (int q = 0; q < 5; ++q) part[blockIdx.x * 6 + q] = sb[0][q];
@@ -251,21 +260,22 @@ __global__ void __launch_bounds__(GRID_THREADS) k_grid_bounds(const double *x, c
     last = atomicAdd(&info[5], 1u) == gridDim.x - 1;
   }
   __syncthreads();
-  if (!last || t != 0) return;
+  if (!last) return;
   __threadfence();
-  double a0 = INFINITY, a1 = INFINITY, a2 = -INFINITY, a3 = -INFINITY, rmax = 0;
-  uint32_t mm = 0;
-  for (unsigned k = 0; k < gridDim.x; ++k) {
-    const volatile double *p = &part[k * 6];
-    uint32_t pm = ((const volatile uint32_t *)&part[k * 6 + 5])[0];
-    if (pm == 0) continue;
-    mm += pm;
-    if (p[0] < a0) a0 = p[0];
-    if (p[2] > a2) a2 = p[2];
-    if (p[1] < a1) a1 = p[1];
-    if (p[3] > a3) a3 = p[3];
-    if (p[4] > rmax) rmax = p[4];
+  double o[5] = {INFINITY, INFINITY, -INFINITY, -INFINITY, 0};
+  m = 0;
+  for (unsigned k = t; k < gridDim.x; k += GRID_THREADS) {
+    const double *p = &part[k * 6];
+    m += __ldcg(reinterpret_cast<const uint32_t *>(&p[5]));
+    for (int q = 0; q < 5; ++q) {
+      const double v = __ldcg(&p[q]);
+      if (q < 2 ? v < o[q] : v > o[q]) o[q] = v;
+    }
   }
+  grid_reduce(o, m, sb, sm);
+  if (t != 0) return;
+  const double a0 = sb[0][0], a1 = sb[0][1], a2 = sb[0][2], a3 = sb[0][3], rmax = sb[0][4];
+  const uint32_t mm = sm[0];
   info[5] = 0;
   info[3] = mm;
   if (mm < 2 || !(rmax > 0)) {
