@@ -43,6 +43,14 @@ constexpr double FMM_MIN_SEP2 = 1e-28;
 constexpr uint32_t FMM_TAB = 2 * FMM_MAX_ORDER + 2;  // rows of the binomial table
 constexpr unsigned LISTS_THREADS = 128;
 constexpr unsigned UP_THREADS = 64, M2L_THREADS = 32, P2P_THREADS = 32, DOWN_THREADS = 64;
+// A P2P list of more than LONG_LIST source leaves (a leaf beside a far denser
+// region) goes by segments of 32; the terms of a segment and 16 targets take a
+// unit of 32 KB, LONG_UNITS_MAX of them at most (256 MB, held once a run wanted
+// some; lists past that, and leaves of more than LONG_POINTS points, go by
+// k_fmm_p2p).
+constexpr uint32_t LONG_LIST = 64, LONG_POINTS = 64, LONG_UNITS_MAX = 8192;
+constexpr uint32_t LONG_UNIT = 32 * 4 * 16;  // terms: source leaf, three pairs and a sum, target
+
 constexpr uint32_t P2P_FEW_CELLS = 4096;  // some 30,000 nodes; measured at k_fmm_p2p
 constexpr uint32_t FMM_STACK = 64;
 
@@ -58,6 +66,7 @@ enum : uint32_t { FI_CELLS = 0, FI_OVERFLOW, FI_LEVELS, FI_POOL_M2L, FI_POOL_P2P
                   FI_LIST_OVERFLOW,              // 1: a pool, 2: a call stack or a wait
                   FI_TICKET,                     // k_fmm_lists' blocks so far
                   FI_LVL = 8,  // FI_LVL + d: first cell of level d
+                  FI_LONG_UNITS = 36, FI_LONGS,  // long P2P lists: units of terms, leaves
                   FI_M = 40,                     // points to act on (0 when the extent is bad)
                   FI_BAD = 41 };                 // 1: the extent is not finite and positive
 
@@ -74,6 +83,10 @@ struct FmmDev {
   FmmTables *tab = nullptr;
   uint32_t tab_p = 0;
   uint32_t *info = nullptr, *arrive = nullptr;
+  uint2 *long_items = nullptr;
+  uint32_t *long_at = nullptr, *longs = nullptr, *long_flags = nullptr;
+  double2 *long_terms = nullptr;
+  uint32_t long_cap = 0, long_want = 0;  // units: held, wanted by the last run
   cudaEvent_t lists_read = nullptr;  // the lists' words are in h_info
   double *square = nullptr;      // box x0, y0, side
   uint32_t *h_info = nullptr;    // pinned mirror of info
@@ -99,6 +112,10 @@ struct FmmArgs {
   uint32_t *m2l, *p2p, *fwd;
   uint32_t *m2l_off, *m2l_cnt, *p2p_off, *p2p_cnt, *fwd_off, *fwd_cnt;
   uint32_t *info, *arrive;
+  uint2 *long_items;  // per unit: the leaf and its item (NONE: not an item's first unit)
+  uint32_t *long_at, *longs, *long_flags;  // per cell: first unit or NONE; the leaves; see there
+  double2 *long_terms;
+  uint32_t long_cap;
   size_t cap_m2l, cap_p2p, cap_fwd;
   uint32_t ncells, p;
   double mac_far, dmax_scaled, dmin_scaled, dmin2, dmax2, inv_w;
@@ -364,6 +381,7 @@ __global__ void __launch_bounds__(32) k_cells_starts(uint32_t ccap, uint32_t *in
   const unsigned used = __ballot_sync(0xffffffffu, x != 0);
   if (lane < CB_LEVELS) info[FI_LVL + lane] = incl - x;
   if (lane == 0) {
+    info[FI_LONG_UNITS] = info[FI_LONGS] = 0;
     info[FI_LVL + CB_LEVELS] = at;
     info[FI_CELLS] = at;
     info[FI_LEVELS] = used ? 32 - __clz(used) : 0;
@@ -824,11 +842,13 @@ __device__ bool reserve_lists(const FmmArgs &a, uint32_t c, uint32_t tm, uint32_
 // their expansion passes the shared lists: lane k expands calls k, k + 32, ...
 // depth first; each call's events are placed after those of the calls before
 // it (a warp scan of the counts). Counts, then a reservation in the pools, then
-// counts again and the writes. Returns the forward list's length.
+// counts again and the writes. Returns the forward list's length; tp the P2P
+// list's.
 __device__ uint32_t expand_long(const FmmArgs &a, uint32_t c, const FCell &A, const uint32_t *in,
-                                uint32_t nin) {
+                                uint32_t nin, uint32_t &tp) {
   const unsigned lane = threadIdx.x & 31;
-  uint32_t tm = 0, tp = 0, tf = 0;
+  uint32_t tm = 0, tf = 0;
+  tp = 0;
   bool ok = true;
   for (uint32_t u0 = 0; u0 < nin; u0 += 32) {
     const uint32_t u = u0 + lane;
@@ -872,13 +892,13 @@ __device__ uint32_t expand_long(const FmmArgs &a, uint32_t c, const FCell &A, co
 // beside a far denser region) takes the depth-first form.
 constexpr uint32_t LIST_CAP = 512;
 __device__ uint32_t expand_cell(const FmmArgs &a, uint32_t c, const FCell &A, const uint32_t *in,
-                                uint32_t nin, uint32_t *buf) {
+                                uint32_t nin, uint32_t *buf, uint32_t &tp) {
   const unsigned lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1;
-  if (nin > LIST_CAP) return expand_long(a, c, A, in, nin);
+  if (nin > LIST_CAP) return expand_long(a, c, A, in, nin, tp);
   for (uint32_t u = lane; u < nin; u += 32) buf[u] = in ? ldg_cg(&in[u]) : 0;
   __syncwarp();
-  uint32_t cnt = nin, tm = 0, tp = 0;
+  uint32_t cnt = nin, tm = 0;
   uint32_t *src = buf, *dst = buf + LIST_CAP;
   for (bool more = true; more;) {
     more = false;
@@ -895,7 +915,7 @@ __device__ uint32_t expand_cell(const FmmArgs &a, uint32_t c, const FCell &A, co
                      b2 = __ballot_sync(0xffffffffu, k & 4);
       const uint32_t at = out + __popc(b0 & lt) + 2 * __popc(b1 & lt) + 4 * __popc(b2 & lt);
       out += __popc(b0) + 2 * __popc(b1) + 4 * __popc(b2);
-      if (out > LIST_CAP) return expand_long(a, c, A, in, nin);
+      if (out > LIST_CAP) return expand_long(a, c, A, in, nin, tp);
       for (uint32_t j = 0; j < k; ++j) dst[at + j] = v + j;
       const uint32_t type = v & ~EV_CELL;
       tm += __popc(__ballot_sync(0xffffffffu, k && type == EV_M2L));
@@ -923,6 +943,26 @@ __device__ uint32_t expand_cell(const FmmArgs &a, uint32_t c, const FCell &A, co
     of += __popc(bf);
   }
   return tf;
+}
+
+// A leaf with a long P2P list (tp > LONG_LIST): its units, if they fit;
+// long_at[c] = the first.
+__device__ void plan_long(const FmmArgs &a, uint32_t c, uint32_t count, uint32_t tp) {
+  const unsigned lane = threadIdx.x & 31;
+  uint32_t at = NONE;
+  if (count <= LONG_POINTS) {
+    const uint32_t per = count <= 16 ? 1 : 2;  // units an item: targets in lanes / 16
+    const uint32_t items = (tp + 31) / 32 * ((count + 31) / 32), units = items * per;
+    if (lane == 0) at = atomicAdd(&a.info[FI_LONG_UNITS], units);
+    at = __shfl_sync(0xffffffffu, at, 0);
+    const bool fits = (size_t)at + units <= a.long_cap;
+    for (uint32_t j = lane; j < units; j += 32)
+      if ((size_t)at + j < a.long_cap)
+        a.long_items[at + j] = make_uint2(fits && j % per == 0 ? c : NONE, j / per);
+    if (!fits) at = NONE;
+    else if (lane == 0) a.longs[atomicAdd(&a.info[FI_LONGS], 1u)] = c;
+  }
+  if (lane == 0) a.long_at[c] = at;
 }
 
 // A warp per cell, in level order (blocks numbered as they start, so a block's
@@ -960,11 +1000,14 @@ __global__ void __launch_bounds__(LISTS_THREADS) k_fmm_lists(FmmArgs a) {
     nin = __shfl_sync(0xffffffffu, nin, 0);
     in = a.fwd + (nin ? ldg_cg(&a.fwd_off[A.parent]) : 0);
   }
-  const uint32_t tf = expand_cell(a, c, A, in, nin, buf[warp]);
+  uint32_t tp = 0;
+  const uint32_t tf = expand_cell(a, c, A, in, nin, buf[warp], tp);
   if (A.nchild) {
     __threadfence();
     __syncwarp();
     if (lane == 0) st_release(&a.fwd_cnt[c], tf);
+  } else if (tp > LONG_LIST) {
+    plan_long(a, c, A.count, tp);
   }
 }
 
@@ -1134,48 +1177,54 @@ struct Sources {
   double x[32], y[32], s[32];
 };
 
-// A target's sums within one source leaf: four pairs per division on two lanes
-// (sum 0: k, k + 2; sum 1: k + 1, k + 3), pairs that cannot go that way added to
-// the velocity one by one.
-// One thread has both sums; `b0` is the chunk's first point.
+// Four pairs of a target by one division, on two lanes (sum 0: k, k + 2; sum 1:
+// k + 1, k + 3); false, with nothing added, if they have to go one by one.
+__device__ inline bool group_four(const FmmArgs &a, uint32_t ti, uint32_t b0, uint32_t k,
+                                  const Sources &src, double xi, double yi, double &ax0, double &ay0,
+                                  double &ax1, double &ay1) {
+  const double xa0 = src.x[k] - xi, xa1 = src.x[k + 1] - xi;
+  const double ya0 = src.y[k] - yi, ya1 = src.y[k + 1] - yi;
+  const double xb0 = src.x[k + 2] - xi, xb1 = src.x[k + 3] - xi;
+  const double yb0 = src.y[k + 2] - yi, yb1 = src.y[k + 3] - yi;
+  const double la0 = xa0 * xa0 + ya0 * ya0, la1 = xa1 * xa1 + ya1 * ya1;
+  const double lb0 = xb0 * xb0 + yb0 * yb0, lb1 = xb1 * xb1 + yb1 * yb1;
+  const double z0 = xa0 * ya0 * xb0 * yb0, z1 = xa1 * ya1 * xb1 * yb1;
+  const double mn = zmin(zmin(la0, lb0), zmin(la1, lb1));
+  if (z0 == 0 || z1 == 0 || !(mn >= a.dmin2) || ti - (b0 + k) < 4) return false;
+  const double pa = la0 * la1, pb = lb0 * lb1;
+  const double inv = 1 / (pa * pb);
+  double wa0 = src.s[k] * la1 * pb * inv, wa1 = src.s[k + 1] * la0 * pb * inv;
+  double wb0 = src.s[k + 2] * lb1 * pa * inv, wb1 = src.s[k + 3] * lb0 * pa * inv;
+  if (a.has_dmax) {
+    if (!(la0 < a.dmax2)) wa0 = 0;
+    if (!(la1 < a.dmax2)) wa1 = 0;
+    if (!(lb0 < a.dmax2)) wb0 = 0;
+    if (!(lb1 < a.dmax2)) wb1 = 0;
+  }
+  ax0 += xa0 * wa0 + xb0 * wb0;
+  ax1 += xa1 * wa1 + xb1 * wb1;
+  ay0 += ya0 * wa0 + yb0 * wb0;
+  ay1 += ya1 * wa1 + yb1 * wb1;
+  return true;
+}
+
+// A target's sums within one source leaf: its groups of four, pairs that cannot
+// go that way added to the velocity one by one. One thread has both sums; `b0`
+// is the chunk's first point.
 __device__ inline void leaf_one(const FmmArgs &a, uint64_t seed, uint32_t ti, uint32_t b0, uint32_t cn,
                                 const Sources &src, double xi, double yi, double &vx, double &vy,
                                 double &ax0, double &ay0, double &ax1, double &ay1) {
   uint32_t k = 0;
   for (; k + 4 <= cn; k += 4) {
-    const double xa0 = src.x[k] - xi, xa1 = src.x[k + 1] - xi;
-    const double ya0 = src.y[k] - yi, ya1 = src.y[k + 1] - yi;
-    const double xb0 = src.x[k + 2] - xi, xb1 = src.x[k + 3] - xi;
-    const double yb0 = src.y[k + 2] - yi, yb1 = src.y[k + 3] - yi;
-    const double la0 = xa0 * xa0 + ya0 * ya0, la1 = xa1 * xa1 + ya1 * ya1;
-    const double lb0 = xb0 * xb0 + yb0 * yb0, lb1 = xb1 * xb1 + yb1 * yb1;
-    const double z0 = xa0 * ya0 * xb0 * yb0, z1 = xa1 * ya1 * xb1 * yb1;
-    const double mn = zmin(zmin(la0, lb0), zmin(la1, lb1));
-    if (z0 == 0 || z1 == 0 || !(mn >= a.dmin2) || ti - (b0 + k) < 4) {
+    if (group_four(a, ti, b0, k, src, xi, yi, ax0, ay0, ax1, ay1)) continue;
 #pragma unroll 1
-      for (uint32_t u = 0; u < 4; ++u) {
-        double tx, ty;
-        if (pair_term(a, seed, ti, b0 + k + u, src.s[k + u], src.x[k + u], src.y[k + u], xi, yi, tx, ty)) {
-          vx += tx;
-          vy += ty;
-        }
+    for (uint32_t u = 0; u < 4; ++u) {
+      double tx, ty;
+      if (pair_term(a, seed, ti, b0 + k + u, src.s[k + u], src.x[k + u], src.y[k + u], xi, yi, tx, ty)) {
+        vx += tx;
+        vy += ty;
       }
-      continue;
     }
-    const double pa = la0 * la1, pb = lb0 * lb1;
-    const double inv = 1 / (pa * pb);
-    double wa0 = src.s[k] * la1 * pb * inv, wa1 = src.s[k + 1] * la0 * pb * inv;
-    double wb0 = src.s[k + 2] * lb1 * pa * inv, wb1 = src.s[k + 3] * lb0 * pa * inv;
-    if (a.has_dmax) {
-      if (!(la0 < a.dmax2)) wa0 = 0;
-      if (!(la1 < a.dmax2)) wa1 = 0;
-      if (!(lb0 < a.dmax2)) wb0 = 0;
-      if (!(lb1 < a.dmax2)) wb1 = 0;
-    }
-    ax0 += xa0 * wa0 + xb0 * wb0;
-    ax1 += xa1 * wa1 + xb1 * wb1;
-    ay0 += ya0 * wa0 + yb0 * wb0;
-    ay1 += ya1 * wa1 + yb1 * wb1;
   }
 #pragma unroll 1
   for (; k < cn; ++k) {
@@ -1282,8 +1331,8 @@ __device__ inline void leaf_many(const FmmArgs &a, uint64_t seed, uint32_t ti, u
 // us at 6,000 nodes (now 52) and 759 us at 1 M (now 620). FEW: four warps
 // a leaf, eight targets each and four lanes a target, where the leaves do not
 // fill the chip: shorter chains for a sixth more work. Against a lane or two a
-// target, evenly spread / clustered: 6,000 nodes 25 / 64 us for 37 / 84; 20,000
-// 39 / 150 for 35 / 200; 80,000 104 / 360 for 68 / 478 (one leaf's long list).
+// target, evenly spread / clustered (long lists included): 6,000 nodes 25 / 64
+// us for 37 / 84; 20,000 39 / 150 for 35 / 200; 80,000 104 / 360 for 68 / 478.
 template <bool FEW>
 __global__ void __launch_bounds__(P2P_THREADS) k_fmm_p2p(FmmArgs a) {
   __shared__ Sources sources[P2P_THREADS / 32];
@@ -1295,7 +1344,7 @@ __global__ void __launch_bounds__(P2P_THREADS) k_fmm_p2p(FmmArgs a) {
   const uint32_t c = FEW ? gw >> 2 : gw, skip = FEW ? (gw & 3) * 8 : 0;
   if (c >= a.ncells) return;
   const uint32_t cnt = a.p2p_cnt[c];
-  if (!cnt) return;
+  if (!cnt || (cnt > LONG_LIST && a.long_at[c] != NONE)) return;
   const uint32_t off = a.p2p_off[c], first = a.cells[c].first, count = a.cells[c].count;
   const bool two = count <= 16;
   for (uint32_t base = first + skip; base < first + count; base += 32) {
@@ -1349,6 +1398,165 @@ __global__ void __launch_bounds__(P2P_THREADS) k_fmm_p2p(FmmArgs a) {
       }
     }
     if (live && (FEW ? lane % 4 == 0 : !two || lane % 2 == 0)) {
+      a.vx[i] = vx;
+      a.vy[i] = vy;
+    }
+  }
+}
+
+// Long lists. A target's velocity is a chain over all pairs of its list, but
+// within a source leaf the chain's terms do not depend on the velocity: the sums
+// of the groups of four, after up to three pairs of their own. So a warp per
+// segment of 32 source leaves writes every leaf's terms (a pair without a term
+// writes -0, which changes nothing), and a warp per leaf then adds them in
+// order; a source leaf with groups that go pair by pair (`long_flags`, a bit a
+// leaf of the segment) is summed there as before. P2P in all, clustered nodes:
+// 20,000 150 -> 99 us, 80,000 478 -> 173, 160,000 329 -> 180.
+constexpr unsigned LONG_THREADS = 64, LONG_BLOCKS = 2368;
+
+__global__ void __launch_bounds__(LONG_THREADS) k_fmm_p2p_terms(FmmArgs a) {
+  __shared__ Sources sources[LONG_THREADS / 32];
+  if (a.info[FI_LIST_OVERFLOW]) return;
+  const unsigned lane = threadIdx.x & 31;
+  Sources &src = sources[threadIdx.x >> 5];
+  const uint64_t seed = (uint64_t)__double_as_longlong(*a.seed);
+  const uint32_t units = min(a.info[FI_LONG_UNITS], a.long_cap);
+  for (uint32_t u = (blockIdx.x * LONG_THREADS + threadIdx.x) >> 5; u < units;
+       u += gridDim.x * LONG_THREADS >> 5) {
+    const uint2 item = a.long_items[u];
+    const uint32_t c = item.x;
+    if (c == NONE) continue;
+    const uint32_t cnt = a.p2p_cnt[c], off = a.p2p_off[c];
+    const uint32_t first = a.cells[c].first, count = a.cells[c].count;
+    const uint32_t nseg = (cnt + 31) / 32, chunk = item.y / nseg, e0 = item.y % nseg * 32;
+    const uint32_t wide = count <= 16 ? 16 : 32;
+    const uint32_t at = first + chunk * 32 + lane;
+    const bool live = at < first + count;  // (lanes past `wide` are not)
+    const uint32_t ti = live ? at : first;
+    const double xi = a.px[ti], yi = a.py[ti];
+    double2 *terms = a.long_terms + (size_t)u * LONG_UNIT;
+    const uint32_t ne = min(32u, cnt - e0);
+    uint32_t lb = 0, ln = 0;
+    if (lane < ne) {
+      const uint32_t B = a.p2p[off + e0 + lane];
+      lb = a.cells[B].first;
+      ln = a.cells[B].count;
+    }
+    uint32_t flags = 0;
+    uint32_t b0 = __shfl_sync(0xffffffffu, lb, 0), bn = __shfl_sync(0xffffffffu, ln, 0);
+    double rx = 0, ry = 0, rs = 0;
+    if (lane < bn) { rx = a.px[b0 + lane]; ry = a.py[b0 + lane]; rs = a.ps[b0 + lane]; }
+    for (uint32_t e = 0; e < ne; ++e) {
+      const uint32_t cb = b0, cn = bn;
+      __syncwarp();
+      src.x[lane] = rx;
+      src.y[lane] = ry;
+      src.s[lane] = rs;
+      __syncwarp();
+      b0 = __shfl_sync(0xffffffffu, lb, (e + 1) & 31);
+      bn = __shfl_sync(0xffffffffu, ln, (e + 1) & 31);
+      if (e + 1 < ne && lane < bn) { rx = a.px[b0 + lane]; ry = a.py[b0 + lane]; rs = a.ps[b0 + lane]; }
+      if (cn > 32) {
+        flags |= 1u << e;
+        continue;
+      }
+      double ax0 = 0, ax1 = 0, ay0 = 0, ay1 = 0;
+      bool bad = false;
+      uint32_t k = 0;
+      for (; k + 4 <= cn; k += 4)
+        bad |= !group_four(a, ti, cb, k, src, xi, yi, ax0, ay0, ax1, ay1);
+      if (bad) flags |= 1u << e;
+      for (uint32_t t = 0; k < cn; ++k, ++t) {
+        double tx, ty;
+        if (!pair_term(a, seed, ti, cb + k, src.s[k], src.x[k], src.y[k], xi, yi, tx, ty)) tx = ty = -0.0;
+        if (live) terms[(e * 4 + t) * wide + lane] = make_double2(tx, ty);
+      }
+      if (live) terms[(e * 4 + 3) * wide + lane] = make_double2(ax0 + ax1, ay0 + ay1);
+    }
+    if (live) a.long_flags[(size_t)u * 16 + lane] = flags;
+  }
+}
+
+__global__ void __launch_bounds__(LONG_THREADS) k_fmm_p2p_add(FmmArgs a) {
+  __shared__ Sources sources[LONG_THREADS / 32];
+  if (a.info[FI_LIST_OVERFLOW]) return;
+  const unsigned lane = threadIdx.x & 31;
+  Sources &src = sources[threadIdx.x >> 5];
+  const uint64_t seed = (uint64_t)__double_as_longlong(*a.seed);
+  const uint32_t longs = 2 * a.info[FI_LONGS];  // two chunks of targets a leaf
+  for (uint32_t w = (blockIdx.x * LONG_THREADS + threadIdx.x) >> 5; w < longs;
+       w += gridDim.x * LONG_THREADS >> 5) {
+    const uint32_t c = a.longs[w >> 1], chunk = w & 1;
+    const uint32_t cnt = a.p2p_cnt[c], off = a.p2p_off[c];
+    const uint32_t first = a.cells[c].first, count = a.cells[c].count;
+    if (chunk * 32 >= count) continue;
+    const uint32_t nseg = (cnt + 31) / 32, per = count <= 16 ? 1 : 2, wide = 16 * per;
+    const uint32_t at = first + chunk * 32 + lane;
+    const bool live = at < first + count;
+    const uint32_t ti = live ? at : first;
+    const uint32_t i = a.perm[ti], row = live ? lane : 0;
+    const double xi = a.px[ti], yi = a.py[ti];
+    double vx = a.vx[i], vy = a.vy[i];
+    for (uint32_t sg = 0; sg < nseg; ++sg) {
+      const uint32_t u = a.long_at[c] + (chunk * nseg + sg) * per;
+      const double2 *terms = a.long_terms + (size_t)u * LONG_UNIT + row;
+      const uint32_t flags = live ? a.long_flags[(size_t)u * 16 + lane] : 0;
+      const uint32_t e0 = sg * 32, ne = min(32u, cnt - e0);
+      uint32_t lb = 0, ln = 0;
+      if (lane < ne) {
+        const uint32_t B = a.p2p[off + e0 + lane];
+        lb = a.cells[B].first;
+        ln = a.cells[B].count;
+      }
+      // four source leaves' terms at a time on their way
+      constexpr uint32_t AHEAD = 4;
+      double2 buf[AHEAD][4];
+#pragma unroll
+      for (uint32_t q = 0; q < AHEAD; ++q)
+#pragma unroll
+        for (uint32_t t = 0; t < 4; ++t) buf[q][t] = terms[(q * 4 + t) * wide];
+      for (uint32_t eb = 0; eb < ne; eb += AHEAD) {
+#pragma unroll
+        for (uint32_t q = 0; q < AHEAD; ++q) {
+          const uint32_t e = eb + q;
+          if (e >= ne) break;
+          const uint32_t b0 = __shfl_sync(0xffffffffu, lb, e), bn = __shfl_sync(0xffffffffu, ln, e);
+          const bool by_pairs = flags >> e & 1u;
+          if (!by_pairs) {
+#pragma unroll
+            for (uint32_t t = 0; t < 3; ++t)
+              if (t < (bn & 3)) {
+                vx += buf[q][t].x;
+                vy += buf[q][t].y;
+              }
+            vx += buf[q][3].x;
+            vy += buf[q][3].y;
+          }
+          if (e + AHEAD < 32)
+#pragma unroll
+            for (uint32_t t = 0; t < 4; ++t) buf[q][t] = terms[((e + AHEAD) * 4 + t) * wide];
+          if (__any_sync(0xffffffffu, by_pairs)) {
+            double ax0 = 0, ax1 = 0, ay0 = 0, ay1 = 0;
+            for (uint32_t o = 0; o < bn; o += 32) {
+              const uint32_t cn = min(32u, bn - o);
+              __syncwarp();
+              if (lane < cn) {
+                src.x[lane] = a.px[b0 + o + lane];
+                src.y[lane] = a.py[b0 + o + lane];
+                src.s[lane] = a.ps[b0 + o + lane];
+              }
+              __syncwarp();
+              if (by_pairs) leaf_one(a, seed, ti, b0 + o, cn, src, xi, yi, vx, vy, ax0, ay0, ax1, ay1);
+            }
+            if (by_pairs) {
+              vx += ax0 + ax1;
+              vy += ay0 + ay1;
+            }
+          }
+        }
+      }
+    }
+    if (live) {
       a.vx[i] = vx;
       a.vy[i] = vy;
     }
@@ -1503,7 +1711,7 @@ int fmm_reserve_cells(FmmDev &f, uint32_t ccap) {
   if (ccap <= f.ccap && f.ccap) return 0;
   cudaFree(f.cells); cudaFree(f.bx0); cudaFree(f.by0); cudaFree(f.bx1); cudaFree(f.by1);
   cudaFree(f.m2l_off); cudaFree(f.m2l_cnt); cudaFree(f.p2p_off);
-  cudaFree(f.p2p_cnt); cudaFree(f.fwd_off); cudaFree(f.fwd_cnt); cudaFree(f.arrive);
+  cudaFree(f.p2p_cnt); cudaFree(f.fwd_off); cudaFree(f.fwd_cnt); cudaFree(f.arrive); cudaFree(f.long_at);
   D3_CUDA_OK(cudaMalloc(&f.cells, ccap * sizeof(FCell)));
   D3_CUDA_OK(cudaMalloc(&f.bx0, ccap * 8ull));
   D3_CUDA_OK(cudaMalloc(&f.by0, ccap * 8ull));
@@ -1516,6 +1724,7 @@ int fmm_reserve_cells(FmmDev &f, uint32_t ccap) {
   D3_CUDA_OK(cudaMalloc(&f.fwd_off, ccap * 4ull));
   D3_CUDA_OK(cudaMalloc(&f.fwd_cnt, ccap * 4ull));
   D3_CUDA_OK(cudaMalloc(&f.arrive, ccap * 4ull));
+  D3_CUDA_OK(cudaMalloc(&f.long_at, ccap * 4ull));
   f.ccap = ccap;
   return 0;
 }
@@ -1529,7 +1738,8 @@ void fmm_free(FastScratch &s) {
   cudaFree(f->m2l_off); cudaFree(f->m2l_cnt); cudaFree(f->p2p_off);
   cudaFree(f->p2p_cnt); cudaFree(f->fwd_off); cudaFree(f->fwd_cnt); cudaFree(f->m2l);
   cudaFree(f->p2p); cudaFree(f->fwd); cudaFree(f->mco); cudaFree(f->lco); cudaFree(f->tab);
-  cudaFree(f->info); cudaFree(f->arrive); cudaFree(f->square); cudaFree(f->geom);
+  cudaFree(f->info); cudaFree(f->arrive); cudaFree(f->long_at); cudaFree(f->longs);
+  cudaFree(f->long_items); cudaFree(f->long_flags); cudaFree(f->long_terms); cudaFree(f->square); cudaFree(f->geom);
   cudaFree(f->cb_count); cudaFree(f->start_of); cudaFree(f->level_of);
   cudaFreeHost(f->h_info); cudaFreeHost(f->h_geom);
   if (f->lists_read) cudaEventDestroy(f->lists_read);
@@ -1703,6 +1913,27 @@ int fmm_run(FastScratch &s, TreeDev &t, const NodeArrays &a, const double *stren
   args.mco = f.mco;
   args.lco = f.lco;
   args.arrive = f.arrive;
+  if (f.long_want > f.long_cap && f.long_cap < LONG_UNITS_MAX) {
+    // what the last run wanted, and a quarter more
+    cudaFree(f.longs); cudaFree(f.long_items); cudaFree(f.long_flags); cudaFree(f.long_terms);
+    f.longs = f.long_flags = nullptr;
+    f.long_items = nullptr;
+    f.long_terms = nullptr;
+    f.long_cap = 0;
+    const uint32_t want = f.long_want + f.long_want / 4;
+    const size_t cap = want < LONG_UNITS_MAX ? want : LONG_UNITS_MAX;
+    D3_CUDA_OK(cudaMalloc(&f.longs, cap * 4));
+    D3_CUDA_OK(cudaMalloc(&f.long_items, cap * sizeof(uint2)));
+    D3_CUDA_OK(cudaMalloc(&f.long_flags, cap * 16 * 4));
+    D3_CUDA_OK(cudaMalloc(&f.long_terms, cap * LONG_UNIT * sizeof(double2)));
+    f.long_cap = (uint32_t)cap;
+  }
+  args.long_items = f.long_items;
+  args.long_at = f.long_at;
+  args.longs = f.longs;
+  args.long_flags = f.long_flags;
+  args.long_terms = f.long_terms;
+  args.long_cap = f.long_cap;
   args.m2l_off = f.m2l_off; args.m2l_cnt = f.m2l_cnt;
   args.p2p_off = f.p2p_off; args.p2p_cnt = f.p2p_cnt;
   args.fwd_off = f.fwd_off; args.fwd_cnt = f.fwd_cnt;
@@ -1727,11 +1958,13 @@ int fmm_run(FastScratch &s, TreeDev &t, const NodeArrays &a, const double *stren
     args.m2l = f.m2l; args.p2p = f.p2p; args.fwd = f.fwd;
     args.cap_m2l = f.cap_m2l; args.cap_p2p = f.cap_p2p; args.cap_fwd = f.cap_fwd;
     if (cudaMemsetAsync(f.info + FI_POOL_M2L, 0, 5 * sizeof(uint32_t), st) != cudaSuccess) return -1;
-    if (attempt && cudaMemsetAsync(f.fwd_cnt, 0xFF, (size_t)ncells * 4, st) != cudaSuccess) return -1;
+    if (attempt && (cudaMemsetAsync(f.fwd_cnt, 0xFF, (size_t)ncells * 4, st) != cudaSuccess ||
+                    cudaMemsetAsync(f.info + FI_LONG_UNITS, 0, 8, st) != cudaSuccess))
+      return -1;
     D3_LAUNCH(k_fmm_lists, blocks_for(ncells, LISTS_THREADS / 32), LISTS_THREADS, 0, st)(args);
     // the rest follows at once (it does nothing where a list overflowed), and
     // the host reads the lists' words while it runs
-    if (cudaMemcpyAsync(f.h_info, f.info, 8 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st) !=
+    if (cudaMemcpyAsync(f.h_info, f.info, 64 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st) !=
             cudaSuccess ||
         cudaEventRecord(f.lists_read, st) != cudaSuccess)
       return -1;
@@ -1740,6 +1973,10 @@ int fmm_run(FastScratch &s, TreeDev &t, const NodeArrays &a, const double *stren
     if (ncells <= P2P_FEW_CELLS)
       D3_LAUNCH(k_fmm_p2p<true>, blocks_for(4 * ncells, P2P_THREADS / 32), P2P_THREADS, 0, st)(args);
     else D3_LAUNCH(k_fmm_p2p<false>, pb, P2P_THREADS, 0, st)(args);
+    if (f.long_cap) {
+      D3_LAUNCH(k_fmm_p2p_terms, LONG_BLOCKS, LONG_THREADS, 0, st)(args);
+      D3_LAUNCH(k_fmm_p2p_add, LONG_BLOCKS / 8, LONG_THREADS, 0, st)(args);
+    }
     if (dflt) D3_LAUNCH(k_fmm_down<FMM_DEFAULT_ORDER>, db, DOWN_THREADS, down_smem(q), st)(args);
     else D3_LAUNCH(k_fmm_down<0>, db, DOWN_THREADS, down_smem(q), st)(args);
     if (cudaEventSynchronize(f.lists_read) != cudaSuccess) return -1;
@@ -1748,6 +1985,7 @@ int fmm_run(FastScratch &s, TreeDev &t, const NodeArrays &a, const double *stren
       f.last_m2l = f.h_info[FI_POOL_M2L];
       f.last_p2p = f.h_info[FI_POOL_P2P];
       f.last_fwd = f.h_info[FI_POOL_FWD];
+      if (f.h_info[FI_LONG_UNITS] > f.long_cap) f.long_want = f.h_info[FI_LONG_UNITS];
       break;
     }
     if ((ovf & 2) || attempt > 8) return -1;  // a call stack overflowed, or a wait ran out

@@ -1,6 +1,7 @@
 """The fast many-body passes where their shapes turn: orders at which the
 lanes per source and the sources side by side change, lists past the shared
-ones (a dense cluster beside sparse leaves) and past the first pools, leaves of
+ones (a dense cluster beside sparse leaves) and past the first pools, long P2P
+lists in segments, leaves of
 16, 17 and 32 points and of more than a warp's chunk, one leaf as the whole
 tree. Positions equal the oracle's bit for bit."""
 
@@ -22,6 +23,11 @@ def _layout(kind, n):
         x[:k], y[:k] = 1700 + 30 * rng.random(k), 1450 + 30 * rng.random(k)
     if kind == "far":  # one node far from the rest: a leaf child of the root
         x[0], y[0] = 4e5, 4e5
+    if kind == "beside":  # nineteen in twenty in a cluster among sparse leaves
+        k = 19 * n // 20
+        x[:k], y[:k] = 1500 + 120 * rng.standard_normal(k), 1500 + 120 * rng.standard_normal(k)
+        x[:40] = x[0] + 0.3 * rng.random(40)
+        y[:40] = y[0] + 0.3 * rng.random(40)
     if kind == "clump":  # 77 nodes on one spot: three chunks of a source leaf
         x[:77], y[:77] = 1234.5, 777.25
     if kind == "blocks":  # leaves of exactly 16, 17 and 32 points on an 8 x 8 grid
@@ -59,6 +65,15 @@ def test_gpu_fmm_orders(ocore, gcore, order):
                                          ("uniform", 33, None), ("uniform", 17, None)])
 def test_gpu_fmm_shapes(ocore, gcore, kind, n, dmax):
     _run(ocore, gcore, kind, n, 3, dmax=dmax)
+
+
+@pytest.mark.parametrize("kind,n,dmax", [("beside", 9000, None), ("beside", 40001, 700.0),
+                                         ("beside", 40001, None)])
+def test_gpu_fmm_long_lists(ocore, gcore, kind, n, dmax):
+    """Leaves beside a dense cluster (lists of hundreds of leaves; clumps closer
+    than distanceMin in it, whose groups go pair by pair), with leaves of up to
+    16 and of more targets: the second tick on has the room for their terms."""
+    _run(ocore, gcore, kind, n, 4, dmax=dmax)
 
 
 def test_gpu_fmm_pools_grow(ocore, gcore):
