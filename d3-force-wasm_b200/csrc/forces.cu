@@ -1033,8 +1033,8 @@ __device__ __forceinline__ LinkPar link_par(const LinkFlowArgs &a, uint32_t p) {
 
 // The pass of a graph whose nodes fit one SM: a block keeps every node's
 // velocity and position in shared memory and takes the links level by level,
-// a barrier between levels. A level costs the chain of one link (about 0.3 us:
-// shared loads, sqrt, division) and the barrier; its links' constants are
+// a barrier between levels. A level costs the chain of one link (shared
+// loads, sqrt, division) and the barrier, about 1 us; its links' constants are
 // loaded during the level before. The node arrays are written only if no link
 // met a jiggle; if one did, they are still the pass's start for the serial
 // pass. A level's links share no node: at most half the nodes, so the block is
@@ -1120,7 +1120,7 @@ constexpr uint32_t LINK_MET_JIGGLE = 1, LINK_GAVE_UP = 2;
 // the links in level order; a link waits (bounded) for the velocities of its
 // two nodes from the links before it there, each a 16-byte message in a place
 // of its own, and hands them on to the links after it. A level costs one
-// message through L2 and one link's arithmetic (1.1 us; 5 us with finished
+// message through L2 and one link's arithmetic (1.6 us; 5 us with finished
 // counts and the velocities read after an acquire). The first link on a node
 // reads its velocity and saves it, the last one writes it. A read message is
 // cleared for the next pass. If a link met a zero or NaN delta or gave up, the
@@ -1269,9 +1269,9 @@ void link_exact(const NodeArrays &a, const LinkArrays &l, LinkPlan &plan, double
   c.levels = plan.levels; c.nodes = plan.nodes; c.alpha = alpha; c.iterations = iterations;
   c.flag = flag; c.rng = rng; c.status = status; c.serial_lcg = serial_lcg;
   c.sleep_ns = wait_sleep_ns();
-  // One SM when its shared memory holds the nodes: a level there takes a third
-  // of a message's time (1,000 nodes, 2,000 links: 12 us for 30; 5,003 nodes,
-  // 10,006 links: 22 us for 38).
+  // One SM when its shared memory holds the nodes: no messages, and the gain
+  // ends about there (block / messages: 77 nodes 13 / 21 us; 1,000 nodes, 2,000
+  // links 16 / 27; 5,003 nodes, two iterations 52 / 56).
   if (plan.nodes <= LINK_BLOCK_NODES) {
     static const bool attr =
         cudaFuncSetAttribute(k_link_block, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -262,8 +262,9 @@ int32_t d3_mlp_infer(const float *x, uint32_t n, const float *params, float *y,
  * batch_create: node_counts[graphs], link_counts[graphs]; src / tgt the
  * links of every graph concatenated, as node indices local to their graph;
  * x / y the start positions of every node, concatenated. Returns a handle
- * (0 on a bad argument or no memory). batch_run: `ticks` ticks, captured
- * into one CUDA graph when `graph` is non-zero; *ms the device time.
+ * (0 on a bad argument or no memory). batch_run: `ticks` ticks, 16
+ * and more captured into one CUDA graph when `graph` is non-zero; *ms the
+ * device time.
  * batch_kick: the many-body kick alone at the current positions (x, y per
  * node, host float[2 x nodes]) and the alpha it used. batch_read: the node
  * state (any pointer may be NULL). batch_set_shape: threads per CTA (256,
