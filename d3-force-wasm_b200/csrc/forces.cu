@@ -5,6 +5,7 @@
 // preorder, so "descend" is c + 1 and "do not descend" is skip[c].
 #include <climits>
 #include <cstdlib>
+#include <cstring>
 #include <vector>
 
 #include <cooperative_groups.h>
@@ -817,17 +818,28 @@ int link_plan_build(LinkPlan &plan, const uint32_t *src, const uint32_t *tgt, ui
       else r.src |= LINK_FIRST;
     }
   link_plan_free(plan);
-  D3_CUDA_OK(cudaMalloc(&plan.order, order.size() * 4));
-  D3_CUDA_OK(cudaMalloc(&plan.level_start, start.size() * 4));
-  D3_CUDA_OK(cudaMalloc(&plan.ends, ends.size() * sizeof(LinkEnds)));
-  D3_CUDA_OK(cudaMalloc(&plan.par, ends.size() * 3 * sizeof(double)));
-  D3_CUDA_OK(cudaMalloc(&plan.msg, ends.size() * 2 * sizeof(double2)));
-  D3_CUDA_OK(cudaMalloc(&plan.tally, 2 * sizeof(uint32_t)));
-  D3_CUDA_OK(cudaMemcpy(plan.order, order.data(), order.size() * 4, cudaMemcpyHostToDevice));
-  D3_CUDA_OK(cudaMemcpy(plan.level_start, start.data(), start.size() * 4, cudaMemcpyHostToDevice));
-  D3_CUDA_OK(cudaMemcpy(plan.ends, ends.data(), ends.size() * sizeof(LinkEnds), cudaMemcpyHostToDevice));
-  D3_CUDA_OK(cudaMemset(plan.msg, 0xff, ends.size() * 2 * sizeof(double2)));  // no message yet
-  D3_CUDA_OK(cudaMemset(plan.tally, 0, 2 * sizeof(uint32_t)));
+  // one allocation and one copy: the plan's tables and the zeroed tally, then
+  // the constants and the messages
+  const auto room = [](size_t bytes) { return (bytes + 255) / 256 * 256; };
+  const size_t at_order = room(ends.size() * sizeof(LinkEnds)),
+               at_start = at_order + room(order.size() * 4), at_tally = at_start + room(start.size() * 4),
+               at_par = at_tally + room(2 * sizeof(uint32_t)),
+               at_msg = at_par + room(ends.size() * 3 * sizeof(double)),
+               msg_bytes = ends.size() * 2 * sizeof(double2);
+  std::vector<unsigned char> image(at_par, 0);
+  memcpy(image.data(), ends.data(), ends.size() * sizeof(LinkEnds));
+  memcpy(image.data() + at_order, order.data(), order.size() * 4);
+  memcpy(image.data() + at_start, start.data(), start.size() * 4);
+  unsigned char *block = nullptr;
+  D3_CUDA_OK(cudaMalloc(&block, at_msg + msg_bytes));
+  plan.ends = reinterpret_cast<LinkEnds *>(block);
+  plan.order = reinterpret_cast<uint32_t *>(block + at_order);
+  plan.level_start = reinterpret_cast<uint32_t *>(block + at_start);
+  plan.tally = reinterpret_cast<uint32_t *>(block + at_tally);
+  plan.par = reinterpret_cast<double *>(block + at_par);
+  plan.msg = reinterpret_cast<double2 *>(block + at_msg);
+  D3_CUDA_OK(cudaMemcpy(block, image.data(), at_par, cudaMemcpyHostToDevice));
+  D3_CUDA_OK(cudaMemset(plan.msg, 0xff, msg_bytes));  // no message yet
   plan.h_level_start = new uint32_t[start.size()];
   for (size_t k = 0; k < start.size(); ++k) plan.h_level_start[k] = start[k];
   plan.m = m;
@@ -840,12 +852,7 @@ int link_plan_build(LinkPlan &plan, const uint32_t *src, const uint32_t *tgt, ui
 }
 
 void link_plan_free(LinkPlan &plan) {
-  cudaFree(plan.order);
-  cudaFree(plan.level_start);
-  cudaFree(plan.ends);
-  cudaFree(plan.par);
-  cudaFree(plan.msg);
-  cudaFree(plan.tally);
+  cudaFree(plan.ends);  // the block of all device arrays
   delete[] plan.h_level_start;
   plan = LinkPlan();
 }
