@@ -764,6 +764,8 @@ void many_body_rerun(TreeDev &t, const NodeArrays &a, const double *strengths,
 // Exact link (link.zig:8-40)
 // ---------------------------------------------------------------------------
 
+static bool link_in_block(uint32_t nodes);
+
 int link_plan_build(LinkPlan &plan, const uint32_t *src, const uint32_t *tgt, uint32_t m) {
   // level(e) = 1 + the largest level of an earlier link sharing a node, so
   // every link sees exactly the velocities its predecessors wrote.
@@ -819,13 +821,13 @@ int link_plan_build(LinkPlan &plan, const uint32_t *src, const uint32_t *tgt, ui
     }
   link_plan_free(plan);
   // one allocation and one copy: the plan's tables and the zeroed tally, then
-  // the constants and the messages
+  // the constants and (for k_link_flow) the messages
   const auto room = [](size_t bytes) { return (bytes + 255) / 256 * 256; };
   const size_t at_order = room(ends.size() * sizeof(LinkEnds)),
                at_start = at_order + room(order.size() * 4), at_tally = at_start + room(start.size() * 4),
                at_par = at_tally + room(2 * sizeof(uint32_t)),
                at_msg = at_par + room(ends.size() * 3 * sizeof(double)),
-               msg_bytes = ends.size() * 2 * sizeof(double2);
+               msg_bytes = link_in_block(nmax) ? 0 : ends.size() * 2 * sizeof(double2);
   std::vector<unsigned char> image(at_par, 0);
   memcpy(image.data(), ends.data(), ends.size() * sizeof(LinkEnds));
   memcpy(image.data() + at_order, order.data(), order.size() * 4);
@@ -839,7 +841,7 @@ int link_plan_build(LinkPlan &plan, const uint32_t *src, const uint32_t *tgt, ui
   plan.par = reinterpret_cast<double *>(block + at_par);
   plan.msg = reinterpret_cast<double2 *>(block + at_msg);
   D3_CUDA_OK(cudaMemcpy(block, image.data(), at_par, cudaMemcpyHostToDevice));
-  D3_CUDA_OK(cudaMemset(plan.msg, 0xff, msg_bytes));  // no message yet
+  if (msg_bytes) D3_CUDA_OK(cudaMemset(plan.msg, 0xff, msg_bytes));  // no message yet
   plan.h_level_start = new uint32_t[start.size()];
   for (size_t k = 0; k < start.size(); ++k) plan.h_level_start[k] = start[k];
   plan.m = m;
@@ -1107,6 +1109,14 @@ __global__ void __launch_bounds__(1024) k_link_block(LinkFlowArgs a) {
   }
 }
 
+// Whether a plan over `nodes` nodes runs in one block.
+static bool link_in_block(uint32_t nodes) {
+  static const bool attr =
+      cudaFuncSetAttribute(k_link_block, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)(LINK_BLOCK_NODES * 2 * sizeof(double2))) == cudaSuccess;
+  return attr && nodes <= LINK_BLOCK_NODES;
+}
+
 // A link's input from the link before it on one of its nodes, or all ones in
 // either half while that has not come. Each half is a 64-bit access and is
 // looked at by itself, so the halves need not arrive together; the value is
@@ -1279,15 +1289,10 @@ void link_exact(const NodeArrays &a, const LinkArrays &l, LinkPlan &plan, double
   // One SM when its shared memory holds the nodes: no messages, and the gain
   // ends about there (block / messages: 77 nodes 13 / 21 us; 1,000 nodes, 2,000
   // links 16 / 27; 5,003 nodes, two iterations 52 / 56).
-  if (plan.nodes <= LINK_BLOCK_NODES) {
-    static const bool attr =
-        cudaFuncSetAttribute(k_link_block, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)(LINK_BLOCK_NODES * 2 * sizeof(double2))) == cudaSuccess;
-    if (attr) {
-      const uint32_t w = plan.width > 1024 ? 1024 : (plan.width + 31) / 32 * 32;
-      D3_LAUNCH(k_link_block, 1, w, plan.nodes * 2 * sizeof(double2), st)(c);
-      return;
-    }
+  if (link_in_block(plan.nodes)) {
+    const uint32_t w = plan.width > 1024 ? 1024 : (plan.width + 31) / 32 * 32;
+    D3_LAUNCH(k_link_block, 1, w, plan.nodes * 2 * sizeof(double2), st)(c);
+    return;
   }
   static int sms = 0, per_sm = 0;
   if (!per_sm) {
