@@ -499,9 +499,9 @@ void radix_sort_u64(uint64_t *keys, uint32_t *vals, uint32_t n, int byte_lo, int
   uint32_t *av = vals, *bv = s.vals_tmp;
   const uint32_t tiles = (n + SORT_TILE - 1) / SORT_TILE;
   const int passes = byte_hi - byte_lo;
-  // hist: the passes' totals, tickets, then 512 words per tile and pass
+  // hist: the passes' totals, tickets, then a word per tile, digit and pass
   uint32_t *tot = s.hist, *ticket = tot + SORT_PASSES * 512, *words = ticket + SORT_PASSES;
-  cudaMemsetAsync(s.hist, 0, (SORT_PASSES * 513 + (size_t)passes * tiles * 512) * 4, st);
+  cudaMemsetAsync(s.hist, 0, (SORT_PASSES * 513 + (size_t)tiles * 256 * (passes + partition_hi_bit)) * 4, st);
   const unsigned hb = blocks_for(n, SORT_THREADS * 2);
   D3_LAUNCH(k_sort_totals, hb < 592 ? hb : 592, SORT_THREADS, 0, st)(keys, vals, n, byte_lo, passes,
                                                                   partition_hi_bit, tot);
@@ -514,7 +514,7 @@ void radix_sort_u64(uint64_t *keys, uint32_t *vals, uint32_t n, int byte_lo, int
     else
       D3_LAUNCH(k_sort_scatter<BYTE>, tiles, SORT_THREADS, 0, st)(ak, av, bk, bv, n, shift,
                                                                  tot + p * 512, words, ticket + p);
-    words += (size_t)tiles * 512;
+    words += (size_t)tiles * 256;  // (the 9-bit digit comes last)
     uint64_t *tk = ak; ak = bk; bk = tk;
     uint32_t *tv = av; av = bv; bv = tv;
   }

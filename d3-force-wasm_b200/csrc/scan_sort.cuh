@@ -112,7 +112,7 @@ void radix_sort_u64(uint64_t *keys, uint32_t *vals, uint32_t n, int byte_lo, int
 inline size_t sort_hist_words(uint32_t n) {
   size_t tiles = (n + SORT_TILE - 1) / SORT_TILE;
   if (!tiles) tiles = 1;
-  return SORT_PASSES * (513 + 512 * tiles) + 1;
+  return SORT_PASSES * 513 + (SORT_PASSES + 1) * 256 * tiles;
 }
 inline size_t scan_partial_words(size_t n) { return blocks_for(n, SCAN_BLOCK * 4) + 2; }
 
