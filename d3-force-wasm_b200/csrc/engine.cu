@@ -420,7 +420,7 @@ int run_link(DSim *s, DForce *f, double alpha) {
   if (f->max_index > s->n) return D3_BAD_ARGUMENT;
   if (f->count == 0) return D3_OK;
   if (f->plan_dirty) {
-    if (link_plan_build(f->plan, f->h_src, f->h_tgt, f->count)) return D3_OUT_OF_MEMORY;
+    if (link_plan_build(f->plan, f->h_src, f->h_tgt, f->count, s->stream)) return D3_OUT_OF_MEMORY;
     f->plan_dirty = false;
   }
   NodeArrays a = nodes_of(s);

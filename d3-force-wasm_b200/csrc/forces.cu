@@ -766,7 +766,8 @@ void many_body_rerun(TreeDev &t, const NodeArrays &a, const double *strengths,
 
 static bool link_in_block(uint32_t nodes);
 
-int link_plan_build(LinkPlan &plan, const uint32_t *src, const uint32_t *tgt, uint32_t m) {
+int link_plan_build(LinkPlan &plan, const uint32_t *src, const uint32_t *tgt, uint32_t m,
+                    cudaStream_t st) {
   // level(e) = 1 + the largest level of an earlier link sharing a node, so
   // every link sees exactly the velocities its predecessors wrote.
   uint32_t nmax = 0;
@@ -821,7 +822,10 @@ int link_plan_build(LinkPlan &plan, const uint32_t *src, const uint32_t *tgt, ui
     }
   link_plan_free(plan);
   // one allocation and one copy: the plan's tables and the zeroed tally, then
-  // the constants and (for k_link_flow) the messages
+  // the constants and (for k_link_flow) the messages. Copy and fill go on the
+  // stream of the launches that read them: it does not wait for the default
+  // stream, where either may still be under way when the call returns, and a
+  // link would take what the memory held before for its velocity.
   const auto room = [](size_t bytes) { return (bytes + 255) / 256 * 256; };
   const size_t at_order = room(ends.size() * sizeof(LinkEnds)),
                at_start = at_order + room(order.size() * 4), at_tally = at_start + room(start.size() * 4),
@@ -840,8 +844,8 @@ int link_plan_build(LinkPlan &plan, const uint32_t *src, const uint32_t *tgt, ui
   plan.tally = reinterpret_cast<uint32_t *>(block + at_tally);
   plan.par = reinterpret_cast<double *>(block + at_par);
   plan.msg = reinterpret_cast<double2 *>(block + at_msg);
-  D3_CUDA_OK(cudaMemcpy(block, image.data(), at_par, cudaMemcpyHostToDevice));
-  if (msg_bytes) D3_CUDA_OK(cudaMemset(plan.msg, 0xff, msg_bytes));  // no message yet
+  D3_CUDA_OK(cudaMemcpyAsync(block, image.data(), at_par, cudaMemcpyHostToDevice, st));
+  if (msg_bytes) D3_CUDA_OK(cudaMemsetAsync(plan.msg, 0xff, msg_bytes, st));  // no message yet
   plan.h_level_start = new uint32_t[start.size()];
   for (size_t k = 0; k < start.size(); ++k) plan.h_level_start[k] = start[k];
   plan.m = m;

@@ -77,7 +77,9 @@ struct LinkPlan {
   double2 *msg = nullptr;           // device: per link its two input messages
   uint32_t *tally = nullptr;        // device: blocks done, failure bits of the running pass
 };
-int link_plan_build(LinkPlan &plan, const uint32_t *src, const uint32_t *tgt, uint32_t m);
+// The device arrays are filled on `st`, where the passes run.
+int link_plan_build(LinkPlan &plan, const uint32_t *src, const uint32_t *tgt, uint32_t m,
+                    cudaStream_t st);
 void link_plan_free(LinkPlan &plan);
 
 struct LinkArrays {
