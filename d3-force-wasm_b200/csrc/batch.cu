@@ -894,7 +894,7 @@ void set_levels(Batch &b) {
     while (L < BMAX_L && (double)b.h_counts[g] / (double)(1u << (2 * L)) > b.leaf_size) ++L;
     b.h_level[g] = (uint8_t)L;
   }
-  cudaMemcpy(b.level, b.h_level.data(), b.graphs, cudaMemcpyHostToDevice);
+  cudaMemcpyAsync(b.level, b.h_level.data(), b.graphs, cudaMemcpyHostToDevice, b.st);
   // what the largest working set takes, up to the cap: more of the SM's
   // memory stays L1 for the loads through the node and link arrays
   b.smem = 0;
@@ -1029,22 +1029,23 @@ uint32_t batch_create(uint32_t graphs, const uint32_t *node_counts, const uint32
             cudaMalloc(&b->x, N * 4ull) == cudaSuccess && cudaMalloc(&b->y, N * 4ull) == cudaSuccess &&
             cudaMalloc(&b->vx, N * 4ull) == cudaSuccess && cudaMalloc(&b->vy, N * 4ull) == cudaSuccess &&
             cudaMalloc(&b->kick, N * sizeof(float2)) == cudaSuccess;
-  ok = ok && cudaMemcpy(b->tab, &T, sizeof T, cudaMemcpyHostToDevice) == cudaSuccess &&
-       cudaMemcpy(b->order, b->h_order.data(), graphs * 4, cudaMemcpyHostToDevice) == cudaSuccess &&
-       cudaMemcpy(b->node_off, b->h_off.data(), (graphs + 1) * 4, cudaMemcpyHostToDevice) == cudaSuccess &&
-       cudaMemcpy(b->adj_off, adj_off.data(), (N + 1) * 4ull, cudaMemcpyHostToDevice) == cudaSuccess &&
-       (links == 0 ||
-        cudaMemcpy(b->adj, adj.data(), 2 * links * sizeof(BLink), cudaMemcpyHostToDevice) ==
-            cudaSuccess) &&
-       cudaMemcpy(b->x, x, N * 4ull, cudaMemcpyHostToDevice) == cudaSuccess &&
-       cudaMemcpy(b->y, y, N * 4ull, cudaMemcpyHostToDevice) == cudaSuccess &&
-       cudaMemset(b->vx, 0, N * 4ull) == cudaSuccess && cudaMemset(b->vy, 0, N * 4ull) == cudaSuccess;
+  // on the batch's stream, which does not wait for the default one
+  auto put = [&](void *to, const void *from, size_t bytes) {
+    return cudaMemcpyAsync(to, from, bytes, cudaMemcpyHostToDevice, b->st) == cudaSuccess;
+  };
+  ok = ok && put(b->tab, &T, sizeof T) && put(b->order, b->h_order.data(), graphs * 4) &&
+       put(b->node_off, b->h_off.data(), (graphs + 1) * 4) &&
+       put(b->adj_off, adj_off.data(), (N + 1) * 4ull) &&
+       (links == 0 || put(b->adj, adj.data(), 2 * links * sizeof(BLink))) &&
+       put(b->x, x, N * 4ull) && put(b->y, y, N * 4ull) &&
+       cudaMemsetAsync(b->vx, 0, N * 4ull, b->st) == cudaSuccess &&
+       cudaMemsetAsync(b->vy, 0, N * 4ull, b->st) == cudaSuccess;
   cudaFuncSetAttribute(k_batch_tick, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)smem_cap(1));
   b->alpha_decay = 1 - std::pow(0.001, 1.0 / 300);
   if (ok) {
     set_levels(*b);
-    ok = ensure_scratch(*b) == 0;
+    ok = ensure_scratch(*b) == 0 && cudaStreamSynchronize(b->st) == cudaSuccess;
   }
   if (!ok) {
     delete b;
@@ -1196,7 +1197,8 @@ int32_t batch_autotune(uint32_t h, uint32_t ticks, double *out) {
   float *save = nullptr;
   if (cudaMalloc(&save, 4 * bytes) != cudaSuccess) return D3_OUT_OF_MEMORY;
   float *arr[4] = {b->x, b->y, b->vx, b->vy};
-  for (int k = 0; k < 4; ++k) cudaMemcpy(save + k * b->nodes, arr[k], bytes, cudaMemcpyDeviceToDevice);
+  for (int k = 0; k < 4; ++k)
+    cudaMemcpyAsync(save + k * b->nodes, arr[k], bytes, cudaMemcpyDeviceToDevice, b->st);
   const double alpha0 = b->alpha;
   const uint32_t tick0 = b->tick;
   double best = 1e30;
@@ -1219,10 +1221,11 @@ int32_t batch_autotune(uint32_t h, uint32_t ticks, double *out) {
           bl = ls;
         }
         for (int k = 0; k < 4; ++k)
-          cudaMemcpy(arr[k], save + k * b->nodes, bytes, cudaMemcpyDeviceToDevice);
+          cudaMemcpyAsync(arr[k], save + k * b->nodes, bytes, cudaMemcpyDeviceToDevice, b->st);
         b->alpha = alpha0;
         b->tick = tick0;
       }
+  if (cudaStreamSynchronize(b->st) != cudaSuccess) rc = D3_WORKER_FAILED;  // the state is back
   cudaFree(save);
   if (rc != D3_OK) return rc;
   batch_set_shape(h, bt, bp, bl);

@@ -1483,7 +1483,7 @@ static void spec_arrays(CollideSpec &s, F f) {
   f((void **)&s.work, 3 * 4ull);  // bigfill, biglink, vwork
 }
 
-int collide_spec_reserve(CollideSpec &s, uint32_t n) {
+int collide_spec_reserve(CollideSpec &s, uint32_t n, cudaStream_t st) {
   if (n <= s.cap && s.cap) return 0;
   uint32_t cap = n < 1024 ? 1024 : n;
   spec_arrays(s, [](void **p, size_t) {
@@ -1492,7 +1492,7 @@ int collide_spec_reserve(CollideSpec &s, uint32_t n) {
   });
   if (!s.counters) {
     D3_CUDA_OK(cudaMalloc(&s.counters, C_COUNTERS * sizeof(uint32_t)));
-    D3_CUDA_OK(cudaMemset(s.counters, 0, C_COUNTERS * sizeof(uint32_t)));
+    D3_CUDA_OK(cudaMemsetAsync(s.counters, 0, C_COUNTERS * sizeof(uint32_t), st));
     D3_CUDA_OK(cudaMalloc(&s.grid_part, 1024 * sizeof(uint32_t)));
   }
   // 16 phase stamps, then attempt 1's per-depth last finish times and turn
@@ -1510,7 +1510,7 @@ int collide_spec_reserve(CollideSpec &s, uint32_t n) {
     cudaGetLastError();
     return D3_OUT_OF_MEMORY;
   }
-  D3_CUDA_OK(cudaMemset(s.push_prev, 0, cap * 8ull));
+  D3_CUDA_OK(cudaMemsetAsync(s.push_prev, 0, cap * 8ull, st));
   s.cap = cap;
   return 0;
 }

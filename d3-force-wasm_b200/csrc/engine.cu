@@ -335,7 +335,7 @@ int take_failure(DSim *s) {
   const uint32_t w = s->h_words[24];
   if (!(w & ST_FATAL)) return D3_OK;
   s->h_words[25] = w & ~ST_FATAL;
-  cudaMemcpy(s->d_words, s->h_words + 25, sizeof(uint32_t), cudaMemcpyHostToDevice);
+  cudaMemcpyAsync(s->d_words, s->h_words + 25, sizeof(uint32_t), cudaMemcpyHostToDevice, s->stream);
   s->h_words[24] = 0;
   return D3_WORKER_FAILED;
 }
@@ -527,7 +527,7 @@ int run_force(DSim *s, DForce *f, double alpha, bool presummed = false, bool fus
       if (fast_mode(s, f)) {
         if (f->max_index > s->n) return D3_BAD_ARGUMENT;
         if (f->csr_dirty || f->csr.n != s->n) {
-          if (fast_link_build(f->csr, f->h_src, f->h_tgt, f->count, s->n)) return D3_OUT_OF_MEMORY;
+          if (fast_link_build(f->csr, f->h_src, f->h_tgt, f->count, s->n, s->stream)) return D3_OUT_OF_MEMORY;
           f->csr_dirty = false;
         }
         LinkArrays l{f->d_f[0], f->d_f[1], f->d_f[2], f->d_src, f->d_tgt, f->count};
@@ -588,8 +588,8 @@ int ensure_cap(DSim *s, uint32_t n) {
       grow_device(s->d_py, 0, cap, st) || grow_device(s->d_svx, 0, cap, st) ||
       grow_device(s->d_svy, 0, cap, st))
     return -1;
-  if (tree_reserve(s->tree, cap) || scratch_reserve(s->scratch, cap) || fast_reserve(s->fast, cap) ||
-      collide_spec_reserve(s->spec, cap))
+  if (tree_reserve(s->tree, cap, st) || scratch_reserve(s->scratch, cap, st) ||
+      fast_reserve(s->fast, cap, st) || collide_spec_reserve(s->spec, cap, st))
     return -1;
   s->cap = cap;
   return 0;
@@ -621,14 +621,17 @@ uint32_t sim_create(void) {
   cudaMallocHost(&s->h_rng, sizeof(Rng));
   cudaMalloc(&s->d_words, 16 * sizeof(uint32_t));
   cudaMallocHost(&s->h_words, 32 * sizeof(uint32_t));
-  cudaMemset(s->d_words, 0, 16 * sizeof(uint32_t));
+  cudaMemsetAsync(s->d_words, 0, 16 * sizeof(uint32_t), s->stream);
   Rng r{};
   r.lcg = 1;
   r.mode = 0;
-  cudaMemcpy(s->d_rng, &r, sizeof(Rng), cudaMemcpyHostToDevice);
+  *s->h_rng = r;
+  cudaMemcpyAsync(s->d_rng, s->h_rng, sizeof(Rng), cudaMemcpyHostToDevice, s->stream);
   cudaEventCreate(&s->ev0);
   cudaEventCreate(&s->ev1);
-  if (tree_reserve(s->tree, 16) || scratch_reserve(s->scratch, 16) || fast_reserve(s->fast, 16)) {
+  // (h_rng is written again by calls that follow)
+  if (tree_reserve(s->tree, 16, s->stream) || scratch_reserve(s->scratch, 16, s->stream) ||
+      fast_reserve(s->fast, 16, s->stream) || cudaStreamSynchronize(s->stream) != cudaSuccess) {
     delete s;
     return 0;
   }
@@ -1121,7 +1124,7 @@ int32_t sim_set_learned(uint32_t h, const float *params, uint32_t len, double to
   DSim *s = get_sim(h);
   if (!s) return D3_BAD_HANDLE;
   if (!(tolerance > 0) || samples == 0 || samples > 4096) return D3_BAD_ARGUMENT;
-  const int r = fmm_tc_set_learned(s->fast, params, len);
+  const int r = fmm_tc_set_learned(s->fast, params, len, s->stream);
   if (r == -3) return D3_BAD_ARGUMENT;
   if (r < 0) return D3_OUT_OF_MEMORY;
   s->fast.learn_tol = tolerance;

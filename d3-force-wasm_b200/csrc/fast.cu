@@ -16,12 +16,12 @@ constexpr uint32_t NO_CELL = 0xffffffffu;
 constexpr unsigned GRID_THREADS = 256;
 constexpr unsigned GRID_BLOCKS_MAX = 592;
 
-int fast_reserve(FastScratch &s, uint32_t n) {
+int fast_reserve(FastScratch &s, uint32_t n, cudaStream_t st) {
   if (!s.seed) {
     D3_CUDA_OK(cudaMalloc(&s.seed, sizeof(double)));
     D3_CUDA_OK(cudaMalloc(&s.g_box, GRID_BLOCKS_MAX * 6 * sizeof(double)));
     D3_CUDA_OK(cudaMalloc(&s.g_info, 8 * sizeof(uint32_t)));
-    D3_CUDA_OK(cudaMemset(s.g_info, 0, 8 * sizeof(uint32_t)));
+    D3_CUDA_OK(cudaMemsetAsync(s.g_info, 0, 8 * sizeof(uint32_t), st));
     D3_CUDA_OK(cudaMalloc(&s.g_geom, 4 * sizeof(double)));
   }
   if (n <= s.cap && s.cap) return 0;
@@ -69,7 +69,8 @@ __device__ inline uint64_t seed_bits(const double *seed) {
 
 // ---- link_fast.zig --------------------------------------------------------
 
-int fast_link_build(FastLink &c, const uint32_t *src, const uint32_t *tgt, uint32_t m, uint32_t n) {
+int fast_link_build(FastLink &c, const uint32_t *src, const uint32_t *tgt, uint32_t m, uint32_t n,
+                    cudaStream_t st) {
   // link_fast.zig:105-130
   std::vector<uint32_t> row(n + 1, 0), adj(m ? 2 * (size_t)m : 1);
   for (uint32_t e = 0; e < m; ++e) {
@@ -95,9 +96,9 @@ int fast_link_build(FastLink &c, const uint32_t *src, const uint32_t *tgt, uint3
   D3_CUDA_OK(cudaMalloc(&c.adj, adj.size() * 4));
   D3_CUDA_OK(cudaMalloc(&c.other, other.size() * 4));
   D3_CUDA_OK(cudaMalloc(&c.scal, 3 * adj.size() * sizeof(double)));
-  D3_CUDA_OK(cudaMemcpy(c.row, row.data(), row.size() * 4, cudaMemcpyHostToDevice));
-  D3_CUDA_OK(cudaMemcpy(c.adj, adj.data(), adj.size() * 4, cudaMemcpyHostToDevice));
-  D3_CUDA_OK(cudaMemcpy(c.other, other.data(), other.size() * 4, cudaMemcpyHostToDevice));
+  D3_CUDA_OK(cudaMemcpyAsync(c.row, row.data(), row.size() * 4, cudaMemcpyHostToDevice, st));
+  D3_CUDA_OK(cudaMemcpyAsync(c.adj, adj.data(), adj.size() * 4, cudaMemcpyHostToDevice, st));
+  D3_CUDA_OK(cudaMemcpyAsync(c.other, other.data(), other.size() * 4, cudaMemcpyHostToDevice, st));
   c.n = n;
   c.m = m;
   c.gathered = false;

@@ -30,7 +30,7 @@ struct FastScratch {
   double learn_checks = 0, learn_fallbacks = 0, learn_last_rms = 0;
 };
 
-int fast_reserve(FastScratch &s, uint32_t n);
+int fast_reserve(FastScratch &s, uint32_t n, cudaStream_t st);
 void fast_free(FastScratch &s);
 
 // The per-run SEED: one draw from the device LCG (src/core.js:221), or a
@@ -51,7 +51,8 @@ struct FastLink {
   double *scal = nullptr;      // per adjacency entry: distance, strength, bias planes
   bool gathered = false;       // scal holds the current link arrays
 };
-int fast_link_build(FastLink &c, const uint32_t *src, const uint32_t *tgt, uint32_t m, uint32_t n);
+int fast_link_build(FastLink &c, const uint32_t *src, const uint32_t *tgt, uint32_t m, uint32_t n,
+                    cudaStream_t st);
 void fast_link_free(FastLink &c);
 void fast_link(const NodeArrays &a, const LinkArrays &l, FastLink &c, double alpha,
                double iterations, const double *seed, cudaStream_t st);
@@ -102,7 +103,7 @@ int fmm_tc_run(FastScratch &s, TreeDev &t, const NodeArrays &a, const double *st
                cudaStream_t st);
 void fmm_tc_free(FastScratch &s);
 // Installs the learned form's network (MLP_PARAMS floats, host): 0, or < 0.
-int fmm_tc_set_learned(FastScratch &s, const float *params, uint32_t len);
+int fmm_tc_set_learned(FastScratch &s, const float *params, uint32_t len, cudaStream_t st);
 // The last precision-form run's per-cell rows (16 floats: features, L'_0, sc,
 // the cell index for leaves or -1) into out when cap >= the cell count;
 // returns the cell count.

@@ -1767,7 +1767,7 @@ int fmm_prepare(FastScratch &s, TreeDev &t, const NodeArrays &a, const double *s
     FmmDev *f = new FmmDev();
     s.fmm = f;
     D3_CUDA_OK(cudaMalloc(&f->info, 64 * sizeof(uint32_t)));
-    D3_CUDA_OK(cudaMemset(f->info, 0, 64 * sizeof(uint32_t)));
+    D3_CUDA_OK(cudaMemsetAsync(f->info, 0, 64 * sizeof(uint32_t), st));
     D3_CUDA_OK(cudaMalloc(&f->square, 4 * sizeof(double)));
     D3_CUDA_OK(cudaMalloc(&f->tab, sizeof(FmmTables)));
     D3_CUDA_OK(cudaMalloc(&f->geom, 4 * sizeof(double)));

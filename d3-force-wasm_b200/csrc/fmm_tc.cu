@@ -2128,12 +2128,12 @@ void fmm_tc_free(FastScratch &s) {
   s.fmm_tc = nullptr;
 }
 
-int fmm_tc_set_learned(FastScratch &s, const float *params, uint32_t len) {
+int fmm_tc_set_learned(FastScratch &s, const float *params, uint32_t len, cudaStream_t st) {
   if (len != (uint32_t)MLP_PARAMS || !params) return -3;
   TcDev *d = tc_dev(s);
   if (!d) return -1;
   if (!d->mlp) D3_CUDA_OK(cudaMalloc(&d->mlp, MLP_PARAMS * 4));
-  return cudaMemcpy(d->mlp, params, MLP_PARAMS * 4, cudaMemcpyHostToDevice) == cudaSuccess ? 0 : -1;
+  return cudaMemcpyAsync(d->mlp, params, MLP_PARAMS * 4, cudaMemcpyHostToDevice, st) == cudaSuccess ? 0 : -1;
 }
 
 int fmm_tc_leaves(FastScratch &s, float *out, uint32_t cap) {

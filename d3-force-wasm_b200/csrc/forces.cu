@@ -21,13 +21,13 @@ size_t csum_rec_bytes(uint32_t n);
 size_t csum_count_words(uint32_t n);
 size_t csum_part_words(uint32_t n);
 
-int scratch_reserve(ForceScratch &s, uint32_t n) {
+int scratch_reserve(ForceScratch &s, uint32_t n, cudaStream_t st) {
   if (!s.counters) {
     D3_CUDA_OK(cudaMalloc(&s.counters, 16 * sizeof(uint32_t)));
-    D3_CUDA_OK(cudaMemset(s.counters, 0, 16 * sizeof(uint32_t)));
+    D3_CUDA_OK(cudaMemsetAsync(s.counters, 0, 16 * sizeof(uint32_t), st));
     D3_CUDA_OK(cudaMalloc(&s.center, 2 * sizeof(double)));
     D3_CUDA_OK(cudaMalloc(&s.csum_stamps, 8 * sizeof(unsigned long long)));
-    D3_CUDA_OK(cudaMemset(s.csum_stamps, 0, 8 * sizeof(unsigned long long)));
+    D3_CUDA_OK(cudaMemsetAsync(s.csum_stamps, 0, 8 * sizeof(unsigned long long), st));
   }
   if (n <= s.cap && s.cap) return 0;
   uint32_t cap = n < 1024 ? 1024 : n;

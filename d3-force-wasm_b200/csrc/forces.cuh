@@ -31,7 +31,7 @@ struct ForceScratch {
   unsigned long long *csum_stamps = nullptr;  // the last center sum's timestamps and counts
 };
 
-int scratch_reserve(ForceScratch &s, uint32_t n);
+int scratch_reserve(ForceScratch &s, uint32_t n, cudaStream_t st);
 
 // A device wait that cannot end, bounded by budget_us: sets ST_WAIT_TIMEOUT.
 void wait_selftest(uint32_t *status, uint32_t budget_us, cudaStream_t st);
@@ -140,7 +140,7 @@ struct CollideSpec {
   unsigned long long *stamps = nullptr;
   int profile = 0;  // per-depth stamps of the first attempt (sim_set_profile)
 };
-int collide_spec_reserve(CollideSpec &s, uint32_t n);
+int collide_spec_reserve(CollideSpec &s, uint32_t n, cudaStream_t st);
 void collide_spec_free(CollideSpec &s);
 // One iteration's node loop, in parallel and bit-identical to the serial
 // order (after collide_setup). `delta`: the guess margin. LCG random only.

@@ -1083,14 +1083,14 @@ __global__ void __launch_bounds__(TREE_SMALL_THREADS) k_tree_small(TreeBuildArgs
   tb_stamp(a, 8);
 }
 
-int tree_reserve(TreeDev &t, uint32_t n) {
+int tree_reserve(TreeDev &t, uint32_t n, cudaStream_t st) {
   if (!t.info) {
     D3_CUDA_OK(cudaMalloc(&t.info, 16 * sizeof(uint32_t)));
-    D3_CUDA_OK(cudaMemset(t.info, 0, 16 * sizeof(uint32_t)));
+    D3_CUDA_OK(cudaMemsetAsync(t.info, 0, 16 * sizeof(uint32_t), st));
     D3_CUDA_OK(cudaMalloc(&t.extent, 4 * sizeof(double)));
     D3_CUDA_OK(cudaMalloc(&t.box_part, BOX_BLOCKS_MAX * sizeof(BoxPart)));
     D3_CUDA_OK(cudaMalloc(&t.stamps, 16 * sizeof(unsigned long long)));
-    D3_CUDA_OK(cudaMemset(t.stamps, 0, 16 * sizeof(unsigned long long)));
+    D3_CUDA_OK(cudaMemsetAsync(t.stamps, 0, 16 * sizeof(unsigned long long), st));
   }
   if (n <= t.cap && t.cap) return 0;
   uint32_t cap = n < 1024 ? 1024 : n;

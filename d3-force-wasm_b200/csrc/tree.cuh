@@ -52,7 +52,7 @@ inline size_t tree_hist_words(uint32_t n) {
   return a > b ? a : b;
 }
 
-int tree_reserve(TreeDev &t, uint32_t n);
+int tree_reserve(TreeDev &t, uint32_t n, cudaStream_t st);
 void tree_free(TreeDev &t);
 
 // Builds the tree over (xs, ys)[0..n) on stream st. Leaves the result in t

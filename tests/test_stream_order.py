@@ -7,6 +7,8 @@ itself cannot be forced to go wrong in a run, so the sources are looked at.)"""
 import os
 import re
 
+import pytest
+
 import helpers as H
 
 CSRC = os.path.join(H.ROOT, "d3-force-wasm_b200", "csrc")
@@ -28,3 +30,18 @@ def function(name, text):
 
 def test_link_plan_is_filled_on_the_stream():
     assert not UNORDERED.search(function("link_plan_build", source("forces.cu")))
+
+
+# the sources whose kernels run on non-blocking streams, and the functions in
+# them whose kernels run on the default stream as well
+STREAMED = {"engine.cu": [], "tree.cu": [], "scan_sort.cu": [], "forces.cu": [], "fast.cu": [],
+            "fmm.cu": [], "collide_spec.cu": [], "noalloc.cu": [], "fmm_tc.cu": ["fmm_tc_stats"],
+            "batch.cu": []}
+
+
+@pytest.mark.parametrize("name", sorted(STREAMED))
+def test_set_up_is_on_the_stream(name):
+    text = source(name)
+    for f in STREAMED[name]:
+        text = text.replace(function(f, text), "")
+    assert [m.group(0) for m in UNORDERED.finditer(text)] == []
