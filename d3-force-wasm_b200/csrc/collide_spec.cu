@@ -1530,8 +1530,7 @@ int collide_parallel(TreeDev &t, const NodeArrays &a, const double *radii, doubl
     int dev = 0, sms = 0, per = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaFuncSetAttribute(k_collide_spec, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)SPEC_DYN_SMEM);
+    open_shared<k_collide_spec>(SPEC_DYN_SMEM);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_collide_spec, SPEC_THREADS, SPEC_DYN_SMEM);
     // blocks per SM: full occupancy (at most 2), or D3_COLLIDE_BLOCKS_PER_SM
     int want = per > 2 ? 2 : per;
@@ -1568,6 +1567,7 @@ int collide_parallel(TreeDev &t, const NodeArrays &a, const double *radii, doubl
   args.rng = rng;
   void *params[] = {&args};
   ++g_launches;
+  if (!open_shared<k_collide_spec>(SPEC_DYN_SMEM)) return -1;
   cudaError_t e = cudaLaunchCooperativeKernel((const void *)k_collide_spec, g_spec_blocks,
                                               SPEC_THREADS, params, SPEC_DYN_SMEM, st);
   return e == cudaSuccess ? 0 : -1;

@@ -13,6 +13,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/d3force_b200.h"
+#include "per_device.cuh"
 
 namespace d3 {
 
@@ -114,6 +115,23 @@ extern unsigned long long g_launches;
 #define D3_LAUNCH(kernel, ...) \
   for (int d3_launch_once_ = (++::d3::g_launches, 0); d3_launch_once_ < 1; ++d3_launch_once_) \
   kernel<<<__VA_ARGS__>>>
+
+// Lets KERNEL take `bytes` of dynamic shared memory on the current device (past
+// 48 KB it has to be allowed, and the attribute is the device's): whether it
+// may. One size per kernel.
+template <auto KERNEL>
+bool open_shared(size_t bytes) {
+  static PerDevice opened;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  return opened(dev, [bytes] {
+    if (cudaFuncSetAttribute((const void *)KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)bytes) == cudaSuccess)
+      return true;
+    cudaGetLastError();
+    return false;
+  });
+}
 
 inline unsigned blocks_for(size_t n, unsigned threads) {
   size_t b = (n + threads - 1) / threads;

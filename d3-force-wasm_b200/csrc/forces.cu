@@ -726,7 +726,7 @@ void many_body_exact(TreeDev &t, const NodeArrays &a, const double *strengths,
     int dev = 0, sms = 0, per = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaFuncSetAttribute(k_mb_draws, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MB_DRAWS_SMEM);
+    open_shared<k_mb_draws>(MB_DRAWS_SMEM);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_mb_draws, 256, MB_DRAWS_SMEM);
     blocks = sms * (per >= 2 ? 2 : (per > 0 ? per : 1));
   }
@@ -742,8 +742,9 @@ void many_body_exact(TreeDev &t, const NodeArrays &a, const double *strengths,
   void *params[] = {&rec, &cells, &perm, &info, &x, &y, &vx, &vy, &strengths, &pp, &nn, &draws,
                     &offsets, &counters, &bsum, &rng, &words};
   ++g_launches;
-  if (cudaLaunchCooperativeKernel((const void *)k_mb_draws, blocks, 256, params, MB_DRAWS_SMEM, st) !=
-      cudaSuccess) {
+  if (!open_shared<k_mb_draws>(MB_DRAWS_SMEM) ||
+      cudaLaunchCooperativeKernel((const void *)k_mb_draws, blocks, 256, params, MB_DRAWS_SMEM, st) !=
+          cudaSuccess) {
     cudaGetLastError();
     scan_u32(s.draws, s.offsets, n, s.scan_part, s.counters, st);
     many_body_rerun(t, a, strengths, p, rng, s, st);
@@ -821,6 +822,7 @@ int link_plan_build(LinkPlan &plan, const uint32_t *src, const uint32_t *tgt, ui
       else r.src |= LINK_FIRST;
     }
   link_plan_free(plan);
+  const bool in_block = link_in_block(nmax);
   // one allocation and one copy: the plan's tables and the zeroed tally, then
   // the constants and (for k_link_flow) the messages. Copy and fill go on the
   // stream of the launches that read them: it does not wait for the default
@@ -831,7 +833,7 @@ int link_plan_build(LinkPlan &plan, const uint32_t *src, const uint32_t *tgt, ui
                at_start = at_order + room(order.size() * 4), at_tally = at_start + room(start.size() * 4),
                at_par = at_tally + room(2 * sizeof(uint32_t)),
                at_msg = at_par + room(ends.size() * 3 * sizeof(double)),
-               msg_bytes = link_in_block(nmax) ? 0 : ends.size() * 2 * sizeof(double2);
+               msg_bytes = in_block ? 0 : ends.size() * 2 * sizeof(double2);
   std::vector<unsigned char> image(at_par, 0);
   memcpy(image.data(), ends.data(), ends.size() * sizeof(LinkEnds));
   memcpy(image.data() + at_order, order.data(), order.size() * 4);
@@ -853,6 +855,7 @@ int link_plan_build(LinkPlan &plan, const uint32_t *src, const uint32_t *tgt, ui
   plan.nodes = nmax;
   plan.width = width;
   plan.self = self;
+  plan.in_block = in_block;
   plan.gathered = false;
   return 0;
 }
@@ -1115,10 +1118,7 @@ __global__ void __launch_bounds__(1024) k_link_block(LinkFlowArgs a) {
 
 // Whether a plan over `nodes` nodes runs in one block.
 static bool link_in_block(uint32_t nodes) {
-  static const bool attr =
-      cudaFuncSetAttribute(k_link_block, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)(LINK_BLOCK_NODES * 2 * sizeof(double2))) == cudaSuccess;
-  return attr && nodes <= LINK_BLOCK_NODES;
+  return nodes <= LINK_BLOCK_NODES && open_shared<k_link_block>(LINK_BLOCK_NODES * 2 * sizeof(double2));
 }
 
 // A link's input from the link before it on one of its nodes, or all ones in
@@ -1293,7 +1293,7 @@ void link_exact(const NodeArrays &a, const LinkArrays &l, LinkPlan &plan, double
   // One SM when its shared memory holds the nodes: no messages, and the gain
   // ends about there (block / messages: 77 nodes 13 / 21 us; 1,000 nodes, 2,000
   // links 16 / 27; 5,003 nodes, two iterations 52 / 56).
-  if (link_in_block(plan.nodes)) {
+  if (plan.in_block) {
     const uint32_t w = plan.width > 1024 ? 1024 : (plan.width + 31) / 32 * 32;
     D3_LAUNCH(k_link_block, 1, w, plan.nodes * 2 * sizeof(double2), st)(c);
     return;
@@ -1940,19 +1940,13 @@ void set_status(uint32_t *status, uint32_t bits, cudaStream_t st) {
 void center_sum(const NodeArrays &a, ForceScratch &s, uint32_t *status, cudaStream_t st) {
   if (a.n == 0) return;
   if (a.n <= CSUM_SERIAL_MAX && ((uintptr_t)a.x & 15) == 0 && ((uintptr_t)a.y & 15) == 0) {
-    static bool sattr = [] {
-      return cudaFuncSetAttribute(k_csum_serial, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)CSUM_SERIAL_SMEM) == cudaSuccess;
-    }();
+    const bool sattr = open_shared<k_csum_serial>(CSUM_SERIAL_SMEM);
     D3_LAUNCH(k_csum_serial, 1, 32, CSUM_SERIAL_SMEM, st)(a.x, a.y, a.n, s.center, status,
                                                           s.csum_stamps);
     if (!sattr || cudaGetLastError() != cudaSuccess) set_status(status, ST_CENTER_RECORDS, st);
     return;
   }
-  static bool attr = [] {
-    return cudaFuncSetAttribute(k_csum_walk, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)CSUM_WALK_SMEM) == cudaSuccess;
-  }();
+  const bool attr = open_shared<k_csum_walk>(CSUM_WALK_SMEM);
   const CsumGeom g = csum_geom(a.n);
   CsumRec *recs = static_cast<CsumRec *>(s.csum_recs);
   uint32_t *counts = s.csum_counts, *offsets = s.csum_counts + 2 * g.nc + 1;

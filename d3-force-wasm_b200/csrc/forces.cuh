@@ -68,6 +68,7 @@ struct LinkPlan {
   uint32_t m = 0, levels = 0, nodes = 0;
   uint32_t width = 0;               // links of the widest level
   bool self = false;                // some link joins a node with itself
+  bool in_block = false;            // runs in one block (no messages)
   bool gathered = false;            // par holds the current link arrays
   uint32_t *order = nullptr;        // device: link ids grouped by level
   uint32_t *level_start = nullptr;  // device: levels + 1 offsets (level 1 first at [1])

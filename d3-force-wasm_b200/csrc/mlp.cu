@@ -443,12 +443,7 @@ __global__ void __launch_bounds__(TT) k_mlp_infer_tc(const float *x, uint32_t n,
 int mlp_infer_tc(const float *x, uint32_t n, const float *params, float *y, uint32_t *err_flag,
                  cudaStream_t st) {
   if (n == 0) return 0;
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(k_mlp_infer_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)sizeof(InferSmem));
-    attr = true;
-  }
+  if (!open_shared<k_mlp_infer_tc>(sizeof(InferSmem))) return -1;
   D3_LAUNCH(k_mlp_infer_tc, blocks_for(n, TT), TT, sizeof(InferSmem), st)(x, n, params, y,
                                                                          err_flag);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
@@ -465,8 +460,6 @@ int grad_ctas(uint32_t n) {
   static int sms = 0;
   if (!sms) {
     int dev = 0, count = 0;
-    cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)sizeof(TrainSmem));
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev);
     sms = count;
@@ -477,6 +470,7 @@ int grad_ctas(uint32_t n) {
 
 int grad_launch(const float *x, const float *y, uint32_t n, const float *params, float *part, int ctas,
                 cudaStream_t st) {
+  if (!open_shared<k_mlp_grad>(sizeof(TrainSmem))) return -1;
   D3_LAUNCH(k_mlp_grad, ctas, GTHREADS, sizeof(TrainSmem), st)(x, y, n, params, (float)n, part);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }

@@ -1185,10 +1185,7 @@ void tree_build_shifted(TreeDev &t, const double *xs, const double *ys, const do
   a.extent = t.extent; a.info = t.info; a.status = status;
   a.stamps = t.stamps;
   if (n > 0 && n <= TREE_SMALL_MAX) {
-    static const bool attr =
-        cudaFuncSetAttribute(k_tree_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sizeof(TreeSmallShared)) == cudaSuccess;
-    if (attr) {
+    if (open_shared<k_tree_small>(sizeof(TreeSmallShared))) {
       unsigned threads = 64;
       while (threads < n) threads <<= 1;
       D3_LAUNCH(k_tree_small, 1, threads, sizeof(TreeSmallShared), st)(a);
