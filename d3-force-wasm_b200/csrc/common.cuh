@@ -116,6 +116,24 @@ extern unsigned long long g_launches;
   for (int d3_launch_once_ = (++::d3::g_launches, 0); d3_launch_once_ < 1; ++d3_launch_once_) \
   kernel<<<__VA_ARGS__>>>
 
+// D3_LAUNCH for a caller that goes another way where the launch does not
+// happen: false then.
+template <class T>
+struct as_declared {
+  using type = T;
+};
+template <class... P>
+bool launch(void (*kernel)(P...), unsigned blocks, unsigned threads, size_t smem, cudaStream_t st,
+            typename as_declared<P>::type... args) {
+  void *params[] = {(void *)&args...};
+  ++g_launches;
+  if (cudaLaunchKernel((const void *)kernel, dim3(blocks), dim3(threads), params, smem, st) ==
+      cudaSuccess)
+    return true;
+  cudaGetLastError();
+  return false;
+}
+
 // Lets KERNEL take `bytes` of dynamic shared memory on the current device (past
 // 48 KB it has to be allowed, and the attribute is the device's): whether it
 // may. One size per kernel.

@@ -684,18 +684,18 @@ constexpr size_t MB_DRAWS_SMEM = 64 * 1024;
 // longest serial visit at 8,000 targets).
 constexpr uint32_t MB_WARP_NODES = 7000;
 
-static void launch_traverse(TreeDev &t, const NodeArrays &a, const double *strengths,
+static bool launch_traverse(TreeDev &t, const NodeArrays &a, const double *strengths,
                             const ManyBodyParams &p, ForceScratch &s, cudaStream_t st) {
   const uint32_t n = a.n;
   const MRec *rec = (const MRec *)t.rec;
   // four warps a block: at most 42 KB (the cell buffers may be larger than n asks for)
   const uint32_t words = mb_warp_words(t.cells_cap);
-  if (n <= MB_WARP_NODES && 16 * words <= 42 * 1024)
-    D3_LAUNCH(k_mb_traverse_warp, blocks_for(n * 32ull, 128), 128, 16 * words, st)(
-        rec, t.cells, t.perm, t.info, a.x, a.y, a.vx, a.vy, strengths, p, n, s.draws, s.counters, words);
-  else
-    D3_LAUNCH(k_mb_traverse, blocks_for(n, 128), 128, 0, st)(rec, t.perm, t.info, a.x, a.y, a.vx, a.vy,
-                                                          strengths, p, n, s.draws, s.counters);
+  if (n <= MB_WARP_NODES && 16 * words <= 42 * 1024 &&
+      launch(k_mb_traverse_warp, blocks_for(n * 32ull, 128), 128, 16 * words, st, rec, t.cells, t.perm,
+             t.info, a.x, a.y, a.vx, a.vy, strengths, p, n, s.draws, s.counters, words))
+    return true;
+  return launch(k_mb_traverse, blocks_for(n, 128), 128, 0, st, rec, t.perm, t.info, a.x, a.y, a.vx,
+                a.vy, strengths, p, n, s.draws, s.counters);
 }
 
 void many_body_exact(TreeDev &t, const NodeArrays &a, const double *strengths,
@@ -707,16 +707,14 @@ void many_body_exact(TreeDev &t, const NodeArrays &a, const double *strengths,
   if (n == 0) return;
   unsigned cb, ct;
   climb_grid(cb, ct, t.cells_cap);
-  if (n <= ACC_BLOCK_NODES)
-    D3_LAUNCH(k_mb_accumulate_block, 1, 512, 0, st)(
-        t.cells, t.parent, t.pnch, t.counter, t.perm, t.skip, a.x, a.y, strengths, p.theta2,
-        (MRec *)t.rec, t.info);
-  else
-    D3_LAUNCH(k_mb_accumulate, cb, ct, 0, st)(t.cells, t.parent, t.pnch, t.counter, t.perm, t.skip, a.x,
-                                       a.y, strengths, p.theta2, (MRec *)t.rec, t.info);
+  bool ran = n <= ACC_BLOCK_NODES &&
+             launch(k_mb_accumulate_block, 1, 512, 0, st, t.cells, t.parent, t.pnch, t.counter, t.perm,
+                    t.skip, a.x, a.y, strengths, p.theta2, (MRec *)t.rec, t.info);
+  ran = ran || launch(k_mb_accumulate, cb, ct, 0, st, t.cells, t.parent, t.pnch, t.counter, t.perm,
+                      t.skip, a.x, a.y, strengths, p.theta2, (MRec *)t.rec, t.info);
   if (mark) mark(1);
   cudaMemsetAsync(s.counters, 0, 2 * sizeof(uint32_t), st);
-  launch_traverse(t, a, strengths, p, s, st);
+  if (!ran || !launch_traverse(t, a, strengths, p, s, st)) tree_failed(t, status, st);
   if (host_draws) {
     scan_u32(s.draws, s.offsets, n, s.scan_part, s.counters, st);
     return;
@@ -1295,8 +1293,7 @@ void link_exact(const NodeArrays &a, const LinkArrays &l, LinkPlan &plan, double
   // links 16 / 27; 5,003 nodes, two iterations 52 / 56).
   if (plan.in_block) {
     const uint32_t w = plan.width > 1024 ? 1024 : (plan.width + 31) / 32 * 32;
-    D3_LAUNCH(k_link_block, 1, w, plan.nodes * 2 * sizeof(double2), st)(c);
-    return;
+    if (launch(k_link_block, 1, w, plan.nodes * 2 * sizeof(double2), st, c)) return;
   }
   static int sms = 0, per_sm = 0;
   if (!per_sm) {
@@ -1312,7 +1309,7 @@ void link_exact(const NodeArrays &a, const LinkArrays &l, LinkPlan &plan, double
     }
     per_sm = want;
   }
-  {
+  if (!plan.in_block) {
     void *params[] = {&c};
     const unsigned most = (unsigned)(sms * per_sm), blocks = blocks_for(l.m, 256);
     ++g_launches;
@@ -1321,7 +1318,7 @@ void link_exact(const NodeArrays &a, const LinkArrays &l, LinkPlan &plan, double
       return;
     cudaGetLastError();
   }
-  // (without a cooperative launch: one launch per level)
+  // (without either launch: one per level)
   cudaMemsetAsync(flag, 0, sizeof(uint32_t), st);
   D3_LAUNCH(k_save_v, blocks_for(n, 256), 256, 0, st)(a.snap_vx, a.snap_vy, a.vx, a.vy, n);
   for (double k = 0; k < iterations; k += 1) {

@@ -180,7 +180,7 @@ extern "C" int32_t d3_many_body_exact_noalloc(const double *x, const double *y, 
   a.n = n;
   ManyBodyParams p{theta2, distance_min2, distance_max2, alpha};
   many_body_exact(t, a, strength, p, rng, s, words, false, st);
-  D3_LAUNCH(k_noalloc_out, 1, 1, 0, st)(rng, t.info, words, words + 8);
+  if (!launch(k_noalloc_out, 1, 1, 0, st, rng, t.info, words, words + 8)) return D3_WORKER_FAILED;
   uint32_t out[3] = {0, 0, 0};
   if (cudaMemcpyAsync(out, words + 8, sizeof out, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
       cudaStreamSynchronize(st) != cudaSuccess)

@@ -489,11 +489,10 @@ __global__ void __launch_bounds__(SB_THREADS) k_sort_block(uint64_t *keys, uint3
 void radix_sort_u64(uint64_t *keys, uint32_t *vals, uint32_t n, int byte_lo, int byte_hi,
                     bool partition_hi_bit, const SortScratch &s, cudaStream_t st) {
   if (n == 0) return;
-  if (n <= SORT_BLOCK_MAX && open_shared<k_sort_block>(SB_SMEM)) {
-    D3_LAUNCH(k_sort_block, 1, SB_THREADS, SB_SMEM, st)(keys, vals, n, byte_lo, byte_hi - byte_lo,
-                                                        partition_hi_bit);
+  if (n <= SORT_BLOCK_MAX && open_shared<k_sort_block>(SB_SMEM) &&
+      launch(k_sort_block, 1, SB_THREADS, SB_SMEM, st, keys, vals, n, byte_lo, byte_hi - byte_lo,
+             partition_hi_bit))
     return;
-  }
   uint64_t *ak = keys, *bk = s.keys_tmp;
   uint32_t *av = vals, *bv = s.vals_tmp;
   const uint32_t tiles = (n + SORT_TILE - 1) / SORT_TILE;

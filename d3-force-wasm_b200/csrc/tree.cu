@@ -731,7 +731,7 @@ __device__ uint32_t tb_run_rank(const uint64_t *keys, const uint32_t *vals, uint
   return pos;
 }
 
-// The tree build's cooperative launch did not happen.
+// A launch of the tree build, or one that reads the tree, did not happen.
 __global__ void k_tree_failed(uint32_t *info, uint32_t *status) {
   info[1] = 0;
   info[5] = 0xffffffffu;
@@ -1143,6 +1143,10 @@ void fast_box(TreeDev &t, const double *xs, const double *ys, uint32_t n, double
                                            square);
 }
 
+void tree_failed(TreeDev &t, uint32_t *status, cudaStream_t st) {
+  D3_LAUNCH(k_tree_failed, 1, 1, 0, st)(t.info, status);
+}
+
 static int g_tree_blocks = 0;
 
 void tree_build(TreeDev &t, const double *xs, const double *ys, uint32_t n, uint32_t *status,
@@ -1185,22 +1189,17 @@ void tree_build_shifted(TreeDev &t, const double *xs, const double *ys, const do
   a.extent = t.extent; a.info = t.info; a.status = status;
   a.stamps = t.stamps;
   if (n > 0 && n <= TREE_SMALL_MAX) {
-    if (open_shared<k_tree_small>(sizeof(TreeSmallShared))) {
-      unsigned threads = 64;
-      while (threads < n) threads <<= 1;
-      D3_LAUNCH(k_tree_small, 1, threads, sizeof(TreeSmallShared), st)(a);
+    unsigned threads = 64;
+    while (threads < n) threads <<= 1;
+    if (open_shared<k_tree_small>(sizeof(TreeSmallShared)) &&
+        launch(k_tree_small, 1, threads, sizeof(TreeSmallShared), st, a))
       return;
-    }
   }
   void *params[] = {&a};
   ++g_launches;
   if (cudaLaunchCooperativeKernel((const void *)k_tree_build, g_tree_blocks, TB_THREADS, params, 0,
-                                  st) != cudaSuccess) {
-    // report it: without the launch the cells, perm and leaf_of are stale,
-    // so the passes that follow see an empty tree (info[1] = 0) and the
-    // launch-failure mark (info[5] = 0xffffffff), which they check
-    D3_LAUNCH(k_tree_failed, 1, 1, 0, st)(t.info, status);
-  }
+                                  st) != cudaSuccess)
+    tree_failed(t, status, st);
 }
 
 }  // namespace d3

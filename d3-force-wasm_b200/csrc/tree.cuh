@@ -52,6 +52,10 @@ inline size_t tree_hist_words(uint32_t n) {
   return a > b ? a : b;
 }
 
+// A launch did not happen, so the cells, perm and leaf_of (or what is made of
+// them) are stale: the passes that follow see an empty tree (info[1] = 0) and
+// the mark for it (info[5] = 0xffffffff), which they check.
+void tree_failed(TreeDev &t, uint32_t *status, cudaStream_t st);
 int tree_reserve(TreeDev &t, uint32_t n, cudaStream_t st);
 void tree_free(TreeDev &t);
 

@@ -1,7 +1,8 @@
 """A kernel's shared-memory attribute belongs to the device that was current
 when it was set: it is set on every device a process uses, not once in the
-process."""
+process, and a launch that another path could stand in for is checked."""
 
+import re
 import subprocess
 
 import pytest
@@ -38,3 +39,12 @@ def test_attributes_are_not_set_once_in_the_process(name):
     # (the set-up of a handle, in the other sources, runs with its device current)
     assert "cudaFuncSetAttribute" not in S.source(name)
 
+
+@pytest.mark.parametrize("name, kernel", [
+    ("tree.cu", "k_tree_small"), ("forces.cu", "k_link_block"), ("forces.cu", "k_mb_accumulate_block"),
+    ("forces.cu", "k_mb_accumulate"), ("forces.cu", "k_mb_traverse_warp"), ("forces.cu", "k_mb_traverse"),
+    ("scan_sort.cu", "k_sort_block"), ("noalloc.cu", "k_noalloc_out")])
+def test_launches_are_checked(name, kernel):
+    text = S.source(name)
+    assert not re.search(r"D3_LAUNCH\(\(?%s[,<]" % kernel, text)
+    assert re.search(r"\blaunch\(%s," % kernel, text)
