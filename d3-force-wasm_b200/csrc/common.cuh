@@ -14,6 +14,7 @@
 
 #include "../../include/d3force_b200.h"
 #include "per_device.cuh"
+#include "room.cuh"
 
 namespace d3 {
 
@@ -154,6 +155,24 @@ bool open_shared(size_t bytes) {
 inline unsigned blocks_for(size_t n, unsigned threads) {
   size_t b = (n + threads - 1) / threads;
   return b ? (unsigned)b : 1u;
+}
+
+// take_all on the device.
+inline bool device_take(std::initializer_list<Want> wants) {
+  return take_all(
+      wants,
+      [](void **p, size_t bytes) {
+        if (cudaMalloc(p, bytes) == cudaSuccess) return true;
+        cudaGetLastError();
+        return false;
+      },
+      [](void *p) { cudaFree(p); });
+}
+
+// Device buffers given back, their pointers null.
+template <class... T>
+void device_give(T *&...p) {
+  ((cudaFree(p), p = nullptr), ...);
 }
 
 // The pause between polls of a device wait after its first few polls, in

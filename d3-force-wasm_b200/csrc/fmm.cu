@@ -46,8 +46,8 @@ constexpr unsigned UP_THREADS = 64, M2L_THREADS = 32, P2P_THREADS = 32, DOWN_THR
 // A P2P list of more than LONG_LIST source leaves (a leaf beside a far denser
 // region) goes by segments of 32; the terms of a segment and 16 targets take a
 // unit of 32 KB, LONG_UNITS_MAX of them at most (256 MB, held once a run wanted
-// some; lists past that, and leaves of more than LONG_POINTS points, go by
-// k_fmm_p2p).
+// some; lists past that or past what the device has left, and leaves of more
+// than LONG_POINTS points, go by k_fmm_p2p).
 constexpr uint32_t LONG_LIST = 64, LONG_POINTS = 64, LONG_UNITS_MAX = 8192;
 constexpr uint32_t LONG_UNIT = 32 * 4 * 16;  // terms: source leaf, three pairs and a sum, target
 
@@ -86,7 +86,7 @@ struct FmmDev {
   uint2 *long_items = nullptr;
   uint32_t *long_at = nullptr, *longs = nullptr, *long_flags = nullptr;
   double2 *long_terms = nullptr;
-  uint32_t long_cap = 0, long_want = 0;  // units: held, wanted by the last run
+  SpareRoom long_room{0, 0, LONG_UNITS_MAX};  // units
   cudaEvent_t lists_read = nullptr;  // the lists' words are in h_info
   double *square = nullptr;      // box x0, y0, side
   uint32_t *h_info = nullptr;    // pinned mirror of info
@@ -1913,27 +1913,19 @@ int fmm_run(FastScratch &s, TreeDev &t, const NodeArrays &a, const double *stren
   args.mco = f.mco;
   args.lco = f.lco;
   args.arrive = f.arrive;
-  if (f.long_want > f.long_cap && f.long_cap < LONG_UNITS_MAX) {
-    // what the last run wanted, and a quarter more
-    cudaFree(f.longs); cudaFree(f.long_items); cudaFree(f.long_flags); cudaFree(f.long_terms);
-    f.longs = f.long_flags = nullptr;
-    f.long_items = nullptr;
-    f.long_terms = nullptr;
-    f.long_cap = 0;
-    const uint32_t want = f.long_want + f.long_want / 4;
-    const size_t cap = want < LONG_UNITS_MAX ? want : LONG_UNITS_MAX;
-    D3_CUDA_OK(cudaMalloc(&f.longs, cap * 4));
-    D3_CUDA_OK(cudaMalloc(&f.long_items, cap * sizeof(uint2)));
-    D3_CUDA_OK(cudaMalloc(&f.long_flags, cap * 16 * 4));
-    D3_CUDA_OK(cudaMalloc(&f.long_terms, cap * LONG_UNIT * sizeof(double2)));
-    f.long_cap = (uint32_t)cap;
-  }
+  f.long_room.grow([&](size_t cap) {
+    device_give(f.longs, f.long_items, f.long_flags, f.long_terms);
+    return device_take({{(void **)&f.longs, cap * 4},
+                        {(void **)&f.long_items, cap * sizeof(uint2)},
+                        {(void **)&f.long_flags, cap * 16 * 4},
+                        {(void **)&f.long_terms, cap * LONG_UNIT * sizeof(double2)}});
+  });
   args.long_items = f.long_items;
   args.long_at = f.long_at;
   args.longs = f.longs;
   args.long_flags = f.long_flags;
   args.long_terms = f.long_terms;
-  args.long_cap = f.long_cap;
+  args.long_cap = f.long_room.cap;
   args.m2l_off = f.m2l_off; args.m2l_cnt = f.m2l_cnt;
   args.p2p_off = f.p2p_off; args.p2p_cnt = f.p2p_cnt;
   args.fwd_off = f.fwd_off; args.fwd_cnt = f.fwd_cnt;
@@ -1973,7 +1965,7 @@ int fmm_run(FastScratch &s, TreeDev &t, const NodeArrays &a, const double *stren
     if (ncells <= P2P_FEW_CELLS)
       D3_LAUNCH(k_fmm_p2p<true>, blocks_for(4 * ncells, P2P_THREADS / 32), P2P_THREADS, 0, st)(args);
     else D3_LAUNCH(k_fmm_p2p<false>, pb, P2P_THREADS, 0, st)(args);
-    if (f.long_cap) {
+    if (f.long_room.cap) {
       D3_LAUNCH(k_fmm_p2p_terms, LONG_BLOCKS, LONG_THREADS, 0, st)(args);
       D3_LAUNCH(k_fmm_p2p_add, LONG_BLOCKS / 8, LONG_THREADS, 0, st)(args);
     }
@@ -1985,7 +1977,7 @@ int fmm_run(FastScratch &s, TreeDev &t, const NodeArrays &a, const double *stren
       f.last_m2l = f.h_info[FI_POOL_M2L];
       f.last_p2p = f.h_info[FI_POOL_P2P];
       f.last_fwd = f.h_info[FI_POOL_FWD];
-      if (f.h_info[FI_LONG_UNITS] > f.long_cap) f.long_want = f.h_info[FI_LONG_UNITS];
+      f.long_room.want = f.h_info[FI_LONG_UNITS];
       break;
     }
     if ((ovf & 2) || attempt > 8) return -1;  // a call stack overflowed, or a wait ran out
