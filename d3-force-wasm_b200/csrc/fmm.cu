@@ -1695,36 +1695,38 @@ int grow(T *&p, size_t &cap, size_t need) {
 int fmm_reserve_points(FmmDev &f, uint32_t n) {
   if (n <= f.pcap && f.pcap) return 0;
   uint32_t cap = n < 1024 ? 1024 : n;
-  cudaFree(f.px); cudaFree(f.py); cudaFree(f.ps); cudaFree(f.ux); cudaFree(f.uy);
-  D3_CUDA_OK(cudaMalloc(&f.px, cap * 8ull));
-  D3_CUDA_OK(cudaMalloc(&f.py, cap * 8ull));
-  D3_CUDA_OK(cudaMalloc(&f.ps, cap * 8ull));
-  D3_CUDA_OK(cudaMalloc(&f.ux, cap * 8ull));
-  D3_CUDA_OK(cudaMalloc(&f.uy, cap * 8ull));
-  cudaFree(f.pt_levels);
-  D3_CUDA_OK(cudaMalloc(&f.pt_levels, cap * 2ull));
+  f.pcap = 0;
+  device_give(f.px, f.py, f.ps, f.ux, f.uy, f.pt_levels);
+  if (!device_take({{(void **)&f.px, cap * 8ull},
+                    {(void **)&f.py, cap * 8ull},
+                    {(void **)&f.ps, cap * 8ull},
+                    {(void **)&f.ux, cap * 8ull},
+                    {(void **)&f.uy, cap * 8ull},
+                    {(void **)&f.pt_levels, cap * 2ull}}))
+    return -1;
   f.pcap = cap;
   return 0;
 }
 
 int fmm_reserve_cells(FmmDev &f, uint32_t ccap) {
   if (ccap <= f.ccap && f.ccap) return 0;
-  cudaFree(f.cells); cudaFree(f.bx0); cudaFree(f.by0); cudaFree(f.bx1); cudaFree(f.by1);
-  cudaFree(f.m2l_off); cudaFree(f.m2l_cnt); cudaFree(f.p2p_off);
-  cudaFree(f.p2p_cnt); cudaFree(f.fwd_off); cudaFree(f.fwd_cnt); cudaFree(f.arrive); cudaFree(f.long_at);
-  D3_CUDA_OK(cudaMalloc(&f.cells, ccap * sizeof(FCell)));
-  D3_CUDA_OK(cudaMalloc(&f.bx0, ccap * 8ull));
-  D3_CUDA_OK(cudaMalloc(&f.by0, ccap * 8ull));
-  D3_CUDA_OK(cudaMalloc(&f.bx1, ccap * 8ull));
-  D3_CUDA_OK(cudaMalloc(&f.by1, ccap * 8ull));
-  D3_CUDA_OK(cudaMalloc(&f.m2l_off, ccap * 4ull));
-  D3_CUDA_OK(cudaMalloc(&f.m2l_cnt, ccap * 4ull));
-  D3_CUDA_OK(cudaMalloc(&f.p2p_off, ccap * 4ull));
-  D3_CUDA_OK(cudaMalloc(&f.p2p_cnt, ccap * 4ull));
-  D3_CUDA_OK(cudaMalloc(&f.fwd_off, ccap * 4ull));
-  D3_CUDA_OK(cudaMalloc(&f.fwd_cnt, ccap * 4ull));
-  D3_CUDA_OK(cudaMalloc(&f.arrive, ccap * 4ull));
-  D3_CUDA_OK(cudaMalloc(&f.long_at, ccap * 4ull));
+  f.ccap = 0;
+  device_give(f.cells, f.bx0, f.by0, f.bx1, f.by1, f.m2l_off, f.m2l_cnt, f.p2p_off, f.p2p_cnt, f.fwd_off,
+              f.fwd_cnt, f.arrive, f.long_at);
+  if (!device_take({{(void **)&f.cells, ccap * sizeof(FCell)},
+                    {(void **)&f.bx0, ccap * 8ull},
+                    {(void **)&f.by0, ccap * 8ull},
+                    {(void **)&f.bx1, ccap * 8ull},
+                    {(void **)&f.by1, ccap * 8ull},
+                    {(void **)&f.m2l_off, ccap * 4ull},
+                    {(void **)&f.m2l_cnt, ccap * 4ull},
+                    {(void **)&f.p2p_off, ccap * 4ull},
+                    {(void **)&f.p2p_cnt, ccap * 4ull},
+                    {(void **)&f.fwd_off, ccap * 4ull},
+                    {(void **)&f.fwd_cnt, ccap * 4ull},
+                    {(void **)&f.arrive, ccap * 4ull},
+                    {(void **)&f.long_at, ccap * 4ull}}))
+    return -1;
   f.ccap = ccap;
   return 0;
 }
@@ -1903,12 +1905,11 @@ int fmm_run(FastScratch &s, TreeDev &t, const NodeArrays &a, const double *stren
   args.bx0 = f.bx0; args.by0 = f.by0; args.bx1 = f.bx1; args.by1 = f.by1;
   args.ncells = ncells;
   if ((size_t)ncells * stride > f.coef_cap || !f.mco) {
-    cudaFree(f.mco);
-    cudaFree(f.lco);
-    f.mco = f.lco = nullptr;
-    f.coef_cap = (size_t)ncells * stride + (size_t)ncells * stride / 4;
-    D3_CUDA_OK(cudaMalloc(&f.mco, f.coef_cap * 8));
-    D3_CUDA_OK(cudaMalloc(&f.lco, f.coef_cap * 8));
+    f.coef_cap = 0;
+    device_give(f.mco, f.lco);
+    const size_t cap = (size_t)ncells * stride + (size_t)ncells * stride / 4;
+    if (!device_take({{(void **)&f.mco, cap * 8}, {(void **)&f.lco, cap * 8}})) return -1;
+    f.coef_cap = cap;
   }
   args.mco = f.mco;
   args.lco = f.lco;

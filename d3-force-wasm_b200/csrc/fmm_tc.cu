@@ -1908,38 +1908,39 @@ int build_tables(TcTabSet &d, uint32_t p, double kappa, cudaStream_t st) {
 int reserve(TcDev &d, uint32_t ncells, uint32_t m) {
   if (ncells > d.ccap) {
     const uint32_t cap = ncells + ncells / 4 + 64;
-    cudaFree(d.cells); cudaFree(d.mco); cudaFree(d.mbf); cudaFree(d.lco); cudaFree(d.near);
-    cudaFree(d.m2l); cudaFree(d.groups); cudaFree(d.loff);
-    D3_CUDA_OK(cudaMalloc(&d.cells, cap * sizeof(TcCell)));
-    D3_CUDA_OK(cudaMalloc(&d.mco, (size_t)cap * 2 * TC_MAXQ * 8));
-    D3_CUDA_OK(cudaMalloc(&d.mbf, (size_t)cap * 64 * 2));
-    D3_CUDA_OK(cudaMalloc(&d.lco, (size_t)cap * TC_KN * 4));
-    D3_CUDA_OK(cudaMalloc(&d.near, (size_t)cap * TC_NEAR_MAX * 4));
-    D3_CUDA_OK(cudaMalloc(&d.m2l, (size_t)cap * TC_SLOT_MAX * 4));
-    D3_CUDA_OK(cudaMalloc(&d.groups, (size_t)cap * 4 * 4));
-    D3_CUDA_OK(cudaMalloc(&d.loff, (size_t)cap * 8 * 4));
-    cudaFree(d.arrive);
-    D3_CUDA_OK(cudaMalloc(&d.arrive, (size_t)cap * 4));
-    cudaFree(d.seg_at);
-    D3_CUDA_OK(cudaMalloc(&d.seg_at, (size_t)cap * 2 * 4));
+    d.ccap = 0;
+    device_give(d.cells, d.mco, d.mbf, d.lco, d.near, d.m2l, d.groups, d.loff, d.arrive, d.seg_at);
+    if (!device_take({{(void **)&d.cells, cap * sizeof(TcCell)},
+                      {(void **)&d.mco, (size_t)cap * 2 * TC_MAXQ * 8},
+                      {(void **)&d.mbf, (size_t)cap * 64 * 2},
+                      {(void **)&d.lco, (size_t)cap * TC_KN * 4},
+                      {(void **)&d.near, (size_t)cap * TC_NEAR_MAX * 4},
+                      {(void **)&d.m2l, (size_t)cap * TC_SLOT_MAX * 4},
+                      {(void **)&d.groups, (size_t)cap * 4 * 4},
+                      {(void **)&d.loff, (size_t)cap * 8 * 4},
+                      {(void **)&d.arrive, (size_t)cap * 4},
+                      {(void **)&d.seg_at, (size_t)cap * 2 * 4}}))
+      return -1;
     d.ccap = cap;
   }
   if (m > d.pcap) {
     const uint32_t cap = m + m / 4 + 1024;
-    cudaFree(d.kick);
-    cudaFree(d.nearbuf);
-    D3_CUDA_OK(cudaMalloc(&d.kick, (size_t)cap * sizeof(double2)));
-    D3_CUDA_OK(cudaMalloc(&d.nearbuf, (size_t)cap * sizeof(float2)));
-    cudaFree(d.leafidx);
-    D3_CUDA_OK(cudaMalloc(&d.leafidx, (size_t)cap * sizeof(uint32_t)));
+    d.pcap = 0;
+    device_give(d.kick, d.nearbuf, d.leafidx);
+    if (!device_take({{(void **)&d.kick, (size_t)cap * sizeof(double2)},
+                      {(void **)&d.nearbuf, (size_t)cap * sizeof(float2)},
+                      {(void **)&d.leafidx, (size_t)cap * sizeof(uint32_t)}}))
+      return -1;
     d.pcap = cap;
   }
   if (d.ccap > d.lcap) {
-    cudaFree(d.feat); cudaFree(d.leaves); cudaFree(d.mlp_x); cudaFree(d.mlp_y);
-    D3_CUDA_OK(cudaMalloc(&d.feat, (size_t)d.ccap * 16 * 4));
-    D3_CUDA_OK(cudaMalloc(&d.leaves, (size_t)d.ccap * 4));
-    D3_CUDA_OK(cudaMalloc(&d.mlp_x, (size_t)d.ccap * 12 * 4));
-    D3_CUDA_OK(cudaMalloc(&d.mlp_y, (size_t)d.ccap * 2 * 4));
+    d.lcap = 0;
+    device_give(d.feat, d.leaves, d.mlp_x, d.mlp_y);
+    if (!device_take({{(void **)&d.feat, (size_t)d.ccap * 16 * 4},
+                      {(void **)&d.leaves, (size_t)d.ccap * 4},
+                      {(void **)&d.mlp_x, (size_t)d.ccap * 12 * 4},
+                      {(void **)&d.mlp_y, (size_t)d.ccap * 2 * 4}}))
+      return -1;
     d.lcap = d.ccap;
   }
   return 0;
@@ -2268,15 +2269,13 @@ int tc_run(FastScratch &s, TreeDev &t, const NodeArrays &a, const double *streng
   size_t need = d.last_pool ? d.last_pool + d.last_pool / 4 + 4096 : (size_t)pr.ncells * 24 + 4096;
   for (int attempt = 0;; ++attempt) {
     if (need > d.pool_cap) {
-      cudaFree(d.pool);
-      d.pool = nullptr;
+      d.pool_cap = 0;
+      device_give(d.pool, d.seg_p2p, d.seg_w);
+      if (!device_take({{(void **)&d.pool, need * 4},
+                        {(void **)&d.seg_p2p, (need / SEG_P2P + 1) * sizeof(uint2)},
+                        {(void **)&d.seg_w, (need / SEG_W + 1) * sizeof(uint2)}}))
+        return -1;
       d.pool_cap = need;
-      cudaFree(d.seg_p2p);
-      cudaFree(d.seg_w);
-      d.seg_p2p = d.seg_w = nullptr;
-      D3_CUDA_OK(cudaMalloc(&d.pool, d.pool_cap * 4));
-      D3_CUDA_OK(cudaMalloc(&d.seg_p2p, (d.pool_cap / SEG_P2P + 1) * sizeof(uint2)));
-      D3_CUDA_OK(cudaMalloc(&d.seg_w, (d.pool_cap / SEG_W + 1) * sizeof(uint2)));
     }
     g.pool = d.pool;
     g.pool_cap = d.pool_cap;
@@ -2315,9 +2314,9 @@ int tc_run(FastScratch &s, TreeDev &t, const NodeArrays &a, const double *streng
   if (samples > CHECK_MAX_SAMPLES) samples = CHECK_MAX_SAMPLES;
   const uint32_t parts = blocks_for(pr.m, CHECK_THREADS * CHECK_PTS);
   if ((size_t)samples * parts > d.chk_cap) {
-    cudaFree(d.chk_part);
-    d.chk_part = nullptr;
-    D3_CUDA_OK(cudaMalloc(&d.chk_part, (size_t)samples * parts * sizeof(double2)));
+    d.chk_cap = 0;
+    device_give(d.chk_part);
+    if (!device_take({{(void **)&d.chk_part, (size_t)samples * parts * sizeof(double2)}})) return -1;
     d.chk_cap = samples * parts;
   }
   D3_LAUNCH(k_tc_check, parts, CHECK_THREADS, 0, st)(g, samples, prm.dmin2, d.chk_part);

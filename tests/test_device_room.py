@@ -6,6 +6,8 @@ have come."""
 import re
 import subprocess
 
+import pytest
+
 import test_stream_order as S
 
 HARNESS = r"""
@@ -98,3 +100,19 @@ def test_long_lists_go_without_their_room():
     text = S.function("fmm_run", S.source("fmm.cu"))
     assert not re.search(r"D3_CUDA_OK\(cudaMalloc\(&f\.long", text)
     assert "long_room.grow(" in text
+
+
+@pytest.mark.parametrize("name, function", [
+    ("fmm.cu", "fmm_run"), ("fmm.cu", "fmm_reserve_points"), ("fmm.cu", "fmm_reserve_cells"),
+    ("fmm_tc.cu", "reserve"), ("fmm_tc.cu", "tc_run")])
+def test_a_size_is_held_when_its_buffers_have_come(name, function):
+    # each group: its size to 0, the old buffers back, all the new ones or a
+    # return, then the size
+    text = S.function(function, S.source(name))
+    assert not re.search(r"\bcudaMalloc\(", text)
+    groups = re.findall(r"(\w)\.(\w*cap) = 0;\s*device_give\(([^)]*)\);(.*?)\1\.\2 = (?!0)", text, re.S)
+    assert len(groups) == len(re.findall(r"\bdevice_give\(", text)) - text.count(".grow([&]")
+    for _, _, given, between in groups:
+        taken = re.findall(r"\(void \*\*\)&(\w\.\w+)", between)
+        assert taken == [p.strip() for p in given.split(",")]
+        assert "return -1;" in between
