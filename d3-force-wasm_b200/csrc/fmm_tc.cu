@@ -157,7 +157,7 @@ struct TcDev {
   uint2 *seg_p2p = nullptr, *seg_w = nullptr;  // pool_cap / SEG_P2P and / SEG_W
   float2 *part_p2p = nullptr;                // SEG_POINTS per segment
   double2 *part_w = nullptr;
-  size_t part_p2p_cap = 0, part_w_cap = 0;   // segments
+  SpareRoom room_p2p, room_w;                // segments
   uint32_t *leafidx = nullptr;               // per sorted point: its leaf's index in the leaf list
   float *mlp = nullptr;              // installed network parameters (device)
   uint32_t ncells_last = 0;
@@ -196,8 +196,8 @@ struct TcArgs {
   uint32_t *leaves;
   uint32_t *seg_at;
   uint2 *seg_p2p, *seg_w;
-  float2 *part_p2p;
-  double2 *part_w;
+  float2 *part_p2p;  // null: the lists are not split
+  double2 *part_w;   // null: the lists are not split
   uint32_t *leafidx;  // per sorted point: its leaf's index in the leaf list (near pass)
   double2 *kick;  // non-null: the many-body kick goes here instead of into vx, vy
   double *vx, *vy;
@@ -1464,7 +1464,7 @@ __global__ void __launch_bounds__(NEAR_THREADS, 8) k_tc_near(TcArgs a, float2 *n
     const uint32_t all = a.loff[(size_t)c * 8 + 1], op = a.loff[(size_t)c * 8];
     // this item's entries of the list
     const uint32_t np0 = it.y * SEG_P2P;
-    const uint32_t np = more_segments(all, A.count, SEG_P2P) ? min(all, np0 + SEG_P2P) : all;
+    const uint32_t np = a.part_p2p && more_segments(all, A.count, SEG_P2P) ? min(all, np0 + SEG_P2P) : all;
     // lane groups: a lane holds two targets (slots gl and W + gl of the
     // round), W = ceil(count / 2) lanes a group, G = 32 / W groups (lanes
     // past G W idle); a leaf of more than 64 points takes several rounds
@@ -1606,13 +1606,13 @@ __global__ void __launch_bounds__(TC_THREADS) k_tc_far(TcArgs a, const float2 *n
     c0i = sc * a.mlp_y[(size_t)e * 2 + 1];
   }
   float wr, wi;
-  const uint32_t mw = more_segments(nw, C.count, SEG_W);
+  const uint32_t mw = a.part_w ? more_segments(nw, C.count, SEG_W) : 0;
   const float2 f = tc_far(a, k, cx, cy, inv_s, a.lco + (size_t)c * TC_KN, c0r, c0i, mw ? SEG_W : nw, ow,
                           mw ? a.part_w + (size_t)a.seg_at[2 * (size_t)c + 1] * SEG_POINTS + (k - C.first)
                              : nullptr,
                           mw, wr, wi);
   float2 nv = nearbuf[k];
-  const uint32_t mp = more_segments(a.loff[(size_t)c * 8 + 1], C.count, SEG_P2P);
+  const uint32_t mp = a.part_p2p ? more_segments(a.loff[(size_t)c * 8 + 1], C.count, SEG_P2P) : 0;
   if (mp) {
     const float2 *part = a.part_p2p + (size_t)a.seg_at[2 * (size_t)c] * SEG_POINTS + (k - C.first);
     for (uint32_t j = 0; j < mp; ++j) {
@@ -1946,17 +1946,16 @@ int reserve(TcDev &d, uint32_t ncells, uint32_t m) {
   return 0;
 }
 
-// Room for `segments` segments' partial sums, with headroom.
+// Room for `segments` segments' partial sums; null where it is not to be had
+// (the lists are then taken whole).
 template <typename T>
-int grow_parts(T *&p, size_t &cap, size_t segments) {
-  if (segments <= cap) return 0;
-  cudaFree(p);
-  p = nullptr;
-  cap = 0;
-  const size_t want = segments + segments / 4 + 64;
-  D3_CUDA_OK(cudaMalloc(&p, want * SEG_POINTS * sizeof(T)));
-  cap = want;
-  return 0;
+T *segment_sums(T *&p, SpareRoom &room, uint32_t segments) {
+  room.want = segments;
+  room.grow([&](size_t cap) {
+    device_give(p);
+    return device_take({{(void **)&p, cap * SEG_POINTS * sizeof(T)}});
+  });
+  return room.cap >= segments ? p : nullptr;
 }
 
 // The table set for (p, kappa): an existing one, else built in the older slot.
@@ -2052,7 +2051,7 @@ int tc_order_pass(TcDev &d, TcArgs &g, const TcTabSet &ts, uint32_t tiles, bool 
     cudaEventRecord(d.ev_lists, st);
     cudaStreamWaitEvent(d.side, d.ev_lists, 0);
     cudaEventRecord(d.ev[7], d.side);
-    const uint32_t segments = d.h_info[TI_SEG_P2P];
+    const uint32_t segments = g.part_p2p ? d.h_info[TI_SEG_P2P] : 0;
     D3_LAUNCH(k_tc_near, blocks_for(((size_t)nleaf + segments) * 32, NEAR_THREADS), NEAR_THREADS, 0,
               d.side)(g, d.nearbuf, segments);
     cudaEventRecord(d.ev[8], d.side);
@@ -2087,7 +2086,7 @@ int tc_order_pass(TcDev &d, TcArgs &g, const TcTabSet &ts, uint32_t tiles, bool 
     D3_LAUNCH(k_tc_features, lw, TC_THREADS, 0, d.side)(g);
     cudaEventRecord(d.ev_feat, d.side);
   }
-  if (const uint32_t segments = d.h_info[TI_SEG_W])
+  if (const uint32_t segments = g.part_w ? d.h_info[TI_SEG_W] : 0)
     D3_LAUNCH(k_tc_m2p_segments, blocks_for(segments * 32ull, 128), 128, 0, st)(g, segments);
   cudaEventRecord(d.ev[11], st);
   if (!far_only) cudaStreamWaitEvent(st, d.ev_near, 0);
@@ -2299,11 +2298,8 @@ int tc_run(FastScratch &s, TreeDev &t, const NodeArrays &a, const double *streng
     if (attempt > 6) return -1;
     need = 2 * (size_t)(used > need ? used : need);
   }
-  if (grow_parts(d.part_p2p, d.part_p2p_cap, d.h_info[TI_SEG_P2P]) ||
-      grow_parts(d.part_w, d.part_w_cap, d.h_info[TI_SEG_W]))
-    return -1;
-  g.part_p2p = d.part_p2p;
-  g.part_w = d.part_w;
+  g.part_p2p = segment_sums(d.part_p2p, d.room_p2p, d.h_info[TI_SEG_P2P]);
+  g.part_w = segment_sums(d.part_w, d.room_w, d.h_info[TI_SEG_W]);
   cudaEventRecord(d.ev[2], st);
   uint32_t tiles = 0;
   for (uint32_t q4 = 0; q4 < 4; ++q4) tiles += (d.h_info[TI_GROUP + q4] + TC_TILE - 1) / TC_TILE;

@@ -102,6 +102,15 @@ def test_long_lists_go_without_their_room():
     assert "long_room.grow(" in text
 
 
+def test_segments_go_without_their_room():
+    text = S.source("fmm_tc.cu")
+    assert "device_take" in S.function("segment_sums", text) and "grow_parts" not in text
+    # a kernel that could meet a split list asks whether there is room for its sums
+    for kernel in ("k_tc_near", "k_tc_far"):
+        for use in re.findall(r"[^;]*\bmore_segments\(", S.function(kernel, text)):
+            assert re.search(r"a\.part_(p2p|w) (&&|\?)", use), use
+
+
 @pytest.mark.parametrize("name, function", [
     ("fmm.cu", "fmm_run"), ("fmm.cu", "fmm_reserve_points"), ("fmm.cu", "fmm_reserve_cells"),
     ("fmm_tc.cu", "reserve"), ("fmm_tc.cu", "tc_run")])
