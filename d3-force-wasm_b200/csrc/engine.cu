@@ -1193,6 +1193,8 @@ double sim_stat(uint32_t h, uint32_t which) {
     fmm_tc_stats(s->fast, out);
     return out[which - 50];
   }
+  // runs of the plain FMM whose list build gave up waiting and took a launch a level
+  if (which == 29) return s->fast.lists_by_level;
   if ((which >= 300 && which < 364) || (which >= 400 && which < 464)) {
     // the last parallel collide's first attempt: 300 + k microseconds from
     // the end of its list build to the last turn of depth k, 400 + k turns

@@ -28,6 +28,7 @@ struct FastScratch {
   double learn_tol = 1e-5;
   uint32_t learn_samples = 64, learn_hold = 0;
   double learn_checks = 0, learn_fallbacks = 0, learn_last_rms = 0;
+  double lists_by_level = 0;  // plain FMM: runs whose lists took a launch a level
 };
 
 int fast_reserve(FastScratch &s, uint32_t n, cudaStream_t st);

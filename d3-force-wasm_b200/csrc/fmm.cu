@@ -29,6 +29,8 @@
 //           against each source leaf of its list in order.
 //  downward per cell with leaf children: L2L along its path from the root and
 //           into the children (fmm.zig:823-849), L2P there (fmm.zig:853-886).
+#include <cstdlib>
+
 #include "fast.cuh"
 #include "scan_sort.cuh"
 
@@ -63,10 +65,11 @@ struct FmmTables {
 
 // info words (device, mirrored to the host after the cell build)
 enum : uint32_t { FI_CELLS = 0, FI_OVERFLOW, FI_LEVELS, FI_POOL_M2L, FI_POOL_P2P, FI_POOL_FWD,
-                  FI_LIST_OVERFLOW,              // 1: a pool, 2: a call stack or a wait
+                  FI_LIST_OVERFLOW,              // 1: a pool, 2: a call stack, 4: a wait ran out
                   FI_TICKET,                     // k_fmm_lists' blocks so far
                   FI_LVL = 8,  // FI_LVL + d: first cell of level d
                   FI_LONG_UNITS = 36, FI_LONGS,  // long P2P lists: units of terms, leaves
+                  FI_DONE,                       // counts on while k_fmm_lists makes progress
                   FI_M = 40,                     // points to act on (0 when the extent is bad)
                   FI_BAD = 41 };                 // 1: the extent is not finite and positive
 
@@ -116,6 +119,8 @@ struct FmmArgs {
   uint32_t *long_at, *longs, *long_flags;  // per cell: first unit or NONE; the leaves; see there
   double2 *long_terms;
   uint32_t long_cap;
+  uint32_t by_level;               // k_fmm_lists: a launch a level, nothing to wait for
+  unsigned long long wait_ns;      // k_fmm_lists: a wait's limit
   size_t cap_m2l, cap_p2p, cap_fwd;
   uint32_t ncells, p;
   double mac_far, dmax_scaled, dmin_scaled, dmin2, dmax2, inv_w;
@@ -969,16 +974,18 @@ __device__ void plan_long(const FmmArgs &a, uint32_t c, uint32_t count, uint32_t
 // cells wait only for cells of running blocks): a cell waits for its parent's
 // forward list (`fwd_cnt`, NONE until the list is there) and no level waits as
 // a whole. With a grid barrier a level and the depth-first form 6,000 nodes
-// took 174 us (now 37), 1 M 584 us (now 151). The wait is bounded
-// (20 ms, then the run fails).
-__global__ void __launch_bounds__(LISTS_THREADS) k_fmm_lists(FmmArgs a) {
+// took 174 us (now 37), 1 M 584 us (now 151). A wait ends after 20 ms in which
+// no counted cell was finished (the first 1,024 and every 64th: a count of all
+// would be a chain of atomics on one word); the lists are then built again with
+// a launch a level (by_level), whose cells find their parents' lists there.
+__global__ void __launch_bounds__(LISTS_THREADS) k_fmm_lists(FmmArgs a, uint32_t c0, uint32_t c1) {
   __shared__ uint32_t buf[LISTS_THREADS / 32][2 * LIST_CAP];
   __shared__ uint32_t ticket;
   const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (threadIdx.x == 0) ticket = atomicAdd(&a.info[FI_TICKET], 1u);
+  if (threadIdx.x == 0) ticket = a.by_level ? blockIdx.x : atomicAdd(&a.info[FI_TICKET], 1u);
   __syncthreads();
-  const uint32_t c = ticket * (LISTS_THREADS / 32) + warp;
-  if (c >= a.ncells) return;
+  const uint32_t c = c0 + ticket * (LISTS_THREADS / 32) + warp;
+  if (c >= c1) return;
   const FCell A = load_cell(a.cells + c);
   const uint32_t *in = nullptr;
   uint32_t nin = 1;
@@ -986,12 +993,18 @@ __global__ void __launch_bounds__(LISTS_THREADS) k_fmm_lists(FmmArgs a) {
     if (lane == 0) {
       nin = ld_acquire(&a.fwd_cnt[A.parent]);
       if (nin == NONE) {
-        const unsigned long long t0 = fmm_timer_ns();
+        unsigned long long t0 = fmm_timer_ns();
+        uint32_t seen = ld_acquire(&a.info[FI_DONE]);
         while ((nin = ld_acquire(&a.fwd_cnt[A.parent])) == NONE) {
-          if (fmm_timer_ns() - t0 > 20000000ull) {
-            atomicOr(&a.info[FI_LIST_OVERFLOW], 2u);
-            nin = 0;
-            break;
+          if (fmm_timer_ns() - t0 > a.wait_ns) {
+            const uint32_t done = ld_acquire(&a.info[FI_DONE]);
+            if (done == seen) {
+              atomicOr(&a.info[FI_LIST_OVERFLOW], 4u);
+              nin = 0;
+              break;
+            }
+            seen = done;
+            t0 = fmm_timer_ns();
           }
           __nanosleep(64);
         }
@@ -1009,6 +1022,7 @@ __global__ void __launch_bounds__(LISTS_THREADS) k_fmm_lists(FmmArgs a) {
   } else if (tp > LONG_LIST) {
     plan_long(a, c, A.count, tp);
   }
+  if (lane == 0 && (c < 1024 || (c & 63) == 0)) atomicAdd(&a.info[FI_DONE], 1u);
 }
 
 // ---- M2L (fmm.zig:561-610) and the unscale of L (fmm.zig:645-657) --------------------
@@ -1749,6 +1763,16 @@ void fmm_free(FastScratch &s) {
   s.fmm = nullptr;
 }
 
+// The limit of a wait in k_fmm_lists: 20 ms, or D3_LISTS_WAIT_NS (0: every wait
+// runs out at once, a test of what follows).
+static unsigned long long lists_wait_ns() {
+  static const unsigned long long v = [] {
+    const char *e = getenv("D3_LISTS_WAIT_NS");
+    return e ? strtoull(e, nullptr, 10) : 20000000ull;
+  }();
+  return v;
+}
+
 // Dynamic shared memory of a block, at q coefficients.
 static int up_smem(uint32_t q) { return (int)(UP_THREADS / 32 * 32 * up_row(2 * q) * 8); }
 static int m2l_smem(uint32_t q) { return (int)(M2L_THREADS / 32 * m2l_words(q) * 8); }
@@ -1944,6 +1968,8 @@ int fmm_run(FastScratch &s, TreeDev &t, const NodeArrays &a, const double *stren
     need_p2p = f.last_p2p + f.last_p2p / 4 + 1024;
     need_fwd = f.last_fwd + f.last_fwd / 4 + 1024;
   }
+  args.by_level = 0;
+  args.wait_ns = lists_wait_ns();
   for (int attempt = 0;; ++attempt) {
     if (grow(f.m2l, f.cap_m2l, need_m2l) || grow(f.p2p, f.cap_p2p, need_p2p) ||
         grow(f.fwd, f.cap_fwd, need_fwd))
@@ -1954,7 +1980,12 @@ int fmm_run(FastScratch &s, TreeDev &t, const NodeArrays &a, const double *stren
     if (attempt && (cudaMemsetAsync(f.fwd_cnt, 0xFF, (size_t)ncells * 4, st) != cudaSuccess ||
                     cudaMemsetAsync(f.info + FI_LONG_UNITS, 0, 8, st) != cudaSuccess))
       return -1;
-    D3_LAUNCH(k_fmm_lists, blocks_for(ncells, LISTS_THREADS / 32), LISTS_THREADS, 0, st)(args);
+    const uint32_t launches = args.by_level ? pr.nlev : 1;
+    for (uint32_t lev = 0; lev < launches; ++lev) {
+      const uint32_t c0 = args.by_level ? pr.lvl[lev] : 0, c1 = args.by_level ? pr.lvl[lev + 1] : ncells;
+      if (c1 > c0)
+        D3_LAUNCH(k_fmm_lists, blocks_for(c1 - c0, LISTS_THREADS / 32), LISTS_THREADS, 0, st)(args, c0, c1);
+    }
     // the rest follows at once (it does nothing where a list overflowed), and
     // the host reads the lists' words while it runs
     if (cudaMemcpyAsync(f.h_info, f.info, 64 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st) !=
@@ -1981,7 +2012,12 @@ int fmm_run(FastScratch &s, TreeDev &t, const NodeArrays &a, const double *stren
       f.long_room.want = f.h_info[FI_LONG_UNITS];
       break;
     }
-    if ((ovf & 2) || attempt > 8) return -1;  // a call stack overflowed, or a wait ran out
+    if ((ovf & 2) || attempt > 8) return -1;  // a call stack overflowed
+    if (ovf & 4) {  // a wait ran out (what it left out also says too little of the pools)
+      args.by_level = 1;
+      s.lists_by_level += 1;
+    }
+    if (!(ovf & 1)) continue;
     need_m2l = 2 * (size_t)(f.h_info[FI_POOL_M2L] > need_m2l ? f.h_info[FI_POOL_M2L] : need_m2l);
     need_p2p = 2 * (size_t)(f.h_info[FI_POOL_P2P] > need_p2p ? f.h_info[FI_POOL_P2P] : need_p2p);
     need_fwd = 2 * (size_t)(f.h_info[FI_POOL_FWD] > need_fwd ? f.h_info[FI_POOL_FWD] : need_fwd);
