@@ -34,6 +34,7 @@ enum : uint32_t {
   ST_COLLIDE_OVERFLOW = 1u << 6, // a guessed set exceeded its capacity
   ST_CENTER_RECORDS = 1u << 7,   // a center-sum launch failed or its records disagreed
   ST_LAUNCH_FAILED = 1u << 8,    // a kernel launch the pass depends on did not happen
+  ST_LINK_GAVE_UP = 1u << 9,     // a link pass waited in vain for a message (it then ran serially)
 };
 
 // Device-side failures (a bounded wait that ran out, a tree or record buffer

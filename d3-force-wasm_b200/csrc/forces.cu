@@ -829,7 +829,7 @@ int link_plan_build(LinkPlan &plan, const uint32_t *src, const uint32_t *tgt, ui
   const auto room = [](size_t bytes) { return (bytes + 255) / 256 * 256; };
   const size_t at_order = room(ends.size() * sizeof(LinkEnds)),
                at_start = at_order + room(order.size() * 4), at_tally = at_start + room(start.size() * 4),
-               at_par = at_tally + room(2 * sizeof(uint32_t)),
+               at_par = at_tally + room(3 * sizeof(uint32_t)),
                at_msg = at_par + room(ends.size() * 3 * sizeof(double)),
                msg_bytes = in_block ? 0 : ends.size() * 2 * sizeof(double2);
   std::vector<unsigned char> image(at_par, 0);
@@ -923,8 +923,8 @@ __global__ void k_save_v(double *svx, double *svy, const double *vx, const doubl
 // link.zig:8-40 on one thread, drawing from the device LCG.
 __device__ void link_serial_lcg(const double *xs, const double *ys, double *vxs, double *vys,
                                 const LinkArrays &l, double alpha, double iterations, Rng *rng,
-                                uint32_t *status) {
-  atomicOr(status, ST_LINK_JIGGLE);
+                                uint32_t *status, uint32_t why = ST_LINK_JIGGLE) {
+  atomicOr(status, why);
   uint32_t s = rng->lcg;
   for (double k = 0; k < iterations; k += 1) {
     for (uint32_t i = 0; i < l.m; ++i) {
@@ -1007,7 +1007,7 @@ struct LinkFlowArgs {
   const double *par;           // distance, strength, bias planes
   const uint32_t *level_start; // k_link_block
   ulonglong2 *msg;             // k_link_flow: two inputs per link, all ones = nothing yet
-  uint32_t *tally;             // k_link_flow: blocks done, failure bits
+  uint32_t *tally;             // k_link_flow: blocks done, failure bits, progress
   uint32_t levels, nodes;
   double alpha, iterations;
   uint32_t *flag;
@@ -1135,9 +1135,9 @@ __device__ __forceinline__ void msg_write(ulonglong2 *p, unsigned long long x, u
 
 constexpr uint32_t LINK_MET_JIGGLE = 1, LINK_GAVE_UP = 2;
 
-// The pass as messages, in one cooperative launch, for any size: threads take
-// the links in level order; a link waits (bounded) for the velocities of its
-// two nodes from the links before it there, each a 16-byte message in a place
+// The pass as messages, in one cooperative launch: threads take the links in
+// level order; a link waits (until no 64th link was done for 20 ms: a chain of
+// any length goes on) for the velocities of its two nodes from the links before it there, each a 16-byte message in a place
 // of its own, and hands them on to the links after it. A level costs one
 // message through L2 and one link's arithmetic (1.6 us; 5 us with finished
 // counts and the velocities read after an acquire). The first link on a node
@@ -1160,7 +1160,7 @@ __global__ void __launch_bounds__(256) k_link_flow(LinkFlowArgs a) {
     ulonglong2 in_s, in_t;
     bool fresh = true;
     unsigned long long t0 = 0;
-    uint32_t polls = 0;
+    uint32_t polls = 0, seen = 0;
     while (p < m) {
       if (fresh) {
         fresh = false;
@@ -1197,7 +1197,12 @@ __global__ void __launch_bounds__(256) k_link_flow(LinkFlowArgs a) {
         if (polls == 0) t0 = globaltimer_ns();
         ++polls;
         if (polls > 8 && a.sleep_ns) __nanosleep(a.sleep_ns);
-        gave_up = (polls & 15) == 0 && globaltimer_ns() - t0 > 20000000ull;
+        if ((polls & 15) == 0 && globaltimer_ns() - t0 > 20000000ull) {
+          const uint32_t done = *(volatile const uint32_t *)&a.tally[2];
+          gave_up = done == seen;  // (counted on from 0: a first look sees any progress)
+          seen = done;
+          t0 = globaltimer_ns();
+        }
       }
       if ((have_s && have_t) || gave_up) {
         const uint32_t s = r.src & ~LINK_FIRST, d = r.tgt & ~LINK_FIRST;
@@ -1220,6 +1225,7 @@ __global__ void __launch_bounds__(256) k_link_flow(LinkFlowArgs a) {
         }
         if (!(r.src & LINK_FIRST)) msg_write(&a.msg[2 * (size_t)p], none, none);
         if (!(r.tgt & LINK_FIRST)) msg_write(&a.msg[2 * (size_t)p + 1], none, none);
+        if ((p & 63) == 0) atomicAdd(&a.tally[2], 1u);
         p += nth;
         fresh = true;
       }
@@ -1237,7 +1243,7 @@ __global__ void __launch_bounds__(256) k_link_flow(LinkFlowArgs a) {
     if (atomicAdd(&a.tally[0], 1u) == gridDim.x - 1) {
       __threadfence();
       bits = atomicExch(&a.tally[1], 0u);
-      a.tally[0] = 0;
+      a.tally[0] = a.tally[2] = 0;
       *a.flag = bits != 0;
     }
   }
@@ -1261,7 +1267,8 @@ __global__ void __launch_bounds__(256) k_link_flow(LinkFlowArgs a) {
   }
   __syncthreads();
   if (a.serial_lcg && threadIdx.x == 0)
-    link_serial_lcg(a.xs, a.ys, a.vxs, a.vys, a.l, a.alpha, a.iterations, a.rng, a.status);
+    link_serial_lcg(a.xs, a.ys, a.vxs, a.vys, a.l, a.alpha, a.iterations, a.rng, a.status,
+                    (bits & LINK_MET_JIGGLE ? ST_LINK_JIGGLE : 0) | (bits & LINK_GAVE_UP ? ST_LINK_GAVE_UP : 0));
 }
 
 __global__ void k_link_flag(uint32_t *flag) { *flag = 1; }

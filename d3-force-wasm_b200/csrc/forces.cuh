@@ -76,7 +76,7 @@ struct LinkPlan {
   LinkEnds *ends = nullptr;         // device, in plan order
   double *par = nullptr;            // device: distance, strength, bias planes in plan order
   double2 *msg = nullptr;           // device: per link its two input messages
-  uint32_t *tally = nullptr;        // device: blocks done, failure bits of the running pass
+  uint32_t *tally = nullptr;        // device: blocks done, failure bits of the running pass, progress
 };
 // The device arrays are filled on `st`, where the passes run.
 int link_plan_build(LinkPlan &plan, const uint32_t *src, const uint32_t *tgt, uint32_t m,
