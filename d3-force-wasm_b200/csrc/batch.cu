@@ -45,6 +45,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "pages.cuh"
 
 namespace d3 {
 namespace {
@@ -718,15 +719,16 @@ void build_btables(BTables &T) {
   }
 }
 
-// Reads of device arrays into the caller's (pageable, often untouched) memory.
-// One cudaMemcpy stages through one thread, which also takes every page fault:
-// 96 MB take 25 ms, 4 GB/s. Here up to READ_WORKERS threads take pieces of
-// READ_PIECE bytes in turn, each with two pinned slots (one being filled by the
-// copy engine while the other is copied out): 9 ms. The slots, 8 MB at most,
-// stay with the batch and go with it. Reads under READ_MIN take cudaMemcpy:
-// pinning the slots costs the first read 4 to 9 ms, which later reads of 32 MB
-// (4.3 ms as they are, 3.1 to 4.6 with the threads: the allocator hands out
-// memory of that size that is mapped already) do not win back.
+// Reads of device arrays into the caller's pageable memory. One cudaMemcpy
+// stages through one thread, which also takes every page fault of memory that
+// was never touched. Here up to READ_WORKERS threads take pieces of READ_PIECE
+// bytes in turn, each with two pinned slots (one being filled by the copy
+// engine while the other is copied out). 96 MB, cudaMemcpy / threads: untouched
+// 49 / 14 ms, touched 4.9 / 4.4 ms. The slots, 8 MB at most, stay with the batch
+// and go with it; pinning them takes the first such read 8 to 18 ms more, so it
+// needs READ_MIN bytes of untouched memory (48 MB: 25 ms by cudaMemcpy, 14 ms
+// with the pinning, 7 ms without); other reads take cudaMemcpy until there are
+// slots.
 constexpr unsigned READ_WORKERS = 8, READ_SLOTS = 2;
 constexpr size_t READ_PIECE = 1u << 19, READ_MIN = 48u << 20;
 
@@ -741,10 +743,12 @@ class Reader {
   // Copies the spans; false on a CUDA error. One call at a time (a second
   // thread waits).
   bool read(const ReadSpan *spans, unsigned count) {
-    size_t total = 0;
+    size_t total = 0, untouched = 0;
     for (unsigned i = 0; i < count; ++i) total += spans[i].bytes;
     std::lock_guard<std::mutex> hold(lock_);
-    if (total < READ_MIN || !reserve()) {
+    if (total >= READ_MIN && !workers_)
+      for (unsigned i = 0; i < count; ++i) untouched += untouched_bytes(spans[i].dst, spans[i].bytes);
+    if (total < READ_MIN || (!workers_ && (untouched < READ_MIN || !reserve()))) {
       for (unsigned i = 0; i < count; ++i)
         if (cudaMemcpy(spans[i].dst, spans[i].src, spans[i].bytes, cudaMemcpyDeviceToHost) !=
             cudaSuccess)
