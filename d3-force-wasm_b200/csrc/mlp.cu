@@ -136,9 +136,12 @@ __global__ void __launch_bounds__(GTHREADS) k_mlp_grad(const float *x, const flo
   if (t < MLP_OUT) S.b3[t] = params[P_B3 + t];
   const float inv = 1.f / norm;
   // gradient sums: W2 tile (rows i0.., columns j0..), W1 (row gj, columns gk ..
-  // gk + 2), W3 and the biases by the threads that take their columns
+  // gk + 2), W3 and the biases by the threads that take their columns (gc: a
+  // thread's one of W3, b2 and b3). A tile's sum is formed by itself and then
+  // added: one chain over all of a CTA's samples would lose bits as it grows
+  // (64 tiles of equal terms: 6e-5 of the sum for 2e-6).
   const int gj = t & 63, gk = (t >> 6) * 3;
-  float gw2[4][4] = {}, gw1[3] = {}, gw3 = 0, gb1 = 0, gb2 = 0, gb3 = 0, my_loss = 0;
+  float gw2[4][4] = {}, gw1[3] = {}, gb1 = 0, gc = 0, my_loss = 0;
   for (uint32_t base = blockIdx.x * GT; base < n; base += gridDim.x * GT) {
     __syncthreads();  // the weights; the last tile's reads
     for (int e = t; e < GT * MLP_IN; e += GTHREADS) {
@@ -215,23 +218,33 @@ __global__ void __launch_bounds__(GTHREADS) k_mlp_grad(const float *x, const flo
 #pragma unroll
       for (int j = 0; j < 4; ++j) v[i][j] *= g1[i][j];
     put_tile(v, i0, j0, S.d1);
-    tile_outer(S.d2, S.a1, i0, j0, gw2);
+    float tw2[4][4] = {};
+    tile_outer(S.d2, S.a1, i0, j0, tw2);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) gw2[i][j] += tw2[i][j];
     __syncthreads();
     // the other gradients, a column of samples each
+    float tw1[3] = {}, tb1 = 0, tc = 0;
     for (int s = 0; s < GT; ++s) {
       const float d = S.d1[s][gj];
-      if (gk == 0) gb1 += d;
+      if (gk == 0) tb1 += d;
 #pragma unroll
-      for (int q = 0; q < 3; ++q) gw1[q] += d * S.x[s][gk + q];
+      for (int q = 0; q < 3; ++q) tw1[q] += d * S.x[s][gk + q];
     }
+    gb1 += tb1;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) gw1[q] += tw1[q];
     if (t < MLP_OUT * MLP_H) {
       const int o = t / MLP_H, k = t % MLP_H;
-      for (int s = 0; s < GT; ++s) gw3 += S.dy[o][s] * S.a2[s][k];
+      for (int s = 0; s < GT; ++s) tc += S.dy[o][s] * S.a2[s][k];
     } else if (t < MLP_OUT * MLP_H + MLP_H) {
-      for (int s = 0; s < GT; ++s) gb2 += S.d2[s][t - MLP_OUT * MLP_H];
+      for (int s = 0; s < GT; ++s) tc += S.d2[s][t - MLP_OUT * MLP_H];
     } else if (t < MLP_OUT * MLP_H + MLP_H + MLP_OUT) {
-      for (int s = 0; s < GT; ++s) gb3 += S.dy[t - MLP_OUT * MLP_H - MLP_H][s];
+      for (int s = 0; s < GT; ++s) tc += S.dy[t - MLP_OUT * MLP_H - MLP_H][s];
     }
+    gc += tc;
   }
   float *g = part + (size_t)blockIdx.x * PART;
 #pragma unroll
@@ -241,9 +254,9 @@ __global__ void __launch_bounds__(GTHREADS) k_mlp_grad(const float *x, const flo
 #pragma unroll
   for (int q = 0; q < 3; ++q) g[P_W1 + gj * MLP_IN + gk + q] = gw1[q];
   if (gk == 0) g[P_B1 + gj] = gb1;
-  if (t < MLP_OUT * MLP_H) g[P_W3 + t] = gw3;
-  else if (t < MLP_OUT * MLP_H + MLP_H) g[P_B2 + t - MLP_OUT * MLP_H] = gb2;
-  else if (t < MLP_OUT * MLP_H + MLP_H + MLP_OUT) g[P_B3 + t - MLP_OUT * MLP_H - MLP_H] = gb3;
+  if (t < MLP_OUT * MLP_H) g[P_W3 + t] = gc;
+  else if (t < MLP_OUT * MLP_H + MLP_H) g[P_B2 + t - MLP_OUT * MLP_H] = gc;
+  else if (t < MLP_OUT * MLP_H + MLP_H + MLP_OUT) g[P_B3 + t - MLP_OUT * MLP_H - MLP_H] = gc;
   for (int o = 16; o > 0; o >>= 1) my_loss += __shfl_xor_sync(0xffffffffu, my_loss, o);
   if ((t & 31) == 0) S.loss[t >> 5] = my_loss;
   __syncthreads();
