@@ -1195,6 +1195,8 @@ double sim_stat(uint32_t h, uint32_t which) {
   }
   // runs of the plain FMM whose list build gave up waiting and took a launch a level
   if (which == 29) return s->fast.lists_by_level;
+  // leaves whose P2P lists the last of them took in segments
+  if (which == 38) return fmm_longs(s->fast);
   if ((which >= 300 && which < 364) || (which >= 400 && which < 464)) {
     // the last parallel collide's first attempt: 300 + k microseconds from
     // the end of its list build to the last turn of depth k, 400 + k turns

@@ -87,6 +87,9 @@ struct FmmPrep {
   uint32_t *info = nullptr;  // device: FI_LVL + d = first cell of level d
 };
 
+// Leaves whose P2P lists the last plain run took in segments.
+uint32_t fmm_longs(const FastScratch &s);
+
 // The fast tree of fmm.zig:247-330 up to the cells: square extent, 16-bit
 // Morton keys, stable sort, gather, level-order cells (fmm.zig:685-717).
 // 1: ready; 2: no point to act on; 0: non-finite extent (the exact kernel

@@ -49,9 +49,20 @@ constexpr unsigned UP_THREADS = 64, M2L_THREADS = 32, P2P_THREADS = 32, DOWN_THR
 // region) goes by segments of 32; the terms of a segment and 16 targets take a
 // unit of 32 KB, LONG_UNITS_MAX of them at most (256 MB, held once a run wanted
 // some; lists past that or past what the device has left, and leaves of more
-// than LONG_POINTS points, go by k_fmm_p2p).
+// than LONG_POINTS points, go by k_fmm_p2p). LONG_LIST 32 / 64 / 128: a tick of
+// 80,000 clustered nodes 494 / 503 / 579 us, 80,000 in tighter clusters 945 /
+// 945 / 1,014.
 constexpr uint32_t LONG_LIST = 64, LONG_POINTS = 64, LONG_UNITS_MAX = 8192;
 constexpr uint32_t LONG_UNIT = 32 * 4 * 16;  // terms: source leaf, three pairs and a sum, target
+
+// The two launches and their chains take 45 to 60 us, which only a list that
+// is long against k_fmm_p2p's own chain gives back: they are taken when the
+// longest list of the last run passed LONG_WORTH, or LONG_WORTH_FEW where the
+// cells are few and k_fmm_p2p has four lanes a target. A tick with / without
+// them, by the longest list. Few cells: 77 leaves 366 / 305 us, 96 408 / 360,
+// 120 424 / 402, 160 404 / 410, 230 421 / 482, 340 450 / 608. More cells: 80
+// 441 / 386, 137 497 / 517, 245 459 / 523, 677 947 / 1,522.
+constexpr uint32_t LONG_WORTH_FEW = 192, LONG_WORTH = 96;
 
 constexpr uint32_t P2P_FEW_CELLS = 4096;  // some 30,000 nodes; measured at k_fmm_p2p
 constexpr uint32_t FMM_STACK = 64;
@@ -68,7 +79,8 @@ enum : uint32_t { FI_CELLS = 0, FI_OVERFLOW, FI_LEVELS, FI_POOL_M2L, FI_POOL_P2P
                   FI_LIST_OVERFLOW,              // 1: a pool, 2: a call stack, 4: a wait ran out
                   FI_TICKET,                     // k_fmm_lists' blocks so far
                   FI_LVL = 8,  // FI_LVL + d: first cell of level d
-                  FI_LONG_UNITS = 36, FI_LONGS,  // long P2P lists: units of terms, leaves
+                  FI_LONG_UNITS = 36, FI_LONGS,  // long P2P lists: units of terms, leaves,
+                  FI_LONG_MAX,                   // the longest list's source leaves
                   FI_DONE,                       // counts on while k_fmm_lists makes progress
                   FI_M = 40,                     // points to act on (0 when the extent is bad)
                   FI_BAD = 41 };                 // 1: the extent is not finite and positive
@@ -90,6 +102,7 @@ struct FmmDev {
   uint32_t *long_at = nullptr, *longs = nullptr, *long_flags = nullptr;
   double2 *long_terms = nullptr;
   SpareRoom long_room{0, 0, LONG_UNITS_MAX};  // units
+  uint32_t long_max = 0, longs_last = 0;      // the last run's longest P2P list, its leaves in segments
   cudaEvent_t lists_read = nullptr;  // the lists' words are in h_info
   double *square = nullptr;      // box x0, y0, side
   uint32_t *h_info = nullptr;    // pinned mirror of info
@@ -386,7 +399,7 @@ __global__ void __launch_bounds__(32) k_cells_starts(uint32_t ccap, uint32_t *in
   const unsigned used = __ballot_sync(0xffffffffu, x != 0);
   if (lane < CB_LEVELS) info[FI_LVL + lane] = incl - x;
   if (lane == 0) {
-    info[FI_LONG_UNITS] = info[FI_LONGS] = 0;
+    info[FI_LONG_UNITS] = info[FI_LONGS] = info[FI_LONG_MAX] = 0;
     info[FI_LVL + CB_LEVELS] = at;
     info[FI_CELLS] = at;
     info[FI_LEVELS] = used ? 32 - __clz(used) : 0;
@@ -1021,6 +1034,7 @@ __global__ void __launch_bounds__(LISTS_THREADS) k_fmm_lists(FmmArgs a, uint32_t
     if (lane == 0) st_release(&a.fwd_cnt[c], tf);
   } else if (tp > LONG_LIST) {
     plan_long(a, c, A.count, tp);
+    if (lane == 0) atomicMax(&a.info[FI_LONG_MAX], tp);
   }
   if (lane == 0 && (c < 1024 || (c & 63) == 0)) atomicAdd(&a.info[FI_DONE], 1u);
 }
@@ -1778,6 +1792,11 @@ static int up_smem(uint32_t q) { return (int)(UP_THREADS / 32 * 32 * up_row(2 * 
 static int m2l_smem(uint32_t q) { return (int)(M2L_THREADS / 32 * m2l_words(q) * 8); }
 static int down_smem(uint32_t q) { return (int)(DOWN_THREADS / 32 * 2 * DOWN_ROWS * up_row(2 * q) * 8); }
 
+uint32_t fmm_longs(const FastScratch &s) {
+  const FmmDev *f = static_cast<const FmmDev *>(s.fmm);
+  return f ? f->longs_last : 0;
+}
+
 static int sync_read(FmmDev &f, cudaStream_t st) {
   if (cudaMemcpyAsync(f.h_info, f.info, 64 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st) !=
           cudaSuccess ||
@@ -1938,7 +1957,8 @@ int fmm_run(FastScratch &s, TreeDev &t, const NodeArrays &a, const double *stren
   args.mco = f.mco;
   args.lco = f.lco;
   args.arrive = f.arrive;
-  f.long_room.grow([&](size_t cap) {
+  const bool few = ncells <= P2P_FEW_CELLS, longs = f.long_max > (few ? LONG_WORTH_FEW : LONG_WORTH);
+  if (longs) f.long_room.grow([&](size_t cap) {
     device_give(f.longs, f.long_items, f.long_flags, f.long_terms);
     return device_take({{(void **)&f.longs, cap * 4},
                         {(void **)&f.long_items, cap * sizeof(uint2)},
@@ -1950,7 +1970,7 @@ int fmm_run(FastScratch &s, TreeDev &t, const NodeArrays &a, const double *stren
   args.longs = f.longs;
   args.long_flags = f.long_flags;
   args.long_terms = f.long_terms;
-  args.long_cap = f.long_room.cap;
+  args.long_cap = longs ? f.long_room.cap : 0;
   args.m2l_off = f.m2l_off; args.m2l_cnt = f.m2l_cnt;
   args.p2p_off = f.p2p_off; args.p2p_cnt = f.p2p_cnt;
   args.fwd_off = f.fwd_off; args.fwd_cnt = f.fwd_cnt;
@@ -1978,7 +1998,7 @@ int fmm_run(FastScratch &s, TreeDev &t, const NodeArrays &a, const double *stren
     args.cap_m2l = f.cap_m2l; args.cap_p2p = f.cap_p2p; args.cap_fwd = f.cap_fwd;
     if (cudaMemsetAsync(f.info + FI_POOL_M2L, 0, 5 * sizeof(uint32_t), st) != cudaSuccess) return -1;
     if (attempt && (cudaMemsetAsync(f.fwd_cnt, 0xFF, (size_t)ncells * 4, st) != cudaSuccess ||
-                    cudaMemsetAsync(f.info + FI_LONG_UNITS, 0, 8, st) != cudaSuccess))
+                    cudaMemsetAsync(f.info + FI_LONG_UNITS, 0, 12, st) != cudaSuccess))
       return -1;
     const uint32_t launches = args.by_level ? pr.nlev : 1;
     for (uint32_t lev = 0; lev < launches; ++lev) {
@@ -1994,10 +2014,10 @@ int fmm_run(FastScratch &s, TreeDev &t, const NodeArrays &a, const double *stren
       return -1;
     if (dflt) D3_LAUNCH(k_fmm_m2l<FMM_DEFAULT_ORDER>, mb, M2L_THREADS, m2l_smem(q), st)(args);
     else D3_LAUNCH(k_fmm_m2l<0>, mb, M2L_THREADS, m2l_smem(q), st)(args);
-    if (ncells <= P2P_FEW_CELLS)
+    if (few)
       D3_LAUNCH(k_fmm_p2p<true>, blocks_for(4 * ncells, P2P_THREADS / 32), P2P_THREADS, 0, st)(args);
     else D3_LAUNCH(k_fmm_p2p<false>, pb, P2P_THREADS, 0, st)(args);
-    if (f.long_room.cap) {
+    if (args.long_cap) {
       D3_LAUNCH(k_fmm_p2p_terms, LONG_BLOCKS, LONG_THREADS, 0, st)(args);
       D3_LAUNCH(k_fmm_p2p_add, LONG_BLOCKS / 8, LONG_THREADS, 0, st)(args);
     }
@@ -2010,6 +2030,8 @@ int fmm_run(FastScratch &s, TreeDev &t, const NodeArrays &a, const double *stren
       f.last_p2p = f.h_info[FI_POOL_P2P];
       f.last_fwd = f.h_info[FI_POOL_FWD];
       f.long_room.want = f.h_info[FI_LONG_UNITS];
+      f.long_max = f.h_info[FI_LONG_MAX];
+      f.longs_last = args.long_cap ? f.h_info[FI_LONGS] : 0;
       break;
     }
     if ((ovf & 2) || attempt > 8) return -1;  // a call stack overflowed
