@@ -49,7 +49,7 @@ THREADED = "tree keys, sort and emission jobs; many-body record pass"
 # DRAM bytes (read + write) of one collide launch (k_collide_spec) on this
 # workload, from an ncu capture of the 11th pass of a 15-tick schedule
 # (profiles/k_collide_spec_exact_50k.md)
-COLLIDE_DRAM_BYTES = 64813568 + 9635072
+COLLIDE_DRAM_BYTES = 65102592 + 9839872
 
 
 def parse():

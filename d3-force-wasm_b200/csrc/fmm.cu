@@ -216,8 +216,6 @@ __global__ void k_fmm_gather(const uint32_t *perm, const double *xs, const doubl
   uy[j] = (y - oy) * inv_w;
 }
 
-// ---- grid-wide helpers --------------------------------------------------------
-
 // ---- cells (fmm.zig:685-717) ---------------------------------------------------
 
 // The child ranges of a cell at depth d: bnd[q] .. bnd[q + 1] holds digit q.
@@ -907,7 +905,10 @@ __device__ uint32_t expand_long(const FmmArgs &a, uint32_t c, const FCell &A, co
 // events are left. Each cell is read once, by as many lanes as there are calls;
 // the depth-first form reads it three times, in one lane's chain of dependent
 // loads a call. `buf` holds two lists of LIST_CAP words; a longer list (a leaf
-// beside a far denser region) takes the depth-first form.
+// beside a far denser region) takes the depth-first form. LIST_CAP 256 / 512 /
+// 1,024: a tick of 200,003 clustered nodes 985 / 992 / 737 us, of 80,000 in
+// tighter clusters 944 / 946 / 637 (their lists pass 512); 6,000 to 80,000
+// clustered or even nodes the same.
 constexpr uint32_t LIST_CAP = 512;
 __device__ uint32_t expand_cell(const FmmArgs &a, uint32_t c, const FCell &A, const uint32_t *in,
                                 uint32_t nin, uint32_t *buf, uint32_t &tp) {
@@ -1438,8 +1439,8 @@ __global__ void __launch_bounds__(P2P_THREADS) k_fmm_p2p(FmmArgs a) {
 // segment of 32 source leaves writes every leaf's terms (a pair without a term
 // writes -0, which changes nothing), and a warp per leaf then adds them in
 // order; a source leaf with groups that go pair by pair (`long_flags`, a bit a
-// leaf of the segment) is summed there as before. P2P in all, clustered nodes:
-// 20,000 150 -> 99 us, 80,000 478 -> 173, 160,000 329 -> 180.
+// leaf of the segment) is summed there as before. Where this pays, and what it
+// measured: at LONG_WORTH.
 constexpr unsigned LONG_THREADS = 64, LONG_BLOCKS = 2368;
 
 __global__ void __launch_bounds__(LONG_THREADS) k_fmm_p2p_terms(FmmArgs a) {
@@ -1895,8 +1896,6 @@ int fmm_run(FastScratch &s, TreeDev &t, const NodeArrays &a, const double *stren
   if (pre == 2) return 1;
   if (pre <= 0) return pre;
   FmmDev &f = *static_cast<FmmDev *>(s.fmm);
-  const uint32_t m = pr.m;
-  (void)m;
   const double w = pr.w;
   uint32_t p = FMM_DEFAULT_ORDER;
   if (prm.order >= 1 && prm.order <= (double)FMM_MAX_ORDER) p = (uint32_t)prm.order;

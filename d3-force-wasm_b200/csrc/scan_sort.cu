@@ -202,7 +202,9 @@ __device__ bool look_back(const uint32_t *words, uint32_t tile, uint32_t d, uint
   return true;
 }
 
-// Stable scatter of one tile of SORT_TILE keys: warp w takes the tile's
+// Stable scatter of one tile of SORT_TILE keys, a launch a pass (the published
+// single-pass prefix with decoupled look-back of Merrill and Garland 2016, and
+// its use in a radix sort, Adinets and Merrill 2022): warp w takes the tile's
 // w-th run of 32 x PER keys, in PER rounds of 32. In a round a key's rank
 // among equal digits is the warp's count of that digit so far plus the lanes
 // below it with the same digit (same_digit). The warps' counts then give

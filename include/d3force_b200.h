@@ -170,7 +170,7 @@ int32_t sim_find(uint32_t h, double x, double y, double radius, uint32_t *index)
  *     collide, 1 its attempts, 2 1 if it fell back to the serial loop;
  *   3 nodes the last exact many-body traversal flagged for jiggle;
  *   4 link levels of the last exact link plan, 5 1 if the last exact link
- *     pass fell back to the serial order (a jiggle);
+ *     pass fell back to the serial order (a jiggle, or a wait in vain);
  *   6 kernels this library launched so far (all simulations);
  *   7, 8 turns of the last parallel collide that met an unguessed head /
  *     overlap, 9 inactive nodes whose turn would have written, 10 turns run
@@ -184,6 +184,9 @@ int32_t sim_find(uint32_t h, double x, double y, double radius, uint32_t *index)
  *     rerun with their entry tests, 25 stretches added one by one, 26
  *     records in all (24-26 are 0 after the serial sums);
  *   27 host milliseconds the last sim_tick spent queueing work;
+ *   29 runs of the plain fast many-body whose list build waited in vain and
+ *     was done again level by level, 38 leaves whose point-to-point lists its
+ *     last run took in segments;
  *   30-37 microseconds of the last tree build's phases (box, keys, sort,
  *     runs, cell counts, their scan, cell owners, the cells);
  *   with profiling on, 300 + k microseconds from the end of the last
